@@ -143,6 +143,61 @@ bool mq_supported(int M, int Q) {
   return false;
 }
 
+// The n-point Gauss rule of the discrete measure sum_q w_q delta(s - s_q),
+// symmetric about 0 (n even, n <= number of points): the three-term recurrence
+// of its orthogonal polynomials by the Stieltjes procedure (Gautschi, Orthogonal
+// Polynomials: Computation and Approximation, 2004), the nodes as the roots of
+// the n-th one, bracketed by the sign changes of the Sturm sequence and
+// bisected, the weights from the orthonormal polynomials' sums of squares.
+static void discrete_gauss(const std::vector<double>& s, const std::vector<double>& w, int n, double* x, double* v) {
+  const size_t Q = s.size();
+  std::vector<double> beta((size_t)n, 0.0);   // the alphas vanish by symmetry
+  std::vector<double> p0(Q, 0.0), p1(Q, 1.0), p2(Q);
+  double nrm = 0.0;
+  for (double wq : w) nrm += wq;
+  beta[0] = nrm;
+  for (int k = 1; k < n; ++k) {
+    double nn = 0.0;
+    for (size_t q = 0; q < Q; ++q) {
+      p2[q] = s[q] * p1[q] - (k > 1 ? beta[(size_t)k - 1] * p0[q] : 0.0);
+      nn += w[q] * p2[q] * p2[q];
+    }
+    beta[(size_t)k] = nn / nrm;
+    nrm = nn;
+    p0.swap(p1);
+    p1.swap(p2);
+  }
+  // number of roots of the n-th polynomial below t (sign changes of the recurrence)
+  auto below = [&](double t) {
+    int c = 0;
+    double d = t;   // p_1 / p_0
+    for (int k = 1;; ++k) {
+      if (d == 0.0) d = 1e-300;
+      if (d > 0.0) ++c;
+      if (k == n) return c;
+      d = t - beta[(size_t)k] / d;
+    }
+  };
+  for (int r = n / 2; r < n; ++r) {
+    double lo = 0.0, hi = 1.0;   // the positive roots; the others mirror them
+    for (int it = 0; it < 100; ++it) {
+      const double m = 0.5 * (lo + hi);
+      (below(m) > r ? hi : lo) = m;
+    }
+    const double t = 0.5 * (lo + hi);
+    double a = 0.0, b = 1.0 / std::sqrt(beta[0]), sum = b * b;   // orthonormal polynomials at t
+    for (int k = 1; k < n; ++k) {
+      const double c = (t * b - (k > 1 ? std::sqrt(beta[(size_t)k - 1]) * a : 0.0)) / std::sqrt(beta[(size_t)k]);
+      a = b;
+      b = c;
+      sum += b * b;
+    }
+    x[r] = t;
+    x[n - 1 - r] = -t;
+    v[r] = v[n - 1 - r] = 1.0 / sum;
+  }
+}
+
 // fortran/fibers.f95:141-145,353-476: quadrature, Legendre, lambda and E_k
 // in double, then the working-precision constants as the REAL*4 program
 // forms them (c, d, D1 and gamma in single precision).
@@ -190,6 +245,47 @@ static Tables make_tables(const rf_config& c) {
       if (2 * q < Q) t.W2[k][q] = make_float2(t.W[k][q], t.W[k][q]);
     }
   }
+  double fx[kFarNodes], fv[kFarNodes];
+  discrete_gauss(pts, wts, kFarNodes, fx, fv);
+  for (int q = 0; q < kFarNodes; ++q) t.far_pts[q] = (float)fx[q];
+  for (int k = 0; k <= M; ++k) {
+    double wk[kFarNodes / 2], big = 0.0;
+    for (int q = 0; q < kFarNodes / 2; ++q) {
+      wk[q] = fv[q] * P(fx[q], k);
+      big = std::max(big, std::fabs(wk[q]));
+    }
+    if (k >= 2 && k % 2 == 0) {
+      // The full rule's weights of P_2 and P_4 sum to zero (those of P_6 and P_8
+      // to a small residue).  Rounded one by one the far ones sum to ~4e-8 more,
+      // and that excess times the nearly constant kernel of a distant pair adds
+      // up over all pairs with one sign (N=1000 dilute: forces 1.3e-5 off FP64,
+      // 2.9e-6 with the 24-point rule).  On the grid of the largest one's FP32
+      // spacing they are FP32 numbers whose sum is exact; the largest one takes
+      // up what is missing.
+      const double g = std::ldexp(1.0, std::ilogb(big) - 23);
+      double sum = 0.0, want = 0.0;
+      for (int q = 0; q < Q; ++q) want += 0.5 * wts[q] * P(pts[q], k);
+      int at = 0;
+      for (int q = 0; q < kFarNodes / 2; ++q) {
+        wk[q] = g * std::nearbyint(wk[q] / g);
+        sum += wk[q];
+        if (std::fabs(wk[q]) > std::fabs(wk[at])) at = q;
+      }
+      wk[at] += want - sum;
+    }
+    for (int q = 0; q < kFarNodes / 2; ++q) {
+      t.far_W[k][q] = (float)wk[q];
+      t.far_W[k][kFarNodes - 1 - q] = (k & 1) ? -t.far_W[k][q] : t.far_W[k][q];
+      t.far_W2[k][q] = make_float2(t.far_W[k][q], t.far_W[k][q]);
+    }
+  }
+  // Centre distance from which the far rule's blocks are the full rule's to
+  // 3e-10 of their largest entry (both in FP64, collinear and random
+  // orientations): below the FP32 rounding of the blocks, ~2e-9.  8 points, M = 5
+  // terms, 24 points per fiber: 2.4e-8 at 3.0, 2.0e-9 at 3.5, 2.6e-10 at 4.0;
+  // M = 8: 6.4e-9 at 5.0, 3.2e-10 at 7.0.  12 and 48 points per fiber: the same.
+  const double far = M <= 5 ? 4.0 : 7.0;
+  t.far_d2 = (float)(far * far);
   const double eps = c.slenderness;
   const double cd = std::log(eps * eps * std::exp(1.0));
   const double dd = -cd;
@@ -319,7 +415,7 @@ struct rf_handle {
   bool use_graphs = true;         // GMRES restart cycles from graphs
   bool use_step_graphs = true;    // rf_step as one graph
   int mv_variant = 0;             // structured matvec kernel (rf_autotune)
-  int asm_variant = 0;            // numerical pair-tile kernel (rf_autotune)
+  int asm_variant = 1;            // numerical pair-tile kernel (rf_autotune): packed FP32
   int64_t ypart_floats = 0;       // capacity of ypart
   bool assembled = false, solved = false;
   int64_t device_bytes = 0;

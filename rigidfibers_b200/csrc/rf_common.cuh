@@ -12,6 +12,7 @@ namespace rf {
 
 constexpr int kMaxTerms = 8;      // Legendre terms supported (closed forms to P_8)
 constexpr int kMaxQuad = 48;      // quadrature points per fiber (16 intervals x 3)
+constexpr int kFarNodes = 8;      // points per fiber of the far rule (Tables::far_pts)
 
 // Per-launch tables, passed by value so every kernel sees them through the
 // constant parameter bank (no module-global state: handles with different
@@ -24,6 +25,15 @@ struct Tables {
   // W2[k][q] = (W[k][q], W[k][q]) for q < Q/2: the weight as the second
   // operand of a packed two-lane FP32 multiply-add
   float2 W2[kMaxTerms + 1][kMaxQuad / 2];
+  // The far rule: the kFarNodes-point Gauss rule of the discrete measure
+  // {pts, w}, which gives that sum exactly for polynomials of degree
+  // 2 kFarNodes - 1, hence the sums against P_0..P_M of any kernel that is
+  // smooth on the fiber.  far_W[k][q] = weight x P_k, far_W2 as W2; pairs with
+  // |x_i - x_j|^2 >= far_d2 take it.
+  float far_pts[kFarNodes];
+  float far_W[kMaxTerms + 1][kFarNodes];
+  float2 far_W2[kMaxTerms + 1][kFarNodes / 2];
+  float far_d2;
   float gamma[kMaxTerms];   // gamma[0] = D1 (force index 0), gamma[k] for k>=1
   float eigen[kMaxTerms];   // E_k; unused for k = 0
   float e2;                 // 2 * eps^2

@@ -32,6 +32,8 @@
 //                storage tile as [tile][sub-tile][j][value][i] so that one
 //                CTA's writes for one j are contiguous and the matvec reads
 //                whole 32-byte sectors (see rf_struct.cu).
+#include <type_traits>
+
 #include "rf_common.cuh"
 #include "rf_kernels.cuh"
 #include "rf_analytic.cuh"
@@ -120,17 +122,18 @@ struct AsmOut {
 // parts (W[k][Q-1-q] = (-1)^k W[k][q]).
 //
 // P2 = true evaluates the two mirror points in the two lanes of packed FP32
-// instructions (add/mul/fma .f32x2) and accumulates the moments in lane pairs
-// (A, B0), (B1, B2) against the duplicated weights W2; every rounding is the
-// same as in the scalar form (all steps are explicit _rn operations, none can
-// be contracted), so both give bit-identical G.
-//
-// FAR: the rule of the far pairs (far_pts, far_W) instead of the full one.
-template <int K1, int Q, int GS, bool P2, bool FAR>
+// instructions (add/mul/fma .f32x2); every rounding is the same as in the scalar
+// form (all steps are explicit _rn operations, none can be contracted), so both
+// give bit-identical G.  Either way the moments of P_2i and P_2i+1 accumulate in
+// the two lanes against the weight pair W2[i][q] (the even part for P_2i, the
+// odd part for P_2i+1), and their six components are recombined and stored as
+// pairs: gcol[(i * 6 + c) * GS2] = (P_2i, P_2i+1).
+// FAR: the rule of the far pairs (far_pts, far_W2) instead of the full one.
+template <int K1, int Q, int GS2, bool P2, bool FAR>
 __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const float p[3], const float4 tj, float e2,
-                                                    float e2x3, float* __restrict__ gcol) {
+                                                    float e2x3, float2* __restrict__ gcol) {
   static_assert(P2 || !FAR, "the far rule runs packed");
-  constexpr int H = Q / 2;
+  constexpr int H = Q / 2, KP = (K1 + 1) / 2;
   const float* const pts = FAR ? tab.far_pts : tab.pts;
   float ss = fmaf(p[0], tj.x, fmaf(p[1], tj.y, p[2] * tj.z));
   float dx = fmaf(-ss, tj.x, p[0]), dy = fmaf(-ss, tj.y, p[1]), dz = fmaf(-ss, tj.z, p[2]);
@@ -140,11 +143,11 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
   dy = fmaf(-dl, tj.y, dy);
   dz = fmaf(-dl, tj.z, dz);
   const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  float2 m01[K1], m23[K1];   // (A_k, B0_k), (B1_k, B2_k)
+  float2 mA[KP], m0[KP], m1[KP], m2[KP];
 #pragma unroll
-  for (int k = 0; k < K1; ++k) m01[k] = m23[k] = make_float2(0.f, 0.f);
-  // the scalar form keeps more live values per point: unrolled less, no spills
-  constexpr int kUnroll = P2 ? H : 3;
+  for (int i = 0; i < KP; ++i) mA[i] = m0[i] = m1[i] = m2[i] = make_float2(0.f, 0.f);
+  // the full rule's 12 folded points unrolled whole would spill
+  constexpr int kUnroll = FAR ? H : 3;
 #pragma unroll kUnroll
   for (int q = 0; q < H; ++q) {
     float2 fa, fb, fc, fd;   // lane x: point q, lane y: point Q-1-q
@@ -185,23 +188,18 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
       fc = make_float2(r[2][0], r[2][1]);
       fd = make_float2(r[3][0], r[3][1]);
     }
-    const float2 e01 = make_float2(__fadd_rn(fa.x, fa.y), __fadd_rn(fb.x, fb.y));
-    const float2 o01 = make_float2(__fsub_rn(fa.x, fa.y), __fsub_rn(fb.x, fb.y));
-    const float2 e23 = make_float2(__fadd_rn(fc.x, fc.y), __fadd_rn(fd.x, fd.y));
-    const float2 o23 = make_float2(__fsub_rn(fc.x, fc.y), __fsub_rn(fd.x, fd.y));
+    // (even, odd) parts
+    const float2 ga = make_float2(__fadd_rn(fa.x, fa.y), __fsub_rn(fa.x, fa.y));
+    const float2 gb = make_float2(__fadd_rn(fb.x, fb.y), __fsub_rn(fb.x, fb.y));
+    const float2 gc = make_float2(__fadd_rn(fc.x, fc.y), __fsub_rn(fc.x, fc.y));
+    const float2 gd = make_float2(__fadd_rn(fd.x, fd.y), __fsub_rn(fd.x, fd.y));
 #pragma unroll
-    for (int k = 0; k < K1; ++k) {
-      if constexpr (P2) {
-        const float2 w2 = FAR ? tab.far_W2[k][FAR ? q : 0] : tab.W2[k][q];
-        m01[k] = __ffma2_rn((k & 1) ? o01 : e01, w2, m01[k]);
-        m23[k] = __ffma2_rn((k & 1) ? o23 : e23, w2, m23[k]);
-      } else {
-        const float w = tab.W[k][q];
-        m01[k].x = __fmaf_rn((k & 1) ? o01.x : e01.x, w, m01[k].x);
-        m01[k].y = __fmaf_rn((k & 1) ? o01.y : e01.y, w, m01[k].y);
-        m23[k].x = __fmaf_rn((k & 1) ? o23.x : e23.x, w, m23[k].x);
-        m23[k].y = __fmaf_rn((k & 1) ? o23.y : e23.y, w, m23[k].y);
-      }
+    for (int i = 0; i < KP; ++i) {
+      const float2 w = FAR ? tab.far_W2[i][FAR ? q : 0] : tab.W2[i][q];
+      mA[i] = __ffma2_rn(ga, w, mA[i]);
+      m0[i] = __ffma2_rn(gb, w, m0[i]);
+      m1[i] = __ffma2_rn(gc, w, m1[i]);
+      m2[i] = __ffma2_rn(gd, w, m2[i]);
     }
   }
   // components in the order (11, 22, 33, 12, 13, 23)
@@ -210,11 +208,14 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
                        fmaf(dx, tj.z, dz * tj.x), fmaf(dy, tj.z, dz * tj.y)};
   const float Tt[6] = {tj.x * tj.x, tj.y * tj.y, tj.z * tj.z, tj.x * tj.y, tj.x * tj.z, tj.y * tj.z};
 #pragma unroll
-  for (int c = 0; c < 6; ++c)
+  for (int c = 0; c < 6; ++c) {
+    const float2 D2 = make_float2(Dd[c], Dd[c]), S2 = make_float2(Sd[c], Sd[c]), T2 = make_float2(Tt[c], Tt[c]);
 #pragma unroll
-    for (int k = 0; k < K1; ++k)
-      gcol[(k * 6 + c) * GS] =
-          fmaf(m01[k].y, Dd[c], fmaf(m23[k].x, Sd[c], fmaf(m23[k].y, Tt[c], c < 3 ? m01[k].x : 0.f)));
+    for (int i = 0; i < KP; ++i) {
+      const float2 t = c < 3 ? __ffma2_rn(m2[i], T2, mA[i]) : __fmul2_rn(m2[i], T2);
+      gcol[(i * 6 + c) * GS2] = __ffma2_rn(m0[i], D2, __ffma2_rn(m1[i], S2, t));
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -234,27 +235,29 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
 template <int M, int Q>
 struct NumShape {
   using A = AsmShape<M, Q>;
-  static constexpr int TI = A::TI, K1 = A::K1, NC = A::NC, NQ32 = A::NQ32;
+  static constexpr int TI = A::TI, K1 = A::K1, NQ32 = A::NQ32;
+  static constexpr int KP = (K1 + 1) / 2;                  // Legendre index pairs (2i, 2i + 1) of fiber j
+  static constexpr int NC2 = 6 * KP;                       // G columns, pairs of floats
   static constexpr int NT = 256;
   static constexpr int FN = kFarNodes;
   // far pairs per batch: 32 (one per lane); 16 where the tile has no more, and
   // for M > 5, whose G and T of 32 pairs would leave one CTA per SM
   static constexpr int PB = (M <= 5 && TI * TI >= 32) ? 32 : 16;
   static constexpr int JB = PB / TI;                       // j of a batch
-  static constexpr int GSF = PB * FN + PB % 32;            // G column stride (words): lanes (col, pair)
-  static constexpr int QP = Q + 1;                         // near: words per slot of a G column
-  static constexpr int GSN = TI * QP + (TI * QP + 1) % 2;  // odd: lanes = columns read distinct banks
-  static constexpr int GFLOATS = (NC * (GSF > GSN ? GSF : GSN) + 3) / 4 * 4;
-  // T of a far batch, structured and matrix-free: [jj][value][i], the j
-  // stride = TI (mod 32) past a multiple of 16 so that 32 pairs hit distinct
-  // banks; dense and near: [pair][value] with AsmShape's padded stride
+  static constexpr int GSF = PB * FN + PB % 32;            // G column stride (float2): lanes (col, pair)
+  static constexpr int QP = Q + 1;                         // near: float2 per slot of a G column
+  static constexpr int GSN = TI * QP + (TI * QP + 1) % 2;  // odd: lanes = columns
+  static constexpr int GFLOATS = (2 * NC2 * (GSF > GSN ? GSF : GSN) + 3) / 4 * 4;
+  // T of a batch.  Structured and matrix-free: [jj][value][i], the storage
+  // record's own order (s32_block), so one j is the contiguous run that a bulk
+  // copy stores; the j stride is TI past a multiple of 16 words so that a
+  // batch's pairs write distinct banks.  Dense: [pair][row, col, component].
   static constexpr int JS = NQ32 * TI + TI;
   static constexpr int TP = A::TP;
-  static constexpr int TF0 = JB * JS, TF1 = PB * TP, TF2 = TI * TP;
-  static constexpr int TFLOATS = TF0 > TF1 ? (TF0 > TF2 ? TF0 : TF2) : (TF1 > TF2 ? TF1 : TF2);
+  static constexpr int TFLOATS = JB * JS > PB * TP ? JB * JS : PB * TP;
   static constexpr size_t kSmem = sizeof(float) * (GFLOATS + TFLOATS);
-  static_assert(PB % TI == 0 && JS % 4 == 0 && TP % 4 == 0, "batches are whole j; T is copied out as float4");
-  static_assert(TI % JB == 0, "batches cover the tile's j");
+  static_assert(PB % TI == 0 && TI % JB == 0 && 32 % PB == 0, "batches are whole j and part of one mask word");
+  static_assert(JS % 4 == 0 && NQ32 * TI % 4 == 0, "a j's values are copied out from a 16-byte boundary");
 };
 
 // Block (rows of fiber a, columns of fiber b) of the dense matrix from the
@@ -281,36 +284,33 @@ template <int M, int Q, int MODE, bool P2>
 __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, const float4* __restrict__ ori,
                                                    const AsmOut& out, int I, int J) {
   using S = NumShape<M, Q>;
-  constexpr int TI = S::TI, K1 = S::K1, NC = S::NC, NT = S::NT, PB = S::PB, JB = S::JB, TP = S::TP, JS = S::JS;
-  constexpr int NQ32 = S::NQ32, NC2 = NC / 2;
+  constexpr int TI = S::TI, K1 = S::K1, NC2 = S::NC2, NT = S::NT, PB = S::PB, JB = S::JB, TP = S::TP, JS = S::JS;
+  constexpr int NQ32 = S::NQ32;
   constexpr int M3 = 3 * M;
   constexpr int FF = K1 * 3;   // force-term floats per fiber
   constexpr bool STRUCT = MODE == kAsmStructF16 || MODE == kAsmStructBF16;
   constexpr bool APPLY = MODE == kAsmApply;
-  constexpr bool QT = MODE != kAsmDense;   // far T as [jj][value][i]
+  constexpr bool QT = MODE != kAsmDense;   // T as [jj][value][i]
   static_assert(Q % 2 == 0, "mirror folding needs an even number of quadrature points");
 
-  __shared__ float4 sTi[TI], sTj[TI];    // orientations
-  __shared__ float sD[TI * TI][3];       // pair jl * TI + il: x_i - x_j, formed in FP64 and rounded once
-  __shared__ unsigned char sFar[TI * TI];
+  __shared__ float4 sTi[TI], sTj[TI];        // orientations
+  __shared__ float sD[TI * TI][3];           // pair jl * TI + il: x_i - x_j, formed in FP64 and rounded once
+  __shared__ unsigned char sKind[TI * TI];   // 0: no such pair, 1: far, 2: near
   __shared__ unsigned char sNear[TI * TI];   // the near pairs, in pair order
-  __shared__ int sNearW[NT / 32];            // near pairs per warp of the classification
+  __shared__ unsigned sMask[NT / 32];        // near pairs as bits
   extern __shared__ __align__(16) float smem_dyn[];
-  float* const sG = smem_dyn;
+  float2* const sG = reinterpret_cast<float2*>(smem_dyn);
   float* const sT = smem_dyn + S::GFLOATS;
   __shared__ float sCoef[kMaxTerms], sEig[kMaxTerms];
-  __shared__ float sFi[TI * FF], sFj[TI * FF];   // force terms of the tile's i and j
-  __shared__ short sMapS[STRUCT ? NQ32 : 1];     // stored value q (s32_block order) -> offset of its T entry
+  __shared__ float sFj[TI * FF];             // force terms of the tile's j
 
   const bool diag = (I == J);
   const int tid = threadIdx.x, lane = tid & 31;
   const int i0 = I * TI, j0 = J * TI;
   // kAsmApply with a vector applies the blocks; without one it forms the force terms
   const bool do_apply = APPLY && out.x != nullptr;
-  const bool do_force = !do_apply;
   constexpr int XW = APPLY ? TI * M3 : 1;
-  __shared__ float sXi[XW], sXj[XW], sZi[XW], sZj[XW];   // x and z rows of the I and J tiles
-  __shared__ float sNz[APPLY ? 2 * TI * M3 : 1];         // near pairs' products of one group
+  __shared__ float sXi[XW], sXj[XW], sZj[XW];   // x rows of the I and J tiles, z of this tile's j
 
   if (tid < M) { sCoef[tid] = tab.gamma[tid]; sEig[tid] = tab.eigen[tid]; }
   if (tid < TI) {
@@ -332,130 +332,132 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
     sD[tid][2] = dz;
     const bool valid = i0 + il < N && j0 + jl < N && (!diag || il < jl);
     near_pair = valid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < tab.far_d2;
-    sFar[tid] = valid && !near_pair;
+    sKind[tid] = near_pair ? 2 : valid ? 1 : 0;
   }
   const unsigned near_mask = __ballot_sync(0xffffffffu, near_pair);
-  if (lane == 0) sNearW[tid >> 5] = __popc(near_mask);
-  for (int k = tid; k < TI * FF; k += NT) sFi[k] = sFj[k] = 0.f;
+  if (lane == 0) sMask[tid >> 5] = near_mask;
   if constexpr (APPLY) {
     if (do_apply) {
       for (int k = tid; k < TI * M3; k += NT) {
         const int f = k / M3, c = k % M3;
         sXi[k] = i0 + f < N ? out.x[(int64_t)(i0 + f) * M3 + c] : 0.f;
         sXj[k] = j0 + f < N ? out.x[(int64_t)(j0 + f) * M3 + c] : 0.f;
-        sZi[k] = sZj[k] = 0.f;
       }
-    }
-  }
-  if constexpr (STRUCT) {
-    for (int q = tid; q < NQ32; q += NT) {
-      const int c = q % 6, blk = q / 6;
-      int row = 0, col = 0;
-      if (blk < M * M) {
-        row = blk / M + 1;
-        col = blk % M + 1;
-      } else if (blk < M * M + K1) {
-        col = blk - M * M;
-      } else {
-        row = blk - M * M - M;
-      }
-      sMapS[q] = (short)((row * K1 + col) * 6 + c);
     }
   }
   const float e2 = tab.e2;
   const float e2x3 = -3.f * e2;
   const float fz = tab.fz_half;
   __syncthreads();
-  int nnear = 0;
-  {
-    int before = 0;
-#pragma unroll
-    for (int w = 0; w < (TI * TI + 31) / 32; ++w) {
-      if (w < (tid >> 5)) before += sNearW[w];
-      nnear += sNearW[w];
-    }
-    // read after the barriers of the far batches
-    if (near_pair) sNear[before + __popc(near_mask & ((1u << lane) - 1))] = (unsigned char)tid;
+  if (near_pair) {   // read after the barriers of the first batch
+    int at = __popc(near_mask & ((1u << lane) - 1));
+    for (int w = 0; w < (tid >> 5); ++w) at += __popc(sMask[w]);
+    sNear[at] = (unsigned char)tid;
   }
 
-  // structured storage: the record of j = j0 + jl
+  // structured storage: the record of j = j0 + jl is rec0 + jl
   constexpr int SUB = kStoreTile / TI;
-  const int64_t rec0 = (((int64_t)(J / SUB) * (J / SUB + 1) / 2 + I / SUB) * SUB * SUB + (I % SUB) * SUB + (J % SUB)) * TI;
-  constexpr int NW = s16_record_words(M);
-  constexpr int NQ16 = AsmShape<M, Q>::NQ16;
-  // words 4 w4 .. 4 w4 + 3 of the 16-bit record whose T entries are t[sMapS[.] * stride]
-  auto words16 = [&](const float* t, int stride, int w4) -> uint4 {
-    uint32_t w[4];
+  const int64_t rec0 =
+      (((int64_t)(J / SUB) * (J / SUB + 1) / 2 + I / SUB) * SUB * SUB + (I % SUB) * SUB + (J % SUB)) * TI;
+
+  // phase 2: T[ki][kj][c] = sum_qi W[ki][qi] G[qi][c][kj], folded over qi, for the
+  // two kj of column (i, c) in the lanes of packed FP32 instructions, into the
+  // pair's T at dst (stride QS per value); lo - hi as fma(hi, -1, lo): the same
+  // rounding as a scalar subtraction
+  auto contract = [&](const float2* g, auto points, auto far, int stride, int col, float* dst) {
+    constexpr int NQ = decltype(points)::value;
+    constexpr bool FAR = decltype(far)::value;
+    constexpr int QS = QT ? TI : 1;
+    float2 acc[K1];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int q2 = 4 * w4 + u;
-      const float lo = q2 < NQ16 ? t[sMapS[2 * q2] * stride] : 0.f;
-      const float hi = q2 < NQ16 ? t[sMapS[2 * q2 + 1] * stride] : 0.f;
-      if constexpr (MODE == kAsmStructF16) {
-        __half2 hv = __floats2half2_rn(lo, hi);
-        w[u] = *reinterpret_cast<uint32_t*>(&hv);
-      } else {
-        __nv_bfloat162 hv = __floats2bfloat162_rn(lo, hi);
-        w[u] = *reinterpret_cast<uint32_t*>(&hv);
+    for (int k = 0; k < K1; ++k) acc[k] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < NQ / 2; ++q) {
+      const float2 lo = g[q * stride], hi = g[(NQ - 1 - q) * stride];
+      const float2 ev = __fadd2_rn(lo, hi), od = __ffma2_rn(hi, make_float2(-1.f, -1.f), lo);
+#pragma unroll
+      for (int k = 0; k < K1; ++k) {
+        const float w = FAR ? tab.far_W[k][FAR ? q : 0] : tab.W[k][q];
+        acc[k] = __ffma2_rn((k & 1) ? od : ev, make_float2(w, w), acc[k]);
       }
     }
-    return make_uint4(w[0], w[1], w[2], w[3]);
+    const int i = col / 6, c = col % 6;
+#pragma unroll
+    for (int lane2 = 0; lane2 < 2; ++lane2) {
+      const int kj = 2 * i + lane2;
+      if (lane2 == 1 && K1 % 2 == 1 && kj == K1) break;   // odd M + 1: no such index
+      // block (k, kj): dense order k K1 + kj; storage order s32_block
+      const int b0 = QT ? M * M + kj : kj;                                     // k = 0
+      const int b1 = QT ? (kj > 0 ? kj - 1 : M * M + K1) : K1 + kj;            // k = 1
+      const int bs = QT ? (kj > 0 ? M : 1) : K1;                               // per k after that
+#pragma unroll
+      for (int k = 0; k < K1; ++k)
+        dst[((k == 0 ? b0 : b1 + (k - 1) * bs) * 6 + c) * QS] = lane2 == 0 ? acc[k].x : acc[k].y;
+    }
   };
+  auto t_of = [&](int jj, int il) { return QT ? sT + jj * JS + il : sT + (jj * TI + il) * TP; };
 
   // i-side sums of task (jj, k, il) = this thread, over the batches: force
   // terms (k <= M) or z (k < M)
   float iacc[3] = {0.f, 0.f, 0.f};
   const int jcount = min(TI, N - j0);
+  int near0 = 0;   // near pairs of the batches done
 
-  // ---- far pairs, JB rows of the tile per batch -----------------------------
   for (int jb = 0; jb < jcount; jb += JB) {
-    // phase 1: G[c][k] = sum_qj K_c(qi, qj) W[k][qj], unit u = qi * PB + pair
+    // ---- far pairs.  Phase 1: G[c][k] = sum_qj K_c(qi, qj) W[k][qj], unit
+    // u = qi * PB + pair; zeros for the others
     if (tid < PB * S::FN) {
       const int p = tid % PB, qi = tid / PB;
-      const int il = p % TI, jl = jb + p / TI;
-      float* const gcol = sG + tid;
-      if (sFar[jl * TI + il]) {
+      const int pr = jb * TI + p, il = p % TI;
+      float2* const gcol = sG + tid;
+      if (sKind[pr] == 1) {
         const float4 ti = sTi[il];
         const float si = tab.far_pts[qi];
-        const float* D = sD[jl * TI + il];
-        const float pp[3] = {fmaf(si, ti.x, D[0]), fmaf(si, ti.y, D[1]), fmaf(si, ti.z, D[2])};
-        stokeslet_moments_G<K1, S::FN, S::GSF, true, true>(tab, pp, sTj[jl], e2, e2x3, gcol);
+        const float pp[3] = {fmaf(si, ti.x, sD[pr][0]), fmaf(si, ti.y, sD[pr][1]), fmaf(si, ti.z, sD[pr][2])};
+        stokeslet_moments_G<K1, S::FN, S::GSF, true, true>(tab, pp, sTj[pr / TI], e2, e2x3, gcol);
       } else {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) gcol[c * S::GSF] = 0.f;
+        for (int c = 0; c < NC2; ++c) gcol[c * S::GSF] = make_float2(0.f, 0.f);
       }
     }
+    // T of the last batch has left shared memory before phase 2 overwrites it
+    if (STRUCT && tid < JB) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncthreads();
-    // phase 2: T[ki][kj][c] = sum_qi W[ki][qi] G[qi][c][kj], folded over qi;
-    // lanes = pairs, a lane takes columns col and col + NC/2 in the two lanes of
-    // packed FP32 instructions
+    // phase 2, lanes = pairs
     for (int task = tid; task < PB * NC2; task += NT) {
       const int col = task / PB, p = task % PB;
-      const float* ga = sG + col * S::GSF + p;
-      const float* gb = ga + NC2 * S::GSF;
-      float2 acc[K1];
-#pragma unroll
-      for (int k = 0; k < K1; ++k) acc[k] = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int q = 0; q < S::FN / 2; ++q) {
-        const float2 lo = make_float2(ga[q * PB], gb[q * PB]);
-        const float2 hi = make_float2(ga[(S::FN - 1 - q) * PB], gb[(S::FN - 1 - q) * PB]);
-        const float2 ev = __fadd2_rn(lo, hi), od = __ffma2_rn(hi, make_float2(-1.f, -1.f), lo);
-#pragma unroll
-        for (int k = 0; k < K1; ++k) acc[k] = __ffma2_rn((k & 1) ? od : ev, tab.far_W2[k][q], acc[k]);
+      contract(sG + col * S::GSF + p, std::integral_constant<int, S::FN>(), std::true_type(), PB, col,
+               t_of(p / TI, p % TI));
+    }
+    // ---- near pairs of these rows, in groups of up to TI, into the same T
+    const unsigned bits = (sMask[jb * TI / 32] >> (jb * TI % 32)) & (PB == 32 ? 0xffffffffu : (1u << PB % 32) - 1u);
+    const int near1 = near0 + __popc(bits);
+    for (int n0 = near0; n0 < near1; n0 += TI) {
+      const int cnt = min(TI, near1 - n0);
+      __syncthreads();   // G is read
+      if (tid < cnt * Q) {
+        const int slot = tid / Q, qi = tid % Q;
+        const int pr = sNear[n0 + slot];
+        const float4 ti = sTi[pr % TI];
+        const float si = tab.pts[qi];
+        const float pp[3] = {fmaf(si, ti.x, sD[pr][0]), fmaf(si, ti.y, sD[pr][1]), fmaf(si, ti.z, sD[pr][2])};
+        stokeslet_moments_G<K1, Q, S::GSN, P2, false>(tab, pp, sTj[pr / TI], e2, e2x3, sG + slot * S::QP + qi);
       }
-      // column col = kj * 6 + c; T entry (k * K1 + kj) * 6 + c = k * NC + col
-      float* const dst = QT ? sT + (p / TI) * JS + p % TI : sT + p * TP;
-      constexpr int QS = QT ? TI : 1;
-#pragma unroll
-      for (int k = 0; k < K1; ++k) {
-        dst[(k * NC + col) * QS] = acc[k].x;
-        dst[(k * NC + col + NC2) * QS] = acc[k].y;
+      __syncthreads();
+      for (int task = tid; task < cnt * NC2; task += NT) {   // lanes = columns
+        const int slot = task / NC2, col = task % NC2;
+        const int pr = sNear[n0 + slot];
+        contract(sG + col * S::GSN + slot * S::QP, std::integral_constant<int, Q>(), std::false_type(), 1, col,
+                 t_of(pr / TI - jb, pr % TI));
       }
     }
+    near0 = near1;
+    // the bulk copy below reads T through the async proxy
+    if (STRUCT) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    // phase 3: the batch's blocks to their destination (the next batch's phase 1
-    // writes G only, and its phase 2 follows a barrier)
+    // ---- phase 3: the batch's blocks to their destination (the next batch's
+    // phase 1 writes G only, and its phase 2 follows a barrier).  Pairs that do
+    // not exist (i >= N, i >= j on a diagonal tile) came out as exact zeros
     if constexpr (MODE == kAsmDense) {
       // block (i, j): rows of fiber i, columns of fiber j
       for (int task = tid; task < PB * M * M; task += NT) {
@@ -470,58 +472,70 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
             for (int a = 0; a < 3; ++a) dst[a + b * out.lda] = (kIp == kJp && a == b) ? 1.f : 0.f;
           continue;
         }
-        if (!sFar[jl * TI + tl]) continue;
-        dense_block(dst, out.lda, sT + (jj * TI + tl) * TP + ((kIp + 1) * K1 + kJp + 1) * 6, sTi[tl], kIp, sCoef[kIp],
-                    sEig[kIp]);
+        if (!sKind[jl * TI + tl]) continue;
+        dense_block(dst, out.lda, t_of(jj, tl) + ((kIp + 1) * K1 + kJp + 1) * 6, sTi[tl], kIp, sCoef[kIp], sEig[kIp]);
       }
       // block (j, i): rows of fiber j, columns of fiber i
       for (int task = tid; task < PB * M * M; task += NT) {
         const int jj = task / (TI * M * M), r0 = task % (TI * M * M);
         const int tl = r0 / (M * M), rem = r0 % (M * M);
         const int kIp = rem / M, kJp = rem % M, jl = jb + jj;
-        if (!sFar[jl * TI + tl]) continue;
+        if (!sKind[jl * TI + tl]) continue;
         float* dst = out.A + (int64_t)((j0 + jl) * M3 + 3 * kJp) + (int64_t)((i0 + tl) * M3 + 3 * kIp) * out.lda;
-        dense_block(dst, out.lda, sT + (jj * TI + tl) * TP + ((kIp + 1) * K1 + kJp + 1) * 6, sTj[jl], kJp, sCoef[kJp],
-                    sEig[kJp]);
+        dense_block(dst, out.lda, t_of(jj, tl) + ((kIp + 1) * K1 + kJp + 1) * 6, sTj[jl], kJp, sCoef[kJp], sEig[kJp]);
       }
     } else if constexpr (STRUCT) {
-      // T is [jj][q][il] with q in (row, col) order, stored in s32_block order:
-      // one j is a contiguous run of NQ32 x TI floats.  Near pairs and pairs
-      // that do not exist (i >= N, i >= j on a diagonal tile) are exact zeros
-      // here (the near pairs' blocks follow below).  No FP32 copy in the
-      // recompute modes (out.S32 null)
+      // FP32: one bulk copy per j (no FP32 copy in the recompute modes: out.S32 null)
       const int jn = min(JB, jcount - jb);
-      if (out.S32 != nullptr) {
-        float4* d32 = reinterpret_cast<float4*>(out.S32 + (rec0 + jb) * (int64_t)(NQ32 * TI));
-        constexpr int V = NQ32 * TI / 4;   // float4 per j
-        for (int v = tid; v < jn * V; v += NT) {
-          const int jj = v / V, r = v % V;
-          const int q = r / (TI / 4), g4 = (r % (TI / 4)) * 4;
-          d32[v] = *reinterpret_cast<const float4*>(sT + jj * JS + sMapS[q] * TI + g4);
-        }
+      if (out.S32 != nullptr && tid < jn) {
+        const float* dst = out.S32 + (rec0 + jb + tid) * (int64_t)(NQ32 * TI);
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                     "r"(static_cast<uint32_t>(__cvta_generic_to_shared(sT + tid * JS))), "r"(NQ32 * TI * 4)
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
-      // 16-bit records [il][NW]: pair il's words are contiguous
+      // 16-bit records [i][NW]: the M^2 operator blocks, which lead the FP32
+      // record, two values per word; lane = pair
+      constexpr int NW = s16_record_words(M), NQ16 = AsmShape<M, Q>::NQ16;
       uint32_t* d16 = out.S16 + (rec0 + jb) * (int64_t)(NW * TI);
-      for (int v = tid; v < jn * (TI * NW / 4); v += NT) {
-        const int jj = v / (TI * NW / 4), r = v % (TI * NW / 4);
-        const int tl = r % TI, w4 = r / TI;
-        *reinterpret_cast<uint4*>(&d16[(jj * TI + tl) * NW + 4 * w4]) = words16(sT + jj * JS + tl, TI, w4);
+      for (int v = tid; v < PB * (NW / 4); v += NT) {
+        const int p = v % PB, w4 = v / PB;
+        if (p / TI >= jn) continue;
+        const float* t = t_of(p / TI, p % TI) + 8 * w4 * TI;
+        uint32_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool in = NQ16 % 4 == 0 || 4 * w4 + u < NQ16;
+          const float lo = in ? t[2 * u * TI] : 0.f, hi = in ? t[(2 * u + 1) * TI] : 0.f;
+          if constexpr (MODE == kAsmStructF16) {
+            __half2 hv = __floats2half2_rn(lo, hi);
+            w[u] = *reinterpret_cast<uint32_t*>(&hv);
+          } else {
+            __nv_bfloat162 hv = __floats2bfloat162_rn(lo, hi);
+            w[u] = *reinterpret_cast<uint32_t*>(&hv);
+          }
+        }
+        *reinterpret_cast<uint4*>(&d16[p * NW + 4 * w4]) = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
     // i side: sums over the thread's own j of each batch; j side: sums over the
     // tile's i by halving shuffles in groups of TI lanes
+    const unsigned grp = ((1u << TI) - 1u) << (lane & ~(TI - 1));
     if (APPLY && do_apply) {
       if constexpr (APPLY) {
+        // z_i[k] += T(k+1, l+1) x_j[l], z_j[k] += T(l+1, k+1) x_i[l] (blocks symmetric)
         for (int task = tid; task < 2 * PB * M; task += NT) {
           const bool iside = task < PB * M;
           const int u = iside ? task : task - PB * M;
           const int jj = u / (TI * M), k = (u / TI) % M, tl = u % TI, jl = jb + jj;
           const float* xv = iside ? sXj + jl * M3 : sXi + tl * M3;
+          const float* t = t_of(jj, tl) + (iside ? k * M : k) * 6 * TI;
+          const int ts = (iside ? 1 : M) * 6 * TI;
           float zs[3] = {0.f, 0.f, 0.f};
 #pragma unroll
           for (int l = 0; l < M; ++l) {
-            const float* t = sT + jj * JS + ((iside ? (k + 1) * K1 + l + 1 : (l + 1) * K1 + k + 1) * 6) * TI + tl;
-            const float T6[6] = {t[0], t[TI], t[2 * TI], t[3 * TI], t[4 * TI], t[5 * TI]};
+            const float* b = t + l * ts;
+            const float T6[6] = {b[0], b[TI], b[2 * TI], b[3 * TI], b[4 * TI], b[5 * TI]};
 #pragma unroll
             for (int a = 0; a < 3; ++a)
               zs[a] = fmaf(sym_get(T6, a, 0), xv[3 * l],
@@ -531,7 +545,6 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
 #pragma unroll
             for (int a = 0; a < 3; ++a) iacc[a] += zs[a];
           } else {
-            const unsigned grp = (TI == 32 ? 0xffffffffu : ((1u << TI) - 1u)) << (lane & ~(TI - 1));
 #pragma unroll
             for (int o = TI / 2; o > 0; o >>= 1)
 #pragma unroll
@@ -549,15 +562,14 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
         const bool iside = task < PB * K1;
         const int u = iside ? task : task - PB * K1;
         const int jj = u / (TI * K1), k = (u / TI) % K1, tl = u % TI, jl = jb + jj;
-        const int q0 = (iside ? k * K1 : k) * 6;
-        const float* t = QT ? sT + jj * JS + q0 * TI + tl : sT + (jj * TI + tl) * TP + q0;
+        const int blk = QT ? (iside ? s32_block(M, k, 0) : s32_block(M, 0, k)) : (iside ? k * K1 : k);
         constexpr int QS = QT ? TI : 1;
+        const float* t = t_of(jj, tl) + blk * 6 * QS;
         float f3[3] = {t[4 * QS], t[5 * QS], t[2 * QS]};
         if (iside) {
 #pragma unroll
           for (int a = 0; a < 3; ++a) iacc[a] = fmaf(f3[a], fz, iacc[a]);
         } else {
-          const unsigned grp = (TI == 32 ? 0xffffffffu : ((1u << TI) - 1u)) << (lane & ~(TI - 1));
 #pragma unroll
           for (int o = TI / 2; o > 0; o >>= 1)
 #pragma unroll
@@ -569,148 +581,28 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
       }
     }
   }
+  if (STRUCT && tid < JB) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 
-  // ---- near pairs, groups of up to TI ----------------------------------------
-  for (int n0 = 0; n0 < nnear; n0 += TI) {
-    const int cnt = min(TI, nnear - n0);
-    __syncthreads();   // G and T of the previous batch or group are read
-    if (tid < cnt * Q) {
-      const int slot = tid / Q, qi = tid % Q;
-      const int pr = sNear[n0 + slot], il = pr % TI, jl = pr / TI;
-      const float4 ti = sTi[il];
-      const float si = tab.pts[qi];
-      const float pp[3] = {fmaf(si, ti.x, sD[pr][0]), fmaf(si, ti.y, sD[pr][1]), fmaf(si, ti.z, sD[pr][2])};
-      stokeslet_moments_G<K1, Q, S::GSN, P2, false>(tab, pp, sTj[jl], e2, e2x3, sG + slot * S::QP + qi);
-    }
-    __syncthreads();
-    // lanes = columns; P2 as in the far phase 2 (lo - hi as fma(hi, -1, lo): the
-    // same rounding as the scalar subtraction)
-    if constexpr (P2) {
-      for (int task = tid; task < cnt * NC2; task += NT) {
-        const int slot = task / NC2, col = task % NC2;
-        const float* ga = sG + col * S::GSN + slot * S::QP;
-        const float* gb = ga + NC2 * S::GSN;
-        float2 acc[K1];
-#pragma unroll
-        for (int k = 0; k < K1; ++k) acc[k] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int q = 0; q < Q / 2; ++q) {
-          const float2 lo = make_float2(ga[q], gb[q]), hi = make_float2(ga[Q - 1 - q], gb[Q - 1 - q]);
-          const float2 ev = __fadd2_rn(lo, hi), od = __ffma2_rn(hi, make_float2(-1.f, -1.f), lo);
-#pragma unroll
-          for (int k = 0; k < K1; ++k) acc[k] = __ffma2_rn((k & 1) ? od : ev, tab.W2[k][q], acc[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < K1; ++k) {
-          sT[slot * TP + k * NC + col] = acc[k].x;
-          sT[slot * TP + k * NC + col + NC2] = acc[k].y;
-        }
-      }
-    } else {
-      for (int task = tid; task < cnt * NC; task += NT) {
-        const int slot = task / NC, col = task % NC;
-        const float* gp = sG + col * S::GSN + slot * S::QP;
-        float acc[K1];
-#pragma unroll
-        for (int k = 0; k < K1; ++k) acc[k] = 0.f;
-#pragma unroll 4
-        for (int q = 0; q < Q / 2; ++q) {
-          const float lo = gp[q], hi = gp[Q - 1 - q];
-          const float ev = __fadd_rn(lo, hi), od = __fsub_rn(lo, hi);
-#pragma unroll
-          for (int k = 0; k < K1; ++k) acc[k] = __fmaf_rn((k & 1) ? od : ev, tab.W[k][q], acc[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < K1; ++k) sT[slot * TP + k * NC + col] = acc[k];
-      }
-    }
-    __syncthreads();
-    if constexpr (MODE == kAsmDense) {
-      for (int task = tid; task < 2 * cnt * M * M; task += NT) {
-        const int side = task / (cnt * M * M), rem = task % (cnt * M * M);
-        const int slot = rem / (M * M), kJp = (rem % (M * M)) / M, kIp = rem % M;
-        const int pr = sNear[n0 + slot], il = pr % TI, jl = pr / TI;
-        const int64_t ri = (int64_t)(i0 + il) * M3 + 3 * kIp, rj = (int64_t)(j0 + jl) * M3 + 3 * kJp;
-        const float* T6 = sT + slot * TP + ((kIp + 1) * K1 + kJp + 1) * 6;
-        if (side == 0) dense_block(out.A + ri + rj * out.lda, out.lda, T6, sTi[il], kIp, sCoef[kIp], sEig[kIp]);
-        else dense_block(out.A + rj + ri * out.lda, out.lda, T6, sTj[jl], kJp, sCoef[kJp], sEig[kJp]);
-      }
-    } else if constexpr (STRUCT) {
-      // over the zeros that the far batches of this CTA stored (ordered by the
-      // barriers above)
-      if (out.S32 != nullptr)
-        for (int v = tid; v < cnt * NQ32; v += NT) {
-          const int slot = v / NQ32, q = v % NQ32;
-          const int pr = sNear[n0 + slot];
-          out.S32[(rec0 + pr / TI) * (int64_t)(NQ32 * TI) + q * TI + pr % TI] = sT[slot * TP + sMapS[q]];
-        }
-      for (int v = tid; v < cnt * (NW / 4); v += NT) {
-        const int slot = v / (NW / 4), w4 = v % (NW / 4);
-        const int pr = sNear[n0 + slot];
-        uint32_t* d16 = out.S16 + ((rec0 + pr / TI) * TI + pr % TI) * (int64_t)NW;
-        *reinterpret_cast<uint4*>(&d16[4 * w4]) = words16(sT + slot * TP, 1, w4);
-      }
-    }
-    if (APPLY && do_apply) {
-      if constexpr (APPLY) {
-        for (int task = tid; task < 2 * cnt * M; task += NT) {
-          const int side = task / (cnt * M), slot = (task % (cnt * M)) / M, k = task % M;
-          const int pr = sNear[n0 + slot];
-          const float* xv = side == 0 ? sXj + (pr / TI) * M3 : sXi + (pr % TI) * M3;
-          float zs[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-          for (int l = 0; l < M; ++l) {
-            const float* T6 = sT + slot * TP + (side == 0 ? (k + 1) * K1 + l + 1 : (l + 1) * K1 + k + 1) * 6;
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-              zs[a] = fmaf(sym_get(T6, a, 0), xv[3 * l],
-                           fmaf(sym_get(T6, a, 1), xv[3 * l + 1], fmaf(sym_get(T6, a, 2), xv[3 * l + 2], zs[a])));
-          }
-#pragma unroll
-          for (int a = 0; a < 3; ++a) sNz[(side * TI + slot) * M3 + 3 * k + a] = zs[a];
-        }
-        __syncthreads();
-        for (int u = tid; u < 2 * M3; u += NT) {
-          const int side = u / M3, c = u % M3;
-          for (int slot = 0; slot < cnt; ++slot) {
-            const int pr = sNear[n0 + slot];
-            (side == 0 ? sZi[(pr % TI) * M3 + c] : sZj[(pr / TI) * M3 + c]) += sNz[(side * TI + slot) * M3 + c];
-          }
-        }
-      }
-    } else if (tid < 2 * FF) {
-      // component a of force term k of one side: the group's pairs in order
-      const int side = tid / FF, k = (tid % FF) / 3, a = tid % 3;
-      const int q0 = (side == 0 ? k * K1 : k) * 6 + (a == 0 ? 4 : a == 1 ? 5 : 2);
-      for (int slot = 0; slot < cnt; ++slot) {
-        const int pr = sNear[n0 + slot];
-        float& f = side == 0 ? sFi[(pr % TI) * FF + 3 * k + a] : sFj[(pr / TI) * FF + 3 * k + a];
-        f = fmaf(sT[slot * TP + q0], fz, f);
-      }
-    }
-  }
-  __syncthreads();
-
-  // ---- i-side sums over the JB rows of a batch, added to the near pairs' -----
+  // ---- i-side sums over the JB rows of a batch (G is free: its last readers
+  // passed a barrier), then the partial rows, each written exactly once
+  float* const red = smem_dyn;
   if (APPLY && do_apply) {
     if constexpr (APPLY) {
       if (tid < PB * M) {
         const int jj = tid / (TI * M), k = (tid / TI) % M, tl = tid % TI;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) sG[(jj * TI + tl) * M3 + 3 * k + a] = iacc[a];
+        for (int a = 0; a < 3; ++a) red[(jj * TI + tl) * M3 + 3 * k + a] = iacc[a];
       }
       __syncthreads();
-      // partial rows of z: the i side of tile (I, J) to slot J, the j side to
-      // slot I (a diagonal tile's j side to slot T): every slot of every fiber
-      // is written exactly once per product
+      // the i side of tile (I, J) to slot J, the j side to slot I (a diagonal
+      // tile's j side to the slot after the last tile)
       const int64_t R = (int64_t)M3 * N;
-      const int T8 = (N + TI - 1) / TI;
       float* zi = out.zpart + (int64_t)J * R + (int64_t)i0 * M3;
-      float* zj = out.zpart + (int64_t)(diag ? T8 : I) * R + (int64_t)j0 * M3;
+      float* zj = out.zpart + (int64_t)(diag ? (N + TI - 1) / TI : I) * R + (int64_t)j0 * M3;
       for (int u = tid; u < TI * M3; u += NT) {
-        float v = sZi[u];
+        float v = red[u];
 #pragma unroll
-        for (int jj = 0; jj < JB; ++jj) v += sG[jj * TI * M3 + u];
+        for (int jj = 1; jj < JB; ++jj) v += red[jj * TI * M3 + u];
         if (i0 + u / M3 < N) zi[u] = v;
         if (j0 + u / M3 < N) zj[u] = sZj[u];
       }
@@ -720,17 +612,18 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
   if (tid < PB * K1) {
     const int jj = tid / (TI * K1), k = (tid / TI) % K1, tl = tid % TI;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) sG[(jj * TI + tl) * FF + 3 * k + a] = iacc[a];
+    for (int a = 0; a < 3; ++a) red[(jj * TI + tl) * FF + 3 * k + a] = iacc[a];
   }
   __syncthreads();
-  // partial force terms: ffpart[X][fiber of Y][k][3] written exactly once
+  // partial force terms ffpart[X][fiber of Y][k][3]
   for (int u = tid; u < TI * FF; u += NT) {
-    float v = sFi[u];
+    float v = red[u];
 #pragma unroll
-    for (int jj = 0; jj < JB; ++jj) v += sG[jj * TI * FF + u];
-    if (diag) v += sFj[u];
+    for (int jj = 1; jj < JB; ++jj) v += red[jj * TI * FF + u];
+    const bool jin = j0 + u / FF < N;
+    if (diag && jin) v += sFj[u];
     if (i0 + u / FF < N) out.ffpart[((int64_t)J * N + i0) * FF + u] = v;
-    if (!diag && j0 + u / FF < N) out.ffpart[((int64_t)I * N + j0) * FF + u] = sFj[u];
+    if (!diag && jin) out.ffpart[((int64_t)I * N + j0) * FF + u] = sFj[u];
   }
 }
 

@@ -242,7 +242,7 @@ static Tables make_tables(const rf_config& c) {
     for (int k = 0; k <= M; ++k) {
       // weight and Legendre value rounded separately, as the REAL*4 tables are
       t.W[k][q] = (float)wts[q] * (float)P(pts[q], k);
-      if (2 * q < Q) t.W2[k][q] = make_float2(t.W[k][q], t.W[k][q]);
+      if (2 * q < Q) (k % 2 ? t.W2[k / 2][q].y : t.W2[k / 2][q].x) = t.W[k][q];
     }
   }
   double fx[kFarNodes], fv[kFarNodes];
@@ -276,7 +276,7 @@ static Tables make_tables(const rf_config& c) {
     for (int q = 0; q < kFarNodes / 2; ++q) {
       t.far_W[k][q] = (float)wk[q];
       t.far_W[k][kFarNodes - 1 - q] = (k & 1) ? -t.far_W[k][q] : t.far_W[k][q];
-      t.far_W2[k][q] = make_float2(t.far_W[k][q], t.far_W[k][q]);
+      (k % 2 ? t.far_W2[k / 2][q].y : t.far_W2[k / 2][q].x) = t.far_W[k][q];
     }
   }
   // Centre distance from which the far rule's blocks are the full rule's to

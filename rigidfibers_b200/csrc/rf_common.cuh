@@ -22,9 +22,9 @@ constexpr int kFarNodes = 8;      // points per fiber of the far rule (Tables::f
 struct Tables {
   float pts[kMaxQuad];
   float W[kMaxTerms + 1][kMaxQuad];   // W[0][q] = w_q
-  // W2[k][q] = (W[k][q], W[k][q]) for q < Q/2: the weight as the second
-  // operand of a packed two-lane FP32 multiply-add
-  float2 W2[kMaxTerms + 1][kMaxQuad / 2];
+  // W2[i][q] = (W[2i][q], W[2i+1][q]) for q < Q/2 (0 past P_M): the weights of an
+  // even and an odd Legendre index as the operand of a packed multiply-add
+  float2 W2[kMaxTerms / 2 + 1][kMaxQuad / 2];
   // The far rule: the kFarNodes-point Gauss rule of the discrete measure
   // {pts, w}, which gives that sum exactly for polynomials of degree
   // 2 kFarNodes - 1, hence the sums against P_0..P_M of any kernel that is
@@ -32,7 +32,7 @@ struct Tables {
   // |x_i - x_j|^2 >= far_d2 take it.
   float far_pts[kFarNodes];
   float far_W[kMaxTerms + 1][kFarNodes];
-  float2 far_W2[kMaxTerms + 1][kFarNodes / 2];
+  float2 far_W2[kMaxTerms / 2 + 1][kFarNodes / 2];
   float far_d2;
   float gamma[kMaxTerms];   // gamma[0] = D1 (force index 0), gamma[k] for k>=1
   float eigen[kMaxTerms];   // E_k; unused for k = 0

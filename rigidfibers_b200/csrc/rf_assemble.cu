@@ -754,40 +754,64 @@ k_assemble_analytical(const Tables tab, int N, const float4* __restrict__ ori, A
   }
 }
 
-// F[i][k] = sum_X ffpart[X][i][k] (fixed order); b[i][k'] = -C_i(k') F[i][k'+1]
-// for unit u = (i, k) of N (M + 1).
-__device__ __forceinline__ void force_term_unit(const Tables& tab, int N, const float4* __restrict__ ori,
-                                                const float* __restrict__ ffpart, int nparts, float* __restrict__ F,
-                                                float* __restrict__ b, int64_t u) {
-  const int M = tab.M, K1 = M + 1, FFn = 3 * K1;
-  {
-    const int i = (int)(u / K1), k = (int)(u % K1);
-    float s[3] = {0.f, 0.f, 0.f};
-    for (int p = 0; p < nparts; ++p) {
-      const float* src = ffpart + ((int64_t)p * N + i) * FFn + 3 * k;
-      s[0] += src[0]; s[1] += src[1]; s[2] += src[2];
-    }
-    float* f = F + (int64_t)i * FFn + 3 * k;
-    f[0] = s[0]; f[1] = s[1]; f[2] = s[2];
-    if (k >= 1) {
-      const int kp = k - 1;
-      const float4 t = ori[i];
-      const float t3[3] = {t.x, t.y, t.z};
-      const float QF = s[0] * t3[0] + s[1] * t3[1] + s[2] * t3[2];
-      const float coef = tab.gamma[kp], E = tab.eigen[kp];
-      float* dst = b + (int64_t)i * 3 * M + 3 * kp;
+// F[i] = sum_X ffpart[X][i] (rows X = g (mod 8) in order for each of 8 groups, then
+// the groups in order) and b[i][k'] = -C_i(k') F[i][k'+1], for the kForceFibers
+// fibers from i0.  Thread (group, component): 8 loads in flight per thread.
+// Bound: the partial rows (N=4000: 144 MB, 227 us with one thread per (i, k)).
+constexpr int kForceFibers = 4, kForceGroups = 8;
+static inline int force_threads(int M) { return kForceFibers * 3 * (M + 1) * kForceGroups; }
+
+__device__ __forceinline__ void force_terms_block(const Tables& tab, int N, const float4* __restrict__ ori,
+                                                  const float* __restrict__ ffpart, int nparts, float* __restrict__ F,
+                                                  float* __restrict__ b, int i0) {
+  __shared__ float red[kForceGroups][kForceFibers * 3 * (kMaxTerms + 1)];
+  __shared__ float sum[kForceFibers * 3 * (kMaxTerms + 1)];
+  const int M = tab.M, FFn = 3 * (M + 1), C = kForceFibers * FFn;
+  const int c = (int)threadIdx.x % C, g = (int)threadIdx.x / C;
+  const bool in = i0 + c / FFn < N;
+  const int64_t row = (int64_t)N * FFn;
+  float s = 0.f;
+  if (in) {
+    const float* src = ffpart + (int64_t)i0 * FFn + c;
+    int p = g;
+    for (; p + 7 * kForceGroups < nparts; p += 8 * kForceGroups) {
+      float v[8];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) dst[a] = kp == 0 ? -coef * t3[a] * QF : -coef * (s[a] - E * t3[a] * QF);
+      for (int u = 0; u < 8; ++u) v[u] = src[(p + u * kForceGroups) * row];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
     }
+    for (; p < nparts; p += kForceGroups) s += src[p * row];
+  }
+  red[g][c] = s;
+  __syncthreads();
+  if (g == 0) {
+    float v = red[0][c];
+#pragma unroll
+    for (int q = 1; q < kForceGroups; ++q) v += red[q][c];
+    sum[c] = v;
+    if (in) F[(int64_t)i0 * FFn + c] = v;
+  }
+  __syncthreads();
+  const int u = (int)threadIdx.x, il = u / M, kp = u % M;
+  if (u >= kForceFibers * M || i0 + il >= N) return;
+  const float* f = sum + il * FFn + 3 * (kp + 1);
+  const float4 t = ori[i0 + il];
+  const float t3[3] = {t.x, t.y, t.z};
+  const float QF = fmaf(f[2], t3[2], fmaf(f[1], t3[1], __fmul_rn(f[0], t3[0])));
+  const float coef = tab.gamma[kp], E = tab.eigen[kp];
+  float* dst = b + (int64_t)(i0 + il) * 3 * M + 3 * kp;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float tq = __fmul_rn(t3[a], QF);
+    dst[a] = __fmul_rn(-coef, kp == 0 ? tq : fmaf(-E, tq, f[a]));
   }
 }
 
 __global__ void k_force_terms(const Tables tab, int N, const float4* __restrict__ ori,
                               const float* __restrict__ ffpart, int nparts, float* __restrict__ F,
                               float* __restrict__ b) {
-  const int64_t n = (int64_t)N * (tab.M + 1);
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
-    force_term_unit(tab, N, ori, ffpart, nparts, F, b, u);
+  force_terms_block(tab, N, ori, ffpart, nparts, F, b, (int)blockIdx.x * kForceFibers);
 }
 
 // ---- packed step: every member of a group (one Tables) in one launch ------
@@ -809,13 +833,14 @@ k_pack_assemble(const Tables tab, const PackStepMember* __restrict__ mem, int n)
   assemble_pair_tile<5, 24, MODE, true>(tab, p.N, p.ori32, out, I, J);
 }
 
-// one block per member: its force terms and right-hand side
-__global__ void __launch_bounds__(256) k_pack_force_terms(const Tables tab, const PackStepMember* __restrict__ mem) {
+// blockIdx.x: member, blockIdx.y: kForceFibers of its fibers (the grid covers
+// the largest member the packed solve takes)
+__global__ void k_pack_force_terms(const Tables tab, const PackStepMember* __restrict__ mem) {
   const PackStepMember& p = mem[blockIdx.x];
-  const int N = p.N;
-  const int64_t n = (int64_t)N * (tab.M + 1);
-  const int nparts = (N + AsmShape<5, 24>::TI - 1) / AsmShape<5, 24>::TI;
-  for (int64_t u = threadIdx.x; u < n; u += blockDim.x) force_term_unit(tab, N, p.ori32, p.ffpart, nparts, p.F, p.b, u);
+  const int i0 = (int)blockIdx.y * kForceFibers;
+  if (i0 >= p.N) return;
+  const int nparts = (p.N + AsmShape<5, 24>::TI - 1) / AsmShape<5, 24>::TI;
+  force_terms_block(tab, p.N, p.ori32, p.ffpart, nparts, p.F, p.b, i0);
 }
 
 int launch_pack_assemble(const Tables& tab, const PackStepMember* members, int n, int64_t blocks, bool bf16,
@@ -834,7 +859,7 @@ int launch_pack_assemble(const Tables& tab, const PackStepMember* members, int n
     k_pack_assemble<kAsmStructF16><<<(unsigned)blocks, NumShape<5, 24>::NT, smem, st>>>(tab, members, n);
   }
   RF_LAUNCH_CHECK();
-  k_pack_force_terms<<<(unsigned)n, 256, 0, st>>>(tab, members);
+  k_pack_force_terms<<<dim3((unsigned)n, kPackMaxFibers / kForceFibers), force_threads(5), 0, st>>>(tab, members);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }
@@ -899,8 +924,7 @@ static int launch_analytical(const Tables& tab, int N, const float4* ori, const 
 
 static int launch_force_terms(const Tables& tab, int N, const float4* ori, const AsmOut& out, float* F, float* b,
                               cudaStream_t st) {
-  const int64_t n = (int64_t)N * (tab.M + 1);
-  k_force_terms<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 148 * 8), 256, 0, st>>>(
+  k_force_terms<<<(unsigned)ceil_div(N, kForceFibers), force_threads(tab.M), 0, st>>>(
       tab, N, ori, out.ffpart, assemble_tiles(tab.M, tab.Q, N), F, b);
   RF_LAUNCH_CHECK();
   return RF_OK;

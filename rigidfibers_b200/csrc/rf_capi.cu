@@ -728,8 +728,8 @@ static int allocate_buffers(rf_handle* h, const rf_config* cfg) {
     }
   }
   // velocities
-  if (!rc) rc = h->alloc((void**)&h->fw, (size_t)N * h->Q * sizeof(float4));
-  if (!rc) rc = h->alloc((void**)&h->vpart, (size_t)velocity_chunks(N) * N * 6 * sizeof(float));
+  if (!rc) rc = h->alloc((void**)&h->fw, (size_t)N * (h->Q + kFarNodes) * sizeof(float4));
+  if (!rc) rc = h->alloc((void**)&h->vpart, (size_t)velocity_rows(N) * N * 6 * sizeof(float));
   if (!rc) rc = h->alloc((void**)&h->vflag, sizeof(int));
   if (!rc && !h->dry && !(h->host_vflag = static_cast<int*>(pinned_pool().get(sizeof(int))))) rc = RF_E_OOM;
   return rc;
@@ -899,12 +899,12 @@ static MatvecFn make_matvec(rf_handle* h, int* launches) {
       }
       rc = launch_struct_matvec(h->tab, h->N, smode, h->S32, h->S16, h->ori32, xa, h->zpart, h->ypart, skip,
                                 &h->ctl->timeout, st, h->recompute ? 0 : h->mv_variant);
-      *launches += 2;
+      *launches += 1;
     } else if (h->mfree) {
       rc = launch_assemble_apply(h->tab, h->N, h->pos32, h->ori32, h->pos64[h->icur], xin, h->zpart, skip,
                                  h->ffpart, h->F, h->b, st, h->asm_variant);
       if (rc == RF_OK) rc = launch_parts_finalize(h->tab, h->N, h->ori32, xin, h->zpart, h->zparts, h->ypart, skip, st);
-      *launches += 2;
+      *launches += 1;
     } else {
       rc = launch_dense_gemv(h->gemv_plan, h->A, h->lda, h->R, xin, h->ypart, skip, st);
     }
@@ -1000,7 +1000,7 @@ int rf_solve(rf_handle* h) {
         RF_TRY(launch_cast_to_float(h->x64, h->x, h->R, h->st));
         h->launches += 1;
       }
-      h->launches += 3 * (br.refinements + 1);   // the FP64 residual of every outer pass
+      h->launches += (h->recompute ? 3 : 2) * (br.refinements + 1);   // the FP64 residual of every outer pass
       h->refinements = br.refinements;
     } else {
       brc = bicgstab_solve(bs, mv, h->b, h->x, h->st, &br);
@@ -1028,7 +1028,7 @@ int rf_solve(rf_handle* h) {
       if (rc2) return rc2;
       h->launches += 1;
     }
-    h->launches += 2 * h->refinements;
+    h->launches += (h->recompute ? 3 : 2) * h->refinements;
   } else {
     rc = gmres_solve(s, mv, h->b, h->x, h->st, &res);
   }
@@ -1045,25 +1045,23 @@ int rf_solve(rf_handle* h) {
   return rc;
 }
 
-// the velocity kernels and the non-finite guard (read by rf_step after its
-// sync); returns the number of kernels in *kernels
+// the velocity kernels; the last one sets the non-finite guard (read by rf_step
+// after its sync); returns the number of kernels in *kernels
 static int enqueue_velocities(rf_handle* h, int* kernels) {
   const int vint = h->cfg.velocity_integration < 0 ? h->cfg.integration : h->cfg.velocity_integration;
   if (vint == RF_ANALYTICAL) {
     RF_TRY(launch_velocity_analytical(h->tab, h->N, h->ori32, h->pos64[h->icur], h->ori64[h->icur], h->x,
-                                      h->vpart, h->tv[h->vcur], h->rv[h->vcur], h->st));
+                                      h->vpart, h->tv[h->vcur], h->rv[h->vcur], h->vflag, h->st));
     *kernels += 2;
   } else if (h->mixed && !h->recompute) {
     RF_TRY(launch_struct_velocity(h->tab, h->N, h->S32, h->ori32, h->F, h->x, h->svpart, h->tv[h->vcur],
-                                  h->rv[h->vcur], h->st));
+                                  h->rv[h->vcur], h->vflag, h->st));
     *kernels += 2;
   } else {
     RF_TRY(launch_velocity_numerical(h->tab, h->N, h->pos64[h->icur], h->ori32, h->x, h->fw, h->vpart, h->tv[h->vcur],
-                                     h->rv[h->vcur], h->st));
+                                     h->rv[h->vcur], h->vflag, h->st));
     *kernels += 3;
   }
-  RF_TRY(launch_check_finite(h->tv[h->vcur], h->rv[h->vcur], h->N, h->vflag, h->st));
-  *kernels += 1;
   return RF_OK;
 }
 
@@ -1148,7 +1146,7 @@ static int build_step_graph(rf_handle* h, int first_step, rf_handle::StepGraph* 
     return gmres_enqueue_cycle(s, mv, resid, h->b, xsol, h->mixed, cond, h->st, &kcycle);
   }, &body);
   if (rc) return fail(rc);
-  kcycle += mvk + (h->mixed ? 3 : 0);   // the FP64 residual's kernels
+  kcycle += mvk + (h->mixed ? (h->recompute ? 3 : 2) : 0);   // the FP64 residual's kernels
   rc = capture_segment(h->st, [&]() -> int {
     if (h->mixed) {
       RF_TRY(launch_cast_to_float(h->x64, h->x, h->R, h->st));

@@ -49,9 +49,8 @@ int launch_assemble_analytical(const Tables& tab, int N, const float4* pos, cons
 int launch_assemble_apply(const Tables& tab, int N, const float4* pos, const float4* ori, const double4* pos64,
                           const float* x, float* zpart, const int* skip, float* ffpart, float* F, float* b,
                           cudaStream_t st, int variant = 0);
-// y = x + C z with z the fixed-order sum of nparts partial rows of zpart
-// (zpart holds nparts + 1 rows: the sum goes to row nparts).
-int launch_parts_finalize(const Tables& tab, int N, const float4* ori, const float* x, float* zpart, int nparts,
+// y = x + C z with z the fixed-order sum of nparts partial rows of zpart.
+int launch_parts_finalize(const Tables& tab, int N, const float4* ori, const float* x, const float* zpart, int nparts,
                           float* y, const int* skip, cudaStream_t st);
 // r = b - (x + C z) with z the sum of nparts FP32 partial-row slots of a
 // matrix-free product (launch_assemble_apply), summed in FP64, x in FP64
@@ -82,7 +81,7 @@ int launch_struct_apply64(const Tables& tab, int N, const float* S32, const floa
                           double* zpart64, float* y, int* err, cudaStream_t st);
 // velocities from the FP32 blocks; vpart: ceil(N/16) x N x 6 floats.
 int launch_struct_velocity(const Tables& tab, int N, const float* S32, const float4* ori, const float* F,
-                           const float* x, float* vpart, float4* tvel, float4* rvel, cudaStream_t st);
+                           const float* x, float* vpart, float4* tvel, float4* rvel, int* vflag, cudaStream_t st);
 int launch_cast_to_float(const double* in, float* out, int64_t n, cudaStream_t st);
 
 // Near-field preconditioner (csrc/rf_precond.cu; M = 5, stored FP32 blocks):
@@ -186,16 +185,57 @@ namespace rf {
 cudaError_t handle_pool(int dev, cudaMemPool_t* out);
 void pools_acquire();
 void pools_release();
-int velocity_chunks(int N);
-// fw: N*Q float4 scratch; vpart: velocity_chunks(N) * N * 6 floats scratch.
-int launch_check_finite(const float4* a, const float4* b, int N, int* flag, cudaStream_t st);
+// fw: N * (Q + kFarNodes) float4 scratch; vpart: velocity_rows(N) * N * 6 floats scratch.
+int velocity_rows(int N);
 // pos64: the FP64 centres, from which the pair separations are formed
 int launch_velocity_numerical(const Tables& tab, int N, const double4* pos64, const float4* ori, const float* x,
-                              float4* fw, float* vpart, float4* tvel, float4* rvel, cudaStream_t st);
+                              float4* fw, float* vpart, float4* tvel, float4* rvel, int* vflag, cudaStream_t st);
 // analytical inner integrals (FP64 moments); vpart as for the numerical kernel
 int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, const double4* pos64,
                                const double4* ori64, const float* x, float* vpart, float4* tvel, float4* rvel,
-                               cudaStream_t st);
+                               int* vflag, cudaStream_t st);
+
+// Sums of the velocity partial rows vpart[row][i][6]: rows row = g (mod 4) in
+// order for each group g, then the groups in order.  velocity_row_sum: component
+// c of fiber i by one thread; velocity_rows_block: 32 fibers from i0 by a block
+// of kVelSumThreads threads (8 loads per thread in flight), the same sums.
+constexpr int kVelSumFibers = 32, kVelSumGroups = 4;
+constexpr int kVelSumThreads = kVelSumFibers * 6 * kVelSumGroups;
+__device__ __forceinline__ float velocity_row_sum(const float* __restrict__ vpart, int nrows, int N, int i, int c) {
+  float r[kVelSumGroups];
+#pragma unroll
+  for (int g = 0; g < kVelSumGroups; ++g) {
+    r[g] = 0.f;
+    for (int p = g; p < nrows; p += kVelSumGroups) r[g] = __fadd_rn(r[g], vpart[((int64_t)p * N + i) * 6 + c]);
+  }
+  return __fadd_rn(__fadd_rn(__fadd_rn(r[0], r[1]), r[2]), r[3]);
+}
+__device__ __forceinline__ void velocity_rows_block(const float* __restrict__ vpart, int nrows, int N, int i0,
+                                                    float (*sums)[7]) {
+  __shared__ float red[kVelSumGroups][kVelSumFibers * 6];
+  const int e = (int)threadIdx.x % (kVelSumFibers * 6), g = (int)threadIdx.x / (kVelSumFibers * 6);
+  float s = 0.f;
+  if (i0 + e / 6 < N) {
+    const float* v = vpart + (int64_t)i0 * 6 + e;
+    int p = g;
+    for (; p + 7 * kVelSumGroups < nrows; p += 8 * kVelSumGroups) {
+      float a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a[u] = v[(int64_t)(p + u * kVelSumGroups) * N * 6];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s = __fadd_rn(s, a[u]);
+    }
+    for (; p < nrows; p += kVelSumGroups) s = __fadd_rn(s, v[(int64_t)p * N * 6]);
+  }
+  red[g][e] = s;
+  __syncthreads();
+  if (g == 0) sums[e / 6][e % 6] = __fadd_rn(__fadd_rn(__fadd_rn(red[0][e], red[1][e]), red[2][e]), red[3][e]);
+  __syncthreads();
+}
+__device__ __forceinline__ bool velocity_finite(const float4& u, const float4& w) {
+  return isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(w.x) && isfinite(w.y) && isfinite(w.z);
+}
+
 // Fiber i's second-order step (fortran/update_fibers.incl; the first step,
 // fortran/update_fibers_firststep.incl, is explicit Euler):
 // x' = 4/3 x - 1/3 x_prev + 2/3 dt (2 U - U_prev), the same for t with W, then

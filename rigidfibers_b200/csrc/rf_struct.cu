@@ -767,62 +767,59 @@ k_struct_r64_bulk(int N, const float* __restrict__ S32, const double* __restrict
   }
 }
 
-// zsum[r] = sum_p zpart[p][r] (fixed order within each of 4 p-groups, then
-// the 4 groups in order).  256 threads = 64 consecutive rows x 4 groups, the
-// p loop unrolled so that 8 loads per thread are in flight.
-template <typename ACC>
-__global__ void __launch_bounds__(256)
-k_sum_parts(const ACC* part, int nparts, int64_t R, ACC* out, const int* __restrict__ skip) {
-  // out may be the last partial row (read by this block before it is written)
-  if (skip != nullptr && *skip) return;
-  __shared__ ACC red[4][64];
-  const int rr = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const int64_t r = (int64_t)blockIdx.x * 64 + rr;
-  ACC s = (ACC)0;
-  if (r < R) {
-    int p = g;
-    for (; p + 28 < nparts; p += 32) {
-      ACC v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = part[(int64_t)(p + 4 * u) * R + r];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) s += v[u];
-    }
-    for (; p < nparts; p += 4) s += part[(int64_t)p * R + r];
-  }
-  red[g][rr] = s;
-  __syncthreads();
-  if (g == 0 && r < R) out[r] = ((red[0][rr] + red[1][rr]) + red[2][rr]) + red[3][rr];
-}
+// z = sum_p zpart[p] in ACC (fixed order: rows p = g (mod 8) in order for each of
+// 8 groups, then the groups in order), then y = x + C z, or r = b - (x + C z).  A
+// block takes 32 (fiber, k) units = 96 consecutive rows x 8 groups, 8 loads per
+// thread in flight.  Bound: the partial rows, from L2 (N=4000: 60 MB, 13 us;
+// as two kernels, the sum and the projection, 20 us).
+constexpr int kFinUnits = 32, kFinGroups = 8;
 
-// y = x + C z (z = sum of partials, added in ACC), or r = b - (x + C z).  One
-// thread per (fiber, k).
 template <typename XT, typename ACC, bool RESIDUAL, typename ZT = ACC>
-__global__ void k_struct_finalize(const Tables tab, int N, const float4* __restrict__ ori, const XT* __restrict__ x,
-                                  const ZT* __restrict__ zpart, int nparts, const float* __restrict__ b,
-                                  float* __restrict__ out, const int* __restrict__ skip) {
+__global__ void __launch_bounds__(3 * kFinUnits * kFinGroups)
+k_parts_finalize(const Tables tab, int N, const float4* __restrict__ ori, const XT* __restrict__ x,
+                 const ZT* __restrict__ zpart, int nparts, const float* __restrict__ b, float* __restrict__ out,
+                 const int* __restrict__ skip) {
   if (skip != nullptr && *skip) return;
+  __shared__ ACC red[kFinGroups][3 * kFinUnits];
   const int M = tab.M;
   const int64_t R = (int64_t)3 * M * N;
-  const int64_t n = (int64_t)N * M;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(u / M), k = (int)(u % M);
-    const int64_t r0 = (int64_t)i * 3 * M + 3 * k;
-    ACC z[3] = {0, 0, 0};
-    for (int p = 0; p < nparts; ++p) {
-      const ZT* s = zpart + (int64_t)p * R + r0;
-      z[0] += (ACC)s[0]; z[1] += (ACC)s[1]; z[2] += (ACC)s[2];
-    }
-    const float4 t = ori[i];
-    const ACC t3[3] = {(ACC)t.x, (ACC)t.y, (ACC)t.z};
-    const ACC tz = t3[0] * z[0] + t3[1] * z[1] + t3[2] * z[2];
-    const ACC coef = (ACC)tab.gamma[k], E = (ACC)tab.eigen[k];
+  const int e = threadIdx.x % (3 * kFinUnits), g = threadIdx.x / (3 * kFinUnits);
+  const int64_t r = (int64_t)blockIdx.x * (3 * kFinUnits) + e;
+  ACC s = (ACC)0;
+  if (r < R) {
+    const ZT* z = zpart + r;
+    int p = g;
+    for (; p + 7 * kFinGroups < nparts; p += 8 * kFinGroups) {
+      ZT v[8];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const ACC cz = k == 0 ? coef * t3[a] * tz : coef * (z[a] - E * t3[a] * tz);
-      const ACC y = (ACC)x[r0 + a] + cz;
-      out[r0 + a] = RESIDUAL ? (float)((ACC)b[r0 + a] - y) : (float)y;
+      for (int u = 0; u < 8; ++u) v[u] = z[(int64_t)(p + u * kFinGroups) * R];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += (ACC)v[u];
     }
+    for (; p < nparts; p += kFinGroups) s += (ACC)z[(int64_t)p * R];
+  }
+  red[g][e] = s;
+  __syncthreads();
+  const int64_t u = (int64_t)blockIdx.x * kFinUnits + threadIdx.x;
+  if (threadIdx.x >= kFinUnits || u >= (int64_t)N * M) return;
+  const int i = (int)(u / M), k = (int)(u % M);
+  ACC z[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    z[a] = red[0][3 * threadIdx.x + a];
+#pragma unroll
+    for (int q = 1; q < kFinGroups; ++q) z[a] += red[q][3 * threadIdx.x + a];
+  }
+  const float4 t = ori[i];
+  const ACC t3[3] = {(ACC)t.x, (ACC)t.y, (ACC)t.z};
+  const ACC tz = t3[0] * z[0] + t3[1] * z[1] + t3[2] * z[2];
+  const ACC coef = (ACC)tab.gamma[k], E = (ACC)tab.eigen[k];
+  const int64_t r0 = 3 * u;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const ACC cz = k == 0 ? coef * t3[a] * tz : coef * (z[a] - E * t3[a] * tz);
+    const ACC y = (ACC)x[r0 + a] + cz;
+    out[r0 + a] = RESIDUAL ? (float)((ACC)b[r0 + a] - y) : (float)y;
   }
 }
 
@@ -901,19 +898,21 @@ __device__ __forceinline__ void struct_velocity_tile(int N, const float* __restr
 
 template <int M, int TI>
 __global__ void __launch_bounds__(256)
-k_struct_velocity(int N, const float* __restrict__ S32, const float* __restrict__ x, float* __restrict__ vpart) {
+k_struct_velocity(int N, const float* __restrict__ S32, const float* __restrict__ x, float* __restrict__ vpart,
+                  int* __restrict__ vflag) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *vflag = 0;
   struct_velocity_tile<M, TI>(N, S32, x, vpart, blockIdx.x);
 }
 
 // U_i = (0.5/d) [ (d+2)F + (d-2)(t.F)t + F_i[P0] + sum u ],
-// W_i = (1.5/d) (I - t t^T) [ F_i[P1] + sum w ]   (fiber i < N).
+// W_i = (1.5/d) (I - t t^T) [ F_i[P1] + sum w ]   (S: the six sums of fiber i).
 // Every rounding is spelled out (fmaf, __fmul_rn, __fadd_rn), so the result
 // does not depend on which multiply-adds the compiler would contract in the
 // kernel it is inlined into: the single-suspension and packed kernels agree
 // bit for bit.
-__device__ __forceinline__ void struct_velocity_fiber(const Tables& tab, int N, const float4* __restrict__ ori,
-                                                      const float* __restrict__ F, const float* __restrict__ vpart,
-                                                      int nparts, int i, float4& tv, float4& rv) {
+__device__ __forceinline__ void struct_velocity_fiber(const Tables& tab, const float4* __restrict__ ori,
+                                                      const float* __restrict__ F, const float* S, int i, float4& tv,
+                                                      float4& rv) {
   const int FFn = 3 * (tab.M + 1);
   const float4 t = ori[i];
   const float d = tab.d;
@@ -921,13 +920,9 @@ __device__ __forceinline__ void struct_velocity_fiber(const Tables& tab, int N, 
   const float tF = __fmul_rn(t.z, Fz);
   const float cF = __fmul_rn(d - 2.f, tF);
   const float* Fi = F + (int64_t)i * FFn;
-  float U[3] = {fmaf(cF, t.x, Fi[0]), fmaf(cF, t.y, Fi[1]), __fadd_rn(fmaf(cF, t.z, __fmul_rn(d + 2.f, Fz)), Fi[2])};
-  float W[3] = {Fi[3], Fi[4], Fi[5]};
-  for (int p = 0; p < nparts; ++p) {
-    const float* v = vpart + ((int64_t)p * N + i) * 6;
-    U[0] += v[0]; U[1] += v[1]; U[2] += v[2];
-    W[0] += v[3]; W[1] += v[4]; W[2] += v[5];
-  }
+  const float U[3] = {__fadd_rn(fmaf(cF, t.x, Fi[0]), S[0]), __fadd_rn(fmaf(cF, t.y, Fi[1]), S[1]),
+                      __fadd_rn(__fadd_rn(fmaf(cF, t.z, __fmul_rn(d + 2.f, Fz)), Fi[2]), S[2])};
+  const float W[3] = {__fadd_rn(Fi[3], S[3]), __fadd_rn(Fi[4], S[4]), __fadd_rn(Fi[5], S[5])};
   const float tW = fmaf(t.z, W[2], fmaf(t.y, W[1], __fmul_rn(t.x, W[0])));
   const float su = 0.5f / d, sr = 1.5f / d;
   tv = make_float4(__fmul_rn(U[0], su), __fmul_rn(U[1], su), __fmul_rn(U[2], su), 0.f);
@@ -935,15 +930,21 @@ __device__ __forceinline__ void struct_velocity_fiber(const Tables& tab, int N, 
                    __fmul_rn(fmaf(-t.z, tW, W[2]), sr), 0.f);
 }
 
-__global__ void k_struct_velocity_finalize(const Tables tab, int N, const float4* __restrict__ ori,
-                                           const float* __restrict__ F, const float* __restrict__ vpart, int nparts,
-                                           float4* __restrict__ tvel, float4* __restrict__ rvel) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
+// the sums over the partial rows, the velocities and the non-finite guard
+// (*vflag was cleared by k_struct_velocity)
+__global__ void __launch_bounds__(kVelSumThreads)
+k_struct_velocity_finalize(const Tables tab, int N, const float4* __restrict__ ori, const float* __restrict__ F,
+                           const float* __restrict__ vpart, int nparts, float4* __restrict__ tvel,
+                           float4* __restrict__ rvel, int* __restrict__ vflag) {
+  __shared__ float sums[kVelSumFibers][7];
+  velocity_rows_block(vpart, nparts, N, blockIdx.x * kVelSumFibers, sums);
+  const int i = blockIdx.x * kVelSumFibers + threadIdx.x;
+  if (threadIdx.x >= kVelSumFibers || i >= N) return;
   float4 tv, rv;
-  struct_velocity_fiber(tab, N, ori, F, vpart, nparts, i, tv, rv);
+  struct_velocity_fiber(tab, ori, F, sums[threadIdx.x], i, tv, rv);
   tvel[i] = tv;
   rvel[i] = rv;
+  if (!velocity_finite(tv, rv)) *vflag = 1;   // every writer stores the same value
 }
 
 // ---- packed step: velocities and update of every member of one group -----
@@ -968,10 +969,13 @@ k_pack_finish(const Tables tab, const PackStepMember* __restrict__ mem) {
   int bad = 0;
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     float4 u, w;
-    struct_velocity_fiber(tab, N, p.ori32, p.F, p.vpart, nparts, i, u, w);
+    float S[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) S[c] = velocity_row_sum(p.vpart, nparts, N, i, c);
+    struct_velocity_fiber(tab, p.ori32, p.F, S, i, u, w);
     p.tv[i] = u;
     p.rv[i] = w;
-    bad |= !(isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(w.x) && isfinite(w.y) && isfinite(w.z));
+    bad |= !velocity_finite(u, w);
     update_fiber(i, p.first, p.dt, p.pos64_prev, p.pos64, p.ori64_prev, p.ori64, p.tv_prev, u, p.rv_prev, w,
                  p.pos32, p.ori32);
   }
@@ -998,6 +1002,16 @@ __global__ void k_cast_to_float(const XT* __restrict__ in, float* __restrict__ o
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+template <typename XT, typename ACC, bool RESIDUAL, typename ZT>
+static int launch_finalize(const Tables& tab, int N, const float4* ori, const XT* x, const ZT* zpart, int nparts,
+                           const float* b, float* out, const int* skip, cudaStream_t st) {
+  k_parts_finalize<XT, ACC, RESIDUAL, ZT><<<(unsigned)ceil_div((int64_t)N * tab.M, kFinUnits),
+                                            3 * kFinUnits * kFinGroups, 0, st>>>(tab, N, ori, x, zpart, nparts, b, out,
+                                                                                 skip);
+  RF_LAUNCH_CHECK();
+  return RF_OK;
+}
+
 static unsigned fin_blocks(int64_t n) { return (unsigned)std::min<int64_t>(ceil_div(n, 256), 148 * 8); }
 
 template <int M, int TI, int SMODE, typename XT, typename ACC>
@@ -1063,39 +1077,20 @@ int launch_struct_matvec(const Tables& tab, int N, int smode, const float* S32, 
 #undef RF_Z_CASE
   }
   if (rc != RF_OK) return rc;
-  const int64_t n = (int64_t)N * tab.M;
-  const int64_t R = 3 * n;
   const int nparts = (int)ceil_div(N, kStoreTile);
-  // the summed rows go to partial slot nparts, which the TMA-staged kernel
-  // also fills (diagonal tiles' j side): each row is read before it is written
-  k_sum_parts<float><<<(unsigned)ceil_div(R, 64), 256, 0, st>>>(zpart, bulk ? nparts + 1 : nparts, R,
-                                                                zpart + (int64_t)nparts * R, skip);
-  RF_LAUNCH_CHECK();
-  k_struct_finalize<float, float, false><<<fin_blocks(n), 256, 0, st>>>(
-      tab, N, ori, x, zpart + (int64_t)nparts * R, 1, nullptr, y, skip);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
+  // the TMA-staged kernel also fills slot nparts (diagonal tiles' j side)
+  return launch_finalize<float, float, false, float>(tab, N, ori, x, zpart, bulk ? nparts + 1 : nparts, nullptr, y, skip,
+                                                     st);
 }
 
-int launch_parts_finalize(const Tables& tab, int N, const float4* ori, const float* x, float* zpart, int nparts,
+int launch_parts_finalize(const Tables& tab, int N, const float4* ori, const float* x, const float* zpart, int nparts,
                           float* y, const int* skip, cudaStream_t st) {
-  const int64_t n = (int64_t)N * tab.M;
-  const int64_t R = 3 * n;
-  k_sum_parts<float><<<(unsigned)ceil_div(R, 64), 256, 0, st>>>(zpart, nparts, R, zpart + (int64_t)nparts * R, skip);
-  RF_LAUNCH_CHECK();
-  k_struct_finalize<float, float, false><<<fin_blocks(n), 256, 0, st>>>(tab, N, ori, x, zpart + (int64_t)nparts * R,
-                                                                        1, nullptr, y, skip);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
+  return launch_finalize<float, float, false, float>(tab, N, ori, x, zpart, nparts, nullptr, y, skip, st);
 }
 
 int launch_parts_residual64(const Tables& tab, int N, const float4* ori, const double* x, const float* zpart,
                             int nparts, const float* b, float* r, const int* skip, cudaStream_t st) {
-  const int64_t n = (int64_t)N * tab.M;
-  k_struct_finalize<double, double, true, float><<<fin_blocks(n), 256, 0, st>>>(tab, N, ori, x, zpart, nparts, b, r,
-                                                                                skip);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
+  return launch_finalize<double, double, true, float>(tab, N, ori, x, zpart, nparts, b, r, skip, st);
 }
 
 template <int M>
@@ -1137,17 +1132,10 @@ int launch_struct_residual64(const Tables& tab, int N, const float* S32, const f
 #undef RF_Z_CASE
   }
   if (rc != RF_OK) return rc;
-  const int64_t n = (int64_t)N * tab.M;
-  const int64_t R = 3 * n;
+  // the bulk kernel also fills slot nparts (diagonal tiles' j side)
   const int nparts = (int)ceil_div(N, kStoreTile);
-  // the bulk kernel also fills slot nparts (diagonal tiles' j side), which is the output row
-  k_sum_parts<double><<<(unsigned)ceil_div(R, 64), 256, 0, st>>>(zpart64, bulk ? nparts + 1 : nparts, R,
-                                                                 zpart64 + (int64_t)nparts * R, skip);
-  RF_LAUNCH_CHECK();
-  k_struct_finalize<double, double, true><<<fin_blocks(n), 256, 0, st>>>(
-      tab, N, ori, x, zpart64 + (int64_t)nparts * R, 1, b, r, skip);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
+  return launch_finalize<double, double, true, double>(tab, N, ori, x, zpart64, bulk ? nparts + 1 : nparts, b, r, skip,
+                                                       st);
 }
 
 int launch_struct_apply64(const Tables& tab, int N, const float* S32, const float4* ori, const double* x,
@@ -1169,33 +1157,26 @@ int launch_struct_apply64(const Tables& tab, int N, const float* S32, const floa
 #undef RF_Z_CASE
   }
   if (rc != RF_OK) return rc;
-  const int64_t n = (int64_t)N * tab.M;
-  const int64_t R = 3 * n;
   const int nparts = (int)ceil_div(N, kStoreTile);
-  k_sum_parts<double><<<(unsigned)ceil_div(R, 64), 256, 0, st>>>(zpart64, bulk ? nparts + 1 : nparts, R,
-                                                                 zpart64 + (int64_t)nparts * R, nullptr);
-  RF_LAUNCH_CHECK();
-  k_struct_finalize<double, double, false><<<fin_blocks(n), 256, 0, st>>>(
-      tab, N, ori, x, zpart64 + (int64_t)nparts * R, 1, nullptr, y, nullptr);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
+  return launch_finalize<double, double, false, double>(tab, N, ori, x, zpart64, bulk ? nparts + 1 : nparts, nullptr, y,
+                                                        nullptr, st);
 }
 
 int launch_struct_velocity(const Tables& tab, int N, const float* S32, const float4* ori, const float* F,
-                           const float* x, float* vpart, float4* tvel, float4* rvel, cudaStream_t st) {
+                           const float* x, float* vpart, float4* tvel, float4* rvel, int* vflag, cudaStream_t st) {
   const unsigned grid = (unsigned)struct_store_tiles(N);
   bool done = false;
 #define RF_V_CASE(MM, QQ)                                                                 \
   if (!done && tab.M == MM && tab.Q == QQ) {                                              \
-    k_struct_velocity<MM, 192 / QQ><<<grid, 256, 0, st>>>(N, S32, x, vpart);              \
+    k_struct_velocity<MM, 192 / QQ><<<grid, 256, 0, st>>>(N, S32, x, vpart, vflag);       \
     done = true;                                                                          \
   }
   RF_FOR_EACH_MQ(RF_V_CASE)
 #undef RF_V_CASE
   if (!done) return RF_E_UNSUPPORTED;
   RF_LAUNCH_CHECK();
-  k_struct_velocity_finalize<<<(unsigned)ceil_div(N, 128), 128, 0, st>>>(tab, N, ori, F, vpart,
-                                                                          (int)ceil_div(N, kStoreTile), tvel, rvel);
+  k_struct_velocity_finalize<<<(unsigned)ceil_div(N, kVelSumFibers), kVelSumThreads, 0, st>>>(
+      tab, N, ori, F, vpart, (int)ceil_div(N, kStoreTile), tvel, rvel, vflag);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }

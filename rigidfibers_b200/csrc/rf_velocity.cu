@@ -17,16 +17,21 @@ namespace rf {
 
 int velocity_chunks(int N);
 
-// fw[j*Q + q] = w_q f_j(s_q) = W[0][q] F/2 + sum_k a_{j,k} W[k+1][q]
-__global__ void k_source_density(const Tables tab, int N, const float* __restrict__ x, float4* __restrict__ fw) {
-  const int Q = tab.Q, M = tab.M;
-  const int64_t n = (int64_t)N * Q;
+// Source densities of both quadrature rules, weight included:
+// fw[j * (Q + FN) + q] = w_q f_j(s_q) = W[0][q] F/2 + sum_k a_{j,k} W[k+1][q] for
+// the Q points of the full rule, then the FN points of the far rule.
+__global__ void k_source_density(const Tables tab, int N, const float* __restrict__ x, float4* __restrict__ fw,
+                                 int* __restrict__ vflag) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *vflag = 0;   // the stage's non-finite guard (k_velocity_finalize)
+  const int Q = tab.Q, M = tab.M, P = Q + kFarNodes;
+  const int64_t n = (int64_t)N * P;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(u / Q), q = (int)(u % Q);
-    float f0 = 0.f, f1 = 0.f, f2 = tab.W[0][q] * tab.fz_half;
+    const int j = (int)(u / P), q = (int)(u % P);
+    auto weight = [&](int k) { return q < Q ? tab.W[k][q] : tab.far_W[k][q - Q]; };
+    float f0 = 0.f, f1 = 0.f, f2 = weight(0) * tab.fz_half;
     const float* a = x + (int64_t)j * 3 * M;
     for (int k = 0; k < M; ++k) {
-      const float w = tab.W[k + 1][q];
+      const float w = weight(k + 1);
       f0 = fmaf(a[3 * k + 0], w, f0);
       f1 = fmaf(a[3 * k + 1], w, f1);
       f2 = fmaf(a[3 * k + 2], w, f2);
@@ -35,116 +40,221 @@ __global__ void k_source_density(const Tables tab, int N, const float* __restric
   }
 }
 
-// One CTA = TI fibers i x one chunk of source fibers j.  Thread u < TI*Q owns
-// (fiber il, quadrature point qi) and accumulates sum_j GF_ij(qi).
-template <int Q>
-__global__ void __launch_bounds__(192, 4)
-k_velocity_numerical(const Tables tab, int N, const double4* __restrict__ pos64, const float4* __restrict__ ori,
-                     const float4* __restrict__ fw, int jchunk, float* __restrict__ vpart) {
-  constexpr int TI = 192 / Q;
-  constexpr int U = TI * Q;
-  // quadrature-point separations (x_i - x_j) + s_qi t_i - s_qj t_j with the
-  // centre difference in FP64, rounded once (as in the assembly): the error
-  // scales with the fibers' distance, not with their distance from the origin
-  __shared__ float4 sP[TI][Q], sF[TI][Q];    // s_q t_j, w_q f_j(s_q)
-  __shared__ double sXi[TI][3], sXj[TI][3];
-  __shared__ float sGs[3][U];
+// acc += K(p - s t) f for one point of fiber j (p relative to its centre).  NR: a
+// Newton step on the reciprocal root (the far rule's 64 kernel values per pair
+// average their roundings less than the full rule's 576).
+template <bool NR>
+__device__ __forceinline__ void stokeslet_apply(float px, float py, float pz, const float4& st, const float4& f,
+                                                float e2, float e2x3, float (&acc)[3]) {
+  const float rx = px - st.x, ry = py - st.y, rz = pz - st.z;
+  const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+  float inv = rsqrtf(r2);
+  if (NR) inv = fmaf(0.5f * inv, fmaf(-r2 * inv, inv, 1.f), inv);
+  const float inv2 = inv * inv;
+  const float inv3 = inv2 * inv;
+  const float inv5 = inv3 * inv2;
+  const float a = fmaf(e2, inv3, inv);
+  const float bb = fmaf(e2x3, inv5, inv3);
+  // K f = a f + bb R (R.f)
+  const float rf = fmaf(rx, f.x, fmaf(ry, f.y, rz * f.z)) * bb;
+  acc[0] = fmaf(a, f.x, fmaf(rf, rx, acc[0]));
+  acc[1] = fmaf(a, f.y, fmaf(rf, ry, acc[1]));
+  acc[2] = fmaf(a, f.z, fmaf(rf, rz, acc[2]));
+}
+
+// Velocity sums of one ordered pair set.  Sources at least sqrt(far_d2) away (the
+// assembly's rule, see make_tables) take the far rule, 64 kernel values per pair
+// instead of Q^2; the others the full rule.  One launch: the first far_blocks
+// blocks are far ones, the rest near ones, so that the few near pairs run beside
+// the far ones.  Bound: FP32 issue; below a few hundred fibers latency, so both
+// parts split the sources into many partial rows (vpart[row][i][6]: far chunks,
+// then near segments).  Sums over one source's points are formed before they are
+// added to the fiber's: the roundings stay those of one pair.
+constexpr int kVelFibers = 32;
+constexpr int kVelThreads = kVelFibers * kFarNodes;
+
+struct VelSplit {
+  int chunks, jchunk, far_blocks;   // far: source chunks, sources per chunk, blocks
+  int segs, jseg, near_blocks;      // near: source segments, sources per segment, blocks
+};
+
+// 32 fibers i x one chunk of sources, thread (fiber, far point of i); the
+// sources pass through shared memory 32 at a time (broadcast reads: lane = fiber)
+__device__ __forceinline__ void velocity_far_block(const Tables& tab, int N, const double4* __restrict__ pos64,
+                                                   const float4* __restrict__ ori, const float4* __restrict__ fw,
+                                                   int tile, int chunk, int jchunk, float* __restrict__ vpart) {
+  constexpr int FN = kFarNodes, B = kVelFibers;
+  __shared__ float4 sP[B][FN], sF[B][FN];    // s_q t_j, w_q f_j(s_q)
+  __shared__ double sXj[B][3];
+  __shared__ float sGs[3][FN][B];
   const int tid = threadIdx.x;
-  const int il = tid / Q, qi = tid % Q;
-  const int i0 = blockIdx.x * TI;
-  const int i = i0 + il;
-  const bool unit_ok = tid < U && i < N;
-  float tix = 0.f, tiy = 0.f, tiz = 0.f;
-  if (unit_ok) {
-    const float4 t = ori[i];
-    const float s = tab.pts[qi];
-    tix = s * t.x; tiy = s * t.y; tiz = s * t.z;
+  const int il = tid % B, qi = tid / B;
+  const int i = tile * B + il;
+  const int P = tab.Q + FN;
+  double xi[3];
+  float si[3];
+  {
+    const double4 x = pos64[min(i, N - 1)];
+    const float4 t = ori[min(i, N - 1)];
+    const float s = tab.far_pts[qi];
+    xi[0] = x.x; xi[1] = x.y; xi[2] = x.z;
+    si[0] = s * t.x; si[1] = s * t.y; si[2] = s * t.z;
   }
-  if (tid < TI) {
-    const double4 x = pos64[min(i0 + tid, N - 1)];
-    sXi[tid][0] = x.x; sXi[tid][1] = x.y; sXi[tid][2] = x.z;
-  }
-  const float e2 = tab.e2, e2x3 = -3.f * tab.e2;
-  float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-  const int jbeg = blockIdx.y * jchunk, jend = min(N, jbeg + jchunk);
-  for (int js = jbeg; js < jend; js += TI) {
+  const float e2 = tab.e2, e2x3 = -3.f * tab.e2, far_d2 = tab.far_d2;
+  float g[3] = {0.f, 0.f, 0.f};
+  const int jbeg = chunk * jchunk, jend = min(N, jbeg + jchunk);
+  for (int js = jbeg; js < jend; js += B) {
     __syncthreads();
-    if (tid < U) {
-      const int jl = tid / Q, q = tid % Q;
+    {
+      const int jl = tid / FN, q = tid % FN;
       const int j = min(js + jl, N - 1);
       const float4 t = ori[j];
-      const float s = tab.pts[q];
+      const float s = tab.far_pts[q];
       sP[jl][q] = make_float4(s * t.x, s * t.y, s * t.z, 0.f);
-      sF[jl][q] = fw[(int64_t)j * Q + q];
+      sF[jl][q] = fw[(int64_t)j * P + tab.Q + q];
       if (q == 0) {
         const double4 x = pos64[j];
         sXj[jl][0] = x.x; sXj[jl][1] = x.y; sXj[jl][2] = x.z;
       }
     }
     __syncthreads();
-    const int jn = min(TI, jend - js);
-    if (unit_ok) {
-      for (int jl = 0; jl < jn; ++jl) {
-        if (js + jl == i) continue;
-        const float pix = (float)(sXi[il][0] - sXj[jl][0]) + tix;
-        const float piy = (float)(sXi[il][1] - sXj[jl][1]) + tiy;
-        const float piz = (float)(sXi[il][2] - sXj[jl][2]) + tiz;
+    const int jn = min(B, jend - js);
+    for (int jl = 0; jl < jn; ++jl) {
+      // the centre difference in FP64, rounded once (as in the assembly): the
+      // error scales with the fibers' distance, not with their distance from the origin
+      const float dx = (float)(xi[0] - sXj[jl][0]), dy = (float)(xi[1] - sXj[jl][1]), dz = (float)(xi[2] - sXj[jl][2]);
+      if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < far_d2) continue;   // near, or i itself
+      float acc[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          const float4 pj = sP[jl][q];
-          const float4 f = sF[jl][q];
-          const float rx = pix - pj.x, ry = piy - pj.y, rz = piz - pj.z;
-          const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-          const float inv = rsqrtf(r2);
-          const float inv2 = inv * inv;
-          const float inv3 = inv2 * inv;
-          const float inv5 = inv3 * inv2;
-          const float a = fmaf(e2, inv3, inv);
-          const float bb = fmaf(e2x3, inv5, inv3);
-          // K f = a f + bb R (R.f)
-          const float rf = fmaf(rx, f.x, fmaf(ry, f.y, rz * f.z)) * bb;
-          g0 = fmaf(a, f.x, fmaf(rf, rx, g0));
-          g1 = fmaf(a, f.y, fmaf(rf, ry, g1));
-          g2 = fmaf(a, f.z, fmaf(rf, rz, g2));
+      for (int q = 0; q < FN; ++q)
+        stokeslet_apply<true>(dx + si[0], dy + si[1], dz + si[2], sP[jl][q], sF[jl][q], e2, e2x3, acc);
+      g[0] += acc[0]; g[1] += acc[1]; g[2] += acc[2];
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) sGs[a][qi][il] = g[a];
+  __syncthreads();
+  // per fiber: sum_qi w_qi gs(qi) and sum_qi w_qi P_1(s_qi) gs(qi)
+  if (tid < B * 6) {
+    const int fl = tid % B, comp = tid / B;
+    const float* w = comp >= 3 ? tab.far_W[1] : tab.far_W[0];
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < FN; ++q) s = fmaf(w[q], sGs[comp % 3][q][fl], s);
+    if (tile * B + fl < N) vpart[((int64_t)chunk * N + tile * B + fl) * 6 + comp] = s;
+  }
+}
+
+// One warp: fiber i's near sources of one segment, found 32 centres at a time and
+// taken in index order, lane = quadrature point of i (Q = 48: two passes)
+template <int Q>
+__device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, const double4* __restrict__ pos64,
+                                                   const float4* __restrict__ ori, const float4* __restrict__ fw,
+                                                   int i, int jbeg, int jend, float* __restrict__ row) {
+  constexpr int NP = (Q + 31) / 32;   // points per lane
+  const int lane = threadIdx.x & 31;
+  const int P = Q + kFarNodes;
+  const double4 xi = pos64[i];
+  const float4 ti = ori[i];
+  const float e2 = tab.e2, e2x3 = -3.f * tab.e2, far_d2 = tab.far_d2;
+  float g[NP][3] = {};
+  for (int js = jbeg; js < jend; js += 32) {
+    const int j = js + lane;
+    float d[3] = {0.f, 0.f, 0.f};
+    bool near = false;
+    if (j < jend) {
+      const double4 xj = pos64[j];
+      d[0] = (float)(xi.x - xj.x); d[1] = (float)(xi.y - xj.y); d[2] = (float)(xi.z - xj.z);
+      near = j != i && fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2])) < far_d2;
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, near); m != 0; m &= m - 1) {
+      const int src = __ffs(m) - 1, jj = js + src;
+      const float dx = __shfl_sync(0xffffffffu, d[0], src), dy = __shfl_sync(0xffffffffu, d[1], src),
+                  dz = __shfl_sync(0xffffffffu, d[2], src);
+      const float4 tj = ori[jj];
+#pragma unroll
+      for (int h = 0; h < NP; ++h) {
+        const int q = lane + 32 * h;
+        if (q < Q) {
+          const float s = tab.pts[q];
+          const float px = dx + s * ti.x, py = dy + s * ti.y, pz = dz + s * ti.z;
+          float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+          for (int p = 0; p < Q; ++p) {
+            const float sp = tab.pts[p];
+            stokeslet_apply<false>(px, py, pz, make_float4(sp * tj.x, sp * tj.y, sp * tj.z, 0.f),
+                                   fw[(int64_t)jj * P + p], e2, e2x3, acc);
+          }
+#pragma unroll
+          for (int a = 0; a < 3; ++a) g[h][a] += acc[a];
         }
       }
     }
   }
-  if (tid < U) { sGs[0][tid] = g0; sGs[1][tid] = g1; sGs[2][tid] = g2; }
-  __syncthreads();
-  // per fiber: sum_qi w_qi gs(qi) and sum_qi w_qi P_1(s_qi) gs(qi)
-  if (tid < TI * 6) {
-    const int fl = tid / 6, comp = tid % 6;
-    const int a = comp % 3;
-    const bool rot = comp >= 3;
-    float s = 0.f;
+  float u[6] = {};
 #pragma unroll
-    for (int q = 0; q < Q; ++q) s = fmaf(rot ? tab.W[1][q] : tab.W[0][q], sGs[a][fl * Q + q], s);
-    if (i0 + fl < N) vpart[((int64_t)blockIdx.y * N + i0 + fl) * 6 + comp] = s;
+  for (int h = 0; h < NP; ++h) {
+    const int q = lane + 32 * h;
+    if (q < Q) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        u[a] = fmaf(tab.W[0][q], g[h][a], u[a]);
+        u[3 + a] = fmaf(tab.W[1][q], g[h][a], u[3 + a]);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int a = 0; a < 6; ++a) u[a] += __shfl_xor_sync(0xffffffffu, u[a], o);
+  if (lane < 6) {
+    float v = u[0];
+#pragma unroll
+    for (int a = 1; a < 6; ++a) v = lane == a ? u[a] : v;
+    row[(int64_t)i * 6 + lane] = v;
   }
 }
 
-// Self term, fixed-order sum over chunks, projection and scaling.
-__global__ void k_velocity_finalize(const Tables tab, int N, const float4* __restrict__ ori,
-                                    const float* __restrict__ vpart, int nchunks, float4* __restrict__ tvel,
-                                    float4* __restrict__ rvel) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
+template <int Q>
+__global__ void __launch_bounds__(kVelThreads)
+k_velocity_numerical(const Tables tab, int N, const double4* __restrict__ pos64, const float4* __restrict__ ori,
+                     const float4* __restrict__ fw, VelSplit v, float* __restrict__ vpart) {
+  const int b = (int)blockIdx.x;
+  if (b < v.far_blocks) {
+    velocity_far_block(tab, N, pos64, ori, fw, b / v.chunks, b % v.chunks, v.jchunk, vpart);
+    return;
+  }
+  const int w = (b - v.far_blocks) * (kVelThreads / 32) + (int)(threadIdx.x >> 5);
+  const int i = w / v.segs, seg = w % v.segs;
+  if (i < N)
+    velocity_near_warp<Q>(tab, N, pos64, ori, fw, i, seg * v.jseg, min(N, (seg + 1) * v.jseg),
+                          vpart + (int64_t)(v.chunks + seg) * N * 6);
+}
+
+// Sum of the partial rows (velocity_rows_block), self term, projection, scaling
+// and the non-finite guard; *vflag was cleared by an earlier kernel of the stage.
+__global__ void __launch_bounds__(kVelSumThreads)
+k_velocity_finalize(const Tables tab, int N, const float4* __restrict__ ori, const float* __restrict__ vpart,
+                    int nrows, float4* __restrict__ tvel, float4* __restrict__ rvel, int* __restrict__ vflag) {
+  __shared__ float sums[kVelSumFibers][7];
+  velocity_rows_block(vpart, nrows, N, blockIdx.x * kVelSumFibers, sums);
+  const int i = blockIdx.x * kVelSumFibers + threadIdx.x;
+  if (threadIdx.x >= kVelSumFibers || i >= N) return;
+  const float* S = sums[threadIdx.x];
   const float4 t = ori[i];
   const float d = tab.d;
   const float Fz = 2.f * tab.fz_half;            // F = (0, 0, -1)
   const float tF = t.z * Fz;
-  float U[3] = {(d - 2.f) * tF * t.x, (d - 2.f) * tF * t.y, (d + 2.f) * Fz + (d - 2.f) * tF * t.z};
-  float W[3] = {0.f, 0.f, 0.f};
-  for (int c = 0; c < nchunks; ++c) {
-    const float* p = vpart + ((int64_t)c * N + i) * 6;
-    U[0] += p[0]; U[1] += p[1]; U[2] += p[2];
-    W[0] += p[3]; W[1] += p[4]; W[2] += p[5];
-  }
+  const float U[3] = {(d - 2.f) * tF * t.x + S[0], (d - 2.f) * tF * t.y + S[1],
+                      (d + 2.f) * Fz + (d - 2.f) * tF * t.z + S[2]};
+  const float W[3] = {S[3], S[4], S[5]};
   const float tW = t.x * W[0] + t.y * W[1] + t.z * W[2];
   const float su = 0.5f / d, sr = 1.5f / d;
-  tvel[i] = make_float4(U[0] * su, U[1] * su, U[2] * su, 0.f);
-  rvel[i] = make_float4((W[0] - t.x * tW) * sr, (W[1] - t.y * tW) * sr, (W[2] - t.z * tW) * sr, 0.f);
+  const float4 u = make_float4(U[0] * su, U[1] * su, U[2] * su, 0.f);
+  const float4 w = make_float4((W[0] - t.x * tW) * sr, (W[1] - t.y * tW) * sr, (W[2] - t.z * tW) * sr, 0.f);
+  tvel[i] = u;
+  rvel[i] = w;
+  if (!velocity_finite(u, w)) *vflag = 1;   // every writer stores the same value
 }
 
 // Analytical variant: the inner integral over fiber j in closed form (FP64),
@@ -155,7 +265,9 @@ __global__ void k_velocity_finalize(const Tables tab, int N, const float4* __res
 template <int M, int Q>
 __global__ void __launch_bounds__(192, 2)
 k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, const double4* __restrict__ ori,
-                      const float* __restrict__ coeff, int jchunk, float* __restrict__ vpart) {
+                      const float* __restrict__ coeff, int jchunk, float* __restrict__ vpart,
+                      int* __restrict__ vflag) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *vflag = 0;
   constexpr int TI = 192 / Q;
   constexpr int U = TI * Q;
   constexpr int M3 = 3 * M;
@@ -207,7 +319,7 @@ k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, 
 
 int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, const double4* pos64,
                                const double4* ori64, const float* x, float* vpart, float4* tvel, float4* rvel,
-                               cudaStream_t st) {
+                               int* vflag, cudaStream_t st) {
   const int chunks = velocity_chunks(N);
   const int jchunk = (int)ceil_div(N, chunks);
   const int TI = 192 / tab.Q;
@@ -215,7 +327,7 @@ int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, cons
   bool done = false;
 #define RF_VA_CASE(MM, QQ)                                                                   \
   if (!done && tab.M == MM && tab.Q == QQ) {                                                 \
-    k_velocity_analytical<MM, QQ><<<grid, 192, 0, st>>>(tab, N, pos64, ori64, x, jchunk, vpart); \
+    k_velocity_analytical<MM, QQ><<<grid, 192, 0, st>>>(tab, N, pos64, ori64, x, jchunk, vpart, vflag); \
     done = true;                                                                             \
   }
   RF_FOR_EACH_MQ(RF_VA_CASE)
@@ -225,7 +337,8 @@ int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, cons
     return RF_E_UNSUPPORTED;
   }
   RF_LAUNCH_CHECK();
-  k_velocity_finalize<<<(unsigned)ceil_div(N, 128), 128, 0, st>>>(tab, N, ori, vpart, chunks, tvel, rvel);
+  k_velocity_finalize<<<(unsigned)ceil_div(N, kVelSumFibers), kVelSumThreads, 0, st>>>(tab, N, ori, vpart, chunks, tvel,
+                                                                                     rvel, vflag);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }
@@ -238,40 +351,43 @@ int velocity_chunks(int N) {
   return chunks;
 }
 
-// flag = 1 if any component of a or b (N float4, xyz used) is not finite
-__global__ void k_check_finite(const float4* __restrict__ a, const float4* __restrict__ b, int N,
-                               int* __restrict__ flag) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    const float4 u = a[i], w = b[i];
-    const bool ok = isfinite(u.x) && isfinite(u.y) && isfinite(u.z) && isfinite(w.x) && isfinite(w.y) && isfinite(w.z);
-    if (!ok) *flag = 1;   // every writer stores the same value
-  }
+// Far: enough 32-fiber x chunk blocks to fill the GPU twice over, at least 8
+// sources each; near: N warps alone leave the GPU idle below a few thousand fibers
+static VelSplit velocity_split(int N) {
+  VelSplit v;
+  const int tiles = (int)ceil_div(N, kVelFibers), most = (int)ceil_div(N, 8);
+  v.chunks = std::max(1, std::min((int)ceil_div(148 * 4 * 4, tiles), most));
+  v.jchunk = (int)ceil_div(N, v.chunks);
+  v.far_blocks = tiles * v.chunks;
+  v.segs = std::max(1, std::min((int)ceil_div(148 * 16, N), most));
+  v.jseg = (int)ceil_div(N, v.segs);
+  v.near_blocks = (int)ceil_div((int64_t)N * v.segs, kVelThreads / 32);
+  return v;
 }
 
-int launch_check_finite(const float4* a, const float4* b, int N, int* flag, cudaStream_t st) {
-  RF_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
-  k_check_finite<<<(unsigned)std::min<int64_t>(ceil_div(N, 256), 592), 256, 0, st>>>(a, b, N, flag);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
+// partial rows of either velocity path (vpart: this many rows of 6 N floats)
+int velocity_rows(int N) {
+  const VelSplit v = velocity_split(N);
+  return std::max(velocity_chunks(N), v.chunks + v.segs);
 }
 
 int launch_velocity_numerical(const Tables& tab, int N, const double4* pos64, const float4* ori, const float* x,
-                              float4* fw, float* vpart, float4* tvel, float4* rvel, cudaStream_t st) {
+                              float4* fw, float* vpart, float4* tvel, float4* rvel, int* vflag, cudaStream_t st) {
   const int Q = tab.Q;
-  k_source_density<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)N * Q, 256), 148 * 16), 256, 0, st>>>(tab, N, x, fw);
+  k_source_density<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)N * (Q + kFarNodes), 256), 148 * 16), 256, 0, st>>>(
+      tab, N, x, fw, vflag);
   RF_LAUNCH_CHECK();
-  const int chunks = velocity_chunks(N);
-  const int jchunk = (int)ceil_div(N, chunks);
-  const int TI = 192 / Q;
-  dim3 grid((unsigned)ceil_div(N, TI), (unsigned)chunks);
+  const VelSplit v = velocity_split(N);
+  const unsigned nb = (unsigned)(v.far_blocks + v.near_blocks);
   switch (Q) {
-    case 12: k_velocity_numerical<12><<<grid, 192, 0, st>>>(tab, N, pos64, ori, fw, jchunk, vpart); break;
-    case 24: k_velocity_numerical<24><<<grid, 192, 0, st>>>(tab, N, pos64, ori, fw, jchunk, vpart); break;
-    case 48: k_velocity_numerical<48><<<grid, 192, 0, st>>>(tab, N, pos64, ori, fw, jchunk, vpart); break;
+    case 12: k_velocity_numerical<12><<<nb, kVelThreads, 0, st>>>(tab, N, pos64, ori, fw, v, vpart); break;
+    case 24: k_velocity_numerical<24><<<nb, kVelThreads, 0, st>>>(tab, N, pos64, ori, fw, v, vpart); break;
+    case 48: k_velocity_numerical<48><<<nb, kVelThreads, 0, st>>>(tab, N, pos64, ori, fw, v, vpart); break;
     default: set_last_error_str("velocity: quadrature size not instantiated"); return RF_E_UNSUPPORTED;
   }
   RF_LAUNCH_CHECK();
-  k_velocity_finalize<<<(unsigned)ceil_div(N, 128), 128, 0, st>>>(tab, N, ori, vpart, chunks, tvel, rvel);
+  k_velocity_finalize<<<(unsigned)ceil_div(N, kVelSumFibers), kVelSumThreads, 0, st>>>(
+      tab, N, ori, vpart, v.chunks + v.segs, tvel, rvel, vflag);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }

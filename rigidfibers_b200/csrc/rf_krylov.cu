@@ -83,7 +83,7 @@ DenseGemvPlan plan_dense_gemv(int64_t R, int num_sms, int ctas_per_sm) {
   p.row_blocks = (int)ceil_div(R, 1024);
   // about ctas_per_sm CTAs of 256 threads per SM in flight
   int splits = (int)ceil_div((int64_t)num_sms * ctas_per_sm, p.row_blocks);
-  splits = std::max(1, std::min<int>(splits, (int)ceil_div(R, 64)));
+  splits = std::max(1, std::min<int>(splits, (int)ceil_div(R, 32)));
   p.cps = ceil_div(R, splits);
   p.splits = (int)ceil_div(R, p.cps);
   return p;
@@ -118,8 +118,13 @@ int launch_dense_gemv(const DenseGemvPlan& p, const float* A, int64_t lda, int64
 }
 
 // ---------------------------------------------------------------------------
-// Block / grid reductions (FP64)
+// Block / grid reductions (FP64), blocks of kKrylovThreads threads.  A block's
+// sums go to part[k * gridDim.x + block]; after a grid sync every block adds a
+// value's partials with one warp (lane-strided, then a butterfly), so all blocks
+// hold the same bits.
 // ---------------------------------------------------------------------------
+constexpr int kKrylovWarps = kKrylovThreads / 32;
+
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* __restrict__ dst /* NV */) {
   __shared__ double red[32][NV];
@@ -144,55 +149,78 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* __re
   __syncthreads();
 }
 
-// Sum of part[b*stride + k] over blocks b, fixed order; every block computes
-// the same value (used after a grid sync).
-__device__ __forceinline__ double sum_parts(const double* __restrict__ part, int nblk, int stride, int k) {
-  double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += part[(int64_t)b * stride + k];
-  return s;
-}
-
-// Dots of w with V[i0 .. i0+NV) (FP64), for the rows this thread owns.
-template <int NV>
-__device__ __forceinline__ void partial_dots(const float* __restrict__ w, const float* __restrict__ V, int64_t ldv,
-                                             int i0, int nv, int64_t R, double (&acc)[NV]) {
+// v[16] summed over the warp by halving exchanges: lanes 2u, 2u + 1 get value u
+__device__ __forceinline__ double warp_sum16(const double (&v)[16], int lane) {
+  double a[8], b[4], c[2];
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < R; r += (int64_t)gridDim.x * blockDim.x) {
-    const double wr = f2d(w[r]);
+  for (int k = 0; k < 8; ++k)
+    a[k] = (b4 ? v[k + 8] : v[k]) + __shfl_xor_sync(0xffffffffu, b4 ? v[k] : v[k + 8], 16);
 #pragma unroll
-    for (int k = 0; k < NV; ++k)
-      if (k < nv) acc[k] = fma(wr, f2d(V[(int64_t)(i0 + k) * ldv + r]), acc[k]);
-  }
+  for (int k = 0; k < 4; ++k)
+    b[k] = (b3 ? a[k + 4] : a[k]) + __shfl_xor_sync(0xffffffffu, b3 ? a[k] : a[k + 4], 8);
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    c[k] = (b2 ? b[k + 2] : b[k]) + __shfl_xor_sync(0xffffffffu, b2 ? b[k] : b[k + 2], 4);
+  const double d = (b1 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, b1 ? c[0] : c[1], 2);
+  return d + __shfl_xor_sync(0xffffffffu, d, 1);
 }
 
-constexpr int kDotGroup = 8;
-
-// All dots w . V[0..nv) into part[blk*stride + i].
-__device__ void grid_partial_dots(const float* __restrict__ w, const float* __restrict__ V, int64_t ldv, int nv,
-                                  int64_t R, double* __restrict__ part, int stride) {
-  for (int i0 = 0; i0 < nv; i0 += kDotGroup) {
-    double acc[kDotGroup];
-    partial_dots<kDotGroup>(w, V, ldv, i0, min(kDotGroup, nv - i0), R, acc);
-    __shared__ double tmp[kDotGroup];
-    block_reduce_store<kDotGroup>(acc, tmp);
-    if (threadIdx.x < kDotGroup && i0 + (int)threadIdx.x < nv)
-      part[(int64_t)blockIdx.x * stride + i0 + threadIdx.x] = tmp[threadIdx.x];
-    __syncthreads();
-  }
-}
-
-__device__ void grid_partial_norm(const float* __restrict__ w, int64_t R, double* __restrict__ part, int stride,
-                                  int slot) {
-  double acc[1] = {0.0};
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < R; r += (int64_t)gridDim.x * blockDim.x) {
-    const double v = f2d(w[r]);
-    acc[0] = fma(v, v, acc[0]);
-  }
-  __shared__ double tmp[1];
-  block_reduce_store<1>(acc, tmp);
-  if (threadIdx.x == 0) part[(int64_t)blockIdx.x * stride + slot] = tmp[0];
+// red[g][warp][16]: the warps' sums of values 16 g ..; value k of n into
+// part[k * gridDim.x + block].  Ends with every thread past the last read of red.
+__device__ __forceinline__ void block_parts(double (*red)[kKrylovWarps][16], int n, double* __restrict__ part) {
   __syncthreads();
+  for (int e = threadIdx.x; e < (n + 15) / 16 * 16 * kKrylovWarps; e += kKrylovThreads) {
+    const int k = e / kKrylovWarps, w = e % kKrylovWarps;
+    double v = red[k / 16][w][k % 16];
+#pragma unroll
+    for (int o = kKrylovWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (w == 0 && k < n) part[(int64_t)k * gridDim.x + blockIdx.x] = v;
+  }
+  __syncthreads();
+}
+
+// out[k] = sum over the blocks of part[k * gridDim.x + .], k < n (shared memory)
+__device__ __forceinline__ void gather_parts(const double* __restrict__ part, int n, double* out) {
+  const int lane = threadIdx.x & 31, nblk = gridDim.x;
+  for (int k = threadIdx.x >> 5; k < n; k += kKrylovWarps) {
+    double s = 0.0;
+    for (int b = lane; b < nblk; b += 32) s += __ldcg(part + (int64_t)k * nblk + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[k] = s;
+  }
+  __syncthreads();
+}
+
+// one or two values per thread, summed over the block, into the block's parts
+__device__ __forceinline__ void block_parts2(double a, double b, int n, double* __restrict__ part) {
+  __shared__ double red[kKrylovWarps][2];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if (lane == 0) {
+    red[wid][0] = a;
+    red[wid][1] = b;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    double v = red[lane % kKrylovWarps][lane / kKrylovWarps];   // lanes 0-15: a, 16-31: b
+#pragma unroll
+    for (int o = kKrylovWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int k = lane / kKrylovWarps;
+    if (lane % kKrylovWarps == 0 && k < n) part[(int64_t)k * gridDim.x + blockIdx.x] = v;
+  }
+  __syncthreads();
+}
+
+// a grid barrier; one block needs only its own
+__device__ __forceinline__ void grid_barrier(cg::grid_group& grid) {
+  if (gridDim.x > 1) grid.sync();
+  else __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
@@ -209,67 +237,85 @@ struct GmresArgs {
   int64_t ldv;
   int64_t R;
   int m;
-  double* part;        // 3 partial buffers, each nblk x stride
-  int stride;
+  double* part;        // 3 partial buffers of gridDim.x * (kMaxRestart + 2)
   double* H;           // (m+1) x m, column j at H[j*(m+1)]
   double* cs;
   double* sn;
   double* g;           // m+1
   GmresCtl* ctl;
+  double tol;          // the solve's parameters, into ctl by the first residual kernel
+  int maxit;
 };
 
 __device__ __forceinline__ float sum_splits(const float* __restrict__ ypart, int nsplit, int64_t R, int64_t r) {
   float s = ypart[r];
-  for (int k = 1; k < nsplit; ++k) s += ypart[(int64_t)k * R + r];
+  int k = 1;
+  for (; k + 7 < nsplit; k += 8) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = ypart[(int64_t)(k + u) * R + r];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
+  for (; k < nsplit; ++k) s += ypart[(int64_t)k * R + r];
   return s;
 }
 
-// Norm of b -> ctl->bnorm; resets the cycle state.
-__global__ void k_gmres_init(GmresArgs a) {
-  cg::grid_group grid = cg::this_grid();
-  grid_partial_norm(a.b, a.R, a.part, a.stride, 0);
-  grid.sync();
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const double bn = sqrt(sum_parts(a.part, gridDim.x, a.stride, 0));
-    a.ctl->bnorm = bn;
-    a.ctl->total_iters = 0;
-    a.ctl->converged = (bn == 0.0) ? 1 : 0;
-    a.ctl->cycle_done = a.ctl->converged;
-    a.ctl->beta = bn;
-    a.ctl->restarts = 0;
-    a.ctl->nan = isfinite(bn) ? 0 : 1;
-  }
-}
-
 // r = b - A x, beta = ||r||; convergence test on the true residual;
-// V[0] = r / beta, g = (beta, 0, ...).  mode 0: x = 0 (r = b); 1: r = b - sum
-// of the matvec partials of A x; 2: V[0] already holds r (written by a
-// residual operator, e.g. FP64-accumulated).
-__global__ void k_gmres_residual(GmresArgs a, int mode) {
+// V[0] = r / beta, g = (beta, 0, ...).  mode 0 opens a solve: sets up the control
+// block, x = 0, r = b, bnorm = beta; 1: r = b - sum of the matvec partials of
+// A x; 2: V[0] already holds r (written by a residual operator, e.g.
+// FP64-accumulated).
+__global__ void __launch_bounds__(kKrylovThreads) k_gmres_residual(GmresArgs a, int mode) {
   cg::grid_group grid = cg::this_grid();
-  if (a.ctl->converged || a.ctl->nan) return;
+  if (mode != 0 && (a.ctl->converged || a.ctl->nan)) return;
+  const int64_t r0 = blockIdx.x * (int64_t)kKrylovThreads + threadIdx.x, stride = (int64_t)gridDim.x * kKrylovThreads;
   float* V0 = a.V;
-  if (mode != 2)
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
-      V0[r] = mode == 0 ? a.b[r] : a.b[r] - sum_splits(a.ypart, a.nsplit, a.R, r);
-  grid_partial_norm(V0, a.R, a.part, a.stride, 0);
-  grid.sync();
-  const double beta = sqrt(sum_parts(a.part, gridDim.x, a.stride, 0));
-  const double bn = a.ctl->bnorm;
-  const bool conv = beta <= a.ctl->tol * bn;
+  const double bn0 = mode != 0 ? a.ctl->bnorm : 0.0;
+  const double tol = mode != 0 ? a.ctl->tol : a.tol;
+  double acc = 0.0;
+  for (int64_t r = r0; r < a.R; r += stride) {
+    float v;
+    if (mode == 2) {
+      v = V0[r];
+    } else {
+      v = mode == 0 ? a.b[r] : a.b[r] - sum_splits(a.ypart, a.nsplit, a.R, r);
+      V0[r] = v;
+    }
+    if (mode == 0) {
+      if (a.x_double) static_cast<double*>(a.x)[r] = 0.0;
+      else static_cast<float*>(a.x)[r] = 0.f;
+    }
+    acc = fma(f2d(v), f2d(v), acc);
+  }
+  block_parts2(acc, 0.0, 1, a.part);
+  grid_barrier(grid);
+  __shared__ double sum[1];
+  gather_parts(a.part, 1, sum);
+  const double beta = sqrt(sum[0]);
+  const double bn = mode == 0 ? beta : bn0;
+  const bool conv = beta <= tol * bn;
   const bool bad = !isfinite(beta);
   if (!conv && !bad) {
     const float inv = (float)(1.0 / beta);
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
-      V0[r] *= inv;
+    for (int64_t r = r0; r < a.R; r += stride) V0[r] *= inv;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (mode != 0) a.ctl->heads += 1;
-    a.ctl->beta = beta;
-    a.ctl->converged = conv ? 1 : 0;
-    a.ctl->nan = bad ? 1 : 0;
-    a.ctl->cycle_done = (conv || bad || a.ctl->total_iters >= a.ctl->maxit) ? 1 : 0;
-    a.ctl->jconv = 0;
+    GmresCtl* ctl = a.ctl;
+    if (mode == 0) {
+      GmresCtl c{};
+      c.tol = a.tol;
+      c.maxit = a.maxit;
+      c.bnorm = bn;
+      *ctl = c;
+    } else {
+      ctl->heads += 1;
+    }
+    ctl->beta = beta;
+    ctl->converged = conv ? 1 : 0;
+    ctl->nan = bad ? 1 : 0;
+    ctl->cycle_done = (conv || bad || ctl->total_iters >= ctl->maxit) ? 1 : 0;
+    ctl->jconv = 0;
     a.g[0] = beta;
     for (int k = 1; k <= a.m; ++k) a.g[k] = 0.0;
   }
@@ -277,92 +323,194 @@ __global__ void k_gmres_residual(GmresArgs a, int mode) {
 
 // One Arnoldi step j: w = A v_j (from ypart) -> CGS2 against V[0..j] -> v_{j+1};
 // Hessenberg column, Givens rotation, residual estimate |g_{j+1}|.
-__global__ void k_gmres_arnoldi(GmresArgs a, int j) {
+//
+// Bound: latency (two grid syncs, reductions).  With a row per thread (ONE) a
+// thread's entries of V[0..j] stay in registers over both passes, so the basis is
+// read once; the dots of a pass leave a warp by halving exchanges (16 values in
+// 16 exchanges); ||w|| after the second pass is ||w'||^2 - sum h2^2 from that
+// pass's own reduction (recomputed from w when that cancels), so a step has two
+// grid syncs.  N=4000, one B200: 40 us with 59 blocks of serial partial sums.
+// NVB: V entries kept per thread (a multiple of 16, at least j + 2 with ||w'||^2).
+template <int NVB, bool ONE>
+__global__ void __launch_bounds__(kKrylovThreads) k_gmres_arnoldi(GmresArgs a, int j) {
   cg::grid_group grid = cg::this_grid();
   if (a.ctl->cycle_done) return;
+  constexpr int NG = NVB / 16;
+  __shared__ double red[NG][kKrylovWarps][16];
+  __shared__ double h[NVB], h2[NVB], rot[2][kMaxRestart];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nv = j + 1;
+  const int64_t r0 = blockIdx.x * (int64_t)kKrylovThreads + tid, stride = (int64_t)gridDim.x * kKrylovThreads;
   float* w = a.V + (int64_t)(j + 1) * a.ldv;
-  double* p0 = a.part;
-  double* p1 = a.part + (int64_t)gridDim.x * a.stride;
-  double* p2 = a.part + 2 * (int64_t)gridDim.x * a.stride;
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
-    w[r] = sum_splits(a.ypart, a.nsplit, a.R, r);
-  grid_partial_dots(w, a.V, a.ldv, nv, a.R, p0, a.stride);
-  grid.sync();
-  __shared__ double h[kMaxRestart + 1], h2[kMaxRestart + 1];
-  for (int k = threadIdx.x; k < nv; k += blockDim.x) h[k] = sum_parts(p0, gridDim.x, a.stride, k);
-  __syncthreads();
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x) {
-    double s = f2d(w[r]);
-    for (int k = 0; k < nv; ++k) s -= h[k] * f2d(a.V[(int64_t)k * a.ldv + r]);
-    w[r] = (float)s;
-  }
-  grid_partial_dots(w, a.V, a.ldv, nv, a.R, p1, a.stride);
-  grid.sync();
-  for (int k = threadIdx.x; k < nv; k += blockDim.x) h2[k] = sum_parts(p1, gridDim.x, a.stride, k);
-  __syncthreads();
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x) {
-    double s = f2d(w[r]);
-    for (int k = 0; k < nv; ++k) s -= h2[k] * f2d(a.V[(int64_t)k * a.ldv + r]);
-    w[r] = (float)s;
-  }
-  grid_partial_norm(w, a.R, p2, a.stride, 0);
-  grid.sync();
-  const double nrm = sqrt(sum_parts(p2, gridDim.x, a.stride, 0));
-  if (nrm > 0.0 && isfinite(nrm)) {
-    const float inv = (float)(1.0 / nrm);
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
-      w[r] *= inv;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const int ldh = a.m + 1;
-    double* Hc = a.H + (int64_t)j * ldh;
-    for (int k = 0; k < nv; ++k) Hc[k] = h[k] + h2[k];
-    Hc[j + 1] = nrm;
-    for (int k = 0; k < j; ++k) {
-      const double x0 = Hc[k], x1 = Hc[k + 1];
-      Hc[k] = a.cs[k] * x0 + a.sn[k] * x1;
-      Hc[k + 1] = -a.sn[k] * x0 + a.cs[k] * x1;
+  const int64_t pstride = (int64_t)gridDim.x * (kMaxRestart + 2);
+  if (blockIdx.x == 0)
+    for (int k = tid; k < j; k += kKrylovThreads) {
+      rot[0][k] = a.cs[k];
+      rot[1][k] = a.sn[k];
     }
-    const double x0 = Hc[j], x1 = Hc[j + 1];
-    const double rr = hypot(x0, x1);
-    const double c = rr > 0.0 ? x0 / rr : 1.0, s = rr > 0.0 ? x1 / rr : 0.0;
+  float vr[ONE ? NVB : 1], wr = 0.f;
+  if constexpr (ONE) {
+    const bool in = r0 < a.R;
+#pragma unroll
+    for (int k = 0; k < NVB; ++k) vr[k] = (in && k < nv) ? a.V[(int64_t)k * a.ldv + r0] : 0.f;
+    if (in) wr = sum_splits(a.ypart, a.nsplit, a.R, r0);
+  } else {
+    for (int64_t r = r0; r < a.R; r += stride) w[r] = sum_splits(a.ypart, a.nsplit, a.R, r);
+  }
+  // dots of w with V[0..nv), and w.w as value nv when asked for
+  auto dots = [&](bool norm, double* part) {
+    const int n = nv + (norm ? 1 : 0);
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      if (16 * g < n) {
+        double acc[16];
+        if constexpr (ONE) {
+          const double wd = f2d(wr);
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+            acc[u] = wd * f2d(norm && 16 * g + u == nv ? wr : vr[16 * g + u]);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 16; ++u) acc[u] = 0.0;
+          for (int64_t r = r0; r < a.R; r += stride) {
+            const float wv = w[r];
+            const double wd = f2d(wv);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+              const int k = 16 * g + u;
+              if (k < n) acc[u] = fma(wd, f2d(k < nv ? a.V[(int64_t)k * a.ldv + r] : wv), acc[u]);
+            }
+          }
+        }
+        const double v = warp_sum16(acc, lane);
+        if ((lane & 1) == 0) red[g][warp][lane >> 1] = v;
+      }
+    }
+    block_parts(red, n, part);
+  };
+  // w -= sum_k c[k] v_k (FP64), times scale
+  auto update = [&](const double* c, float scale) {
+    if constexpr (ONE) {
+      double s = f2d(wr);
+#pragma unroll
+      for (int k = 0; k < NVB; ++k)
+        if (k < nv) s -= c[k] * f2d(vr[k]);
+      wr = (float)s * scale;
+    } else {
+      for (int64_t r = r0; r < a.R; r += stride) {
+        double s = f2d(w[r]);
+        for (int k = 0; k < nv; ++k) s -= c[k] * f2d(a.V[(int64_t)k * a.ldv + r]);
+        w[r] = (float)s * scale;
+      }
+    }
+  };
+  dots(false, a.part);
+  grid_barrier(grid);
+  gather_parts(a.part, nv, h);
+  update(h, 1.f);
+  dots(true, a.part + pstride);
+  grid_barrier(grid);
+  gather_parts(a.part + pstride, nv + 1, h2);
+  double sub = 0.0;
+  for (int k = 0; k < nv; ++k) sub = fma(h2[k], h2[k], sub);
+  const double ww = h2[nv];
+  double nrm2 = ww - sub;
+  float scale = 1.f;
+  if (nrm2 > 1e-3 * ww && isfinite(nrm2)) {
+    scale = (float)(1.0 / sqrt(nrm2));
+    update(h2, scale);
+  } else {
+    // little is left of w (or nothing finite): its norm from its entries; the
+    // same branch in every block
+    update(h2, 1.f);
+    double acc = 0.0;
+    if constexpr (ONE) {
+      acc = f2d(wr) * f2d(wr);
+    } else {
+      for (int64_t r = r0; r < a.R; r += stride) acc = fma(f2d(w[r]), f2d(w[r]), acc);
+    }
+    block_parts2(acc, 0.0, 1, a.part + 2 * pstride);
+    grid_barrier(grid);
+    __shared__ double sum[1];
+    gather_parts(a.part + 2 * pstride, 1, sum);
+    nrm2 = sum[0];
+    if (nrm2 > 0.0 && isfinite(nrm2)) {
+      scale = (float)(1.0 / sqrt(nrm2));
+      if constexpr (ONE) wr *= scale;
+      else
+        for (int64_t r = r0; r < a.R; r += stride) w[r] *= scale;
+    }
+  }
+  if constexpr (ONE) {
+    if (r0 < a.R) w[r0] = wr;
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    const double nrm = sqrt(nrm2);
+    double* Hc = a.H + (int64_t)j * (a.m + 1);
+    double top = h[0] + h2[0];
+    for (int k = 0; k < j; ++k) {
+      const double x1 = h[k + 1] + h2[k + 1];
+      Hc[k] = rot[0][k] * top + rot[1][k] * x1;
+      top = -rot[1][k] * top + rot[0][k] * x1;
+    }
+    const double rr = hypot(top, nrm);
+    const double c = rr > 0.0 ? top / rr : 1.0, s = rr > 0.0 ? nrm / rr : 0.0;
     a.cs[j] = c;
     a.sn[j] = s;
     Hc[j] = rr;
     Hc[j + 1] = 0.0;
-    a.g[j + 1] = -s * a.g[j];
-    a.g[j] = c * a.g[j];
+    const double gj = a.g[j];
+    a.g[j + 1] = -s * gj;
+    a.g[j] = c * gj;
     GmresCtl* ctl = a.ctl;
-    ctl->total_iters += 1;
+    const int total = ctl->total_iters + 1;
+    ctl->total_iters = total;
     ctl->jconv = j + 1;
-    const double est = fabs(a.g[j + 1]);
+    const double est = fabs(-s * gj);
     ctl->estimate = est;
     const bool bad = !isfinite(est);
     if (bad) ctl->nan = 1;
-    if (bad || est <= ctl->tol * ctl->bnorm || j + 1 >= a.m || ctl->total_iters >= ctl->maxit || nrm == 0.0)
+    if (bad || est <= ctl->tol * ctl->bnorm || j + 1 >= a.m || total >= ctl->maxit || nrm == 0.0)
       ctl->cycle_done = 1;
   }
 }
 
-// x += V y, H y = g (upper triangular, size jconv).
-__global__ void k_gmres_update(GmresArgs a) {
+// x += V y, H y = g (upper triangular, size jconv): the triangle into shared
+// memory, one warp eliminates column by column, lane = row.
+__global__ void __launch_bounds__(kKrylovThreads) k_gmres_update(GmresArgs a) {
   if (a.ctl->converged || a.ctl->nan) return;
   const int jc = a.ctl->jconv;
   if (jc == 0) return;
-  __shared__ double y[kMaxRestart];
-  if (threadIdx.x == 0) {
-    const int ldh = a.m + 1;
-    for (int i = jc - 1; i >= 0; --i) {
-      double s = a.g[i];
-      for (int k = i + 1; k < jc; ++k) s -= a.H[(int64_t)k * ldh + i] * y[k];
-      y[i] = s / a.H[(int64_t)i * ldh + i];
+  __shared__ double y[kMaxRestart], Hs[kMaxRestart * (kMaxRestart + 1) / 2];   // column k at k (k + 1) / 2
+  const int tid = threadIdx.x, lane = tid & 31, ldh = a.m + 1;
+  for (int e = tid; e < jc * jc; e += kKrylovThreads) {
+    const int k = e / jc, i = e % jc;
+    if (i <= k) Hs[k * (k + 1) / 2 + i] = a.H[(int64_t)k * ldh + i];
+  }
+  if (tid < jc) y[tid] = a.g[tid];
+  __syncthreads();
+  if (tid < 32) {
+    for (int k = jc - 1; k >= 0; --k) {
+      const double* col = Hs + k * (k + 1) / 2;
+      const double yk = y[k] / col[k];
+      __syncwarp();
+      if (lane == 0) y[k] = yk;
+      for (int i = lane; i < k; i += 32) y[i] -= col[i] * yk;
+      __syncwarp();
     }
   }
   __syncthreads();
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t r = blockIdx.x * (int64_t)kKrylovThreads + tid; r < a.R; r += (int64_t)gridDim.x * kKrylovThreads) {
     double s = 0.0;
-    for (int k = 0; k < jc; ++k) s += y[k] * f2d(a.Z[(int64_t)k * a.ldv + r]);
+    int k = 0;
+    for (; k + 8 <= jc; k += 8) {
+      float z[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) z[u] = a.Z[(int64_t)(k + u) * a.ldv + r];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += y[k + u] * f2d(z[u]);
+    }
+    for (; k < jc; ++k) s += y[k] * f2d(a.Z[(int64_t)k * a.ldv + r]);
     if (a.x_double) {
       double* x = static_cast<double*>(a.x);
       x[r] += s;
@@ -371,7 +519,7 @@ __global__ void k_gmres_update(GmresArgs a) {
       x[r] = (float)(f2d(x[r]) + s);
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->restarts += 1;
+  if (blockIdx.x == 0 && tid == 0) a.ctl->restarts += 1;
 }
 
 template <typename T>
@@ -400,14 +548,56 @@ void GmresGraphCache::release() {
 }
 
 int krylov_coop_blocks(int64_t R, int num_sms) {
-  // 256-thread blocks; at most 2 per SM (always co-resident), fewer for small systems
-  int want = (int)ceil_div(R, 256 * 4);
-  int n = std::max(1, std::min(want, 2 * num_sms));
+  // a row per thread up to one block per SM (always co-resident)
+  int n = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(R, kKrylovThreads), num_sms));
   // Handles that share the device with other handles' cooperative grids keep
   // the sum of all grids within one block per SM, so every grid can become
   // fully resident once the non-cooperative kernels beside it drain.
   if (t_coop_cap > 0) n = std::min(n, t_coop_cap);
   return n;
+}
+
+static GmresArgs gmres_args(const GmresSetup& s, const float* b, void* x, bool x_double) {
+  GmresArgs a;
+  a.ypart = s.ypart;
+  a.nsplit = s.nsplit;
+  a.b = b;
+  a.x = x;
+  a.x_double = x_double ? 1 : 0;
+  a.V = s.V;
+  a.Z = s.Z ? s.Z : s.V;
+  a.ldv = s.ldv;
+  a.R = s.R;
+  a.m = s.m;
+  a.part = s.part;
+  a.H = s.H;
+  a.cs = s.cs;
+  a.sn = s.sn;
+  a.g = s.g;
+  a.ctl = s.ctl;
+  a.tol = s.tol;
+  a.maxit = s.maxit;
+  return a;
+}
+
+static int launch_residual(GmresArgs& a, int mode, int nblk, cudaStream_t st) {
+  void* args[] = {&a, &mode};
+  return coop_launch((const void*)k_gmres_residual, nblk, kKrylovThreads, args, st);
+}
+
+// Arnoldi step j.  ONE where the grid has a thread per row; NVB by the values of
+// the second pass (j + 1 dots and the norm).
+static int launch_arnoldi(GmresArgs& a, int j, int nblk, cudaStream_t st) {
+  const bool one = (int64_t)nblk * kKrylovThreads >= a.R;
+  const void* fn = nullptr;
+  switch ((j + 2 + 15) / 16) {
+    case 1: fn = one ? (const void*)k_gmres_arnoldi<16, true> : (const void*)k_gmres_arnoldi<16, false>; break;
+    case 2: fn = one ? (const void*)k_gmres_arnoldi<32, true> : (const void*)k_gmres_arnoldi<32, false>; break;
+    case 3: fn = one ? (const void*)k_gmres_arnoldi<48, true> : (const void*)k_gmres_arnoldi<48, false>; break;
+    default: fn = one ? (const void*)k_gmres_arnoldi<80, true> : (const void*)k_gmres_arnoldi<80, false>; break;
+  }
+  void* args[] = {&a, &j};
+  return coop_launch(fn, nblk, kKrylovThreads, args, st);
 }
 
 int gmres_solve(const GmresSetup& s, const MatvecFn& matvec, const float* b, float* x, cudaStream_t st,
@@ -422,40 +612,9 @@ int gmres_solve_ex(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn
     set_last_error_str("gmres: restart length out of range");
     return RF_E_INPUT;
   }
-  GmresArgs a;
-  a.ypart = s.ypart;
-  a.nsplit = s.nsplit;
-  a.b = b;
-  a.x = x;
-  a.x_double = x_double ? 1 : 0;
-  a.V = s.V;
-  a.Z = s.Z ? s.Z : s.V;
-  a.ldv = s.ldv;
-  a.R = s.R;
-  a.m = m;
-  a.part = s.part;
-  a.stride = kMaxRestart + 2;
-  a.H = s.H;
-  a.cs = s.cs;
-  a.sn = s.sn;
-  a.g = s.g;
-  a.ctl = s.ctl;
+  GmresArgs a = gmres_args(s, b, x, x_double);
   const int nblk = s.coop_blocks;
-  GmresCtl init{};
-  init.tol = s.tol;
-  init.maxit = s.maxit;
-  RF_CUDA_TRY(cudaMemcpyAsync(s.ctl, &init, sizeof(GmresCtl), cudaMemcpyHostToDevice, st));
-  if (x_double)
-    k_fill_zero<double><<<std::min<int64_t>(ceil_div(s.R, 256), 1024), 256, 0, st>>>(static_cast<double*>(x), s.R);
-  else
-    k_fill_zero<float><<<std::min<int64_t>(ceil_div(s.R, 256), 1024), 256, 0, st>>>(static_cast<float*>(x), s.R);
-  RF_LAUNCH_CHECK();
-  {
-    void* args[] = {&a};
-    int rc = coop_launch((const void*)k_gmres_init, nblk, 256, args, st);
-    if (rc) return rc;
-  }
-  res->launches = 2;
+  res->launches = 0;
   GmresCtl h{};
   int cycles_run = 0;
   // Pieces of the restart cycles, each launched directly or replayed from a
@@ -476,8 +635,7 @@ int gmres_solve_ex(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn
       mode = residual ? 2 : 1;
     }
     if (v <= 1) {
-      void* args[] = {&a, &mode};
-      const int rc = coop_launch((const void*)k_gmres_residual, nblk, 256, args, st);
+      const int rc = launch_residual(a, mode, nblk, st);
       if (rc) return rc;
     }
     if (v == 1) return RF_OK;
@@ -485,12 +643,11 @@ int gmres_solve_ex(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn
     for (int j = j0; j < j1; ++j) {
       int rc = matvec(s.V + (int64_t)j * s.ldv, &s.ctl->cycle_done, st);
       if (rc) return rc;
-      void* args[] = {&a, &j};
-      rc = coop_launch((const void*)k_gmres_arnoldi, nblk, 256, args, st);
+      rc = launch_arnoldi(a, j, nblk, st);
       if (rc) return rc;
     }
     if (v == 0) {
-      k_gmres_update<<<nblk, 256, 0, st>>>(a);
+      k_gmres_update<<<nblk, kKrylovThreads, 0, st>>>(a);
       RF_LAUNCH_CHECK();
     }
     return RF_OK;
@@ -574,7 +731,7 @@ int gmres_solve_ex(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn
       if (h.cycle_done || h.nan || h.timeout) break;
     }
     if (h.nan || h.timeout) break;
-    k_gmres_update<<<nblk, 256, 0, st>>>(a);
+    k_gmres_update<<<nblk, kKrylovThreads, 0, st>>>(a);
     RF_LAUNCH_CHECK();
     res->launches += 1;
     if (cycle > s.maxit + 2) break;
@@ -597,13 +754,6 @@ int gmres_solve_ex(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn
 // ---------------------------------------------------------------------------
 // GMRES as a graph with a device-side restart loop
 // ---------------------------------------------------------------------------
-__global__ void k_gmres_ctl_init(GmresCtl* ctl, double tol, int maxit) {
-  GmresCtl c{};
-  c.tol = tol;
-  c.maxit = maxit;
-  *ctl = c;
-}
-
 // another restart cycle is needed: not converged, no failure, iterations left
 __global__ void k_gmres_loop_cond(cudaGraphConditionalHandle cond, GmresCtl* ctl) {
   const bool more = !ctl->converged && !ctl->nan && !ctl->timeout && ctl->total_iters < ctl->maxit &&
@@ -612,40 +762,17 @@ __global__ void k_gmres_loop_cond(cudaGraphConditionalHandle cond, GmresCtl* ctl
   cudaGraphSetConditional(cond, more ? 1u : 0u);
 }
 
-static GmresArgs gmres_args(const GmresSetup& s, const float* b, void* x, bool x_double) {
-  GmresArgs a;
-  a.ypart = s.ypart;
-  a.nsplit = s.nsplit;
-  a.b = b;
-  a.x = x;
-  a.x_double = x_double ? 1 : 0;
-  a.V = s.V;
-  a.Z = s.Z ? s.Z : s.V;
-  a.ldv = s.ldv;
-  a.R = s.R;
-  a.m = s.m;
-  a.part = s.part;
-  a.stride = kMaxRestart + 2;
-  a.H = s.H;
-  a.cs = s.cs;
-  a.sn = s.sn;
-  a.g = s.g;
-  a.ctl = s.ctl;
-  return a;
-}
-
 // m x (matvec + Arnoldi step) of the cycle whose first basis vector is in V[0]
 static int enqueue_arnoldi_steps(const GmresSetup& s, GmresArgs& a, const MatvecFn& matvec, cudaStream_t st,
                                  int* kernels) {
   for (int j = 0; j < s.m; ++j) {
     int rc = matvec(s.V + (int64_t)j * s.ldv, &s.ctl->cycle_done, st);
     if (rc) return rc;
-    void* args[] = {&a, &j};
-    rc = coop_launch((const void*)k_gmres_arnoldi, s.coop_blocks, 256, args, st);
+    rc = launch_arnoldi(a, j, s.coop_blocks, st);
     if (rc) return rc;
     *kernels += 1;
   }
-  k_gmres_update<<<s.coop_blocks, 256, 0, st>>>(a);
+  k_gmres_update<<<s.coop_blocks, kKrylovThreads, 0, st>>>(a);
   RF_LAUNCH_CHECK();
   *kernels += 1;
   return RF_OK;
@@ -658,19 +785,8 @@ int gmres_enqueue_first(const GmresSetup& s, const MatvecFn& matvec, const Resid
     return RF_E_INPUT;
   }
   GmresArgs a = gmres_args(s, b, x, x_double);
-  k_gmres_ctl_init<<<1, 1, 0, st>>>(s.ctl, s.tol, s.maxit);
-  if (x_double)
-    k_fill_zero<double><<<std::min<int64_t>(ceil_div(s.R, 256), 1024), 256, 0, st>>>(static_cast<double*>(x), s.R);
-  else
-    k_fill_zero<float><<<std::min<int64_t>(ceil_div(s.R, 256), 1024), 256, 0, st>>>(static_cast<float*>(x), s.R);
-  RF_LAUNCH_CHECK();
-  *kernels += 2;
-  void* args0[] = {&a};
-  if (int rc = coop_launch((const void*)k_gmres_init, s.coop_blocks, 256, args0, st)) return rc;
-  int mode = 0;
-  void* args1[] = {&a, &mode};
-  if (int rc = coop_launch((const void*)k_gmres_residual, s.coop_blocks, 256, args1, st)) return rc;
-  *kernels += 2;
+  if (int rc = launch_residual(a, 0, s.coop_blocks, st)) return rc;
+  *kernels += 1;
   if (int rc = enqueue_arnoldi_steps(s, a, matvec, st, kernels)) return rc;
   k_gmres_loop_cond<<<1, 1, 0, st>>>(cond, s.ctl);
   RF_LAUNCH_CHECK();
@@ -685,9 +801,7 @@ int gmres_enqueue_cycle(const GmresSetup& s, const MatvecFn& matvec, const Resid
   const int rc0 = residual ? residual(x, s.V, &s.ctl->converged, st)
                            : matvec(static_cast<const float*>(x), &s.ctl->converged, st);
   if (rc0) return rc0;
-  int mode = residual ? 2 : 1;
-  void* args1[] = {&a, &mode};
-  if (int rc = coop_launch((const void*)k_gmres_residual, s.coop_blocks, 256, args1, st)) return rc;
+  if (int rc = launch_residual(a, residual ? 2 : 1, s.coop_blocks, st)) return rc;
   *kernels += 1;
   if (int rc = enqueue_arnoldi_steps(s, a, matvec, st, kernels)) return rc;
   k_gmres_loop_cond<<<1, 1, 0, st>>>(cond, s.ctl);
@@ -730,24 +844,20 @@ struct BicgArgs {
   float* sv;
   float* t;
   int64_t R;
-  double* part;
-  int stride;
+  double* part;        // 2 partial buffers of gridDim.x * (kMaxRestart + 2)
   BicgCtl* ctl;
 };
 
-// a.b and c.d partial dots of this block into part[blk*stride + slot], slot+1
+// a.b and c.d over the grid: this block's partial sums
 __device__ void grid_partial_dot2(const float* __restrict__ a, const float* __restrict__ b,
                                   const float* __restrict__ c, const float* __restrict__ d, int64_t R,
-                                  double* __restrict__ part, int stride, int slot) {
+                                  double* __restrict__ part) {
   double acc[2] = {0.0, 0.0};
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < R; r += (int64_t)gridDim.x * blockDim.x) {
     acc[0] = fma(f2d(a[r]), f2d(b[r]), acc[0]);
     acc[1] = fma(f2d(c[r]), f2d(d[r]), acc[1]);
   }
-  __shared__ double tmp[2];
-  block_reduce_store<2>(acc, tmp);
-  if (threadIdx.x < 2) part[(int64_t)blockIdx.x * stride + slot + threadIdx.x] = tmp[threadIdx.x];
-  __syncthreads();
+  block_parts2(acc[0], acc[1], 2, part);
 }
 
 __device__ __forceinline__ bool bicg_stopped(const BicgCtl* c) {
@@ -755,7 +865,7 @@ __device__ __forceinline__ bool bicg_stopped(const BicgCtl* c) {
 }
 
 // ||b||, x = 0, r = r0 = p = b, rho = ||b||^2
-__global__ void k_bicg_init(BicgArgs a) {
+__global__ void __launch_bounds__(kKrylovThreads) k_bicg_init(BicgArgs a) {
   cg::grid_group grid = cg::this_grid();
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x) {
     const float bv = a.b[r];
@@ -764,10 +874,12 @@ __global__ void k_bicg_init(BicgArgs a) {
     a.r0[r] = bv;
     a.p[r] = bv;
   }
-  grid_partial_norm(a.b, a.R, a.part, a.stride, 0);
-  grid.sync();
+  grid_partial_dot2(a.b, a.b, a.b, a.b, a.R, a.part);
+  grid_barrier(grid);
+  __shared__ double sum[2];
+  gather_parts(a.part, 2, sum);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const double bb = sum_parts(a.part, gridDim.x, a.stride, 0);
+    const double bb = sum[0];
     BicgCtl* c = a.ctl;
     c->bnorm = sqrt(bb);
     c->rho = bb;
@@ -782,7 +894,7 @@ __global__ void k_bicg_init(BicgArgs a) {
 }
 
 // after the matvec of x: r = b - A x, r0 = p = r, rho = ||r||^2
-__global__ void k_bicg_restart(BicgArgs a) {
+__global__ void __launch_bounds__(kKrylovThreads) k_bicg_restart(BicgArgs a) {
   cg::grid_group grid = cg::this_grid();
   if (a.ctl->converged || a.ctl->nan || !a.ctl->need_restart) return;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x) {
@@ -791,10 +903,12 @@ __global__ void k_bicg_restart(BicgArgs a) {
     a.r0[r] = rv;
     a.p[r] = rv;
   }
-  grid_partial_norm(a.r, a.R, a.part, a.stride, 0);
-  grid.sync();
+  grid_partial_dot2(a.r, a.r, a.r, a.r, a.R, a.part);
+  grid_barrier(grid);
+  __shared__ double sum[2];
+  gather_parts(a.part, 2, sum);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const double rr = sum_parts(a.part, gridDim.x, a.stride, 0);
+    const double rr = sum[0];
     a.ctl->rho = rr;
     a.ctl->need_restart = 0;
     a.ctl->last_restart = a.ctl->iters;
@@ -804,15 +918,17 @@ __global__ void k_bicg_restart(BicgArgs a) {
 }
 
 // after v = A p: alpha = rho / (v . r0), s = r - alpha v
-__global__ void k_bicg_step1(BicgArgs a) {
+__global__ void __launch_bounds__(kKrylovThreads) k_bicg_step1(BicgArgs a) {
   cg::grid_group grid = cg::this_grid();
   if (bicg_stopped(a.ctl)) return;
   const double rho = a.ctl->rho;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
     a.v[r] = sum_splits(a.ypart, a.nsplit, a.R, r);
-  grid_partial_dot2(a.v, a.r0, a.v, a.v, a.R, a.part, a.stride, 0);
-  grid.sync();
-  const double vr0 = sum_parts(a.part, gridDim.x, a.stride, 0);
+  grid_partial_dot2(a.v, a.r0, a.v, a.v, a.R, a.part);
+  grid_barrier(grid);
+  __shared__ double sum[2];
+  gather_parts(a.part, 2, sum);
+  const double vr0 = sum[0];
   const double alpha = rho / vr0;
   const float af = (float)alpha;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
@@ -825,7 +941,7 @@ __global__ void k_bicg_step1(BicgArgs a) {
 
 // after t = A s: omega = (t.s)/(t.t), x += alpha p + omega s, r = s - omega t,
 // rho' = r.r0, ||r||; convergence; beta; p = r + beta (p - omega v)
-__global__ void k_bicg_step2(BicgArgs a) {
+__global__ void __launch_bounds__(kKrylovThreads) k_bicg_step2(BicgArgs a) {
   cg::grid_group grid = cg::this_grid();
   if (bicg_stopped(a.ctl)) return;
   // every block reads the control block before the first grid sync; block 0
@@ -834,23 +950,26 @@ __global__ void k_bicg_step2(BicgArgs a) {
   const double rho = c->rho, alpha = c->alpha, bnorm = c->bnorm, tol = c->tol;
   const int it = c->iters + 1, last_restart = c->last_restart, restart_every = c->restart_every;
   double* p0 = a.part;
-  double* p1 = a.part + (int64_t)gridDim.x * a.stride;
+  double* p1 = a.part + (int64_t)gridDim.x * (kMaxRestart + 2);
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x)
     a.t[r] = sum_splits(a.ypart, a.nsplit, a.R, r);
-  grid_partial_dot2(a.t, a.sv, a.t, a.t, a.R, p0, a.stride, 0);
-  grid.sync();
-  const double ts = sum_parts(p0, gridDim.x, a.stride, 0);
-  const double tt = sum_parts(p0, gridDim.x, a.stride, 1);
+  grid_partial_dot2(a.t, a.sv, a.t, a.t, a.R, p0);
+  grid_barrier(grid);
+  __shared__ double sum[2], sum1[2];
+  gather_parts(p0, 2, sum);
+  const double ts = sum[0];
+  const double tt = sum[1];
   const double omega = tt > 0.0 ? ts / tt : 0.0;
   const float af = (float)alpha, of = (float)omega;
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.R; r += (int64_t)gridDim.x * blockDim.x) {
     a.x[r] = a.x[r] + af * a.p[r] + of * a.sv[r];
     a.r[r] = a.sv[r] - of * a.t[r];
   }
-  grid_partial_dot2(a.r, a.r0, a.r, a.r, a.R, p1, a.stride, 0);
-  grid.sync();
-  const double rho_new = sum_parts(p1, gridDim.x, a.stride, 0);
-  const double rnorm = sqrt(sum_parts(p1, gridDim.x, a.stride, 1));
+  grid_partial_dot2(a.r, a.r0, a.r, a.r, a.R, p1);
+  grid_barrier(grid);
+  gather_parts(p1, 2, sum1);
+  const double rho_new = sum1[0];
+  const double rnorm = sqrt(sum1[1]);
   const bool conv = rnorm / bnorm < tol;
   const double beta = (rho_new / rho) * (alpha / omega);
   const bool restart = !conv && (rho_new == 0.0 || omega == 0.0 || (it - 1) - last_restart > restart_every);
@@ -888,7 +1007,6 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
   a.t = s.work + 5 * s.ldv;
   a.R = s.R;
   a.part = s.part;
-  a.stride = kMaxRestart + 2;
   a.ctl = s.ctl;
   const int nblk = s.coop_blocks;
   BicgCtl init{};
@@ -898,7 +1016,7 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
   RF_CUDA_TRY(cudaMemcpyAsync(s.ctl, &init, sizeof(BicgCtl), cudaMemcpyHostToDevice, st));
   {
     void* args[] = {&a};
-    int rc = coop_launch((const void*)k_bicg_init, nblk, 256, args, st);
+    int rc = coop_launch((const void*)k_bicg_init, nblk, kKrylovThreads, args, st);
     if (rc) return rc;
   }
   res->launches = 1;
@@ -910,11 +1028,11 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
       int rc = matvec(a.p, (const int*)&s.ctl->stop_word, st);
       if (rc) return rc;
       void* args[] = {&a};
-      rc = coop_launch((const void*)k_bicg_step1, nblk, 256, args, st);
+      rc = coop_launch((const void*)k_bicg_step1, nblk, kKrylovThreads, args, st);
       if (rc) return rc;
       rc = matvec(a.sv, (const int*)&s.ctl->stop_word, st);
       if (rc) return rc;
-      rc = coop_launch((const void*)k_bicg_step2, nblk, 256, args, st);
+      rc = coop_launch((const void*)k_bicg_step2, nblk, kKrylovThreads, args, st);
       if (rc) return rc;
       // the matvec kernels read one word: fold the stop conditions into it
       k_bicg_stopword<<<1, 1, 0, st>>>(s.ctl);
@@ -929,7 +1047,7 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
       int rc = matvec(x, nullptr, st);
       if (rc) return rc;
       void* args[] = {&a};
-      rc = coop_launch((const void*)k_bicg_restart, nblk, 256, args, st);
+      rc = coop_launch((const void*)k_bicg_restart, nblk, kKrylovThreads, args, st);
       if (rc) return rc;
       k_bicg_stopword<<<1, 1, 0, st>>>(s.ctl);
       RF_LAUNCH_CHECK();

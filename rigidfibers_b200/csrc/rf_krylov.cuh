@@ -7,6 +7,7 @@
 namespace rf {
 
 constexpr int kMaxRestart = 64;
+constexpr int kKrylovThreads = 512;   // threads per block of the cooperative Krylov kernels
 
 // Device control block of one solve; the host reads it once per cycle.
 struct GmresCtl {

@@ -64,8 +64,8 @@ __device__ __forceinline__ void stokeslet_apply(float px, float py, float pz, co
 
 // Velocity sums of one ordered pair set.  Sources at least sqrt(far_d2) away (the
 // assembly's rule, see make_tables) take the far rule, 64 kernel values per pair
-// instead of Q^2; the others the full rule.  One launch: the first far_blocks
-// blocks are far ones, the rest near ones, so that the few near pairs run beside
+// instead of Q^2; the others the full rule.  One launch: the first near_blocks
+// blocks are near ones, the rest far ones, so that the few near pairs run beside
 // the far ones.  Bound: FP32 issue; below a few hundred fibers latency, so both
 // parts split the sources into many partial rows (vpart[row][i][6]: far chunks,
 // then near segments).  Sums over one source's points are formed before they are
@@ -74,8 +74,8 @@ constexpr int kVelFibers = 32;
 constexpr int kVelThreads = kVelFibers * kFarNodes;
 
 struct VelSplit {
-  int chunks, jchunk, far_blocks;   // far: source chunks, sources per chunk, blocks
   int segs, jseg, near_blocks;      // near: source segments, sources per segment, blocks
+  int chunks, jchunk, far_blocks;   // far: source chunks, sources per chunk, blocks
 };
 
 // 32 fibers i x one chunk of sources, thread (fiber, far point of i); the
@@ -219,12 +219,12 @@ template <int Q>
 __global__ void __launch_bounds__(kVelThreads)
 k_velocity_numerical(const Tables tab, int N, const double4* __restrict__ pos64, const float4* __restrict__ ori,
                      const float4* __restrict__ fw, VelSplit v, float* __restrict__ vpart) {
-  const int b = (int)blockIdx.x;
-  if (b < v.far_blocks) {
+  const int b = (int)blockIdx.x - v.near_blocks;
+  if (b >= 0) {
     velocity_far_block(tab, N, pos64, ori, fw, b / v.chunks, b % v.chunks, v.jchunk, vpart);
     return;
   }
-  const int w = (b - v.far_blocks) * (kVelThreads / 32) + (int)(threadIdx.x >> 5);
+  const int w = (int)blockIdx.x * (kVelThreads / 32) + (int)(threadIdx.x >> 5);
   const int i = w / v.segs, seg = w % v.segs;
   if (i < N)
     velocity_near_warp<Q>(tab, N, pos64, ori, fw, i, seg * v.jseg, min(N, (seg + 1) * v.jseg),

@@ -39,25 +39,30 @@ __device__ void analytic_G(const double R0[3], const double tj[3], double e2, fl
     double psu = 1.0, psl = -1.0;
 #pragma unroll
     for (int n = 2; n <= M + 2; ++n) {
-      I1[n + 1] = (psu * uu) / n - (psl * ul) / n + ((1.0 - 2.0 * n) * b) / (2.0 * n) * I1[n] -
-                  ((double)(n - 1) * l) / n * I1[n - 1];
+      const double rn = 1.0 / n;   // a constant of the unrolled step
+      I1[n + 1] = (psu * uu) * rn - (psl * ul) * rn + (1.0 - 2.0 * n) * (0.5 * rn) * b * I1[n] -
+                  (double)(n - 1) * rn * l * I1[n - 1];
       I3[n + 1] = I1[n - 1] - b * I3[n] - l * I3[n - 1];
       I5[n + 1] = I3[n - 1] - b * I5[n] - l * I5[n - 1];
       psl = -psl;   // s_lower^(n) with s_lower = -1; s_upper^n = 1
     }
   } else {
     double i1n2 = 0, i1n1 = 0, i3n2 = 0, i3n1 = 0, i5n2 = 0, i5n1 = 0;
+    // i1n0 = (n + 2) / ((n + 1) l) [(uu - (-1)^(n+1) ul) / (n + 2) + (1 - 2 (n + 2)) /
+    // (2 (n + 2)) b i1n1 - i1n2] with the quotients of integers as constants of
+    // the unrolled steps: a division costs as much as the rest of a step
+    const double dsum = uu + ul, ddif = uu - ul;
+#pragma unroll
     for (int n = 27; n >= 2; --n) {
-      const double np2 = n + 2.0, np1 = n + 1.0;
-      const double sln = ((n + 1) & 1) ? -1.0 : 1.0;   // (-1)^(n+1)
-      const double i1n0 = np2 / (np1 * l) * ((uu / np2) - ((sln * ul) / np2) +
-                                              ((1.0 - 2.0 * np2) / (2.0 * np2)) * b * i1n1 - i1n2);
+      const double rn1 = 1.0 / (n + 1.0);
+      const double i1n0 = invL * (rn1 * (((n + 1) & 1) ? dsum : ddif) - (n + 1.5) * rn1 * b * i1n1 -
+                                  (n + 2.0) * rn1 * i1n2);
       const double i3n0 = invL * (i1n0 - b * i3n1 - i3n2);
       const double i5n0 = invL * (i3n0 - b * i5n1 - i5n2);
-      if (n < M + 3) {
-#pragma unroll
-        for (int q = 3; q < NI; ++q)
-          if (q == n + 1) { I1[q] = i1n0; I3[q] = i3n0; I5[q] = i5n0; }
+      if (n + 1 < NI) {   // n >= 2: entries 3 and up
+        I1[n + 1 < NI ? n + 1 : 3] = i1n0;
+        I3[n + 1 < NI ? n + 1 : 3] = i3n0;
+        I5[n + 1 < NI ? n + 1 : 3] = i5n0;
       }
       i1n2 = i1n1; i1n1 = i1n0;
       i3n2 = i3n1; i3n1 = i3n0;

@@ -56,28 +56,12 @@ enum AsmMode { kAsmDense = 0, kAsmStructF16 = 1, kAsmStructBF16 = 2, kAsmApply =
 template <int M, int Q>
 struct AsmShape {
   static constexpr int TI = 192 / Q;     // fibers per tile side
-  static constexpr int U = TI * Q;       // (fiber, quadrature point) units = threads used
   static constexpr int K1 = M + 1;       // P_0..P_M
-  static constexpr int NC = 6 * K1;      // G columns per unit
-  static constexpr int H = Q / 2;        // folded quadrature points
-  static constexpr int NT = 192;         // threads per CTA
-  // dynamic shared memory: G as NC columns of U units (unit u = qi * TI + il),
-  // then the T blocks (6 floats each).  The column stride is TI (mod 32)
-  // words: phase 2 has lanes (col, tl), TI consecutive tl per column and
-  // 32 / TI columns per warp, and reads 32 distinct banks.
-  static constexpr int GS = (U + 31) / 32 * 32 + TI;
-  // the T blocks start on a 16-byte boundary (they are copied out as float4);
-  // NC * GS is odd for odd M + 1
-  static constexpr int GOFF = (NC * GS + 3) / 4 * 4;
-  static constexpr size_t kGBytes = sizeof(float) * GOFF;
-  // T pair stride padded so that 8 consecutive pairs start on distinct banks
-  // that are multiples of 4 (stride = 4 * odd mod 32)
+  static constexpr int NC = 6 * K1;      // G columns per unit (a point of i against a fiber j)
+  // T of one pair as [value] padded so that 8 consecutive pairs start on
+  // distinct banks that are multiples of 4 (stride = 4 * odd mod 32)
   static constexpr int TP = (K1 * K1 * 6 + 7) / 8 * 8 + 4;
-  static constexpr size_t kTBytes = sizeof(float) * TI * TP;
-  static constexpr size_t kSmem = kGBytes + 2 * kTBytes;   // T double-buffered across j
-  static_assert(GOFF % 4 == 0 && TP % 4 == 0, "T buffers must be 16-byte aligned");
   // structured storage
-  static constexpr int SUB = kStoreTile / TI;      // assembly tiles per storage-tile side
   static constexpr int NQ32 = K1 * K1 * 6;         // FP32 values per pair
   static constexpr int NQ16 = M * M * 6 / 2;       // 16-bit pairs per pair (M*M*6 is even)
   static_assert(kStoreTile % TI == 0, "assembly tile must divide the storage tile");
@@ -637,92 +621,202 @@ k_assemble_pairs(const Tables tab, int N, const float4* __restrict__ ori, AsmOut
 }
 
 // ---------------------------------------------------------------------------
-// Analytical pair tiles: ordered pairs (the inner integral over fiber j is
-// exact, the outer one over fiber i a quadrature, so the blocks of (i, j) and
-// (j, i) are different numbers), dense output only.
+// Analytical assembly: ordered pairs (the inner integral over fiber j is exact,
+// the outer one over fiber i a quadrature, so the blocks of (i, j) and (j, i)
+// are different numbers), dense output only.  Bound: FP64 issue and latency of
+// the closed form (analytic_G), so far pairs evaluate it at the far rule's 8
+// outer points instead of Q (the outer integrand is as smooth as the numerical
+// path's).  One launch: the first N blocks take the near pairs of one fiber i
+// each, the others the far pairs of a tile; kept apart, neither waits for the
+// other's barriers.  N=777, one B200: 4.09 ms with Q points for every pair and
+// divisions in analytic_G, 1.70 ms with the near pairs inside the tiles.
 // ---------------------------------------------------------------------------
+template <int M, int Q>
+struct AnaShape {
+  using A = AsmShape<M, Q>;
+  static constexpr int TI = A::TI, K1 = A::K1, NC = A::NC, TP = A::TP;
+  static constexpr int NT = 192;
+  static constexpr int FN = kFarNodes;
+  static constexpr int JB = TI == 8 ? 3 : TI == 4 ? 4 : 1;   // rows of a far batch: PB x FN <= NT units
+  static constexpr int PB = JB * TI;
+  static constexpr int GSF = (PB * FN + 31) / 32 * 32 + PB;  // lanes (column, pair)
+  static constexpr int NS = 192 / Q;                         // near pairs per group
+  static constexpr int QP = Q + 1;
+  static constexpr int GSN = NS * QP + (NS * QP + 1) % 2;    // near: lanes = columns
+  static constexpr int GFLOATS = (NC * (GSF > GSN ? GSF : GSN) + 3) / 4 * 4;
+  static constexpr size_t kSmem = sizeof(float) * (GFLOATS + (PB > NS ? PB : NS) * TP);
+  static_assert(PB * FN <= NT && NS * Q <= NT, "one unit per thread");
+};
+
+// the closed-form integrals G[c][k] over fiber j for the point s of fiber i, into
+// column k * 6 + c of g (column stride cs)
+template <int M>
+__device__ __forceinline__ void closed_form(const AsmOut& out, float eps, int i, int j, float s, float* g, int cs) {
+  const double4 xi = out.pos64[i], ti = out.ori64[i], xj = out.pos64[j], tj4 = out.ori64[j];
+  const double sd = (double)s;
+  const double R0[3] = {xi.x + sd * ti.x - xj.x, xi.y + sd * ti.y - xj.y, xi.z + sd * ti.z - xj.z};
+  const double tj[3] = {tj4.x, tj4.y, tj4.z};
+  float v[6][M + 1];
+  analytic_G<M>(R0, tj, 2.0 * (double)eps * (double)eps, v);
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+#pragma unroll
+    for (int k = 0; k <= M; ++k) g[(k * 6 + c) * cs] = v[c][k];
+}
+
+// dst[k * NC] = sum_qi W[k][qi] g[qi * stride], folded over qi
+template <int K1, int NQ, bool FAR>
+__device__ __forceinline__ void fold_points(const Tables& tab, const float* g, int stride, float* dst) {
+  float acc[K1];
+#pragma unroll
+  for (int k = 0; k < K1; ++k) acc[k] = 0.f;
+#pragma unroll 4
+  for (int q = 0; q < NQ / 2; ++q) {
+    const float lo = g[q * stride], hi = g[(NQ - 1 - q) * stride];
+    const float ev = __fadd_rn(lo, hi), od = __fsub_rn(lo, hi);
+#pragma unroll
+    for (int k = 0; k < K1; ++k)
+      acc[k] = __fmaf_rn((k & 1) ? od : ev, FAR ? tab.far_W[k][FAR ? q : 0] : tab.W[k][q], acc[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < K1; ++k) dst[k * 6 * K1] = acc[k];
+}
+
+__device__ __forceinline__ float centre_dist2(const double4& a, const double4& b) {
+  const float dx = (float)(a.x - b.x), dy = (float)(a.y - b.y), dz = (float)(a.z - b.z);
+  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
+// The near pairs (i, j) of fiber i, found NT centres at a time and taken in index
+// order in groups of NS; their force terms to partial row T
+template <int M, int Q>
+__device__ __forceinline__ void analytical_near(const Tables& tab, int N, const float4* __restrict__ ori,
+                                                const AsmOut& out, int i, int T, float* smem) {
+  using S = AnaShape<M, Q>;
+  constexpr int K1 = S::K1, NC = S::NC, TP = S::TP, NT = S::NT, NS = S::NS, M3 = 3 * M, FF = 3 * K1;
+  constexpr int QUEUE = NT + NS;
+  __shared__ int queue[QUEUE];
+  __shared__ int warp_near[NT / 32];
+  float* const sG = smem;
+  float* const sT = smem + S::GFLOATS;   // [slot][TP]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double4 xi = out.pos64[i];
+  float facc = 0.f;                      // component tid % 3 of F_i[tid / 3]
+  int count = 0;
+  for (int js = 0; js < N; js += NT) {
+    const int j = js + tid;
+    const bool near = j < N && j != i && centre_dist2(xi, out.pos64[j]) < tab.far_d2;
+    const unsigned m = __ballot_sync(0xffffffffu, near);
+    if (lane == 0) warp_near[warp] = __popc(m);
+    __syncthreads();
+    int at = count, total = count;
+    for (int w = 0; w < NT / 32; ++w) {
+      if (w < warp) at += warp_near[w];
+      total += warp_near[w];
+    }
+    if (near) queue[at + __popc(m & ((1u << lane) - 1))] = j;
+    __syncthreads();
+    count = total;
+    const bool last = js + NT >= N;
+    int done = 0;
+    for (; count - done >= NS || (last && done < count); done += NS) {
+      const int cnt = min(NS, count - done);
+      if (tid < cnt * Q) {
+        const int slot = tid / Q, qi = tid % Q;
+        closed_form<M>(out, tab.eps, i, queue[done + slot], tab.pts[qi], sG + slot * S::QP + qi, S::GSN);
+      }
+      __syncthreads();
+      for (int task = tid; task < cnt * NC; task += NT) {   // lanes = columns
+        const int slot = task / NC, col = task % NC;
+        fold_points<K1, Q, false>(tab, sG + col * S::GSN + slot * S::QP, 1, sT + slot * TP + col);
+      }
+      __syncthreads();
+      for (int task = tid; task < cnt * M * M; task += NT) {
+        const int slot = task / (M * M), kJp = task % (M * M) / M, kIp = task % M;
+        float* dst = out.A + (int64_t)i * M3 + 3 * kIp + ((int64_t)queue[done + slot] * M3 + 3 * kJp) * out.lda;
+        dense_block(dst, out.lda, sT + slot * TP + ((kIp + 1) * K1 + kJp + 1) * 6, ori[i], kIp, tab.gamma[kIp],
+                    tab.eigen[kIp]);
+      }
+      if (tid < FF) {
+        const int a = tid % 3;
+        for (int slot = 0; slot < cnt; ++slot)
+          facc = fmaf(sT[slot * TP + (tid / 3) * NC + (a == 0 ? 4 : a == 1 ? 5 : 2)], tab.fz_half, facc);
+      }
+      __syncthreads();
+    }
+    // what is left of the queue (fewer than NS) to its front
+    const int left = max(0, count - done);
+    const int keep = tid < left ? queue[done + tid] : 0;
+    __syncthreads();
+    if (tid < left) queue[tid] = keep;
+    count = left;
+  }
+  if (tid < FF) out.ffpart[((int64_t)T * N + i) * FF + tid] = facc;
+}
+
 template <int M, int Q>
 __global__ void __launch_bounds__(192, 2)
 k_assemble_analytical(const Tables tab, int N, const float4* __restrict__ ori, AsmOut out) {
-  using S = AsmShape<M, Q>;
-  constexpr int TI = S::TI, K1 = S::K1, NC = S::NC, H = S::H, TP = S::TP;
+  using S = AnaShape<M, Q>;
+  constexpr int TI = S::TI, K1 = S::K1, NC = S::NC, TP = S::TP, NT = S::NT, JB = S::JB, PB = S::PB;
   constexpr int M3 = 3 * M;
   constexpr int FF = K1 * 3;
-  __shared__ float4 sTi[TI];
   extern __shared__ __align__(16) float smem_dyn[];
-  float (*sG)[S::GS] = reinterpret_cast<float (*)[S::GS]>(smem_dyn);   // [NC][GS]
-  float* const sTbase = smem_dyn + S::GOFF;                            // 2 x [TI][TP]
-  __shared__ float sCoef[kMaxTerms], sEig[kMaxTerms];
   const int T = (N + TI - 1) / TI;
-  const int I = blockIdx.x / T, J = blockIdx.x % T;
+  if ((int)blockIdx.x < N) {
+    analytical_near<M, Q>(tab, N, ori, out, (int)blockIdx.x, T, smem_dyn);
+    return;
+  }
+  __shared__ float4 sTi[TI];
+  __shared__ unsigned char sKind[TI * TI];   // pair jl * TI + il.  0: no such pair, 1: far, 2: near
+  float* const sG = smem_dyn;
+  float* const sT = smem_dyn + S::GFLOATS;   // [pair of the batch][TP]
+  __shared__ float sCoef[kMaxTerms], sEig[kMaxTerms];
+  const int I = ((int)blockIdx.x - N) / T, J = ((int)blockIdx.x - N) % T;
   const bool diag = (I == J);
   const int tid = threadIdx.x;
   const int i0 = I * TI, j0 = J * TI;
   if (tid < M) { sCoef[tid] = tab.gamma[tid]; sEig[tid] = tab.eigen[tid]; }
   if (tid < TI) sTi[tid] = ori[min(i0 + tid, N - 1)];
-  // own unit: u = qi * TI + il (a warp holds 32 / TI points of TI fibers)
-  const int il = tid % TI, qi = tid / TI;
-  const int i = i0 + il;
-  const bool unit_ok = (tid < S::U) && (i < N);
+  for (int pr = tid; pr < TI * TI; pr += NT) {
+    const int il = pr % TI, jl = pr / TI;
+    const bool valid = i0 + il < N && j0 + jl < N && (!diag || il != jl);
+    const float d2 = centre_dist2(out.pos64[min(i0 + il, N - 1)], out.pos64[min(j0 + jl, N - 1)]);
+    sKind[pr] = !valid ? 0 : d2 < tab.far_d2 ? 2 : 1;
+  }
   const float fz = tab.fz_half;
   // force-term accumulator of task (tl, k) = (tid / K1, tid % K1): F_i[k]
   float facc[3] = {0.f, 0.f, 0.f};
   __syncthreads();
   const int jcount = min(TI, N - j0);
-  for (int jl = 0; jl < jcount; ++jl) {
-    // T is double-buffered: phase 2 of step jl+1 may run while phase 3 of
-    // step jl still reads, so one barrier per step suffices after phase 2
-    float* const sT = sTbase + (jl & 1) * (TI * TP);
-    const bool pair_ok = unit_ok && (!diag || il != jl);
-    // ---- phase 1: the closed-form integrals G[c][k] of this unit
-    float* const gcol = &sG[0][0] + tid;
-    if (tid < S::U) {
-      float g[6][K1];
+  for (int jb = 0; jb < jcount; jb += JB) {
+    const int jn = min(JB, jcount - jb);
+    // phase 1: unit u = qi * PB + pair; zeros for the pairs that are not far
+    if (tid < PB * S::FN) {
+      const int p = tid % PB, qi = tid / PB;
+      const int pr = jb * TI + p;
+      float* const gcol = sG + tid;
+      if (p < jn * TI && sKind[pr] == 1) {
+        closed_form<M>(out, tab.eps, i0 + pr % TI, j0 + pr / TI, tab.far_pts[qi], gcol, S::GSF);
+      } else {
 #pragma unroll
-      for (int c = 0; c < 6; ++c)
-#pragma unroll
-        for (int k = 0; k < K1; ++k) g[c][k] = 0.f;
-      if (pair_ok) {
-        const double4 xi4 = out.pos64[i], ti4 = out.ori64[i];
-        const double4 xj4 = out.pos64[j0 + jl], tj4 = out.ori64[j0 + jl];
-        const double s = (double)tab.pts[qi];
-        const double R0[3] = {xi4.x + s * ti4.x - xj4.x, xi4.y + s * ti4.y - xj4.y, xi4.z + s * ti4.z - xj4.z};
-        const double tj[3] = {tj4.x, tj4.y, tj4.z};
-        analytic_G<M>(R0, tj, 2.0 * (double)tab.eps * (double)tab.eps, g);
+        for (int c = 0; c < NC; ++c) gcol[c * S::GSF] = 0.f;
       }
-#pragma unroll
-      for (int c = 0; c < 6; ++c)
-#pragma unroll
-        for (int k = 0; k < K1; ++k) gcol[(k * 6 + c) * S::GS] = g[c][k];
     }
     __syncthreads();
-    // ---- phase 2: T[ki][kj][c] = sum_qi W[ki][qi] G[qi][c][kj], folded over qi
-    // lanes (col, tl), tl fastest; column col = kj * 6 + c
-    for (int task = tid; task < TI * NC; task += S::NT) {
-      const int col = task / TI, tl = task % TI;
-      const float* gp = &sG[col][tl];
-      float acc[K1];
-#pragma unroll
-      for (int k = 0; k < K1; ++k) acc[k] = 0.f;
-#pragma unroll
-      for (int q = 0; q < H; ++q) {
-        const float lo = gp[q * TI], hi = gp[(Q - 1 - q) * TI];
-        const float ev = __fadd_rn(lo, hi), od = __fsub_rn(lo, hi);
-#pragma unroll
-        for (int k = 0; k < K1; ++k) acc[k] = __fmaf_rn((k & 1) ? od : ev, tab.W[k][q], acc[k]);
-      }
-#pragma unroll
-      for (int k = 0; k < K1; ++k) sT[tl * TP + k * NC + col] = acc[k];
+    // phase 2: lanes (column, pair), pair fastest
+    for (int task = tid; task < PB * NC; task += NT) {
+      const int col = task / PB, p = task % PB;
+      fold_points<K1, S::FN, true>(tab, sG + col * S::GSF + p, PB, sT + p * TP + col);
     }
     __syncthreads();
-    // ---- phase 3: block (i, j) -- rows of fiber i, columns of fiber j
-    const int j = j0 + jl;
-    for (int task = tid; task < TI * M * M; task += S::NT) {
-      const int kJp = task / (TI * M), rem = task % (TI * M);
-      const int tl = rem / M, kIp = rem % M;
-      const int ii = i0 + tl;
-      if (ii >= N) continue;
-      float* dst = out.A + (int64_t)(i0 * M3 + 3 * rem) + (int64_t)(j * M3 + 3 * kJp) * out.lda;
+    // phase 3: block (i, j) -- rows of fiber i, columns of fiber j (the next
+    // batch's phase 1 writes G only, and its phase 2 follows a barrier)
+    for (int task = tid; task < jn * TI * M * M; task += NT) {
+      const int jj = task / (TI * M * M), r0 = task % (TI * M * M);
+      const int kJp = r0 / (TI * M), rem = r0 % (TI * M);
+      const int tl = rem / M, kIp = rem % M, jl = jb + jj;
+      float* dst = out.A + (int64_t)(i0 * M3 + 3 * rem) + (int64_t)((j0 + jl) * M3 + 3 * kJp) * out.lda;
       if (diag && tl == jl) {
 #pragma unroll
         for (int b = 0; b < 3; ++b)
@@ -730,20 +824,23 @@ k_assemble_analytical(const Tables tab, int N, const float4* __restrict__ ori, A
           for (int a = 0; a < 3; ++a) dst[a + b * out.lda] = (kIp == kJp && a == b) ? 1.f : 0.f;
         continue;
       }
-      dense_block(dst, out.lda, sT + tl * TP + ((kIp + 1) * K1 + kJp + 1) * 6, sTi[tl], kIp, sCoef[kIp], sEig[kIp]);
+      if (sKind[jl * TI + tl] != 1) continue;
+      dense_block(dst, out.lda, sT + (jj * TI + tl) * TP + ((kIp + 1) * K1 + kJp + 1) * 6, sTi[tl], kIp, sCoef[kIp],
+                  sEig[kIp]);
     }
-    // ---- force terms F_i[k] += T^{ij}[k][P0] F/2 (F/2 = (0, 0, fz): column z of the block)
+    // force terms F_i[k] += T^{ij}[k][P0] F/2 (F/2 = (0, 0, fz): column z of the
+    // block; zeros for the pairs that are not far)
     if (tid < TI * K1) {
       const int tl = tid / K1, k = tid % K1;
-      if (i0 + tl < N && (!diag || tl != jl)) {
-        const float* t = sT + tl * TP + k * NC;
+      for (int jj = 0; jj < jn; ++jj) {
+        const float* t = sT + (jj * TI + tl) * TP + k * NC;
         facc[0] = fmaf(t[4], fz, facc[0]);
         facc[1] = fmaf(t[5], fz, facc[1]);
         facc[2] = fmaf(t[2], fz, facc[2]);
       }
     }
   }
-  // ---- partial force terms: ffpart[J][fiber of I][k][3] written exactly once
+  // partial force terms: ffpart[J][fiber of I][k][3] written exactly once
   if (tid < TI * K1) {
     const int tl = tid / K1, k = tid % K1;
     if (i0 + tl < N) {
@@ -912,20 +1009,20 @@ static int launch_pairs(const Tables& tab, int N, const float4* ori, const AsmOu
 
 template <int M, int Q>
 static int launch_analytical(const Tables& tab, int N, const float4* ori, const AsmOut& out, cudaStream_t st) {
-  using S = AsmShape<M, Q>;
+  using S = AnaShape<M, Q>;
   const int64_t T = ceil_div(N, S::TI);
   static const cudaError_t attr = cudaFuncSetAttribute(k_assemble_analytical<M, Q>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
   RF_CUDA_TRY(attr);
-  k_assemble_analytical<M, Q><<<(unsigned)(T * T), S::NT, S::kSmem, st>>>(tab, N, ori, out);
+  k_assemble_analytical<M, Q><<<(unsigned)(N + T * T), S::NT, S::kSmem, st>>>(tab, N, ori, out);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }
 
-static int launch_force_terms(const Tables& tab, int N, const float4* ori, const AsmOut& out, float* F, float* b,
-                              cudaStream_t st) {
+static int launch_force_terms(const Tables& tab, int N, const float4* ori, const AsmOut& out, int nparts, float* F,
+                              float* b, cudaStream_t st) {
   k_force_terms<<<(unsigned)ceil_div(N, kForceFibers), force_threads(tab.M), 0, st>>>(
-      tab, N, ori, out.ffpart, assemble_tiles(tab.M, tab.Q, N), F, b);
+      tab, N, ori, out.ffpart, nparts, F, b);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }
@@ -947,7 +1044,7 @@ static int dispatch_assemble(const Tables& tab, int N, const float4* ori, const 
   if (rc == RF_E_UNSUPPORTED) set_last_error_str("assemble: (M, Q) combination not instantiated");
   if (rc != RF_OK) return rc;
   if (MODE == kAsmApply && out.x != nullptr) return RF_OK;   // the product: no force terms
-  return launch_force_terms(tab, N, ori, out, F, b, st);
+  return launch_force_terms(tab, N, ori, out, assemble_tiles(tab.M, tab.Q, N), F, b, st);
 }
 
 int launch_assemble_numerical(const Tables& tab, int N, const float4* pos, const float4* ori, const double4* pos64,
@@ -978,7 +1075,8 @@ int launch_assemble_analytical(const Tables& tab, int N, const float4* pos, cons
 #undef RF_ASM_CASE
   if (rc == RF_E_UNSUPPORTED) set_last_error_str("assemble: (M, Q) combination not instantiated");
   if (rc != RF_OK) return rc;
-  return launch_force_terms(tab, N, ori, out, F, b, st);
+  // one partial row per tile column, and the near pairs'
+  return launch_force_terms(tab, N, ori, out, assemble_tiles(tab.M, tab.Q, N) + 1, F, b, st);
 }
 
 int launch_assemble_apply(const Tables& tab, int N, const float4* pos, const float4* ori, const double4* pos64,

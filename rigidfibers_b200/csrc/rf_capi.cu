@@ -670,7 +670,8 @@ static int allocate_buffers(rf_handle* h, const rf_config* cfg) {
   if (!rc) rc = h->alloc((void**)&h->x, (size_t)R * sizeof(float));
   const int tiles = assemble_tiles(h->M, h->Q, N);
   const size_t ffn = (size_t)N * 3 * (h->M + 1);
-  if (!rc) rc = h->alloc((void**)&h->ffpart, (size_t)tiles * ffn * sizeof(float));
+  // one row per tile column; one more for the analytical assembly's near pairs
+  if (!rc) rc = h->alloc((void**)&h->ffpart, (size_t)(tiles + 1) * ffn * sizeof(float));
   if (!rc) rc = h->alloc((void**)&h->F, ffn * sizeof(float));
   // Krylov
   const int m = (h->mixed && cfg->refinement_restart > 0) ? cfg->refinement_restart : cfg->gmres_restart;

@@ -32,7 +32,7 @@ int assemble_tiles(int M, int Q, int N);
 // give bit-identical results): 0 scalar FP32, 1 packed two-lane FP32
 // (add/mul/fma .f32x2) for the two mirror points of each folded pair.
 constexpr int kAsmVariants = 2;
-// Numerical assembly.  ffpart: assemble_tiles(M,Q,N) x N x 3(M+1) floats of
+// Numerical assembly.  ffpart: (assemble_tiles(M,Q,N) + 1) x N x 3(M+1) floats of
 // scratch; F: N x 3(M+1) force terms sum_j T^{ij}[k][P0] F/2; b: R.  pos64:
 // the FP64 centres, from which the pair separations are formed.
 int launch_assemble_numerical(const Tables& tab, int N, const float4* pos, const float4* ori, const double4* pos64,

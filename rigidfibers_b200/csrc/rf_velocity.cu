@@ -15,8 +15,6 @@
 
 namespace rf {
 
-int velocity_chunks(int N);
-
 // Source densities of both quadrature rules, weight included:
 // fw[j * (Q + FN) + q] = w_q f_j(s_q) = W[0][q] F/2 + sum_k a_{j,k} W[k+1][q] for
 // the Q points of the full rule, then the FN points of the far rule.
@@ -145,6 +143,37 @@ __device__ __forceinline__ void velocity_far_block(const Tables& tab, int N, con
   }
 }
 
+// dst[0..5] = sum_q W[0][q] g(q), sum_q W[1][q] g(q) over a warp whose lane l holds
+// the points l, l + 32 of one fiber
+template <int Q>
+__device__ __forceinline__ void near_row_sums(const Tables& tab, const float (&g)[(Q + 31) / 32][3],
+                                              float* __restrict__ dst) {
+  constexpr int NP = (Q + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  float u[6] = {};
+#pragma unroll
+  for (int h = 0; h < NP; ++h) {
+    const int q = lane + 32 * h;
+    if (q < Q) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        u[a] = fmaf(tab.W[0][q], g[h][a], u[a]);
+        u[3 + a] = fmaf(tab.W[1][q], g[h][a], u[3 + a]);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int a = 0; a < 6; ++a) u[a] += __shfl_xor_sync(0xffffffffu, u[a], o);
+  if (lane < 6) {
+    float v = u[0];
+#pragma unroll
+    for (int a = 1; a < 6; ++a) v = lane == a ? u[a] : v;
+    dst[lane] = v;
+  }
+}
+
 // One warp: fiber i's near sources of one segment, found 32 centres at a time and
 // taken in index order, lane = quadrature point of i (Q = 48: two passes)
 template <int Q>
@@ -191,28 +220,7 @@ __device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, con
       }
     }
   }
-  float u[6] = {};
-#pragma unroll
-  for (int h = 0; h < NP; ++h) {
-    const int q = lane + 32 * h;
-    if (q < Q) {
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        u[a] = fmaf(tab.W[0][q], g[h][a], u[a]);
-        u[3 + a] = fmaf(tab.W[1][q], g[h][a], u[3 + a]);
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int a = 0; a < 6; ++a) u[a] += __shfl_xor_sync(0xffffffffu, u[a], o);
-  if (lane < 6) {
-    float v = u[0];
-#pragma unroll
-    for (int a = 1; a < 6; ++a) v = lane == a ? u[a] : v;
-    row[(int64_t)i * 6 + lane] = v;
-  }
+  near_row_sums<Q>(tab, g, row + (int64_t)i * 6);
 }
 
 template <int Q>
@@ -258,77 +266,137 @@ k_velocity_finalize(const Tables tab, int N, const float4* __restrict__ ori, con
 }
 
 // Analytical variant: the inner integral over fiber j in closed form (FP64),
-// GF_ij(qi) = G_0(qi) F/2 + sum_k G_{k+1}(qi) a_{j,k}; the outer quadrature
-// over fiber i as in the numerical kernel.  This is how the reference's
-// 100_analytic_* golden files were produced (its committed
-// fortran/update_velocities.incl integrates numerically in both modes).
-template <int M, int Q>
-__global__ void __launch_bounds__(192, 2)
-k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, const double4* __restrict__ ori,
-                      const float* __restrict__ coeff, int jchunk, float* __restrict__ vpart,
-                      int* __restrict__ vflag) {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *vflag = 0;
-  constexpr int TI = 192 / Q;
-  constexpr int U = TI * Q;
-  constexpr int M3 = 3 * M;
-  __shared__ float sGs[3][U];
-  const int tid = threadIdx.x;
-  const int il = tid / Q, qi = tid % Q;
-  const int i0 = blockIdx.x * TI;
-  const int i = i0 + il;
-  const bool unit_ok = tid < U && i < N;
-  const double e2 = 2.0 * (double)tab.eps * (double)tab.eps;
-  const float fz = tab.fz_half;
-  float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-  const int jbeg = blockIdx.y * jchunk, jend = min(N, jbeg + jchunk);
-  if (unit_ok) {
-    const double4 xi4 = pos[i], ti4 = ori[i];
-    const double s = (double)tab.pts[qi];
-    for (int j = jbeg; j < jend; ++j) {
-      if (j == i) continue;
-      const double4 xj4 = pos[j], tj4 = ori[j];
-      const double R0[3] = {xi4.x + s * ti4.x - xj4.x, xi4.y + s * ti4.y - xj4.y, xi4.z + s * ti4.z - xj4.z};
-      const double tj[3] = {tj4.x, tj4.y, tj4.z};
-      float G[6][M + 1];
-      analytic_G<M>(R0, tj, e2, G);
-      // F/2 = (0, 0, fz): column z of G_0
-      float f0 = G[4][0] * fz, f1 = G[5][0] * fz, f2 = G[2][0] * fz;
-      const float* a = coeff + (int64_t)j * M3;
+// GF_ij(qi) = G_0(qi) F/2 + sum_k G_{k+1}(qi) a_{j,k}; the outer quadrature over
+// fiber i as in the numerical kernel, the far rule's points for far sources.
+// This is how the reference's 100_analytic_* golden files were produced (its
+// committed fortran/update_velocities.incl integrates numerically in both
+// modes).  Bound: FP64 issue of the closed form.
+template <int M>
+__device__ __forceinline__ void analytic_apply(const double (&R0)[3], const double4& tj4, const float* __restrict__ a,
+                                               double e2, float fz, float (&g)[3]) {
+  const double tj[3] = {tj4.x, tj4.y, tj4.z};
+  float G[6][M + 1];
+  analytic_G<M>(R0, tj, e2, G);
+  // F/2 = (0, 0, fz): column z of G_0
+  float f0 = G[4][0] * fz, f1 = G[5][0] * fz, f2 = G[2][0] * fz;
 #pragma unroll
-      for (int k = 0; k < M; ++k) {
-        const float a0 = a[3 * k], a1 = a[3 * k + 1], a2 = a[3 * k + 2];
-        f0 += G[0][k + 1] * a0 + G[3][k + 1] * a1 + G[4][k + 1] * a2;
-        f1 += G[3][k + 1] * a0 + G[1][k + 1] * a1 + G[5][k + 1] * a2;
-        f2 += G[4][k + 1] * a0 + G[5][k + 1] * a1 + G[2][k + 1] * a2;
+  for (int k = 0; k < M; ++k) {
+    const float a0 = a[3 * k], a1 = a[3 * k + 1], a2 = a[3 * k + 2];
+    f0 += G[0][k + 1] * a0 + G[3][k + 1] * a1 + G[4][k + 1] * a2;
+    f1 += G[3][k + 1] * a0 + G[1][k + 1] * a1 + G[5][k + 1] * a2;
+    f2 += G[4][k + 1] * a0 + G[5][k + 1] * a1 + G[2][k + 1] * a2;
+  }
+  g[0] += f0; g[1] += f1; g[2] += f2;
+}
+
+// Far blocks (after the near ones): 16 fibers x 8 far points x one chunk of
+// sources, lane = fiber.  Near blocks: one warp per (fiber, segment), lane =
+// quadrature point.  Partial rows as the numerical kernel's.
+constexpr int kAnaFibers = 16;
+constexpr int kAnaThreads = kAnaFibers * kFarNodes;
+
+template <int M, int Q>
+__global__ void __launch_bounds__(kAnaThreads, 3)
+k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, const double4* __restrict__ ori,
+                      const float* __restrict__ coeff, VelSplit v, float* __restrict__ vpart,
+                      int* __restrict__ vflag) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *vflag = 0;
+  constexpr int M3 = 3 * M, FN = kFarNodes, B = kAnaFibers;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const double e2 = 2.0 * (double)tab.eps * (double)tab.eps;
+  const float fz = tab.fz_half, far_d2 = tab.far_d2;
+  auto dist2 = [](const double4& a, const double4& b) {
+    const float dx = (float)(a.x - b.x), dy = (float)(a.y - b.y), dz = (float)(a.z - b.z);
+    return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+  };
+  const int b = (int)blockIdx.x - v.near_blocks;
+  if (b >= 0) {
+    __shared__ float sGs[3][FN][B];
+    const int tile = b / v.chunks, chunk = b % v.chunks;
+    const int il = tid % B, qi = tid / B, i = tile * B + il;
+    float g[3] = {0.f, 0.f, 0.f};
+    if (i < N) {
+      const double4 xi = pos[i], ti = ori[i];
+      const double s = (double)tab.far_pts[qi];
+      const double pt[3] = {xi.x + s * ti.x, xi.y + s * ti.y, xi.z + s * ti.z};
+      const int jend = min(N, (chunk + 1) * v.jchunk);
+      for (int j = chunk * v.jchunk; j < jend; ++j) {
+        const double4 xj = pos[j];
+        if (j == i || dist2(xi, xj) < far_d2) continue;
+        const double R0[3] = {pt[0] - xj.x, pt[1] - xj.y, pt[2] - xj.z};
+        analytic_apply<M>(R0, ori[j], coeff + (int64_t)j * M3, e2, fz, g);
       }
-      g0 += f0; g1 += f1; g2 += f2;
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) sGs[a][qi][il] = g[a];
+    __syncthreads();
+    if (tid < B * 6) {
+      const int fl = tid % B, comp = tid / B;
+      const float* w = comp >= 3 ? tab.far_W[1] : tab.far_W[0];
+      float acc = 0.f;
+#pragma unroll
+      for (int q = 0; q < FN; ++q) acc = fmaf(w[q], sGs[comp % 3][q][fl], acc);
+      if (tile * B + fl < N) vpart[((int64_t)chunk * N + tile * B + fl) * 6 + comp] = acc;
+    }
+    return;
+  }
+  const int w = (int)blockIdx.x * (kAnaThreads / 32) + (tid >> 5);
+  const int i = w / v.segs, seg = w % v.segs;
+  if (i >= N) return;
+  constexpr int NP = (Q + 31) / 32;
+  const double4 xi = pos[i], ti = ori[i];
+  float g[NP][3] = {};
+  const int jend = min(N, (seg + 1) * v.jseg);
+  for (int js = seg * v.jseg; js < jend; js += 32) {
+    const int j = js + lane;
+    const bool near = j < jend && j != i && dist2(xi, pos[j]) < far_d2;
+    for (unsigned m = __ballot_sync(0xffffffffu, near); m != 0; m &= m - 1) {
+      const int jj = js + __ffs(m) - 1;
+      const double4 xj = pos[jj], tj = ori[jj];
+#pragma unroll
+      for (int h = 0; h < NP; ++h) {
+        const int q = lane + 32 * h;
+        if (q < Q) {
+          const double s = (double)tab.pts[q];
+          const double R0[3] = {xi.x + s * ti.x - xj.x, xi.y + s * ti.y - xj.y, xi.z + s * ti.z - xj.z};
+          analytic_apply<M>(R0, tj, coeff + (int64_t)jj * M3, e2, fz, g[h]);
+        }
+      }
     }
   }
-  if (tid < U) { sGs[0][tid] = g0; sGs[1][tid] = g1; sGs[2][tid] = g2; }
-  __syncthreads();
-  if (tid < TI * 6) {
-    const int fl = tid / 6, comp = tid % 6;
-    const int a = comp % 3;
-    const bool rot = comp >= 3;
-    float acc = 0.f;
-#pragma unroll
-    for (int q = 0; q < Q; ++q) acc = fmaf(rot ? tab.W[1][q] : tab.W[0][q], sGs[a][fl * Q + q], acc);
-    if (i0 + fl < N) vpart[((int64_t)blockIdx.y * N + i0 + fl) * 6 + comp] = acc;
-  }
+  near_row_sums<Q>(tab, g, vpart + (int64_t)(v.chunks + seg) * N * 6 + (int64_t)i * 6);
+}
+
+// Far: enough fiber-tile x chunk blocks to fill the GPU four times over, at least 8
+// sources each; near: N warps alone leave the GPU idle below a few thousand fibers
+static VelSplit velocity_split(int N, int fibers, int threads) {
+  VelSplit v;
+  const int tiles = (int)ceil_div(N, fibers), most = (int)ceil_div(N, 8);
+  v.chunks = std::max(1, std::min((int)ceil_div(148 * 4 * 4, tiles), most));
+  v.jchunk = (int)ceil_div(N, v.chunks);
+  v.far_blocks = tiles * v.chunks;
+  v.segs = std::max(1, std::min((int)ceil_div(148 * 16, N), most));
+  v.jseg = (int)ceil_div(N, v.segs);
+  v.near_blocks = (int)ceil_div((int64_t)N * v.segs, threads / 32);
+  return v;
+}
+
+// partial rows of either velocity path (vpart: this many rows of 6 N floats)
+int velocity_rows(int N) {
+  const VelSplit n = velocity_split(N, kVelFibers, kVelThreads), a = velocity_split(N, kAnaFibers, kAnaThreads);
+  return std::max(n.chunks + n.segs, a.chunks + a.segs);
 }
 
 int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, const double4* pos64,
                                const double4* ori64, const float* x, float* vpart, float4* tvel, float4* rvel,
                                int* vflag, cudaStream_t st) {
-  const int chunks = velocity_chunks(N);
-  const int jchunk = (int)ceil_div(N, chunks);
-  const int TI = 192 / tab.Q;
-  dim3 grid((unsigned)ceil_div(N, TI), (unsigned)chunks);
+  const VelSplit v = velocity_split(N, kAnaFibers, kAnaThreads);
+  const unsigned nb = (unsigned)(v.far_blocks + v.near_blocks);
   bool done = false;
-#define RF_VA_CASE(MM, QQ)                                                                   \
-  if (!done && tab.M == MM && tab.Q == QQ) {                                                 \
-    k_velocity_analytical<MM, QQ><<<grid, 192, 0, st>>>(tab, N, pos64, ori64, x, jchunk, vpart, vflag); \
-    done = true;                                                                             \
+#define RF_VA_CASE(MM, QQ)                                                                              \
+  if (!done && tab.M == MM && tab.Q == QQ) {                                                            \
+    k_velocity_analytical<MM, QQ><<<nb, kAnaThreads, 0, st>>>(tab, N, pos64, ori64, x, v, vpart, vflag); \
+    done = true;                                                                                        \
   }
   RF_FOR_EACH_MQ(RF_VA_CASE)
 #undef RF_VA_CASE
@@ -337,38 +405,10 @@ int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, cons
     return RF_E_UNSUPPORTED;
   }
   RF_LAUNCH_CHECK();
-  k_velocity_finalize<<<(unsigned)ceil_div(N, kVelSumFibers), kVelSumThreads, 0, st>>>(tab, N, ori, vpart, chunks, tvel,
-                                                                                     rvel, vflag);
+  k_velocity_finalize<<<(unsigned)ceil_div(N, kVelSumFibers), kVelSumThreads, 0, st>>>(
+      tab, N, ori, vpart, v.chunks + v.segs, tvel, rvel, vflag);
   RF_LAUNCH_CHECK();
   return RF_OK;
-}
-
-int velocity_chunks(int N) {
-  // enough CTAs to fill 148 SMs several times over for any N
-  const int tiles = (int)ceil_div(N, 8);
-  int chunks = (int)ceil_div(148 * 8, tiles);
-  chunks = std::max(1, std::min(chunks, (int)ceil_div(N, 8)));
-  return chunks;
-}
-
-// Far: enough 32-fiber x chunk blocks to fill the GPU twice over, at least 8
-// sources each; near: N warps alone leave the GPU idle below a few thousand fibers
-static VelSplit velocity_split(int N) {
-  VelSplit v;
-  const int tiles = (int)ceil_div(N, kVelFibers), most = (int)ceil_div(N, 8);
-  v.chunks = std::max(1, std::min((int)ceil_div(148 * 4 * 4, tiles), most));
-  v.jchunk = (int)ceil_div(N, v.chunks);
-  v.far_blocks = tiles * v.chunks;
-  v.segs = std::max(1, std::min((int)ceil_div(148 * 16, N), most));
-  v.jseg = (int)ceil_div(N, v.segs);
-  v.near_blocks = (int)ceil_div((int64_t)N * v.segs, kVelThreads / 32);
-  return v;
-}
-
-// partial rows of either velocity path (vpart: this many rows of 6 N floats)
-int velocity_rows(int N) {
-  const VelSplit v = velocity_split(N);
-  return std::max(velocity_chunks(N), v.chunks + v.segs);
 }
 
 int launch_velocity_numerical(const Tables& tab, int N, const double4* pos64, const float4* ori, const float* x,
@@ -377,7 +417,7 @@ int launch_velocity_numerical(const Tables& tab, int N, const double4* pos64, co
   k_source_density<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)N * (Q + kFarNodes), 256), 148 * 16), 256, 0, st>>>(
       tab, N, x, fw, vflag);
   RF_LAUNCH_CHECK();
-  const VelSplit v = velocity_split(N);
+  const VelSplit v = velocity_split(N, kVelFibers, kVelThreads);
   const unsigned nb = (unsigned)(v.far_blocks + v.near_blocks);
   switch (Q) {
     case 12: k_velocity_numerical<12><<<nb, kVelThreads, 0, st>>>(tab, N, pos64, ori, fw, v, vpart); break;

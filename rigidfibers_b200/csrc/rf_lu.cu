@@ -915,8 +915,14 @@ int lu_factor_solve(const LuSetup& s, const float* A, const float* b, float* x, 
       RF_TRY_RF(launch_residual64(s, A, b, st));
       k_norm2_pair<<<1, 256, 0, st>>>(s.r64, b, R, s.norms);
       RF_LAUNCH_CHECK();
+      int st_word = 0;
       RF_CUDA_TRY(cudaMemcpyAsync(h, s.norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+      if (tcf) RF_CUDA_TRY(cudaMemcpyAsync(&st_word, s.flags + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
       RF_CUDA_TRY(cudaStreamSynchronize(st));
+      if (st_word < 0) {   // a triangular solve's bounded wait gave up
+        set_last_error_str("lu: a bounded device-side wait timed out");
+        return RF_E_TIMEOUT;
+      }
       rel = h[1] > 0 ? std::sqrt(h[0] / h[1]) : 0.0;
       // factors without row exchanges that do not refine (non-finite, stalled
       // or out of steps) are replaced by partially pivoted ones

@@ -41,18 +41,17 @@
 // from the column-major matrix, where each column's k-run is contiguous.
 // Every wait is bounded (%globaltimer); a wait that gives up records -1 in
 // the status word, and the kernel drains what it issued before freeing TMEM.
-#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
+#include <utility>
 
 #include "rf_common.cuh"
 #include "rf_lu.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace rf {
 
@@ -663,166 +662,310 @@ constexpr size_t tc_smem() {
 
 // ---------------------------------------------------------------------------
 // The w x w diagonal block (w <= 128) at (k, k): factored in shared memory
-// without row exchanges (multiplier a * (1 / pivot), then fmaf(-l, u, a), as
-// the pivoted panel does) and written back; the largest |l| into lmax, a zero
+// without row exchanges and written back; the largest |l| into lmax, a zero
 // pivot into status.  The inverses of its factors follow in k_lu_diag_inv.
 //
-// 32 warps, warp w owning columns w, w + 32, w + 64, w + 96, lane l rows
-// l, l + 32, l + 64, l + 96 of each.  No step waits for the whole CTA: the
-// owner of column j + 1 applies step j to that column first, scales it and
-// publishes it through flag[j + 1] (a bounded spin in shared memory), then
-// applies step j to its other columns; every warp applies the steps to its
-// columns in order.
+// One CTA, latency-bound: column by column (a step of the whole block per
+// column) it took 116 us.  Blocked by 32 columns instead: one warp factors the
+// 32 x 32 diagonal sub-block in registers (lane = row, pivot rows by shuffles);
+// then every thread takes one row of L21 or one column of U12 (32 values in
+// registers, the sub-block read as 16-byte broadcasts); then the rest of the
+// block is updated from shared memory (lane = row).
 // ---------------------------------------------------------------------------
-constexpr int kDiagLd = kPanel + 1;
-constexpr uint32_t kDiagSpin = 1u << 26;
+constexpr int kDiagLd = kPanel + 4;      // rows 16-byte aligned; 8 rows of float4 on distinct banks
+constexpr int kSub = 32;                 // sub-panel width
+constexpr int kDiagThreads = 512;
+constexpr size_t kDiagSmem = sizeof(float) * kPanel * kDiagLd;
+constexpr int kInvLd = kSub + 4;
+constexpr int kInvThreads = 256;
+// diagonal sub-block inverses, the column block of the inverse, one product
+constexpr size_t kDiagInvSmem = sizeof(float) * (kPanel * kDiagLd + 2 * kPanel * kInvLd + kSub * kInvLd);
 
-__global__ void __launch_bounds__(1024) k_lu_diag(float* __restrict__ A, int64_t lda, int64_t k, int w,
-                                                  unsigned int* __restrict__ lmax, int* __restrict__ status) {
-  extern __shared__ float sm[];
-  float* a = sm;                          // [128][129] row-major block
-  __shared__ volatile int flag[kPanel];   // 1: column j scaled, 2: abort
-  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
-  for (int e = tid; e < kPanel * kPanel; e += nt) {
-    const int r = e % kPanel, c = e / kPanel;   // coalesced over r (column-major source)
-    a[r * kDiagLd + c] = (r < w && c < w) ? A[(k + r) + (k + c) * lda] : (r == c ? 1.f : 0.f);
-  }
-  if (tid < kPanel) flag[tid] = 0;
-  __syncthreads();
-  float vmax = 0.f;
-  bool abort = false;
-  // scale column j below the diagonal (the warp owning it); false on a zero pivot
-  auto scale = [&](int j) -> bool {
-    const float piv = a[j * kDiagLd + j];
-    if (piv == 0.f) return false;
-    const float inv = 1.f / piv;
-    for (int r = (j + 1) >> 5; r < 4; ++r) {
-      const int i = lane + 32 * r;
-      if (i > j && i < w) {
-        const float l = a[i * kDiagLd + j] * inv;
-        a[i * kDiagLd + j] = l;
-        vmax = fmaxf(vmax, fabsf(l));
+// rest of the block after sub-panel O: a[r][c] -= sum_k L[r][k] U[k][c]
+template <int O>
+__device__ __forceinline__ void diag_trailing(float* a) {
+  constexpr int F = O + kSub, N2 = kPanel - F;   // first row / column, size
+  if constexpr (N2 > 0) {
+    constexpr int TR = N2 / 32, TC = N2 / 16;    // 512 threads: lane = row (mod 32), warp = TC columns
+    const int lane = threadIdx.x & 31, c0 = F + (int)(threadIdx.x >> 5) * TC;
+    float acc[TR][TC];
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+      for (int j = 0; j < TC; ++j) acc[i][j] = a[(F + lane + 32 * i) * kDiagLd + c0 + j];
+#pragma unroll 2
+    for (int k = 0; k < kSub; k += 4) {
+      float l[TR][4];
+#pragma unroll
+      for (int i = 0; i < TR; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(a + (F + lane + 32 * i) * kDiagLd + O + k);
+        l[i][0] = v.x; l[i][1] = v.y; l[i][2] = v.z; l[i][3] = v.w;
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        const float* u = a + (O + k + kk) * kDiagLd + c0;
+#pragma unroll
+        for (int j = 0; j < TC; ++j) {
+          const float uj = u[j];
+#pragma unroll
+          for (int i = 0; i < TR; ++i) acc[i][j] = fmaf(-l[i][kk], uj, acc[i][j]);
+        }
       }
     }
-    return true;
-  };
-  auto publish = [&](int j, int v) {
-    __syncwarp();
-    __threadfence_block();
-    if (lane == 0) flag[j] = v;
-  };
-  // step j applied to column c (rows > j)
-  auto apply = [&](int j, int c) {
-    const float u = a[j * kDiagLd + c];
-    for (int r = (j + 1) >> 5; r < 4; ++r) {
-      const int i = lane + 32 * r;
-      if (i > j && i < w) a[i * kDiagLd + c] = fmaf(-a[i * kDiagLd + j], u, a[i * kDiagLd + c]);
-    }
-  };
-  if (w > 0 && warp == 0) {
-    const bool ok = scale(0);
-    publish(0, ok ? 1 : 2);
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+      for (int j = 0; j < TC; ++j) a[(F + lane + 32 * i) * kDiagLd + c0 + j] = acc[i][j];
   }
-  for (int j = 0; j < w && !abort; ++j) {
-    // wait for column j (bounded)
-    uint32_t spins = 0;
-    int f;
-    while ((f = flag[j]) == 0) {
-      if (++spins > kDiagSpin) { f = 3; break; }
-    }
-    __syncwarp();
-    __threadfence_block();
-    if (f != 1) {
-      if (lane == 0) atomicExch(status, f == 3 ? -1 : 2);
-      abort = true;
-      // the owners of later columns must not wait for this one
-      if (j + 1 < w && ((j + 1) & 31) == warp) publish(j + 1, 2);
-      break;
-    }
-    const int jn = j + 1;
-    if (jn < w && (jn & 31) == warp) {
-      apply(j, jn);
-      __syncwarp();
-      const bool ok = scale(jn);
-      publish(jn, ok ? 1 : 2);
+}
+
+// the block at (k, k) into a (row-major), the identity outside w x w
+__device__ __forceinline__ void load_diag(const float* __restrict__ A, int64_t lda, int64_t k, int w, float* a) {
+  // thread: row r, every (blockDim / 128)-th column, 16 loads in flight; coalesced
+  // over r (column-major source)
+  const int r = threadIdx.x % kPanel, cs = blockDim.x / kPanel;
+  const float* src = A + k + r + k * lda;
+  for (int c0 = threadIdx.x / kPanel; c0 < kPanel; c0 += 16 * cs) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int c = c0 + u * cs;
+      v[u] = (r < w && c < w) ? src[(int64_t)c * lda] : (r == c ? 1.f : 0.f);
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = warp + 32 * q;
-      if (c > j && c < w && c != jn) apply(j, c);
-    }
-    __syncwarp();
+    for (int u = 0; u < 16; ++u) a[r * kDiagLd + c0 + u * cs] = v[u];
   }
-  // every thread leaves here or none does (the barriers below need all of them)
-  if (__syncthreads_or(abort)) return;
+}
+
+// f(integral_constant<int, 0>), .., f(integral_constant<int, N - 1>): loops whose
+// register arrays need compile-time indexes
+template <class F, int... I>
+__device__ __forceinline__ void static_for_(F& f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>()), ...);
+}
+template <int N, class F>
+__device__ __forceinline__ void static_for(F f) {
+  static_for_(f, std::make_integer_sequence<int, N>());
+}
+
+__global__ void __launch_bounds__(kDiagThreads) k_lu_diag(float* __restrict__ A, int64_t lda, int64_t k, int w,
+                                                          unsigned int* __restrict__ lmax,
+                                                          int* __restrict__ status) {
+  extern __shared__ __align__(16) float sm[];
+  float* a = sm;                          // [128][132] row-major block
+  __shared__ float rdiag[kSub];           // reciprocals of the sub-block's pivots
+  __shared__ int zero_pivot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  load_diag(A, lda, k, w, a);
+  if (tid == 0) zero_pivot = 0;
+  __syncthreads();
+  float vmax = 0.f;
+  for (int o = 0; o < kPanel; o += kSub) {
+    if (warp == 0) {
+      // the 32 x 32 sub-block: lane = row
+      float r[kSub];
+#pragma unroll
+      for (int c = 0; c < kSub; c += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(a + (o + lane) * kDiagLd + o + c);
+        r[c] = v.x; r[c + 1] = v.y; r[c + 2] = v.z; r[c + 3] = v.w;
+      }
+      bool zero = false;
+      static_for<kSub>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        const float piv = __shfl_sync(0xffffffffu, r[j], j);
+        zero |= piv == 0.f;
+        const float inv = 1.f / piv;
+        if (lane == j) rdiag[j] = inv;
+        const float l = r[j] * inv;
+        const bool below = lane > j;
+#pragma unroll
+        for (int c = j + 1; c < kSub; ++c) {
+          const float u = __shfl_sync(0xffffffffu, r[c], j);
+          if (below) r[c] = fmaf(-l, u, r[c]);
+        }
+        if (below) {
+          r[j] = l;
+          vmax = fmaxf(vmax, fabsf(l));
+        }
+      });
+#pragma unroll
+      for (int c = 0; c < kSub; c += 4)
+        *reinterpret_cast<float4*>(a + (o + lane) * kDiagLd + o + c) = make_float4(r[c], r[c + 1], r[c + 2], r[c + 3]);
+      if (zero && lane == 0) zero_pivot = 1;
+    }
+    __syncthreads();
+    if (zero_pivot) {   // every thread leaves here or none does
+      if (tid == 0) atomicExch(status, 2);
+      return;
+    }
+    const int f = o + kSub, n2 = kPanel - f;
+    if (warp < 4 && tid < n2) {
+      // row f + tid of L21: x U11 = a
+      float* row = a + (f + tid) * kDiagLd + o;
+      float x[kSub];
+#pragma unroll
+      for (int c = 0; c < kSub; c += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + c);
+        x[c] = v.x; x[c + 1] = v.y; x[c + 2] = v.z; x[c + 3] = v.w;
+      }
+      static_for<kSub>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        x[j] *= rdiag[j];
+        vmax = fmaxf(vmax, fabsf(x[j]));
+#pragma unroll
+        for (int c = 0; c < kSub; c += 4) {
+          if (c + 3 <= j) continue;
+          const float4 u = *reinterpret_cast<const float4*>(a + (o + j) * kDiagLd + o + c);
+          if (c > j) x[c] = fmaf(-x[j], u.x, x[c]);
+          if (c + 1 > j) x[c + 1] = fmaf(-x[j], u.y, x[c + 1]);
+          if (c + 2 > j) x[c + 2] = fmaf(-x[j], u.z, x[c + 2]);
+          if (c + 3 > j) x[c + 3] = fmaf(-x[j], u.w, x[c + 3]);
+        }
+      });
+#pragma unroll
+      for (int c = 0; c < kSub; c += 4)
+        *reinterpret_cast<float4*>(row + c) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
+    } else if (warp >= 4 && warp < 8 && tid - 128 < n2) {
+      // column f + tid - 128 of U12: L11 x = a (unit diagonal)
+      float* col = a + o * kDiagLd + f + (tid - 128);
+      float x[kSub];
+#pragma unroll
+      for (int i = 0; i < kSub; ++i) x[i] = col[i * kDiagLd];
+      static_for<kSub>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < kSub; c += 4) {
+          if (c >= i) continue;
+          const float4 l = *reinterpret_cast<const float4*>(a + (o + i) * kDiagLd + o + c);
+          s[0] = fmaf(l.x, x[c], s[0]);
+          if (c + 1 < i) s[1] = fmaf(l.y, x[c + 1], s[1]);
+          if (c + 2 < i) s[2] = fmaf(l.z, x[c + 2], s[2]);
+          if (c + 3 < i) s[3] = fmaf(l.w, x[c + 3], s[3]);
+        }
+        x[i] -= (s[0] + s[1]) + (s[2] + s[3]);
+      });
+#pragma unroll
+      for (int i = 1; i < kSub; ++i) col[i * kDiagLd] = x[i];
+    }
+    __syncthreads();
+    if (o == 0) diag_trailing<0>(a);
+    else if (o == 32) diag_trailing<32>(a);
+    else if (o == 64) diag_trailing<64>(a);
+    __syncthreads();
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-  if (lane == 0) atomicMax(lmax, __float_as_uint(vmax));
-  for (int e = tid; e < w * w; e += nt) {
-    const int r = e % w, c = e / w;
-    A[(k + r) + (k + c) * lda] = a[r * kDiagLd + c];
+  if (lane == 0 && vmax > 0.f) atomicMax(lmax, __float_as_uint(vmax));
+  for (int e = tid; e < kPanel * kPanel; e += kDiagThreads) {
+    const int r = e % kPanel, c = e / kPanel;
+    if (r < w && c < w) A[(k + r) + (k + c) * lda] = a[r * kDiagLd + c];
   }
 }
 
 // The inverses of the factored diagonal block (written back by k_lu_diag):
-// 8 CTAs, CTAs 0-3 columns 32b.. of L11^-1, CTAs 4-7 those of U11^-1, one warp
-// per column (lane l: rows l, l + 32, l + 64, l + 96), so the eight run side
-// by side on eight SMs.  L11^-1: column c starts as e_c; step j (from c on)
-// subtracts l_ij x_jc from the rows below j.  U11^-1: step j (from c down to
-// 0) divides x_jc by u_jj and subtracts u_ij x_jc from the rows above j.
-// Outputs: Linv row-major, UinvT (row n = column n of U11^-1), LinvC (both
-// column-major); zero outside w x w.
-__global__ void __launch_bounds__(1024) k_lu_diag_inv(const float* __restrict__ A, int64_t lda, int64_t k, int w,
-                                                      float* __restrict__ Linv, float* __restrict__ UinvT,
-                                                      float* __restrict__ LinvC, const int* __restrict__ status) {
+// 8 CTAs, CTA b < 4 the 32 columns 32b.. of L11^-1, CTA 4 + b those of U11^-1.
+// The 32 x 32 diagonal sub-blocks are inverted by a warp each (lane = column,
+// substitution along the rows), then the column block is filled sub-block by
+// sub-block, X_ij = -X_ii sum_k T_ik X_kj (k between j and i), as small products
+// from shared memory.  Outputs: Linv row-major, UinvT (row n = column n of
+// U11^-1), LinvC (both column-major); zero outside w x w.
+__global__ void __launch_bounds__(kInvThreads) k_lu_diag_inv(const float* __restrict__ A, int64_t lda, int64_t k,
+                                                             int w, float* __restrict__ Linv,
+                                                             float* __restrict__ UinvT, float* __restrict__ LinvC,
+                                                             const int* __restrict__ status) {
   if (*status != 0) return;   // a zero pivot: the factors are discarded
-  extern __shared__ float sm[];
-  float* a = sm;                          // [128][129] the factored block
-  float* x = sm + kPanel * kDiagLd;       // [128][33]  this CTA's 32 columns
-  constexpr int kXLd = 33;
+  extern __shared__ __align__(16) float sm[];
+  float* a = sm;                            // [128][132] the factored block
+  float* xd = a + kPanel * kDiagLd;         // [4][32][36] inverses of the diagonal sub-blocks
+  float* x = xd + kPanel * kInvLd;          // [128][36] this CTA's 32 columns
+  float* t = x + kPanel * kInvLd;           // [32][36] a product
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool upper = blockIdx.x >= 4;
-  const int c = (blockIdx.x & 3) * 32 + warp;
-  for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {
-    const int r = e % kPanel, cc = e / kPanel;
-    a[r * kDiagLd + cc] = (r < w && cc < w) ? A[(k + r) + (k + cc) * lda] : (r == cc ? 1.f : 0.f);
-  }
+  const int jb = blockIdx.x & 3;
+  load_diag(A, lda, k, w, a);
+  for (int e = tid; e < kPanel * kInvLd; e += kInvThreads) x[e] = 0.f;
   __syncthreads();
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = lane + 32 * r;
-    x[i * kXLd + warp] = (i == c && c < w) ? 1.f : 0.f;
-  }
-  __syncwarp();
-  if (c < w) {
+  if (warp < 4 && (upper ? warp <= jb : warp >= jb)) {
+    // column `lane` of the inverse of diagonal sub-block `warp`
+    const float* d = a + warp * kSub * (kDiagLd + 1);
+    const float rd = 1.f / d[lane * (kDiagLd + 1)];   // the division off the substitution's chain
+    float v[kSub];
     if (!upper) {
-      for (int j = c; j < w - 1; ++j) {
-        const float v = x[j * kXLd + warp];
-        for (int r = (j + 1) >> 5; r < 4; ++r) {
-          const int i = lane + 32 * r;
-          if (i > j && i < w) x[i * kXLd + warp] = fmaf(-a[i * kDiagLd + j], v, x[i * kXLd + warp]);
+      static_for<kSub>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < kSub; c += 4) {
+          if (c >= i) continue;
+          const float4 l = *reinterpret_cast<const float4*>(d + i * kDiagLd + c);
+          s[0] = fmaf(l.x, v[c], s[0]);
+          if (c + 1 < i) s[1] = fmaf(l.y, v[c + 1], s[1]);
+          if (c + 2 < i) s[2] = fmaf(l.z, v[c + 2], s[2]);
+          if (c + 3 < i) s[3] = fmaf(l.w, v[c + 3], s[3]);
         }
-        __syncwarp();
-      }
+        v[i] = (i == lane ? 1.f : 0.f) - ((s[0] + s[1]) + (s[2] + s[3]));
+      });
     } else {
-      for (int j = c; j >= 0; --j) {
-        const float v = x[j * kXLd + warp] / a[j * kDiagLd + j];
-        __syncwarp();
-        if (lane == (j & 31)) x[j * kXLd + warp] = v;
-        for (int r = 0; r <= (j >> 5); ++r) {
-          const int i = lane + 32 * r;
-          if (i < j) x[i * kXLd + warp] = fmaf(-a[i * kDiagLd + j], v, x[i * kXLd + warp]);
+      static_for<kSub>([&](auto ic) {
+        constexpr int i = kSub - 1 - decltype(ic)::value;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < kSub; c += 4) {
+          if (c + 3 <= i) continue;
+          const float4 u = *reinterpret_cast<const float4*>(d + i * kDiagLd + c);
+          if (c > i) s[0] = fmaf(u.x, v[c], s[0]);
+          if (c + 1 > i) s[1] = fmaf(u.y, v[c + 1], s[1]);
+          if (c + 2 > i) s[2] = fmaf(u.z, v[c + 2], s[2]);
+          if (c + 3 > i) s[3] = fmaf(u.w, v[c + 3], s[3]);
         }
-        __syncwarp();
-      }
+        v[i] = ((i == lane ? 1.f : 0.f) - ((s[0] + s[1]) + (s[2] + s[3]))) * __shfl_sync(0xffffffffu, rd, i);
+      });
+    }
+#pragma unroll
+    for (int i = 0; i < kSub; ++i) {
+      xd[(warp * kSub + i) * kInvLd + lane] = v[i];
+      if (warp == jb) x[(jb * kSub + i) * kInvLd + lane] = v[i];
     }
   }
   __syncthreads();
+  const int pr = tid >> 3, pc = (tid & 7) * 4;   // product element (pr, pc .. pc + 3)
+  for (int step = 1; step < 4; ++step) {
+    const int ib = upper ? jb - step : jb + step;
+    if (ib < 0 || ib > 3) break;                 // the same in every thread
+    const int k0 = upper ? (ib + 1) * kSub : jb * kSub, k1 = upper ? (jb + 1) * kSub : ib * kSub;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* row = a + (ib * kSub + pr) * kDiagLd;
+#pragma unroll 8
+    for (int kk = k0; kk < k1; ++kk) {
+      const float l = row[kk];
+      const float4 v = *reinterpret_cast<const float4*>(x + kk * kInvLd + pc);
+      s[0] = fmaf(l, v.x, s[0]);
+      s[1] = fmaf(l, v.y, s[1]);
+      s[2] = fmaf(l, v.z, s[2]);
+      s[3] = fmaf(l, v.w, s[3]);
+    }
+    *reinterpret_cast<float4*>(t + pr * kInvLd + pc) = make_float4(s[0], s[1], s[2], s[3]);
+    __syncthreads();
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* xrow = xd + (ib * kSub + pr) * kInvLd;
+#pragma unroll 8
+    for (int kk = 0; kk < kSub; ++kk) {
+      const float l = xrow[kk];
+      const float4 v = *reinterpret_cast<const float4*>(t + kk * kInvLd + pc);
+      y[0] = fmaf(-l, v.x, y[0]);
+      y[1] = fmaf(-l, v.y, y[1]);
+      y[2] = fmaf(-l, v.z, y[2]);
+      y[3] = fmaf(-l, v.w, y[3]);
+    }
+    *reinterpret_cast<float4*>(x + (ib * kSub + pr) * kInvLd + pc) = make_float4(y[0], y[1], y[2], y[3]);
+    __syncthreads();
+  }
   // write this CTA's 32 columns (rows 0..127)
-  const int cb = (blockIdx.x & 3) * 32;
-  for (int e = tid; e < kPanel * 32; e += blockDim.x) {
+  const int cb = jb * kSub;
+  for (int e = tid; e < kPanel * kSub; e += kInvThreads) {
     const int i = e & (kPanel - 1), cl = e >> 7;   // column-major: coalesced over i
-    const float v = x[i * kXLd + cl];
+    const float v = cb + cl < w ? x[i * kInvLd + cl] : 0.f;
     if (!upper) {
       LinvC[(cb + cl) * kPanel + i] = v;
     } else {
@@ -831,83 +974,139 @@ __global__ void __launch_bounds__(1024) k_lu_diag_inv(const float* __restrict__ 
     }
   }
   if (!upper) {
-    for (int e = tid; e < kPanel * 32; e += blockDim.x) {
+    for (int e = tid; e < kPanel * kSub; e += kInvThreads) {
       const int cl = e & 31, i = e >> 5;   // row-major rows of L11^-1: 32 consecutive columns
-      Linv[i * kPanel + cb + cl] = x[i * kXLd + cl];
+      Linv[i * kPanel + cb + cl] = cb + cl < w ? x[i * kInvLd + cl] : 0.f;
     }
   }
 }
 
 // ---------------------------------------------------------------------------
 // Triangular solves with the factors of lu_factor_tc (no permutation): one
-// cooperative kernel per factor, 128-row blocks owned cyclically by the CTAs.
-// Step b: the owner of block b turns y_b into x_b = D_b^-1 y_b with the stored
-// inverse of the diagonal block (a 128 x 128 matvec), then a grid sync, then
-// every CTA subtracts L[rows, block b] x_b (U[rows, block b] x_b) from the
-// blocks it owns below (above) block b.  The owner of the next block updated
-// that block itself, so one grid sync per block suffices.
+// cooperative kernel per factor (every CTA resident), 128-row blocks owned
+// cyclically by the CTAs, each block's right-hand side in its owner's shared
+// memory.  x_b = D_b^-1 y_b with the stored inverse of the diagonal block, then
+// y_r -= L[r, b] x_b (U[r, b] x_b) for the rows below (above).
+//
+// Bound: the chain x_b -> y_{b+1} -> x_{b+1}.  With a grid sync per block it took
+// 5.6 us a block.  Now the owner of a block publishes x_b with a flag of its own
+// (release / acquire, bounded spin) and only that chain is on the critical path:
+// a CTA has the 128 x 128 values of its next block against b, and the inverse it
+// will need, in registers before x_b arrives, updates the next block first,
+// publishes, and then sees to its other blocks.
 // ---------------------------------------------------------------------------
 struct TrsvArgs {
   const float* LU;
   int64_t lda, R;
   const float* sinv;   // per block: L^-1 column-major, then U^-1 column-major (2 x 128 x 128)
   float* y;            // right-hand side in, solution out
+  int* flag;           // nblocks words, zero on entry: x_b is in y
+  int* status;         // -1 on a timed-out wait
+  uint64_t wait_ns;
   int nblocks;
   int lower;
 };
 
 // 512 threads: row i = tid % 128 of a block, quarter h = tid / 128 of its
-// 128 columns; each thread loads its 32 matrix values before the first
-// multiply-add, so a CTA has the whole 128 x 128 block in flight at once
+// 128 columns (32 values per thread)
 constexpr int kTrsvThreads = 512;
+constexpr int kTrsvMaxSmem = 200 * 1024;   // 400 owned blocks of a CTA
 
-__global__ void __launch_bounds__(kTrsvThreads) k_trsv_tc(TrsvArgs a) {
-  cg::grid_group grid = cg::this_grid();
+__global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
+  extern __shared__ float ys[];            // [owned blocks][128]
   __shared__ float xs[kPanel];
   __shared__ float part[4][kPanel];
+  __shared__ int fail;
   const int tid = threadIdx.x, i = tid & (kPanel - 1), h = tid >> 7;
-  const int P = gridDim.x, nb = a.nblocks;
+  const int P = gridDim.x, nb = a.nblocks, p = blockIdx.x;
   const int64_t R = a.R;
-  for (int s = 0; s < nb; ++s) {
-    const int b = a.lower ? s : nb - 1 - s;
-    const int64_t r0 = (int64_t)b * kPanel;
-    const int nr = (int)min((int64_t)kPanel, R - r0);
-    if (b % P == (int)blockIdx.x) {
-      if (tid < kPanel) xs[tid] = tid < nr ? a.y[r0 + tid] : 0.f;
-      __syncthreads();
-      const float* inv = a.sinv + (int64_t)b * 2 * kPanel * kPanel + (a.lower ? 0 : kPanel * kPanel);
-      float m[32];
+  // position q of the sweep is block q (lower) or nb - 1 - q (upper); this CTA
+  // owns the positions p, p + P, ..
+  auto block_at = [&](int q) { return a.lower ? q : nb - 1 - q; };
+  auto rows_of = [&](int b) { return (int)min((int64_t)kPanel, R - (int64_t)b * kPanel); };
+  for (int q = p, o = 0; q < nb; q += P, ++o) {
+    const int b = block_at(q);
+    if (tid < kPanel) ys[o * kPanel + tid] = tid < rows_of(b) ? a.y[(int64_t)b * kPanel + tid] : 0.f;
+  }
+  if (tid == 0) fail = 0;
+  __syncthreads();
+  auto load_block = [&](int rb, int cb, float (&m)[32]) {   // rows of block rb, columns of block cb
+    const int nq = rows_of(rb), nr = rows_of(cb);
+    const float* col = a.LU + ((int64_t)rb * kPanel + i) + ((int64_t)cb * kPanel + h * 32) * a.lda;
 #pragma unroll
-      for (int q = 0; q < 32; ++q) m[q] = __ldcs(inv + (int64_t)(h * 32 + q) * kPanel + i);
-      float v = 0.f;
+    for (int c = 0; c < 32; ++c) m[c] = (i < nq && h * 32 + c < nr) ? __ldcs(col + (int64_t)c * a.lda) : 0.f;
+  };
+  // y -= m xs for the owned block o (thread (i, h) holds 32 columns of row i)
+  auto update = [&](const float (&m)[32], int o) {
+    float v = 0.f;
 #pragma unroll
-      for (int q = 0; q < 32; ++q) v = fmaf(m[q], xs[h * 32 + q], v);
-      part[h][i] = v;
-      __syncthreads();
-      if (tid < nr) a.y[r0 + tid] = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
-    }
-    grid.sync();
-    // x_b into shared memory, then the owned blocks on the far side of b
-    if (tid < kPanel) xs[tid] = tid < nr ? __ldcg(a.y + r0 + tid) : 0.f;
+    for (int c = 0; c < 32; ++c) v = fmaf(m[c], xs[h * 32 + c], v);
+    part[h][i] = v;
     __syncthreads();
-    const int first = a.lower ? b + 1 : 0, last = a.lower ? nb - 1 : b - 1;
-    int bb = first + ((int)blockIdx.x - first % P + P) % P;
-    for (; bb <= last; bb += P) {
-      const int64_t q0 = (int64_t)bb * kPanel;
-      const int nq = (int)min((int64_t)kPanel, R - q0);
-      float v = 0.f;
-      if (i < nq) {
-        const float* col = a.LU + (q0 + i) + (r0 + h * 32) * a.lda;
-        float m[32];
+    if (tid < kPanel) ys[o * kPanel + tid] -= (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+    __syncthreads();
+  };
+  float inv[32];
+  auto load_inv = [&](int b) {
+    const float* s = a.sinv + (int64_t)b * 2 * kPanel * kPanel + (a.lower ? 0 : kPanel * kPanel);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) m[c] = (h * 32 + c < nr) ? __ldcs(col + (int64_t)c * a.lda) : 0.f;
+    for (int q = 0; q < 32; ++q) inv[q] = __ldcs(s + (int64_t)(h * 32 + q) * kPanel + i);
+  };
+  // x_b from the owned block o: into y and xs, then the flag
+  auto publish = [&](int b, int o) {
+    float v = 0.f;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v = fmaf(m[c], xs[h * 32 + c], v);
+    for (int q = 0; q < 32; ++q) v = fmaf(inv[q], ys[o * kPanel + h * 32 + q], v);
+    part[h][i] = v;
+    __syncthreads();
+    if (tid < kPanel) {
+      const float xv = (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+      if (tid < rows_of(b)) __stcg(a.y + (int64_t)b * kPanel + tid, xv);
+      __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(a.flag + b), "r"(1) : "memory");
+  };
+  int mine = p, own = 0;   // this CTA's next position to solve, and its slot
+  if (mine == 0) {
+    load_inv(block_at(0));
+    publish(block_at(0), 0);
+    mine += P;
+    own = 1;
+  }
+  for (int q = 0; q < nb && mine < nb; ++q) {
+    const int b = block_at(q);
+    const bool next = mine == q + 1;
+    float m[32];
+    load_block(block_at(mine), b, m);
+    if (next) load_inv(block_at(mine));
+    if (tid == 0) {
+      const uint64_t t0 = now_ns();
+      for (;;) {
+        int f;
+        asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(f) : "l"(a.flag + b) : "memory");
+        if (f != 0) break;
+        if (now_ns() - t0 > a.wait_ns) {
+          fail = 1;
+          atomicExch(a.status, -1);
+          break;
+        }
       }
-      part[h][i] = v;
-      __syncthreads();
-      if (tid < nq) a.y[q0 + tid] -= (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
-      __syncthreads();
+    }
+    __syncthreads();
+    if (fail) return;   // the same in every thread
+    if (tid < kPanel) xs[tid] = tid < rows_of(b) ? __ldcg(a.y + (int64_t)b * kPanel + tid) : 0.f;
+    __syncthreads();
+    update(m, own);
+    int q2 = mine + P, o2 = own + 1;
+    if (next) {
+      publish(block_at(mine), own);
+      mine += P;
+      ++own;
+    }
+    for (; q2 < nb; q2 += P, ++o2) {
+      load_block(block_at(q2), b, m);
+      update(m, o2);
     }
   }
 }
@@ -1032,20 +1231,29 @@ int lu_solve_tc(const LuSetup& s, const float* rhs, float* x, cudaStream_t st) {
   t.sinv = s.sinv;
   t.y = x;
   t.nblocks = (int)ceil_div(R, kPanel);
-  // every CTA must be resident (grid syncs): at most what the SMs hold
-  static int occ = -1;
-  static int sms = 0;
-  if (occ < 0) {
-    int dev = 0;
-    RF_CUDA_TRY(cudaGetDevice(&dev));
-    RF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    RF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trsv_tc, kTrsvThreads, 0));
+  t.flag = s.ipiv;   // unused by these factors (no row exchanges); R >= nblocks words
+  t.status = s.flags + 1;
+  const int64_t lim = device_wait_limit();
+  t.wait_ns = lim < 0 ? 1000000000ull : (uint64_t)lim;
+  // every CTA must be resident (they wait for one another): at most what the SMs
+  // hold, one per SM
+  int dev = 0, sms = 0;
+  RF_CUDA_TRY(cudaGetDevice(&dev));
+  RF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int P = std::max(1, std::min(std::min(s.coop_blocks, t.nblocks), sms));
+  const size_t smem = sizeof(float) * kPanel * (size_t)ceil_div(t.nblocks, P);
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_trsv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrsvMaxSmem);
+  RF_CUDA_TRY(attr);
+  if (smem > (size_t)kTrsvMaxSmem) {
+    set_last_error_str("lu: too many row blocks per multiprocessor");
+    return RF_E_UNSUPPORTED;
   }
-  const int P = std::max(1, std::min(std::min(s.coop_blocks, t.nblocks), std::max(1, occ) * sms));
   for (int lower = 1; lower >= 0; --lower) {
     t.lower = lower;
+    RF_CUDA_TRY(cudaMemsetAsync(t.flag, 0, (size_t)t.nblocks * sizeof(int), st));
     void* args[] = {&t};
-    RF_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_tc, dim3(P), dim3(kTrsvThreads), args, 0, st));
+    RF_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_tc, dim3(P), dim3(kTrsvThreads), args, smem, st));
   }
   return RF_OK;
 }
@@ -1088,10 +1296,8 @@ int lu_factor_tc(const LuSetup& s, cudaStream_t st, bool* clean, int* launches, 
   const int64_t lim = device_wait_limit();
   const uint64_t wait_ns = lim < 0 ? 1000000000ull : (uint64_t)lim;
   static const cudaError_t diag_attr[2] = {
-      cudaFuncSetAttribute(k_lu_diag, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(kPanel * kDiagLd * sizeof(float))),
-      cudaFuncSetAttribute(k_lu_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)((kPanel * kDiagLd + kPanel * 33) * sizeof(float)))};
+      cudaFuncSetAttribute(k_lu_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem),
+      cudaFuncSetAttribute(k_lu_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagInvSmem)};
   RF_CUDA_TRY(diag_attr[0]);
   RF_CUDA_TRY(diag_attr[1]);
   int nl = 0;
@@ -1107,9 +1313,9 @@ int lu_factor_tc(const LuSetup& s, cudaStream_t st, bool* clean, int* launches, 
   // factor the panel at column k (width w): diagonal block, then L21 for rows
   // k + w .. R into the matrix and into LT columns lt_col .. lt_col + 128
   auto panel = [&](int64_t k, int w, int lt_col) -> int {
-    k_lu_diag<<<1, 1024, kPanel * kDiagLd * sizeof(float), st>>>(s.LU, lda, k, w, lmax, status);
+    k_lu_diag<<<1, kDiagThreads, kDiagSmem, st>>>(s.LU, lda, k, w, lmax, status);
     RF_LAUNCH_CHECK();
-    k_lu_diag_inv<<<8, 1024, (kPanel * kDiagLd + kPanel * 33) * sizeof(float), st>>>(
+    k_lu_diag_inv<<<8, kInvThreads, kDiagInvSmem, st>>>(
         s.LU, lda, k, w, Linv, UinvT, s.sinv + (k / kPanel) * 2 * kPanel * kPanel, status);
     RF_LAUNCH_CHECK();
     ++nl;

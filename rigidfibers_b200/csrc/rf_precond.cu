@@ -29,13 +29,18 @@ constexpr int kNfNQ32 = (kNfM + 1) * (kNfM + 1) * 6;
 constexpr int kNfStride = 16;                 // floats per column of a fiber's stored rows
 
 // k nearest fibers of fiber i (centre distance, ties by index): nb[i][0] = i,
-// nb[i][1..k]; slots past N - 1 neighbours hold -1.  One thread per fiber,
-// the centres streamed through shared memory.
-__global__ void __launch_bounds__(128) k_nf_neighbours(const float4* __restrict__ pos, int N, int k,
-                                                       int* __restrict__ nb) {
+// nb[i][1..k] in order; slots past N - 1 neighbours (or without one: non-finite
+// centres) hold i.  One warp per fiber: every lane keeps the nearest of its 32nd
+// of the centres (streamed through shared memory), then k rounds take the warp's
+// nearest head.  N=4000: 780 us with a thread per fiber.
+constexpr int kNfWarps = 8;
+
+__global__ void __launch_bounds__(kNfWarps * 32) k_nf_neighbours(const float4* __restrict__ pos, int N, int k,
+                                                                 int* __restrict__ nb) {
   constexpr int kChunk = 1024;
   __shared__ float4 sp[kChunk];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int i = (int)blockIdx.x * kNfWarps + (int)(threadIdx.x >> 5);
   float bd[kNfMaxNeighbours];
   int bi[kNfMaxNeighbours];
 #pragma unroll
@@ -49,131 +54,166 @@ __global__ void __launch_bounds__(128) k_nf_neighbours(const float4* __restrict_
     __syncthreads();
     for (int u = threadIdx.x; u < cn; u += blockDim.x) sp[u] = pos[c0 + u];
     __syncthreads();
-    if (i < N) {
-      for (int u = 0; u < cn; ++u) {
-        const int j = c0 + u;
-        if (j == i) continue;
-        const float dx = sp[u].x - pi.x, dy = sp[u].y - pi.y, dz = sp[u].z - pi.z;
-        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        // insertion into the sorted list (the last slot in use is k - 1)
-        if (d2 < bd[k - 1] || (d2 == bd[k - 1] && j < bi[k - 1])) {
-          int s = k - 1;
+    for (int u = lane; u < cn; u += 32) {
+      const int j = c0 + u;
+      const float dx = sp[u].x - pi.x, dy = sp[u].y - pi.y, dz = sp[u].z - pi.z;
+      const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      if (j != i && d2 < bd[kNfMaxNeighbours - 1]) {
+        // insertion into the sorted list (a lane meets its candidates in index order)
+        float d = d2;
+        int id = j;
 #pragma unroll
-          for (int t = kNfMaxNeighbours - 1; t > 0; --t) {
-            if (t <= s && (bd[t - 1] > d2 || (bd[t - 1] == d2 && bi[t - 1] > j))) {
-              bd[t] = bd[t - 1];
-              bi[t] = bi[t - 1];
-              s = t - 1;
-            }
+        for (int t = 0; t < kNfMaxNeighbours; ++t) {
+          if (d < bd[t]) {
+            const float td = bd[t];
+            const int ti = bi[t];
+            bd[t] = d;
+            bi[t] = id;
+            d = td;
+            id = ti;
           }
-          bd[s] = d2;
-          bi[s] = j;
         }
       }
     }
   }
-  if (i < N) {
-    nb[(int64_t)i * (k + 1)] = i;
-    for (int s = 0; s < k; ++s) nb[(int64_t)i * (k + 1) + 1 + s] = bi[s];
+  if (i >= N) return;
+  if (lane == 0) nb[(int64_t)i * (k + 1)] = i;
+  for (int s = 0; s < k; ++s) {
+    float d = bd[0];
+    int id = bi[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float od = __shfl_xor_sync(0xffffffffu, d, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, id, o);
+      if (oi >= 0 && (id < 0 || od < d || (od == d && oi < id))) {
+        d = od;
+        id = oi;
+      }
+    }
+    if (lane == 0) nb[(int64_t)i * (k + 1) + 1 + s] = id >= 0 ? id : i;
+    if (id >= 0 && bi[0] == id) {   // the lane that had it moves on
+#pragma unroll
+      for (int t = 0; t + 1 < kNfMaxNeighbours; ++t) {
+        bd[t] = bd[t + 1];
+        bi[t] = bi[t + 1];
+      }
+      bd[kNfMaxNeighbours - 1] = 3.0e38f;
+      bi[kNfMaxNeighbours - 1] = -1;
+    }
   }
-}
-
-// S (the symmetric 3x3 component c) of T^{pq}[kp][kq] for fibers p != q with
-// kp p's force term: the record of the unordered pair, transposed when p > q
-__device__ __forceinline__ float nf_block(const float* __restrict__ S32, int p, int q, int kp, int kq, int c) {
-  const int a = min(p, q), b = max(p, q);
-  const int ka = p < q ? kp : kq, kb = p < q ? kq : kp;
-  const int I = a / 8, J = b / 8;
-  const int64_t I16 = I / 2, J16 = J / 2;
-  const int sub = (I % 2) * 2 + (J % 2);
-  const int64_t L16 = J16 * (J16 + 1) / 2 + I16;
-  const int64_t rec = (L16 * 4 + sub) * 8 + (b % 8);
-  return S32[(rec * kNfNQ32 + (ka * kNfM + kb) * 6 + c) * 8 + (a % 8)];
-}
-
-__device__ __forceinline__ int sym_index(int d, int e) {
-  // (11, 22, 33, 12, 13, 23)
-  if (d == e) return d;
-  const int lo = min(d, e), hi = max(d, e);
-  return lo == 0 ? (hi == 1 ? 3 : 4) : 5;
 }
 
 // One CTA per fiber i: Gauss-Jordan elimination without row exchanges on
 // [B_i^T | E] (E: the first 15 columns of the identity), so that the right
 // part ends as the transpose of fiber i's rows of B_i^-1; those rows go to
 // W[i] as [column c][row r] (kNfStride floats per column).  A pivot below
-// 1e-6 in magnitude or a non-finite entry leaves fiber i unpreconditioned
-// (its rows of the identity).
-__global__ void __launch_bounds__(256) k_nf_setup(const Tables tab, int N, int k, const float4* __restrict__ ori,
-                                                  const float* __restrict__ S32, const int* __restrict__ nb,
-                                                  float* __restrict__ W) {
-  extern __shared__ float nsm[];
-  const int i = blockIdx.x;
-  const int kk = min(k, N - 1);
-  const int n = (kk + 1) * kNfM3;            // rows of B_i
-  const int ld = n + kNfM3;                  // [B^T | E] row length
-  float* aug = nsm;                          // n x ld
-  float* fcol = nsm + (size_t)n * ld;        // n: the pivot column
-  __shared__ int snb[kNfMaxNeighbours + 1];
-  __shared__ float4 st[kNfMaxNeighbours + 1];
-  __shared__ int bad;
-  if (threadIdx.x <= kk) {
-    snb[threadIdx.x] = nb[(int64_t)i * (k + 1) + threadIdx.x];
-    st[threadIdx.x] = ori[snb[threadIdx.x]];
-  }
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
-  // aug[r][c] = B(c, r) for c < n; B(row of fiber a, term ka, comp d;
-  // column of fiber b, term kb, comp e) = delta when a == b, else
-  // [C_{a,ka} S^{ab}_{ka,kb}]_{d,e}, C_k(S) = k == 0 ? g t (t^T S) : g (S - E t (t^T S))
-  for (int u = threadIdx.x; u < n * n; u += blockDim.x) {
-    const int r = u / n, c = u % n;          // aug row r (a column of B), aug column c (a row of B)
-    const int la = c / kNfM3, lb = r / kNfM3;
-    const int ka = (c % kNfM3) / 3, d = c % 3, kb = (r % kNfM3) / 3, e = r % 3;
-    float v;
-    if (la == lb) {
-      v = (ka == kb && d == e) ? 1.f : 0.f;
-    } else {
-      const int a = snb[la], b = snb[lb];
-      const float4 t = st[la];
-      const float t3[3] = {t.x, t.y, t.z};
-      // (t^T S)_e and S_de of the symmetric block
-      float tS = 0.f;
+// 1e-6 in magnitude or a non-finite one leaves fiber i unpreconditioned (its
+// rows of the identity).
+//
+// Thread = column, its n entries in registers.  A step needs one column of
+// multipliers (published by its thread, read as 16-byte broadcasts) and one
+// barrier; the rows rotate by one per step, so the pivot row is always entry 0,
+// the loop over the steps is not unrolled and the register indexes are
+// constants.  After n steps the rows are back in order.  N=4000, k = 4: 3.63 ms
+// with the block in shared memory and a flat index over its entries.
+template <int KK>
+struct NfShape {
+  static constexpr int n = (KK + 1) * kNfM3;               // rows of B_i
+  static constexpr int NT = (n + kNfM3 + 1 + 31) / 32 * 32;   // columns of [B^T | E], one more for the padding
+  static constexpr int n4 = (n + 3) / 4 * 4;
+};
+
+template <int KK>
+__global__ void __launch_bounds__(NfShape<KK>::NT)
+k_nf_setup(const Tables tab, int k, const float4* __restrict__ ori, const float* __restrict__ S32,
+           const int* __restrict__ nb, float* __restrict__ W) {
+  using S = NfShape<KK>;
+  constexpr int n = S::n, n4 = S::n4;
+  __shared__ __align__(16) float mult[2][n4];   // the pivot column, by turns
+  const int i = blockIdx.x, c = threadIdx.x;
+  float col[n4];                                // col[r] = [B^T | E][r][c]
 #pragma unroll
-      for (int f = 0; f < 3; ++f) tS = fmaf(t3[f], nf_block(S32, a, b, ka, kb, sym_index(f, e)), tS);
-      const float Sde = nf_block(S32, a, b, ka, kb, sym_index(d, e));
-      const float g = tab.gamma[ka];
-      v = ka == 0 ? g * t3[d] * tS : g * (Sde - tab.eigen[ka] * t3[d] * tS);
+  for (int r = 0; r < n4; ++r) col[r] = 0.f;
+  if (c < n) {
+    // row c of B: fiber a, term ka, component d.  B(row; column of fiber b, term kb,
+    // component e) = delta when a == b, else [C_{a,ka} S^{ab}_{ka,kb}]_{d,e},
+    // C_k(S) = k == 0 ? g t (t^T S) : g (S - E t (t^T S)); S the stored symmetric
+    // block of the unordered pair (p, q), p < q (kp p's term): record
+    // ((L16 * 4 + sub) * 8 + q % 8), value ((kp M + kq) 6 + component) of pair p % 8
+    const int la = c / kNfM3, ka = (c % kNfM3) / 3, d = c % 3;
+    const int a = nb[(int64_t)i * (k + 1) + la];
+    const float4 t4 = ori[a];
+    const float t3[3] = {t4.x, t4.y, t4.z};
+    const float td = d == 0 ? t3[0] : d == 1 ? t3[1] : t3[2];
+    const float g = tab.gamma[ka], E = tab.eigen[ka];
+#pragma unroll
+    for (int lb = 0; lb <= KK; ++lb) {
+      const int b = nb[(int64_t)i * (k + 1) + lb];
+      const int p = min(a, b), q = max(a, b);
+      const int I = p / 8, J = q / 8;
+      const int64_t L16 = (int64_t)(J / 2) * (J / 2 + 1) / 2 + I / 2;
+      const int64_t rec = (L16 * 4 + (I % 2) * 2 + (J % 2)) * 8 + (q % 8);
+      const float* base = S32 + rec * (kNfNQ32 * 8) + (p % 8);
+#pragma unroll
+      for (int kb = 0; kb < kNfM; ++kb) {
+        float s[6];
+#pragma unroll
+        for (int e = 0; e < 6; ++e)
+          s[e] = lb == la ? 0.f : base[((a < b ? ka * kNfM + kb : kb * kNfM + ka) * 6 + e) * 8];
+        // rows of S and t^T S
+        const float S3[3][3] = {{s[0], s[3], s[4]}, {s[3], s[1], s[5]}, {s[4], s[5], s[2]}};
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          const float tS = fmaf(t3[2], S3[2][e], fmaf(t3[1], S3[1][e], t3[0] * S3[0][e]));
+          const float Sde = d == 0 ? S3[0][e] : d == 1 ? S3[1][e] : S3[2][e];
+          const float v = ka == 0 ? g * td * tS : g * (Sde - E * td * tS);
+          col[lb * kNfM3 + kb * 3 + e] = lb == la ? (kb == ka && e == d ? 1.f : 0.f) : v;
+        }
+      }
     }
-    aug[(size_t)r * ld + c] = v;
+  } else {
+    // column c - n of E
+#pragma unroll
+    for (int r = 0; r < kNfM3; ++r) col[r] = c - n == r ? 1.f : 0.f;
   }
-  for (int u = threadIdx.x; u < n * kNfM3; u += blockDim.x) {
-    const int r = u / kNfM3, c = u % kNfM3;
-    aug[(size_t)r * ld + n + c] = r == c ? 1.f : 0.f;
+  if (c == 0) {
+#pragma unroll
+    for (int r = 0; r < n4; r += 4)
+      *reinterpret_cast<float4*>(&mult[0][r]) = make_float4(col[r], col[r + 1], col[r + 2], col[r + 3]);
   }
   __syncthreads();
+  bool bad = false;
   for (int piv = 0; piv < n; ++piv) {
-    const float p = aug[(size_t)piv * ld + piv];
-    if (threadIdx.x == 0 && (!(fabsf(p) >= 1e-6f) || !isfinite(p))) bad = 1;
-    __syncthreads();
-    if (bad) break;
-    const float inv = 1.f / p;
-    for (int c = threadIdx.x; c < ld; c += blockDim.x) aug[(size_t)piv * ld + c] *= inv;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) fcol[r] = aug[(size_t)r * ld + piv];
-    __syncthreads();
-    for (int u = threadIdx.x; u < n * ld; u += blockDim.x) {
-      const int r = u / ld, c = u % ld;
-      if (r != piv) aug[u] = fmaf(-fcol[r], aug[(size_t)piv * ld + c], aug[u]);
+    const float* m = mult[piv & 1];
+    const float p = m[0];
+    if (!(fabsf(p) >= 1e-6f) || !isfinite(p)) {   // the same in every thread
+      bad = true;
+      break;
+    }
+    const float u = col[0] * (1.f / p);
+#pragma unroll
+    for (int r = 0; r < n; r += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(m + r);
+      if (r > 0) col[r - 1] = fmaf(-v.x, u, col[r]);
+      if (r + 1 < n) col[r] = fmaf(-v.y, u, col[r + 1]);
+      if (r + 2 < n) col[r + 1] = fmaf(-v.z, u, col[r + 2]);
+      if (r + 3 < n) col[r + 2] = fmaf(-v.w, u, col[r + 3]);
+    }
+    col[n - 1] = u;
+    if (c == piv + 1) {
+#pragma unroll
+      for (int r = 0; r < n4; r += 4)
+        *reinterpret_cast<float4*>(&mult[(piv + 1) & 1][r]) =
+            make_float4(col[r], col[r + 1], col[r + 2], col[r + 3]);
     }
     __syncthreads();
   }
-  // W[i][c][r] = (B^-1)[r][c] = X[c][r], X the right part of aug
-  float* wi = W + (size_t)i * (kNfMaxNeighbours + 1) * kNfM3 * kNfStride;
-  for (int u = threadIdx.x; u < n * kNfStride; u += blockDim.x) {
-    const int c = u / kNfStride, r = u % kNfStride;
-    float v = 0.f;
-    if (r < kNfM3) v = bad ? (c == r ? 1.f : 0.f) : aug[(size_t)c * ld + n + r];
-    wi[u] = v;
+  // W[i][r][e] = (B^-1)[e][r] = X[r][e]: column n + e of the eliminated system
+  const int e = c - n;
+  if (e >= 0 && e < kNfStride) {
+    float* wi = W + (size_t)i * (kNfMaxNeighbours + 1) * kNfM3 * kNfStride;
+#pragma unroll
+    for (int r = 0; r < n; ++r) wi[r * kNfStride + e] = e >= kNfM3 ? 0.f : bad ? (r == e ? 1.f : 0.f) : col[r];
   }
 }
 
@@ -205,13 +245,15 @@ int64_t nf_w_floats(int N) { return (int64_t)N * (kNfMaxNeighbours + 1) * kNfM3 
 int launch_nf_setup(const Tables& tab, int N, int k, const float4* pos, const float4* ori, const float* S32, int* nb,
                     float* W, cudaStream_t st) {
   if (tab.M != kNfM || k < 1 || k > kNfMaxNeighbours || N < 1) return RF_E_UNSUPPORTED;
-  k_nf_neighbours<<<(unsigned)ceil_div(N, 128), 128, 0, st>>>(pos, N, k, nb);
+  k_nf_neighbours<<<(unsigned)ceil_div(N, kNfWarps), kNfWarps * 32, 0, st>>>(pos, N, k, nb);
   RF_LAUNCH_CHECK();
-  const int kk = std::min(k, N - 1);
-  const int n = (kk + 1) * kNfM3;
-  const size_t smem = sizeof(float) * ((size_t)n * (n + kNfM3) + n);
-  RF_CUDA_TRY(cudaFuncSetAttribute(k_nf_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_nf_setup<<<(unsigned)N, 256, smem, st>>>(tab, N, k, ori, S32, nb, W);
+  switch (std::min(k, N - 1)) {
+#define RF_NF_CASE(KK)                                                                                     \
+  case KK: k_nf_setup<KK><<<(unsigned)N, NfShape<KK>::NT, 0, st>>>(tab, k, ori, S32, nb, W); break;
+    RF_NF_CASE(0) RF_NF_CASE(1) RF_NF_CASE(2) RF_NF_CASE(3) RF_NF_CASE(4)
+    RF_NF_CASE(5) RF_NF_CASE(6) RF_NF_CASE(7) RF_NF_CASE(8)
+#undef RF_NF_CASE
+  }
   RF_LAUNCH_CHECK();
   return RF_OK;
 }

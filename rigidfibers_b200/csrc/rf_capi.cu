@@ -410,7 +410,7 @@ struct rf_handle {
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     int state = 0;
-    int pre_kernels = 0, cycle_kernels = 0, post_kernels = 0;
+    int pre_kernels = 0, cycle_kernels = 0, step_kernels = 0, post_kernels = 0;   // step: one Arnoldi step
   } step_graph[2];
   bool use_graphs = true;         // GMRES restart cycles from graphs
   bool use_step_graphs = true;    // rf_step as one graph
@@ -1092,42 +1092,64 @@ static bool step_graph_eligible(const rf_handle* h) {
          h->cfg.solver == RF_SOLVER_GMRES;
 }
 
-// Capture one stream segment into a graph (nothing runs during the capture).
-static int capture_segment(cudaStream_t st, const std::function<int()>& fn, cudaGraph_t* out) {
-  *out = nullptr;
-  if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+// Arnoldi steps per conditional node of a step graph.  A step that converged
+// earlier costs its launches (three of ~2.2 us, mixed modes), an IF node a few
+// microseconds whether its body runs or not.
+constexpr int kStepChunk = 4;
+
+// Capture fn's work on st into `graph` (nothing runs during the capture).
+static int capture_into(cudaStream_t st, cudaGraph_t graph, const std::function<int()>& fn) {
+  if (cudaStreamBeginCaptureToGraph(st, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     cudaGetLastError();
     return RF_E_CUDA;
   }
   int rc = fn();
   cudaGraph_t g = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(st, &g);
-  if (rc == RF_OK && (e != cudaSuccess || !g)) rc = RF_E_CUDA;
-  if (rc != RF_OK) {
-    if (g) cudaGraphDestroy(g);
-    cudaGetLastError();
-    return rc;
-  }
-  *out = g;
+  const cudaError_t e = cudaStreamEndCapture(st, &g);   // g == graph
+  if (rc == RF_OK && (e != cudaSuccess || g != graph)) rc = RF_E_CUDA;
+  if (rc != RF_OK) cudaGetLastError();
+  return rc;
+}
+
+// A conditional node after everything st has captured so far; *body receives its
+// (empty) body graph, to be filled once the capture of the enclosing graph ends.
+static int capture_conditional(cudaStream_t st, cudaGraphConditionalHandle handle, cudaGraphConditionalNodeType type,
+                               cudaGraph_t* body) {
+  cudaStreamCaptureStatus status;
+  cudaGraph_t graph = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  RF_CUDA_TRY(cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &ndeps));
+  if (status != cudaStreamCaptureStatusActive) return RF_E_CUDA;
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = handle;
+  cp.conditional.type = type;
+  cp.conditional.size = 1;
+  cudaGraphNode_t node;
+  RF_CUDA_TRY(cudaGraphAddNode(&node, graph, deps, ndeps, &cp));
+  RF_CUDA_TRY(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+  *body = cp.conditional.phGraph_out[0];
   return RF_OK;
 }
 
-// The step graph: [assembly, first GMRES cycle, loop condition] ->
-// WHILE(condition) { later cycle, loop condition } -> [solution cast,
-// velocities, fiber update].  The WHILE node runs the restart cycles on the
-// device, so a step is one graph launch and one read of the control block.
+// The step graph: [assembly, opening of the solve, first restart cycle, loop
+// condition] -> WHILE(condition) { later cycle, loop condition } -> [solution cast,
+// velocities, fiber update].  The restart cycles run on the device, so a step
+// is one graph launch and one read of the control block.  A cycle's Arnoldi
+// steps come in chunks, each inside the IF node that the one before it sets, so
+// the steps after convergence are not launched.
 static int build_step_graph(rf_handle* h, int first_step, rf_handle::StepGraph* sg) {
-  cudaGraph_t G = nullptr, pre = nullptr, body = nullptr, post = nullptr;
+  cudaGraph_t G = nullptr;
   auto fail = [&](int rc) {
-    for (cudaGraph_t g : {pre, body, post, G})
-      if (g) cudaGraphDestroy(g);
+    if (G) cudaGraphDestroy(G);
     cudaGetLastError();
     sg->state = -1;
     return rc;
   };
   if (cudaGraphCreate(&G, 0) != cudaSuccess) return fail(RF_E_CUDA);
-  cudaGraphConditionalHandle cond;
-  if (cudaGraphConditionalHandleCreate(&cond, G, 1, cudaGraphCondAssignDefault) != cudaSuccess)
+  cudaGraphConditionalHandle loop;
+  if (cudaGraphConditionalHandleCreate(&loop, G, 1, cudaGraphCondAssignDefault) != cudaSuccess)
     return fail(RF_E_CUDA);
   GmresSetup s = gmres_setup(h);
   s.graphs = nullptr;
@@ -1136,42 +1158,60 @@ static int build_step_graph(rf_handle* h, int first_step, rf_handle::StepGraph* 
   ResidualFn resid = h->mixed ? make_residual(h) : ResidualFn();
   void* xsol = h->mixed ? static_cast<void*>(h->x64) : static_cast<void*>(h->x);
   int kpre = 2, kcycle = 0, kpost = 1;
-  int rc = capture_segment(h->st, [&]() -> int {
+  // the chunk of steps from j0 into the graph under capture; what follows it in
+  // *rest (an IF node's body) for later
+  struct Rest {
+    cudaGraph_t graph;
+    int j0;
+  };
+  std::vector<Rest> rest;
+  auto chunk = [&](cudaGraph_t graph, int j0) -> int {
+    const int j1 = std::min(s.m, j0 + kStepChunk);
+    cudaGraphConditionalHandle more = 0;
+    if (j1 < s.m) RF_CUDA_TRY(cudaGraphConditionalHandleCreate(&more, graph, 0, cudaGraphCondAssignDefault));
+    RF_TRY(gmres_enqueue_steps(s, mv, h->b, xsol, h->mixed, j0, j1, more, h->st));
+    if (j1 < s.m) {
+      cudaGraph_t body = nullptr;
+      RF_TRY(capture_conditional(h->st, more, cudaGraphCondTypeIf, &body));
+      rest.push_back({body, j1});
+    }
+    return RF_OK;
+  };
+  cudaGraph_t later = nullptr;
+  int rc = capture_into(h->st, G, [&]() -> int {
     RF_TRY(enqueue_assemble(h));
-    return gmres_enqueue_first(s, mv, resid, h->b, xsol, h->mixed, cond, h->st, &kpre);
-  }, &pre);
-  if (rc) return fail(rc);
-  kpre += mvk;
-  mvk = 0;
-  rc = capture_segment(h->st, [&]() -> int {
-    return gmres_enqueue_cycle(s, mv, resid, h->b, xsol, h->mixed, cond, h->st, &kcycle);
-  }, &body);
-  if (rc) return fail(rc);
-  kcycle += mvk + (h->mixed ? (h->recompute ? 3 : 2) : 0);   // the FP64 residual's kernels
-  rc = capture_segment(h->st, [&]() -> int {
+    RF_TRY(gmres_enqueue_first(s, h->b, xsol, h->mixed, h->st, &kpre));
+    RF_TRY(chunk(G, 0));
+    RF_TRY(gmres_enqueue_tail(s, h->b, xsol, h->mixed, loop, h->st, &kpre));
+    RF_TRY(capture_conditional(h->st, loop, cudaGraphCondTypeWhile, &later));
     if (h->mixed) {
       RF_TRY(launch_cast_to_float(h->x64, h->x, h->R, h->st));
       ++kpost;
     }
     RF_TRY(enqueue_velocities(h, &kpost));
     return enqueue_update_fibers(h, first_step, &h->ctl->halt);
-  }, &post);
+  });
   if (rc) return fail(rc);
-  cudaGraphNode_t npre, ncond, nbody, npost;
-  cudaGraphNodeParams cp = {};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = cond;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  if (cudaGraphAddChildGraphNode(&npre, G, nullptr, 0, pre) != cudaSuccess ||
-      cudaGraphAddNode(&ncond, G, &npre, 1, &cp) != cudaSuccess ||
-      cudaGraphAddChildGraphNode(&nbody, cp.conditional.phGraph_out[0], nullptr, 0, body) != cudaSuccess ||
-      cudaGraphAddChildGraphNode(&npost, G, &ncond, 1, post) != cudaSuccess ||
-      cudaGraphInstantiate(&sg->exec, G, 0) != cudaSuccess) {
+  sg->step_kernels = mvk / std::min(s.m, kStepChunk) + 1;
+  mvk = 0;
+  rc = capture_into(h->st, later, [&]() -> int {
+    RF_TRY(gmres_enqueue_head(s, mv, resid, h->b, xsol, h->mixed, h->st, &kcycle));
+    kcycle += mvk;
+    RF_TRY(chunk(later, 0));
+    return gmres_enqueue_tail(s, h->b, xsol, h->mixed, loop, h->st, &kcycle);
+  });
+  if (rc) return fail(rc);
+  kcycle += h->mixed ? (h->recompute ? 3 : 2) : 0;   // the FP64 residual's kernels
+  for (size_t k = 0; k < rest.size(); ++k) {          // grows while it is walked
+    const Rest r = rest[k];
+    rc = capture_into(h->st, r.graph, [&]() { return chunk(r.graph, r.j0); });
+    if (rc) return fail(rc);
+  }
+  if (cudaGraphInstantiate(&sg->exec, G, 0) != cudaSuccess) {
     sg->exec = nullptr;
     return fail(RF_E_CUDA);
   }
-  for (cudaGraph_t g : {pre, body, post, G}) cudaGraphDestroy(g);
+  cudaGraphDestroy(G);
   sg->pre_kernels = kpre;
   sg->cycle_kernels = kcycle;
   sg->post_kernels = kpost;
@@ -1217,7 +1257,7 @@ static int run_step_graph(rf_handle* h, const rf_handle::StepGraph& g) {
   const GmresCtl c = *h->host_ctl;
   GmresResult res;
   const int rc = gmres_result_from_ctl(c, h->mixed, &res);
-  h->launches = g.pre_kernels + c.heads * g.cycle_kernels + g.post_kernels;
+  h->launches = g.pre_kernels + c.heads * g.cycle_kernels + c.launched * g.step_kernels + g.post_kernels;
   h->matvecs_done = res.matvecs;
   h->mv_used = 0;
   h->refinements = h->mixed ? res.residual_calls : 0;

@@ -331,10 +331,17 @@ __global__ void __launch_bounds__(kKrylovThreads) k_gmres_residual(GmresArgs a, 
 // pass's own reduction (recomputed from w when that cancels), so a step has two
 // grid syncs.  N=4000, one B200: 40 us with 59 blocks of serial partial sums.
 // NVB: V entries kept per thread (a multiple of 16, at least j + 2 with ||w'||^2).
+// more: a graph condition that receives whether the cycle goes on (0: none).
 template <int NVB, bool ONE>
-__global__ void __launch_bounds__(kKrylovThreads) k_gmres_arnoldi(GmresArgs a, int j) {
+__global__ void __launch_bounds__(kKrylovThreads)
+k_gmres_arnoldi(GmresArgs a, int j, cudaGraphConditionalHandle more) {
   cg::grid_group grid = cg::this_grid();
-  if (a.ctl->cycle_done) return;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  if (lead) a.ctl->launched += 1;
+  if (a.ctl->cycle_done) {
+    if (lead && more) cudaGraphSetConditional(more, 0);
+    return;
+  }
   constexpr int NG = NVB / 16;
   __shared__ double red[NG][kKrylovWarps][16];
   __shared__ double h[NVB], h2[NVB], rot[2][kMaxRestart];
@@ -444,7 +451,7 @@ __global__ void __launch_bounds__(kKrylovThreads) k_gmres_arnoldi(GmresArgs a, i
   if constexpr (ONE) {
     if (r0 < a.R) w[r0] = wr;
   }
-  if (blockIdx.x == 0 && tid == 0) {
+  if (lead) {
     const double nrm = sqrt(nrm2);
     double* Hc = a.H + (int64_t)j * (a.m + 1);
     double top = h[0] + h2[0];
@@ -470,8 +477,9 @@ __global__ void __launch_bounds__(kKrylovThreads) k_gmres_arnoldi(GmresArgs a, i
     ctl->estimate = est;
     const bool bad = !isfinite(est);
     if (bad) ctl->nan = 1;
-    if (bad || est <= ctl->tol * ctl->bnorm || j + 1 >= a.m || total >= ctl->maxit || nrm == 0.0)
-      ctl->cycle_done = 1;
+    const bool done = bad || est <= ctl->tol * ctl->bnorm || j + 1 >= a.m || total >= ctl->maxit || nrm == 0.0;
+    if (done) ctl->cycle_done = 1;
+    if (more) cudaGraphSetConditional(more, done ? 0u : 1u);
   }
 }
 
@@ -587,7 +595,7 @@ static int launch_residual(GmresArgs& a, int mode, int nblk, cudaStream_t st) {
 
 // Arnoldi step j.  ONE where the grid has a thread per row; NVB by the values of
 // the second pass (j + 1 dots and the norm).
-static int launch_arnoldi(GmresArgs& a, int j, int nblk, cudaStream_t st) {
+static int launch_arnoldi(GmresArgs& a, int j, int nblk, cudaStream_t st, cudaGraphConditionalHandle more = 0) {
   const bool one = (int64_t)nblk * kKrylovThreads >= a.R;
   const void* fn = nullptr;
   switch ((j + 2 + 15) / 16) {
@@ -596,7 +604,7 @@ static int launch_arnoldi(GmresArgs& a, int j, int nblk, cudaStream_t st) {
     case 3: fn = one ? (const void*)k_gmres_arnoldi<48, true> : (const void*)k_gmres_arnoldi<48, false>; break;
     default: fn = one ? (const void*)k_gmres_arnoldi<80, true> : (const void*)k_gmres_arnoldi<80, false>; break;
   }
-  void* args[] = {&a, &j};
+  void* args[] = {&a, &j, &more};
   return coop_launch(fn, nblk, kKrylovThreads, args, st);
 }
 
@@ -762,51 +770,46 @@ __global__ void k_gmres_loop_cond(cudaGraphConditionalHandle cond, GmresCtl* ctl
   cudaGraphSetConditional(cond, more ? 1u : 0u);
 }
 
-// m x (matvec + Arnoldi step) of the cycle whose first basis vector is in V[0]
-static int enqueue_arnoldi_steps(const GmresSetup& s, GmresArgs& a, const MatvecFn& matvec, cudaStream_t st,
-                                 int* kernels) {
-  for (int j = 0; j < s.m; ++j) {
-    int rc = matvec(s.V + (int64_t)j * s.ldv, &s.ctl->cycle_done, st);
-    if (rc) return rc;
-    rc = launch_arnoldi(a, j, s.coop_blocks, st);
-    if (rc) return rc;
-    *kernels += 1;
-  }
-  k_gmres_update<<<s.coop_blocks, kKrylovThreads, 0, st>>>(a);
-  RF_LAUNCH_CHECK();
-  *kernels += 1;
-  return RF_OK;
-}
-
-int gmres_enqueue_first(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn& residual, const float* b,
-                        void* x, bool x_double, cudaGraphConditionalHandle cond, cudaStream_t st, int* kernels) {
+int gmres_enqueue_first(const GmresSetup& s, const float* b, void* x, bool x_double, cudaStream_t st, int* kernels) {
   if (s.m < 1 || s.m > kMaxRestart) {
     set_last_error_str("gmres: restart length out of range");
     return RF_E_INPUT;
   }
   GmresArgs a = gmres_args(s, b, x, x_double);
-  if (int rc = launch_residual(a, 0, s.coop_blocks, st)) return rc;
   *kernels += 1;
-  if (int rc = enqueue_arnoldi_steps(s, a, matvec, st, kernels)) return rc;
-  k_gmres_loop_cond<<<1, 1, 0, st>>>(cond, s.ctl);
-  RF_LAUNCH_CHECK();
-  *kernels += 1;
-  (void)residual;
-  return RF_OK;
+  return launch_residual(a, 0, s.coop_blocks, st);
 }
 
-int gmres_enqueue_cycle(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn& residual, const float* b,
-                        void* x, bool x_double, cudaGraphConditionalHandle cond, cudaStream_t st, int* kernels) {
+int gmres_enqueue_head(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn& residual, const float* b, void* x,
+                       bool x_double, cudaStream_t st, int* kernels) {
   GmresArgs a = gmres_args(s, b, x, x_double);
   const int rc0 = residual ? residual(x, s.V, &s.ctl->converged, st)
                            : matvec(static_cast<const float*>(x), &s.ctl->converged, st);
   if (rc0) return rc0;
-  if (int rc = launch_residual(a, residual ? 2 : 1, s.coop_blocks, st)) return rc;
   *kernels += 1;
-  if (int rc = enqueue_arnoldi_steps(s, a, matvec, st, kernels)) return rc;
+  return launch_residual(a, residual ? 2 : 1, s.coop_blocks, st);
+}
+
+int gmres_enqueue_steps(const GmresSetup& s, const MatvecFn& matvec, const float* b, void* x, bool x_double, int j0,
+                        int j1, cudaGraphConditionalHandle more, cudaStream_t st) {
+  GmresArgs a = gmres_args(s, b, x, x_double);
+  for (int j = j0; j < j1; ++j) {
+    int rc = matvec(s.V + (int64_t)j * s.ldv, &s.ctl->cycle_done, st);
+    if (rc) return rc;
+    rc = launch_arnoldi(a, j, s.coop_blocks, st, j + 1 == j1 ? more : 0);
+    if (rc) return rc;
+  }
+  return RF_OK;
+}
+
+int gmres_enqueue_tail(const GmresSetup& s, const float* b, void* x, bool x_double, cudaGraphConditionalHandle cond,
+                       cudaStream_t st, int* kernels) {
+  GmresArgs a = gmres_args(s, b, x, x_double);
+  k_gmres_update<<<s.coop_blocks, kKrylovThreads, 0, st>>>(a);
+  RF_LAUNCH_CHECK();
   k_gmres_loop_cond<<<1, 1, 0, st>>>(cond, s.ctl);
   RF_LAUNCH_CHECK();
-  *kernels += 1;
+  *kernels += 2;
   return RF_OK;
 }
 

@@ -21,6 +21,8 @@ struct GmresCtl {
   int timeout;        // a bounded device-side wait gave up (set by kernels)
   int heads;          // restart cycles opened from the residual of x (after the first)
   int halt;           // the solve failed (non-finite or timed out): later stages skip
+  int launched;       // Arnoldi steps launched (those after convergence return at once)
+  int pad;
   double tol;
   double bnorm;
   double beta;        // true residual norm at the last cycle start
@@ -103,15 +105,19 @@ int gmres_solve_ex(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn
 
 // The same solve as launches without host synchronisation, for capture into a
 // graph whose restart loop is a conditional WHILE node (handle `cond`):
-// gmres_enqueue_first enqueues the control-block set-up, x = 0, ||b||, the
-// first cycle and the loop condition; gmres_enqueue_cycle one later cycle
-// (residual of x, m Arnoldi steps, update) and the loop condition.  Steps after
-// convergence return at once on the device.  *kernels counts the kernels
-// these functions launch themselves (the callbacks count theirs).
-int gmres_enqueue_first(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn& residual, const float* b,
-                        void* x, bool x_double, cudaGraphConditionalHandle cond, cudaStream_t st, int* kernels);
-int gmres_enqueue_cycle(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn& residual, const float* b,
-                        void* x, bool x_double, cudaGraphConditionalHandle cond, cudaStream_t st, int* kernels);
+// gmres_enqueue_first opens the solve (control block, x = 0, ||b||),
+// gmres_enqueue_head a later cycle (residual of x); gmres_enqueue_steps enqueues
+// Arnoldi steps [j0, j1), the last of which sets `more` (when not 0) to whether
+// the cycle goes on, so that the steps after it can sit in a conditional IF node;
+// gmres_enqueue_tail the solution update and the loop condition.  *kernels counts
+// the kernels these functions launch themselves (the callbacks count theirs).
+int gmres_enqueue_first(const GmresSetup& s, const float* b, void* x, bool x_double, cudaStream_t st, int* kernels);
+int gmres_enqueue_head(const GmresSetup& s, const MatvecFn& matvec, const ResidualFn& residual, const float* b, void* x,
+                       bool x_double, cudaStream_t st, int* kernels);
+int gmres_enqueue_steps(const GmresSetup& s, const MatvecFn& matvec, const float* b, void* x, bool x_double, int j0,
+                        int j1, cudaGraphConditionalHandle more, cudaStream_t st);
+int gmres_enqueue_tail(const GmresSetup& s, const float* b, void* x, bool x_double, cudaGraphConditionalHandle cond,
+                       cudaStream_t st, int* kernels);
 // The solve's outcome from a host copy of its control block (after such a
 // graph ran); returns the status gmres_solve_ex would have returned.
 int gmres_result_from_ctl(const GmresCtl& h, bool has_residual, GmresResult* res);

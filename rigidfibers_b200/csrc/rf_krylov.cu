@@ -893,6 +893,7 @@ __global__ void __launch_bounds__(kKrylovThreads) k_bicg_init(BicgArgs a) {
     c->nan = isfinite(bb) ? 0 : 1;
     c->need_restart = 0;
     c->restarts = 0;
+    c->stop_word = bicg_stopped(c) ? 1 : 0;
   }
 }
 
@@ -917,6 +918,7 @@ __global__ void __launch_bounds__(kKrylovThreads) k_bicg_restart(BicgArgs a) {
     a.ctl->last_restart = a.ctl->iters;
     a.ctl->restarts += 1;
     if (!isfinite(rr)) a.ctl->nan = 1;
+    a.ctl->stop_word = bicg_stopped(a.ctl) ? 1 : 0;
   }
 }
 
@@ -938,7 +940,10 @@ __global__ void __launch_bounds__(kKrylovThreads) k_bicg_step1(BicgArgs a) {
     a.sv[r] = a.r[r] - af * a.v[r];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.ctl->alpha = alpha;
-    if (!isfinite(alpha)) a.ctl->nan = 1;
+    if (!isfinite(alpha)) {
+      a.ctl->nan = 1;
+      a.ctl->stop_word = 1;
+    }
   }
 }
 
@@ -988,11 +993,8 @@ __global__ void __launch_bounds__(kKrylovThreads) k_bicg_step2(BicgArgs a) {
     if (conv) c->converged = 1;
     if (restart) c->need_restart = 1;
     if (!isfinite(rnorm)) c->nan = 1;
+    c->stop_word = bicg_stopped(c) ? 1 : 0;   // what the matvec kernels read
   }
-}
-
-__global__ void k_bicg_stopword(BicgCtl* c) {
-  c->stop_word = (c->converged || c->nan || c->need_restart || c->iters >= c->maxit) ? 1 : 0;
 }
 
 int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, float* x, cudaStream_t st,
@@ -1025,7 +1027,9 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
   res->launches = 1;
   res->matvecs = 0;
   BicgCtl h{};
-  const int chunk = 10;   // iterations between host checks
+  // iterations between host checks: a check costs ~12 us, an iteration past the
+  // stop its six launches of ~2.2 us (inner solves of the mixed modes take 2 to 4)
+  const int chunk = 4;
   for (int guard = 0; guard < s.maxit + 4 * (s.maxit / std::max(1, s.restart_every) + 2); ++guard) {
     for (int k = 0; k < chunk; ++k) {
       int rc = matvec(a.p, (const int*)&s.ctl->stop_word, st);
@@ -1037,10 +1041,7 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
       if (rc) return rc;
       rc = coop_launch((const void*)k_bicg_step2, nblk, kKrylovThreads, args, st);
       if (rc) return rc;
-      // the matvec kernels read one word: fold the stop conditions into it
-      k_bicg_stopword<<<1, 1, 0, st>>>(s.ctl);
-      RF_LAUNCH_CHECK();
-      res->launches += 5;
+      res->launches += 2;
     }
     RF_CUDA_TRY(cudaMemcpyAsync(s.host_ctl, s.ctl, sizeof(BicgCtl), cudaMemcpyDeviceToHost, st));
     RF_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1052,9 +1053,7 @@ int bicgstab_solve(const BicgSetup& s, const MatvecFn& matvec, const float* b, f
       void* args[] = {&a};
       rc = coop_launch((const void*)k_bicg_restart, nblk, kKrylovThreads, args, st);
       if (rc) return rc;
-      k_bicg_stopword<<<1, 1, 0, st>>>(s.ctl);
-      RF_LAUNCH_CHECK();
-      res->launches += 2;
+      res->launches += 1;
       ++res->matvecs;
     }
   }

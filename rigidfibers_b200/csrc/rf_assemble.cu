@@ -211,26 +211,33 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
 // FP32 rounding).  The others take the full rule.
 //
 // Bound: FP32 issue in the matrix-free product, HBM stores in the structured
-// assembly.  The far pairs run in batches of 32 (four j of the tile at once:
-// 32 pairs x 8 points = the CTA's 256 threads), so that every phase has one
-// unit per thread and lane = pair keeps shared memory free of conflicts; the
-// near pairs are compacted per tile and run in groups of TI pairs x Q points.
+// assembly.  The far pairs run in batches of whole j (2 or 4 of the tile: 16 or
+// 32 pairs x 8 points = the CTA's threads), so that every phase has one unit per
+// thread and lane = pair keeps shared memory free of conflicts; the near pairs
+// of those rows are compacted and run in groups of up to TI pairs x Q points.
 // ---------------------------------------------------------------------------
-template <int M, int Q>
+// Threads per CTA.  Structured output: 128 (six CTAs per SM instead of three of
+// 256: barriers of four warps, more CTAs to fill them; N=4000 3.09 -> 2.42 ms).
+// Matrix-free product and dense output: 256, where the product's 160 and the
+// block stores' 800 tasks of a batch split better (N=2500 product 0.90 against
+// 1.23 ms, N=2000 dense 1.55 against 1.77); 128 for more than 5 terms, whose G
+// and T of 32 pairs would leave one CTA per SM.
+constexpr int num_threads(int M, int mode) { return mode == kAsmStructF16 || mode == kAsmStructBF16 || M > 5 ? 128 : 256; }
+
+template <int M, int Q, int NTH>
 struct NumShape {
   using A = AsmShape<M, Q>;
   static constexpr int TI = A::TI, K1 = A::K1, NQ32 = A::NQ32;
   static constexpr int KP = (K1 + 1) / 2;                  // Legendre index pairs (2i, 2i + 1) of fiber j
   static constexpr int NC2 = 6 * KP;                       // G columns, pairs of floats
-  static constexpr int NT = 256;
+  static constexpr int NT = NTH;
   static constexpr int FN = kFarNodes;
-  // far pairs per batch: 32 (one per lane); 16 where the tile has no more, and
-  // for M > 5, whose G and T of 32 pairs would leave one CTA per SM
-  static constexpr int PB = (M <= 5 && TI * TI >= 32) ? 32 : 16;
+  static constexpr int PB = NT / FN < TI * TI ? NT / FN : TI * TI;   // far pairs per batch
   static constexpr int JB = PB / TI;                       // j of a batch
   static constexpr int GSF = PB * FN + PB % 32;            // G column stride (float2): lanes (col, pair)
+  static constexpr int NS = NT / Q < TI ? NT / Q : TI;     // near pairs per group
   static constexpr int QP = Q + 1;                         // near: float2 per slot of a G column
-  static constexpr int GSN = TI * QP + (TI * QP + 1) % 2;  // odd: lanes = columns
+  static constexpr int GSN = NS * QP + (NS * QP + 1) % 2;  // odd: lanes = columns
   static constexpr int GFLOATS = (2 * NC2 * (GSF > GSN ? GSF : GSN) + 3) / 4 * 4;
   // T of a batch.  Structured and matrix-free: [jj][value][i], the storage
   // record's own order (s32_block), so one j is the contiguous run that a bulk
@@ -267,7 +274,7 @@ __device__ __forceinline__ void dense_block(float* __restrict__ dst, int64_t lda
 template <int M, int Q, int MODE, bool P2>
 __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, const float4* __restrict__ ori,
                                                    const AsmOut& out, int I, int J) {
-  using S = NumShape<M, Q>;
+  using S = NumShape<M, Q, num_threads(M, MODE)>;
   constexpr int TI = S::TI, K1 = S::K1, NC2 = S::NC2, NT = S::NT, PB = S::PB, JB = S::JB, TP = S::TP, JS = S::JS;
   constexpr int NQ32 = S::NQ32;
   constexpr int M3 = 3 * M;
@@ -281,7 +288,7 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
   __shared__ float sD[TI * TI][3];           // pair jl * TI + il: x_i - x_j, formed in FP64 and rounded once
   __shared__ unsigned char sKind[TI * TI];   // 0: no such pair, 1: far, 2: near
   __shared__ unsigned char sNear[TI * TI];   // the near pairs, in pair order
-  __shared__ unsigned sMask[NT / 32];        // near pairs as bits
+  __shared__ unsigned sMask[(TI * TI + 31) / 32];   // near pairs as bits
   extern __shared__ __align__(16) float smem_dyn[];
   float2* const sG = reinterpret_cast<float2*>(smem_dyn);
   float* const sT = smem_dyn + S::GFLOATS;
@@ -301,25 +308,28 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
     sTi[tid] = ori[min(i0 + tid, N - 1)];
     sTj[tid] = ori[min(j0 + tid, N - 1)];
   }
-  bool near_pair = false;
-  if (tid < TI * TI) {
+  for (int pr0 = 0; pr0 < TI * TI; pr0 += NT) {
     // the separation of quadrature points is formed as (x_i - x_j) + s_qi t_i -
     // s_qj t_j with the centre difference taken in FP64 and rounded once, so
     // its error scales with the fibers' distance rather than with their
     // distance from the origin (FP32 points x + s t far from the origin lose
     // ~1e-6 absolutely, which for nearly touching fibers is ~1e-4 of the kernel)
-    const int il = tid % TI, jl = tid / TI;
-    const double4 xi = out.pos64[min(i0 + il, N - 1)], xj = out.pos64[min(j0 + jl, N - 1)];
-    const float dx = (float)(xi.x - xj.x), dy = (float)(xi.y - xj.y), dz = (float)(xi.z - xj.z);
-    sD[tid][0] = dx;
-    sD[tid][1] = dy;
-    sD[tid][2] = dz;
-    const bool valid = i0 + il < N && j0 + jl < N && (!diag || il < jl);
-    near_pair = valid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < tab.far_d2;
-    sKind[tid] = near_pair ? 2 : valid ? 1 : 0;
+    const int pr = pr0 + tid;
+    bool near_pair = false;
+    if (pr < TI * TI) {
+      const int il = pr % TI, jl = pr / TI;
+      const double4 xi = out.pos64[min(i0 + il, N - 1)], xj = out.pos64[min(j0 + jl, N - 1)];
+      const float dx = (float)(xi.x - xj.x), dy = (float)(xi.y - xj.y), dz = (float)(xi.z - xj.z);
+      sD[pr][0] = dx;
+      sD[pr][1] = dy;
+      sD[pr][2] = dz;
+      const bool valid = i0 + il < N && j0 + jl < N && (!diag || il < jl);
+      near_pair = valid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < tab.far_d2;
+      sKind[pr] = near_pair ? 2 : valid ? 1 : 0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, near_pair);
+    if (lane == 0 && pr < TI * TI) sMask[pr / 32] = m;
   }
-  const unsigned near_mask = __ballot_sync(0xffffffffu, near_pair);
-  if (lane == 0) sMask[tid >> 5] = near_mask;
   if constexpr (APPLY) {
     if (do_apply) {
       for (int k = tid; k < TI * M3; k += NT) {
@@ -333,11 +343,12 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
   const float e2x3 = -3.f * e2;
   const float fz = tab.fz_half;
   __syncthreads();
-  if (near_pair) {   // read after the barriers of the first batch
-    int at = __popc(near_mask & ((1u << lane) - 1));
-    for (int w = 0; w < (tid >> 5); ++w) at += __popc(sMask[w]);
-    sNear[at] = (unsigned char)tid;
-  }
+  for (int pr = tid; pr < TI * TI; pr += NT)   // read after the barriers of the first batch
+    if (sKind[pr] == 2) {
+      int at = __popc(sMask[pr / 32] & ((1u << lane) - 1));
+      for (int w = 0; w < pr / 32; ++w) at += __popc(sMask[w]);
+      sNear[at] = (unsigned char)pr;
+    }
 
   // structured storage: the record of j = j0 + jl is rec0 + jl
   constexpr int SUB = kStoreTile / TI;
@@ -413,11 +424,11 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
       contract(sG + col * S::GSF + p, std::integral_constant<int, S::FN>(), std::true_type(), PB, col,
                t_of(p / TI, p % TI));
     }
-    // ---- near pairs of these rows, in groups of up to TI, into the same T
+    // ---- near pairs of these rows, in groups of up to NS, into the same T
     const unsigned bits = (sMask[jb * TI / 32] >> (jb * TI % 32)) & (PB == 32 ? 0xffffffffu : (1u << PB % 32) - 1u);
     const int near1 = near0 + __popc(bits);
-    for (int n0 = near0; n0 < near1; n0 += TI) {
-      const int cnt = min(TI, near1 - n0);
+    for (int n0 = near0; n0 < near1; n0 += S::NS) {
+      const int cnt = min(S::NS, near1 - n0);
       __syncthreads();   // G is read
       if (tid < cnt * Q) {
         const int slot = tid / Q, qi = tid % Q;
@@ -612,7 +623,7 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
 }
 
 template <int M, int Q, int MODE, bool P2>
-__global__ void __launch_bounds__(256, M <= 5 ? 3 : 2)
+__global__ void __launch_bounds__(num_threads(M, MODE), M > 5 ? 4 : num_threads(M, MODE) == 128 ? 6 : 3)
 k_assemble_pairs(const Tables tab, int N, const float4* __restrict__ ori, AsmOut out) {
   if (MODE == kAsmApply && out.skip != nullptr && *out.skip) return;
   int I, J;
@@ -916,7 +927,7 @@ __global__ void k_force_terms(const Tables tab, int N, const float4* __restrict_
 // blocks run exactly the single-suspension kernel's tile code, so a member's
 // system is bit for bit the one k_assemble_pairs forms.
 template <int MODE>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(128, 6)
 k_pack_assemble(const Tables tab, const PackStepMember* __restrict__ mem, int n) {
   const int L = (int)blockIdx.x;
   const PackStepMember& p = mem[pack_member_of(n, L, [&](int m) { return mem[m].asm_start; })];
@@ -943,17 +954,18 @@ __global__ void k_pack_force_terms(const Tables tab, const PackStepMember* __res
 int launch_pack_assemble(const Tables& tab, const PackStepMember* members, int n, int64_t blocks, bool bf16,
                          cudaStream_t st) {
   if (tab.M != 5 || tab.Q != 24 || n < 1 || blocks < 1) return RF_E_UNSUPPORTED;
-  constexpr size_t smem = NumShape<5, 24>::kSmem;
+  using S = NumShape<5, 24, num_threads(5, kAsmStructF16)>;
+  constexpr size_t smem = S::kSmem;
   if (bf16) {
     static const cudaError_t attr = cudaFuncSetAttribute(k_pack_assemble<kAsmStructBF16>,
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     RF_CUDA_TRY(attr);
-    k_pack_assemble<kAsmStructBF16><<<(unsigned)blocks, NumShape<5, 24>::NT, smem, st>>>(tab, members, n);
+    k_pack_assemble<kAsmStructBF16><<<(unsigned)blocks, S::NT, smem, st>>>(tab, members, n);
   } else {
     static const cudaError_t attr = cudaFuncSetAttribute(k_pack_assemble<kAsmStructF16>,
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     RF_CUDA_TRY(attr);
-    k_pack_assemble<kAsmStructF16><<<(unsigned)blocks, NumShape<5, 24>::NT, smem, st>>>(tab, members, n);
+    k_pack_assemble<kAsmStructF16><<<(unsigned)blocks, S::NT, smem, st>>>(tab, members, n);
   }
   RF_LAUNCH_CHECK();
   k_pack_force_terms<<<dim3((unsigned)n, kPackMaxFibers / kForceFibers), force_threads(5), 0, st>>>(tab, members);
@@ -995,7 +1007,7 @@ int64_t struct_words16(int M, int N) {
 
 template <int M, int Q, int MODE, bool P2>
 static int launch_pairs(const Tables& tab, int N, const float4* ori, const AsmOut& out, cudaStream_t st) {
-  using S = NumShape<M, Q>;
+  using S = NumShape<M, Q, num_threads(M, MODE)>;
   const int64_t T = ceil_div(N, S::TI);
   // once per process (thread-safe static initialisation; handles of a serving
   // loop launch from several threads)

@@ -11,7 +11,7 @@
 // Work of a member is cut into kParts = 8 fixed parts whatever C is: storage
 // tile L belongs to partition L mod 8, whose partial rows are summed in tile
 // order; row slice s is fibers [s N / 8, (s + 1) N / 8), whose dot-product
-// partial one warp sums.  A CTA of the cluster owns 8 / C consecutive
+// partial its owner's warps sum in a fixed order.  A CTA of the cluster owns 8 / C consecutive
 // partitions and slices; the partitions' partial rows and the slices'
 // partials are added in part order through distributed shared memory after a
 // cluster barrier.  So a member's solution is the same bits for any C, alone
@@ -19,8 +19,8 @@
 // pack can give its large members more SMs when the GPU has them to spare.
 //
 // Per Arnoldi step each CTA stages v in shared memory, walks its storage
-// tiles (one thread per pair of a 16 x 16 tile, the pair's 16-byte aligned
-// record read with 16-byte loads), reduces z over the tile's lanes (halving
+// tiles (one thread per pair of a 16 x 16 tile, the records brought to shared
+// memory by bulk copies one tile ahead), reduces z over the tile's lanes (halving
 // exchanges) and adds the tile's partial rows into its partition's rows; the
 // Krylov basis stays in the suspension's V (L2-resident at these sizes), each
 // CTA writing its own rows of it.
@@ -45,13 +45,41 @@ constexpr int kPM = 5;                                // force terms of the pack
 constexpr int kPM3 = 3 * kPM;
 constexpr int kNW = s16_record_words(kPM);            // 16-bit record words per pair
 constexpr int kNQ32 = (kPM + 1) * (kPM + 1) * 6;      // FP32 values per pair
+constexpr int kTileDoubles = 8 * 16 * 16 + 16 * 16;   // a tile's partial sums (i side, j side)
+static_assert(kTileDoubles >= 8 * 80, "the warp partials of one slice at the longest restart");
+constexpr int kRecU = kNW / 4;                        // 16-byte units of a pair's 16-bit record
+constexpr int kWarpU = 32 * kRecU;                    // units of a warp's 32 records of a tile
+static_assert(kNW % 4 == 0 && kRecU % 2 == 1, "16-byte reads of eight consecutive records hit different banks");
 
-__device__ __forceinline__ void pack_tile(int L, int& I, int& J) {
-  int j = (int)((sqrtf(8.f * (float)L + 1.f) - 1.f) * 0.5f);
-  while ((j + 1) * (j + 2) / 2 <= L) ++j;
-  while (j * (j + 1) / 2 > L) --j;
-  J = j;
-  I = L - j * (j + 1) / 2;
+// Shared memory offsets: the 16-bit products' sums are FP32, so the records are
+// staged from the upper half of the partition rows on, and past their end where
+// the rows are short.
+__host__ __device__ __forceinline__ int pack_stage_offset(int Rmax, int slots) {   // in 16-byte units
+  return ((2 + slots) * Rmax + 3) / 4;
+}
+__host__ __device__ __forceinline__ int pack_tail_offset(int Rmax, int slots) {    // in doubles
+  const int rows = (1 + slots) * Rmax, staged = 2 * (pack_stage_offset(Rmax, slots) + kPT / 32 * kWarpU);
+  return rows > staged ? rows : staged;
+}
+
+__device__ __forceinline__ uint32_t psmem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// wait for an mbarrier's phase; false after a second
+__device__ __forceinline__ bool pack_wait(uint64_t* bar, uint32_t parity) {
+  uint64_t t0 = 0, now;
+  for (int n = 0;; ++n) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(psmem(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((n & 63) == 63) {
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      if (now - t0 > 1000000000ull) return false;
+    }
+  }
 }
 
 template <typename T>
@@ -124,10 +152,11 @@ __device__ __forceinline__ void ppair16(const uint32_t (&w)[kNW], const float (&
     }
 }
 
-// Shared memory (doubles): [staged vector Rmax][partition rows: 8/C x Rmax]
-// [i-side tile partials 8 x 16 x 16][j-side tile sums 16 x 16][H (m+1) x m]
-// [cs m][sn m][g m+1][y m][h m+1][h2 m+1][reduction partials 3 x 8 x (m+1)]
-// [scalar 2][flags]
+// Shared memory (doubles): [staged vector Rmax][partition rows: 8/C x Rmax, or
+// FP32 rows and a tile's records][i-side tile partials 8 x 16 x 16][j-side tile
+// sums 16 x 16][H: column j of j + 2 entries]
+// [cs m][sn m][g m+1][y m][h m+1][h2 m+2][slice partials 3 x 8 x (m+2)]
+// [scalar 2][flags]; the dot products' warp partials use the tile sums' room
 // kClustered: launched with clusters of 2, 4 or 8 CTAs; otherwise one CTA per
 // member (the same arithmetic in the same order, without cluster barriers and
 // distributed shared memory)
@@ -145,7 +174,6 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
   const int R = kPM3 * N;
   const int T16 = (N + 15) / 16;
   const int ntiles = T16 * (T16 + 1) / 2;
-  const int ldh = m + 1;
   const int spc = kParts / C;                                   // partitions (and row slices) per CTA
   const int p0 = rank * spc;                                    // this CTA's first partition
   const int q0 = kPM3 * ((rank * N) / C), q1 = kPM3 * (((rank + 1) * N) / C);   // its rows
@@ -153,27 +181,39 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
   float* sxf = reinterpret_cast<float*>(psm);
   double* zpd = sxd + Rmax;                                     // partition rows, slot stride Rmax
   float* zpf = reinterpret_cast<float*>(zpd);
-  double* tail = zpd + (size_t)spc * Rmax;
+  double* tail = sxd + pack_tail_offset(Rmax, spc);
   double (*zip)[16][16] = reinterpret_cast<double (*)[16][16]>(tail);
   float (*zipf)[16][16] = reinterpret_cast<float (*)[16][16]>(tail);
   double (*zjs)[16] = reinterpret_cast<double (*)[16]>(tail + 8 * 16 * 16);
   float (*zjsf)[16] = reinterpret_cast<float (*)[16]>(tail + 8 * 16 * 16);
-  double* H = tail + 8 * 16 * 16 + 16 * 16;
-  double* cs = H + (size_t)ldh * m;
+  double* H = tail + kTileDoubles;
+  double* cs = H + m * (m + 3) / 2;
   double* sn = cs + m;
   double* g = sn + m;
   double* yv = g + m + 1;
   double* hh = yv + m;
-  double* hh2 = hh + m + 1;
-  double* dpart = hh2 + m + 1;                                  // [3][kParts][m+1]
-  double* scal = dpart + 3 * kParts * (m + 1);
+  double* hh2 = hh + m + 1;                                     // m + 2: dots and the norm
+  double* dpart = hh2 + m + 2;                                  // [3][kParts][m+2]
+  double* red = tail;                                           // warp partials, outside the products
+  double* scal = dpart + 3 * kParts * (m + 2);
   int* flags = reinterpret_cast<int*>(scal + 2);                // [0] cycle done, [1] converged, [2] non-finite
   float* V = P.V;
   const int64_t ldv = P.ldv;
   const int i16 = t & 15, j16 = t >> 4;
   const int sub = (i16 >> 3) * 2 + (j16 >> 3);
-  const int rec16 = (sub * 8 + (j16 & 7)) * 8 + (i16 & 7);   // record of pair (i16, j16) in a storage tile
+  // a warp's pairs (16 i, 2 j) are two runs of 16 records of a storage tile
+  uint4* stage = reinterpret_cast<uint4*>(psm) + pack_stage_offset(Rmax, spc) + warp * kWarpU;
+  const uint4* mine = stage + ((i16 >> 3) * 16 + (j16 & 1) * 8 + (i16 & 7)) * kRecU;
   const int rec32 = sub * 8 + (j16 & 7);                       // FP32 record (8 pairs, [value][i])
+  __shared__ uint64_t copied[kPT / 32];                        // a warp's records have arrived
+  if (t < kPT / 32) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(psmem(&copied[t])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  uint32_t phase = 0;                                          // of this warp's copies
+  bool lost = false;                                           // one of them never arrived
   int rb = 0;                                                  // reduction buffer in use (of 3)
   // a cluster barrier, or the block barrier when the member has one CTA
   auto csync = [&]() {
@@ -186,74 +226,143 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     else return p;
   };
 
-  // out[k] = sum over the member's rows of a[r] * V_k[r] for k < nv (square:
-  // nv = 1 and a[r]^2), FP64.  Slice s's partial is one warp's (lane-strided
-  // sums, then a butterfly), written into the owning CTA's buffer; after the
-  // cluster barrier every CTA adds the 8 partials in slice order.  Three
+  // out[k] = sum over the member's rows of a[r] * V_k[r] for k < nv, FP64, and with
+  // `norm` out[nv] = sum of a[r]^2.  A slice's partial is that of up to 8 virtual
+  // warps: lane l of virtual warp w adds rows 32 w + l, 32 (w + 8) + l, .. of the
+  // slice (all basis loads of 16 values in flight), the lanes meet in halving
+  // exchanges, the virtual warps add in order; the CTA's warps share all its
+  // slices' virtual warps.  The partials go into the owning CTA's buffer; after
+  // the cluster barrier every CTA adds the 8 of them in slice order.  Three
   // buffers in turn: a buffer is written again only after two more cluster
   // barriers, when every CTA has read it.
-  auto cdots = [&](const float* a, int nv, bool square, double* out) {
+  const int nvw = min(8, (kPM3 * ((N + kParts - 1) / kParts) + 31) / 32);
+  auto cdots = [&](const float* a, int nv, bool norm, double* out) {
     __syncthreads();                                           // this CTA's rows of a are written
-    double* part = dpart + (size_t)rb * kParts * (m + 1);
-    const int ng = (nv + 3) / 4;
-    for (int task = warp; task < spc * ng; task += kPT / 32) {
-      const int s = p0 + task % spc, k0 = 4 * (task / spc);
-      const int r0 = kPM3 * ((s * N) / kParts), r1 = kPM3 * (((s + 1) * N) / kParts);
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int r = r0 + lane; r < r1; r += 32) {
-        const double ar = (double)a[r];
+    double* part = dpart + (size_t)rb * kParts * (m + 2);
+    const int n = nv + (norm ? 1 : 0);
+    const int npad = (n + 15) / 16 * 16;
+    const int per = min(spc, kTileDoubles / (nvw * npad));     // slices whose warp partials fit at once
+    for (int s0 = 0; s0 < spc; s0 += per) {
+      const int cnt = min(per, spc - s0);
+      for (int e = warp; e < cnt * nvw; e += kPT / 32) {
+        const int s = p0 + s0 + e / nvw;
+        const int r0 = kPM3 * ((s * N) / kParts), r1 = kPM3 * (((s + 1) * N) / kParts);
+        for (int g = 0; g < npad; g += 16) {
+          double acc[16];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (k0 + u < nv) {
-            const float* vk = square ? a : V + (int64_t)(k0 + u) * ldv;
-            acc[u] = fma(ar, (double)vk[r], acc[u]);
+          for (int u = 0; u < 16; ++u) acc[u] = 0.0;
+          for (int r = r0 + (e % nvw) * 32 + lane; r < r1; r += 8 * 32) {
+            const float af = a[r];
+            const double ar = (double)af;
+            float v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+              const int k = g + u;
+              v[u] = k < nv ? V[(int64_t)k * ldv + r] : k < n ? af : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 16; ++u) acc[u] = fma(ar, (double)v[u], acc[u]);
           }
+          // lane l gets the warp's sum of value l & 15 (of both half-warps)
+          double v = psum16(acc, lane);
+          v += pshfl(v, 16);
+          if (lane < 16) red[(size_t)e * npad + g + lane] = v;
+        }
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        double v = acc[u];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += pshfl(v, o);
-        if (lane == 0 && k0 + u < nv) part[s * (m + 1) + k0 + u] = v;
+      __syncthreads();
+      for (int e = t; e < cnt * n; e += kPT) {
+        const int sl = e / n, k = e % n;
+        const double* rp = red + (size_t)sl * nvw * npad + k;
+        double v = rp[0];
+        for (int w = 1; w < nvw; ++w) v += rp[w * npad];
+        part[(p0 + s0 + sl) * (m + 2) + k] = v;
       }
+      __syncthreads();
     }
     csync();
-    for (int k = t; k < nv; k += kPT) {
+    for (int k = t; k < n; k += kPT) {
       double sum = 0.0;
-      for (int s = 0; s < kParts; ++s) sum += at_rank(part, s / spc)[s * (m + 1) + k];
+#pragma unroll
+      for (int s = 0; s < kParts; ++s) sum += at_rank(part, s / spc)[s * (m + 2) + k];
       out[k] = sum;
     }
     __syncthreads();
     rb = rb == 2 ? 0 : rb + 1;
   };
+  // sum of a[r]^2
   auto sumsq = [&](const float* a) -> double {
-    cdots(a, 1, true, scal);
+    cdots(a, 0, true, scal);
     return scal[0];
   };
-  // w = v + C (T v) with the 16-bit blocks, FP32 sums; this CTA writes its rows of w
-  auto matvec16 = [&](const float* v, float* w) {
-    for (int q = t; q < spc * Rmax; q += kPT) zpf[q] = 0.f;
+  // this CTA's next storage tile after L, in tile order: partitions p0 .. p0 + spc - 1
+  auto next_own = [&](int L) {
+    const int p = (L + 1) % kParts;
+    return p >= p0 && p < p0 + spc ? L + 1 : L + 1 + (p0 - p + kParts) % kParts;
+  };
+  // this warp's records of storage tile L into its part of the stage
+  auto fetch = [&](int L) {
+    if (lane < 2) {
+      constexpr uint32_t bytes = 16 * kRecU * 16;
+      const int rec = ((lane * 2 + (warp >> 2)) * 8 + ((2 * warp) & 7)) * 8;
+      asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(psmem(&copied[warp])), "r"(bytes)
+                   : "memory");
+      asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       psmem(stage + lane * 16 * kRecU)),
+                   "l"(reinterpret_cast<const uint4*>(P.S16) + ((int64_t)L * 256 + rec) * kRecU), "r"(bytes),
+                   "r"(psmem(&copied[warp]))
+                   : "memory");
+    }
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(psmem(&copied[warp])) : "memory");
+  };
+  // v into shared memory, this CTA's rows of T v cleared and the first tile's
+  // records on their way; meanwhile one thread runs `aside`
+  auto stage_vector = [&](const float* v, auto&& aside) {
+    if (p0 < ntiles) fetch(p0);
     csync();                                                   // every CTA's rows of v are written
+    if (t == kPT - 1) aside();
     for (int r = t; r < R; r += kPT) sxf[r] = v[r];
+    for (int q = t; q < spc * Rmax; q += kPT) zpf[q] = 0.f;
     __syncthreads();
-    for (int L = 0; L < ntiles; ++L) {
-      const int p = L % kParts;
-      if (p / spc != rank) continue;
-      float* zs = zpf + (size_t)(p - p0) * Rmax;
-      int I, J;
-      pack_tile(L, I, J);
+  };
+  // the staged product is not wanted: take in the records that were fetched
+  auto unstage = [&]() {
+    if (p0 < ntiles) {
+      lost |= !pack_wait(&copied[warp], phase);
+      phase ^= 1;
+    }
+  };
+  // w = v + C (T v) of the staged v with the 16-bit blocks, FP32 sums; this CTA
+  // writes its rows of w
+  //
+  // A thread reading its pair's 304-byte record from memory puts 32 cache lines
+  // behind each of a warp's 19 loads: 7.4k cycles a tile of 256 pairs, against
+  // ~2.4k of arithmetic.  The warp's records are two contiguous runs, so two bulk
+  // copies bring the next tile's to shared memory as soon as this one's are in
+  // registers (16-byte reads 19 units apart: no bank conflicts): 4.2k cycles.
+  // The same through 16-byte asynchronous copies: 6.9k, their issue alone 2.8k.
+  auto matvec16 = [&](float* w) {
+    int L = p0, I = p0, J = 0;
+    while (L < ntiles) {
+      float* zs = zpf + (size_t)(L % kParts - p0) * Rmax;
+      while (I > J) I -= ++J;   // storage tile L = J (J + 1) / 2 + I
       const int i = I * 16 + i16, j = J * 16 + j16;
+      lost |= !pack_wait(&copied[warp], phase);
+      phase ^= 1;
+      uint32_t wv[kNW];
+#pragma unroll
+      for (int u = 0; u < kRecU; ++u) {
+        const uint4 q4 = mine[u];
+        wv[4 * u] = q4.x; wv[4 * u + 1] = q4.y; wv[4 * u + 2] = q4.z; wv[4 * u + 3] = q4.w;
+      }
+      __syncwarp();
+      const int Ln = next_own(L);
+      if (Ln < ntiles) fetch(Ln);
       float zi[16], zj[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) zi[q] = zj[q] = 0.f;
       if (i < j && j < N) {
-        uint32_t wv[kNW];
-        const uint4* pw = reinterpret_cast<const uint4*>(P.S16 + ((int64_t)L * 256 + rec16) * kNW);
-#pragma unroll
-        for (int u = 0; u < kNW / 4; ++u) {
-          const uint4 q4 = pw[u];
-          wv[4 * u] = q4.x; wv[4 * u + 1] = q4.y; wv[4 * u + 2] = q4.z; wv[4 * u + 3] = q4.w;
-        }
         float xi[kPM3], xj[kPM3];
 #pragma unroll
         for (int q = 0; q < kPM3; ++q) {
@@ -263,6 +372,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
         if (P.smode == 2) ppair16<__nv_bfloat16>(wv, xi, xj, zi, zj);
         else ppair16<__half>(wv, xi, xj, zi, zj);
       }
+      if (lost) zj[0] = nanf("");   // the solve ends as non-finite
       const float sj = psum16(zj, lane);   // z_j over this half-warp's 16 i
       const bool b4 = lane & 16;
       float u8[8];                          // z_i over this warp's two j: one halving exchange
@@ -278,12 +388,16 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
       __syncthreads();
       if (t < 16 * kPM3) {
         const int f = t / kPM3, q = t % kPM3;
-        float si = 0.f;
-        for (int w8 = 0; w8 < 8; ++w8) si += zipf[w8][f][q];
+        float s8[8];
+#pragma unroll
+        for (int w8 = 0; w8 < 8; ++w8) s8[w8] = zipf[w8][f][q];
+        const float si = ((s8[0] + s8[1]) + (s8[2] + s8[3])) + ((s8[4] + s8[5]) + (s8[6] + s8[7]));
         const int fi = I * 16 + f, fj = J * 16 + f;
         if (fi < N) zs[fi * kPM3 + q] += si;
         if (fj < N) zs[fj * kPM3 + q] += zjsf[f][q];
       }
+      I += Ln - L;
+      L = Ln;
     }
     csync();                                                   // every partition's rows are complete
     for (int u = t; u < (q1 - q0) / 3; u += kPT) {
@@ -313,12 +427,10 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     csync();                                                   // every CTA's rows of x are written
     for (int q = t; q < R; q += kPT) sxd[q] = P.x64[q];
     __syncthreads();
-    for (int L = 0; L < ntiles; ++L) {
-      const int p = L % kParts;
-      if (p / spc != rank) continue;
-      double* zs = zpd + (size_t)(p - p0) * Rmax;
-      int I, J;
-      pack_tile(L, I, J);
+    int I = p0, J = 0;
+    for (int L = p0; L < ntiles;) {
+      double* zs = zpd + (size_t)(L % kParts - p0) * Rmax;
+      while (I > J) I -= ++J;
       const int i = I * 16 + i16, j = J * 16 + j16;
       double zi[16], zj[16];
 #pragma unroll
@@ -327,16 +439,28 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
         const float* base = P.S32 + ((int64_t)L * 32 + rec32) * (kNQ32 * 8) + (i16 & 7);
         const double* xi = sxd + i * kPM3;
         const double* xj = sxd + j * kPM3;
+        // a row of blocks (30 loads) on its way while the one before is summed
+        float next[6 * kPM];
 #pragma unroll
-        for (int kI = 0; kI < kPM; ++kI)
+        for (int c = 0; c < 6 * kPM; ++c) next[c] = base[c * 8];
+#pragma unroll
+        for (int kI = 0; kI < kPM; ++kI) {
+          float row[6 * kPM];
+#pragma unroll
+          for (int c = 0; c < 6 * kPM; ++c) row[c] = next[c];
+          if (kI + 1 < kPM) {
+#pragma unroll
+            for (int c = 0; c < 6 * kPM; ++c) next[c] = base[((kI + 1) * 6 * kPM + c) * 8];
+          }
 #pragma unroll
           for (int kJ = 0; kJ < kPM; ++kJ) {
             double tv[6];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) tv[c] = (double)base[((kI * kPM + kJ) * 6 + c) * 8];
+            for (int c = 0; c < 6; ++c) tv[c] = (double)row[6 * kJ + c];
             psym(tv, xj + 3 * kJ, zi + 3 * kI);
             psym(tv, xi + 3 * kI, zj + 3 * kJ);
           }
+        }
       }
       const double sj = psum16(zj, lane);
       const bool b4 = lane & 16;
@@ -353,13 +477,19 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
       __syncthreads();
       if (t < 16 * kPM3) {
         const int f = t / kPM3, q = t % kPM3;
-        double si = 0.0;
-        for (int w8 = 0; w8 < 8; ++w8) si += zip[w8][f][q];
+        double s8[8];
+#pragma unroll
+        for (int w8 = 0; w8 < 8; ++w8) s8[w8] = zip[w8][f][q];
+        const double si = ((s8[0] + s8[1]) + (s8[2] + s8[3])) + ((s8[4] + s8[5]) + (s8[6] + s8[7]));
         const int fi = I * 16 + f, fj = J * 16 + f;
         if (fi < N) zs[fi * kPM3 + q] += si;
         if (fj < N) zs[fj * kPM3 + q] += zjs[f][q];
       }
+      const int Ln = next_own(L);
+      I += Ln - L;
+      L = Ln;
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the next records land on these rows
     csync();
     for (int u = t; u < (q1 - q0) / 3; u += kPT) {
       const int r0 = q0 + 3 * u, i = r0 / kPM3, k = (r0 % kPM3) / 3;
@@ -410,63 +540,83 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     }
     __syncthreads();
     int jc = 0;
-    for (int j = 0; j < m; ++j) {
-      float* w = V + (int64_t)(j + 1) * ldv;
-      matvec16(V + (int64_t)j * ldv, w);
-      const int nv = j + 1;
+    double nrm = 0.0;
+    // column j's rotation and the decision to stop, by one thread: the same
+    // values in every CTA of the cluster, so the same decisions
+    auto rotate = [&](int j) {
+      double* Hc = H + j * (j + 3) / 2;
+      for (int k = 0; k <= j; ++k) Hc[k] = hh[k] + hh2[k];
+      for (int k = 0; k < j; ++k) {
+        const double x0 = Hc[k], x1 = Hc[k + 1];
+        Hc[k] = cs[k] * x0 + sn[k] * x1;
+        Hc[k + 1] = -sn[k] * x0 + cs[k] * x1;
+      }
+      const double x0 = Hc[j], x1 = nrm;
+      const double rr = hypot(x0, x1);
+      const double c = rr > 0.0 ? x0 / rr : 1.0, s = rr > 0.0 ? x1 / rr : 0.0;
+      cs[j] = c;
+      sn[j] = s;
+      Hc[j] = rr;
+      g[j + 1] = -s * g[j];
+      g[j] = c * g[j];
+      const double est = fabs(g[j + 1]);
+      const bool nf = !isfinite(est);
+      flags[2] = nf ? 1 : 0;
+      flags[0] = (nf || est <= tol || j + 1 >= m || total >= P.maxit || nrm == 0.0) ? 1 : 0;
+    };
+    for (;;) {
+      // the last column's rotation runs beside the staging of the next product
+      stage_vector(V + (int64_t)jc * ldv, [&]() {
+        if (jc > 0) rotate(jc - 1);
+      });
+      if (jc > 0) {
+        bad = flags[2];
+        if (flags[0]) {
+          unstage();
+          break;
+        }
+      }
+      float* w = V + (int64_t)(jc + 1) * ldv;
+      matvec16(w);
+      const int nv = jc + 1;
       cdots(w, nv, false, hh);
       for (int q = q0 + t; q < q1; q += kPT) {
         double s = (double)w[q];
         for (int k = 0; k < nv; ++k) s -= hh[k] * (double)V[(int64_t)k * ldv + q];
         w[q] = (float)s;
       }
-      cdots(w, nv, false, hh2);
+      // ||w|| after the second pass is ||w'||^2 - sum h2^2 from that pass's own
+      // sums, from the entries when that cancels (the same in every CTA)
+      cdots(w, nv, true, hh2);
+      double nrm2 = hh2[nv];
+      const double ww = nrm2;
+      for (int k = 0; k < nv; ++k) nrm2 = fma(-hh2[k], hh2[k], nrm2);
+      const bool direct = nrm2 > 1e-3 * ww && isfinite(nrm2);
+      nrm = sqrt(nrm2);
+      const float sc = direct ? (float)(1.0 / nrm) : 1.f;
       for (int q = q0 + t; q < q1; q += kPT) {
         double s = (double)w[q];
         for (int k = 0; k < nv; ++k) s -= hh2[k] * (double)V[(int64_t)k * ldv + q];
-        w[q] = (float)s;
+        w[q] = (float)s * sc;
       }
-      const double nrm = sqrt(sumsq(w));
-      if (nrm > 0.0 && isfinite(nrm)) {
-        const float winv = (float)(1.0 / nrm);
-        for (int q = q0 + t; q < q1; q += kPT) w[q] *= winv;
-      }
-      if (t == 0) {   // the same values in every CTA of the cluster: the same decisions
-        double* Hc = H + (int64_t)j * ldh;
-        for (int k = 0; k < nv; ++k) Hc[k] = hh[k] + hh2[k];
-        Hc[j + 1] = nrm;
-        for (int k = 0; k < j; ++k) {
-          const double x0 = Hc[k], x1 = Hc[k + 1];
-          Hc[k] = cs[k] * x0 + sn[k] * x1;
-          Hc[k + 1] = -sn[k] * x0 + cs[k] * x1;
+      if (!direct) {
+        nrm2 = sumsq(w);
+        nrm = sqrt(nrm2);
+        if (nrm2 > 0.0 && isfinite(nrm2)) {
+          const float winv = (float)(1.0 / nrm);
+          for (int q = q0 + t; q < q1; q += kPT) w[q] *= winv;
         }
-        const double x0 = Hc[j], x1 = Hc[j + 1];
-        const double rr = hypot(x0, x1);
-        const double c = rr > 0.0 ? x0 / rr : 1.0, s = rr > 0.0 ? x1 / rr : 0.0;
-        cs[j] = c;
-        sn[j] = s;
-        Hc[j] = rr;
-        Hc[j + 1] = 0.0;
-        g[j + 1] = -s * g[j];
-        g[j] = c * g[j];
-        const double est = fabs(g[j + 1]);
-        const bool nf = !isfinite(est);
-        flags[2] = nf ? 1 : 0;
-        flags[0] = (nf || est <= tol || j + 1 >= m || total + 1 >= P.maxit || nrm == 0.0) ? 1 : 0;
       }
-      __syncthreads();
       ++total;
-      jc = j + 1;
-      if (flags[2]) bad = true;
-      if (flags[0]) break;
+      ++jc;
     }
     if (bad) break;
     // x += V y, H y = g (upper triangular, jc x jc)
     if (t == 0) {
       for (int i = jc - 1; i >= 0; --i) {
         double s = g[i];
-        for (int k = i + 1; k < jc; ++k) s -= H[(int64_t)k * ldh + i] * yv[k];
-        yv[i] = s / H[(int64_t)i * ldh + i];
+        for (int k = i + 1; k < jc; ++k) s -= H[k * (k + 3) / 2 + i] * yv[k];
+        yv[i] = s / H[i * (i + 3) / 2 + i];
       }
     }
     __syncthreads();
@@ -517,8 +667,10 @@ void pack_plan_ctas(const int* fibers, int n, int sms, int* ctas, int max_cluste
 
 size_t pack_smem_bytes(int Rmax, int m, int csize) {
   const size_t slots = (size_t)(kParts / csize);
-  const size_t doubles = (1 + slots) * (size_t)Rmax + 8 * 16 * 16 + 16 * 16 + (size_t)(m + 1) * m + 2 * (size_t)m +
-                         (size_t)(m + 1) + (size_t)m + 2 * (size_t)(m + 1) + 3 * kParts * (size_t)(m + 1) + 2;
+  const size_t doubles = (size_t)pack_tail_offset(Rmax, (int)slots) + kTileDoubles + (size_t)(m * (m + 3) / 2) +
+                         2 * (size_t)m +
+                         (size_t)(m + 1) + (size_t)m + (size_t)(m + 1) + (size_t)(m + 2) +
+                         3 * kParts * (size_t)(m + 2) + 2;
   return doubles * sizeof(double) + 4 * sizeof(int);
 }
 

@@ -421,6 +421,8 @@ struct rf_handle {
   int64_t device_bytes = 0;
   std::vector<void*> allocations;
 
+  void* host_io = nullptr;   // page-locked: state and results on their way
+  size_t io_size = 0;
   bool dry = false;          // count bytes only (rf_device_bytes_estimate)
   bool pooled = false;       // counted in the device pools' live handles
   // Stream-ordered allocations: creating or destroying a handle does not
@@ -469,6 +471,7 @@ struct rf_handle {
     pp.put(host_bctl, sizeof(BicgCtl));
     pp.put(host_ir_norm, sizeof(double));
     pp.put(host_vflag, sizeof(int));
+    pp.put(host_io, io_size);
     pp.put(lu.host_ipiv, (size_t)lu.R * sizeof(int));
     pp.put(lu.host_perm, (size_t)lu.R * sizeof(int));
     if (pooled) pools_release();
@@ -585,28 +588,27 @@ const char* rf_status_string(int s) {
 
 const char* rf_last_error(void) { return g_last_error.c_str(); }
 
-static void to_double4(const double* src, int N, std::vector<double>& out) {
-  out.assign((size_t)N * 4, 0.0);
-  for (int i = 0; i < N; ++i)
-    for (int a = 0; a < 3; ++a) out[(size_t)i * 4 + a] = src[(size_t)i * 3 + a];
+// State and results pass through the handle's page-locked block, a chunk of
+// fibers at a time where it is smaller than they are (5400 fibers at 256 KB).
+// Not counted in kernel_launches: that is the step's.
+constexpr size_t kIoBytes = 256 << 10;
+static size_t io_bytes(int N, int64_t R) {
+  return std::min(kIoBytes, std::max((size_t)N * 6 * sizeof(double), (size_t)R * sizeof(float)));
 }
 
 int rf_set_state(rf_handle* h, const double* pos, const double* ori) {
   if (!h || !pos || !ori) return RF_E_INPUT;
-  std::vector<double> p4, o4;
-  to_double4(pos, h->N, p4);
-  to_double4(ori, h->N, o4);
-  std::vector<float> p32((size_t)h->N * 4), o32((size_t)h->N * 4);
-  for (size_t k = 0; k < p4.size(); ++k) { p32[k] = (float)p4[k]; o32[k] = (float)o4[k]; }
-  const size_t b64 = (size_t)h->N * sizeof(double4), b32 = (size_t)h->N * sizeof(float4);
-  for (int s = 0; s < 2; ++s) {   // previous == current at the first step
-    const int idx = s == 0 ? h->icur : h->iprev;
-    RF_CUDA_TRY(cudaMemcpyAsync(h->pos64[idx], p4.data(), b64, cudaMemcpyHostToDevice, h->st));
-    RF_CUDA_TRY(cudaMemcpyAsync(h->ori64[idx], o4.data(), b64, cudaMemcpyHostToDevice, h->st));
+  double* io = static_cast<double*>(h->host_io);
+  const int per = (int)(io_bytes(h->N, h->R) / (6 * sizeof(double)));
+  for (int i0 = 0; i0 < h->N; i0 += per) {
+    const int n = std::min(per, h->N - i0);
+    std::memcpy(io, pos + 3 * (size_t)i0, (size_t)n * 3 * sizeof(double));
+    std::memcpy(io + 3 * (size_t)n, ori + 3 * (size_t)i0, (size_t)n * 3 * sizeof(double));
+    // previous == current at the first step
+    RF_TRY(launch_state_in(io, n, i0, h->pos64[h->icur], h->pos64[h->iprev], h->ori64[h->icur], h->ori64[h->iprev],
+                           h->pos32, h->ori32, h->st));
+    RF_CUDA_TRY(cudaStreamSynchronize(h->st));
   }
-  RF_CUDA_TRY(cudaMemcpyAsync(h->pos32, p32.data(), b32, cudaMemcpyHostToDevice, h->st));
-  RF_CUDA_TRY(cudaMemcpyAsync(h->ori32, o32.data(), b32, cudaMemcpyHostToDevice, h->st));
-  RF_CUDA_TRY(cudaStreamSynchronize(h->st));
   h->assembled = h->solved = false;
   h->vel_fresh = false;
   return RF_OK;
@@ -733,6 +735,8 @@ static int allocate_buffers(rf_handle* h, const rf_config* cfg) {
   if (!rc) rc = h->alloc((void**)&h->vpart, (size_t)velocity_rows(N) * N * 6 * sizeof(float));
   if (!rc) rc = h->alloc((void**)&h->vflag, sizeof(int));
   if (!rc && !h->dry && !(h->host_vflag = static_cast<int*>(pinned_pool().get(sizeof(int))))) rc = RF_E_OOM;
+  h->io_size = io_bytes(N, R);
+  if (!rc && !h->dry && !(h->host_io = pinned_pool().get(h->io_size))) rc = RF_E_OOM;
   return rc;
 }
 
@@ -1373,6 +1377,9 @@ static int pack_order_streams(rf_handle** hs, int n, cudaStream_t st) {
   for (int i = 0; i < n; ++i) {
     rf_handle* h = hs[i];
     if (h->st == st) continue;
+    const cudaError_t idle = cudaStreamQuery(h->st);
+    if (idle == cudaSuccess) continue;   // nothing to wait for: the usual case, the last pack was waited for
+    if (idle == cudaErrorNotReady) (void)cudaGetLastError();
     if (!h->order_ev) RF_CUDA_TRY(cudaEventCreateWithFlags(&h->order_ev, cudaEventDisableTiming));
     RF_CUDA_TRY(cudaEventRecord(h->order_ev, h->st));
     RF_CUDA_TRY(cudaStreamWaitEvent(st, h->order_ev, 0));
@@ -1665,42 +1672,41 @@ int rf_run(rf_handle* h, int first_timestep, int nsteps) {
   return RF_OK;
 }
 
-static int fetch3(rf_handle* h, const void* dev, bool is_double, double* out) {
-  const int N = h->N;
-  if (is_double) {
-    std::vector<double> tmp((size_t)N * 4);
-    RF_CUDA_TRY(cudaMemcpyAsync(tmp.data(), dev, tmp.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+// 3 doubles a fiber of u and of v (double4 or float4 a fiber on the device)
+static int fetch_rows(rf_handle* h, const void* u, const void* v, bool is_double, double* out_u, double* out_v) {
+  double* io = static_cast<double*>(h->host_io);
+  const int per = (int)(io_bytes(h->N, h->R) / (6 * sizeof(double)));
+  for (int i0 = 0; i0 < h->N; i0 += per) {
+    const int n = std::min(per, h->N - i0);
+    RF_TRY(is_double ? launch_rows_out(static_cast<const double4*>(u), static_cast<const double4*>(v), n, i0, io, h->st)
+                     : launch_rows_out(static_cast<const float4*>(u), static_cast<const float4*>(v), n, i0, io, h->st));
     RF_CUDA_TRY(cudaStreamSynchronize(h->st));
-    for (int i = 0; i < N; ++i)
-      for (int a = 0; a < 3; ++a) out[(size_t)i * 3 + a] = tmp[(size_t)i * 4 + a];
-  } else {
-    std::vector<float> tmp((size_t)N * 4);
-    RF_CUDA_TRY(cudaMemcpyAsync(tmp.data(), dev, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, h->st));
-    RF_CUDA_TRY(cudaStreamSynchronize(h->st));
-    for (int i = 0; i < N; ++i)
-      for (int a = 0; a < 3; ++a) out[(size_t)i * 3 + a] = tmp[(size_t)i * 4 + a];
+    std::memcpy(out_u + 3 * (size_t)i0, io, (size_t)n * 3 * sizeof(double));
+    std::memcpy(out_v + 3 * (size_t)i0, io + 3 * (size_t)n, (size_t)n * 3 * sizeof(double));
   }
   return RF_OK;
 }
 
 int rf_get_state(rf_handle* h, double* pos, double* ori) {
   if (!h || !pos || !ori) return RF_E_INPUT;
-  RF_TRY(fetch3(h, h->pos64[h->icur], true, pos));
-  return fetch3(h, h->ori64[h->icur], true, ori);
+  return fetch_rows(h, h->pos64[h->icur], h->ori64[h->icur], true, pos, ori);
 }
 
 int rf_get_velocities(rf_handle* h, double* tvel, double* rvel) {
   if (!h || !tvel || !rvel) return RF_E_INPUT;
   if (h->vlast < 0) { set_last_error_str("no velocities computed yet"); return RF_E_STATE; }
-  RF_TRY(fetch3(h, h->tv[h->vlast], false, tvel));
-  return fetch3(h, h->rv[h->vlast], false, rvel);
+  return fetch_rows(h, h->tv[h->vlast], h->rv[h->vlast], false, tvel, rvel);
 }
 
 static int fetch_vec(rf_handle* h, const float* dev, double* out) {
-  std::vector<float> tmp((size_t)h->R);
-  RF_CUDA_TRY(cudaMemcpyAsync(tmp.data(), dev, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, h->st));
-  RF_CUDA_TRY(cudaStreamSynchronize(h->st));
-  for (int64_t r = 0; r < h->R; ++r) out[r] = tmp[r];
+  float* io = static_cast<float*>(h->host_io);
+  const int64_t per = (int64_t)(io_bytes(h->N, h->R) / sizeof(float));
+  for (int64_t r0 = 0; r0 < h->R; r0 += per) {
+    const int64_t n = std::min(per, h->R - r0);
+    RF_TRY(launch_vector_out(dev + r0, (int)n, io, h->st));
+    RF_CUDA_TRY(cudaStreamSynchronize(h->st));
+    for (int64_t r = 0; r < n; ++r) out[r0 + r] = io[r];
+  }
   return RF_OK;
 }
 

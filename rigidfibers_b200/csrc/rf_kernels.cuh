@@ -285,4 +285,10 @@ __device__ __forceinline__ void update_fiber(int i, int first, double dt, double
 int launch_update_fibers(int N, int first, double dt, double4* pp, double4* cp, double4* po, double4* co,
                          float4* ptv, const float4* ctv, float4* prv, const float4* crv, float4* pos32, float4* ori32,
                          const int* halt, cudaStream_t st);
+// State and results between page-locked host memory and the device
+int launch_state_in(const double* host, int n, int i0, double4* p0, double4* p1, double4* o0, double4* o1, float4* p32,
+                    float4* o32, cudaStream_t st);
+int launch_rows_out(const double4* u, const double4* v, int n, int i0, double* host, cudaStream_t st);
+int launch_rows_out(const float4* u, const float4* v, int n, int i0, double* host, cudaStream_t st);
+int launch_vector_out(const float* x, int n, float* host, cudaStream_t st);
 }  // namespace rf

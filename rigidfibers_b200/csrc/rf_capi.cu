@@ -377,6 +377,7 @@ struct rf_handle {
   GmresCtl* ctl = nullptr;
   GmresCtl* host_ctl = nullptr;
   LuSetup lu{};                   // direct solver workspace
+  LuLane lu_lane;
   float* bicg_work = nullptr;     // BiCGSTAB vectors r, r0, p, v, s, t
   BicgCtl* bctl = nullptr;
   BicgCtl* host_bctl = nullptr;
@@ -464,6 +465,7 @@ struct rf_handle {
     gmres_graphs.release();
     release_step_graphs();
     for (auto e : mv_events) cudaEventDestroy(e);
+    lu_lane.release();
     for (void* p : allocations) cudaFreeAsync(p, st);
     if (st) cudaStreamSynchronize(st);
     PinnedPool& pp = pinned_pool();
@@ -696,6 +698,7 @@ static int allocate_buffers(rf_handle* h, const rf_config* cfg) {
   if (!rc && !h->dry && !(h->host_ctl = static_cast<GmresCtl*>(pinned_pool().get(sizeof(GmresCtl))))) rc = RF_E_OOM;
   if (cfg->solver == RF_SOLVER_DIRECT) {
     LuSetup& L = h->lu;
+    L.lane = &h->lu_lane;
     L.R = R;
     L.lda = h->lda;
     L.tol = cfg->refinement_tolerance;
@@ -2142,6 +2145,8 @@ int rf_dense_lu_solve(const float* A, const float* b, float* x, int64_t R, doubl
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaStream_t st = (cudaStream_t)stream;
   LuSetup L{};
+  LuLane lane;
+  L.lane = &lane;
   L.R = R;
   L.lda = R;
   L.ldlu = ceil_div(R, 32) * 32;   // factors with 128-byte aligned columns (the tensor-core path's TMA needs
@@ -2186,6 +2191,7 @@ int rf_dense_lu_solve(const float* A, const float* b, float* x, int64_t R, doubl
   L.host_perm = hp.data();
   LuResult lr;
   if (!rc) rc = lu_factor_solve(L, A, b, x, st, &lr);
+  lane.release();
   for (void* p : mem) cudaFreeAsync(p, st);
   cudaStreamSynchronize(st);
   return rc;

@@ -7,6 +7,14 @@ namespace rf {
 // column splits of the refinement residual (bounds the rpart buffer)
 constexpr int kLuResidualSplits = 32;
 
+// The side stream of the tensor-core factorization and its events.
+struct LuLane {
+  cudaStream_t side = nullptr;
+  cudaEvent_t forked = nullptr, rows = nullptr, right = nullptr;
+  int open();        // created on first use
+  void release();    // waits for the side stream first
+};
+
 struct LuSetup {
   int64_t R;
   int64_t lda;        // leading dimension of A
@@ -36,6 +44,7 @@ struct LuSetup {
   float* inv = nullptr;    // lu_tc_inv_floats(): the diagonal block's L^-1 and U^-T
   int* flags = nullptr;    // 2: largest |l| (float bits), status
   float* sinv = nullptr;   // lu_tc_sinv_floats(R): each diagonal block's L^-1 and U^-1 (triangular solves)
+  LuLane* lane = nullptr;
   bool use_tc = true;
 };
 

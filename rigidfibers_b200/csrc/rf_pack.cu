@@ -316,13 +316,24 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     if (lane == 0)
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(psmem(&copied[warp])) : "memory");
   };
+  // a member's vector into shared memory, 8 loads in flight
+  auto copy_in = [&](auto* dst, const auto* src) {
+    for (int r0 = t; r0 < R; r0 += 8 * kPT) {
+      std::remove_reference_t<decltype(*dst)> v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = r0 + u * kPT < R ? src[r0 + u * kPT] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r0 + u * kPT < R) dst[r0 + u * kPT] = v[u];
+    }
+  };
   // v into shared memory, this CTA's rows of T v cleared and the first tile's
   // records on their way; meanwhile one thread runs `aside`
   auto stage_vector = [&](const float* v, auto&& aside) {
     if (p0 < ntiles) fetch(p0);
     csync();                                                   // every CTA's rows of v are written
     if (t == kPT - 1) aside();
-    for (int r = t; r < R; r += kPT) sxf[r] = v[r];
+    copy_in(sxf, v);
     for (int q = t; q < spc * Rmax; q += kPT) zpf[q] = 0.f;
     __syncthreads();
   };
@@ -425,7 +436,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
   auto residual64 = [&](float* r) {
     for (int q = t; q < spc * Rmax; q += kPT) zpd[q] = 0.0;
     csync();                                                   // every CTA's rows of x are written
-    for (int q = t; q < R; q += kPT) sxd[q] = P.x64[q];
+    copy_in(sxd, static_cast<const double*>(P.x64));
     __syncthreads();
     int I = p0, J = 0;
     for (int L = p0; L < ntiles;) {

@@ -242,9 +242,11 @@ typedef struct rf_tune_report {
   int panel_blocks;         /* direct solver: blocks of the LU panel kernel (one
                                grid sync per column): SMs, SMs/2, SMs/4 tried */
   double panel_ms[3];       /* first panel's time per candidate (-1: rows do not fit) */
-  int asm_variant;          /* numerical assembly's pair-tile kernel: 0 scalar FP32,
-                               1 packed two-lane FP32 (f32x2) for mirror points; both
-                               give bit-identical operators */
+  int asm_variant;          /* numerical assembly's pair-tile kernel, for the pairs
+                               whose blocks take the full quadrature (the distant
+                               ones have one kernel): 0 scalar FP32, 1 packed two-lane
+                               FP32 (f32x2) for mirror points; both give
+                               bit-identical operators */
   double asm_ms[2];         /* one assembly per candidate (-1: not tried, analytical) */
 } rf_tune_report;
 int rf_autotune(rf_handle* h, rf_tune_report* report);

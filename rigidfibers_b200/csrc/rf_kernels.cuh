@@ -30,7 +30,8 @@ int assemble_tiles(int M, int Q, int N);
 
 // Kernel variants of the numerical pair tiles (rf_autotune picks one; both
 // give bit-identical results): 0 scalar FP32, 1 packed two-lane FP32
-// (add/mul/fma .f32x2) for the two mirror points of each folded pair.
+// (add/mul/fma .f32x2) for the two mirror points of each folded pair.  Only the
+// near pairs differ: the far ones are evaluated packed in both.
 constexpr int kAsmVariants = 2;
 // Numerical assembly.  ffpart: (assemble_tiles(M,Q,N) + 1) x N x 3(M+1) floats of
 // scratch; F: N x 3(M+1) force terms sum_j T^{ij}[k][P0] F/2; b: R.  pos64:

@@ -9,7 +9,7 @@
 // and only the M^2 blocks of each unordered pair (150 values at M = 5) have to
 // be read: 2.4 GB in FP16 at N = 4000 against 14.4 GB for dense FP32.
 //
-// Storage (written by k_assemble_numerical in structured mode): 16x16 fiber
+// Storage (written by k_assemble_pairs in structured mode): 16x16 fiber
 // storage tiles over the upper triangle; inside, (16/TI)^2 assembly
 // sub-tiles of TI x TI pairs.  FP32 blocks as [j][value][i] (values in
 // s32_block order: the operator blocks lead), so a warp reads whole 32-byte

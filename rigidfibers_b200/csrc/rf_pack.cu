@@ -11,10 +11,10 @@
 // Work of a member is cut into kParts = 8 fixed parts whatever C is: storage
 // tile L belongs to partition L mod 8, whose partial rows are summed in tile
 // order; row slice s is fibers [s N / 8, (s + 1) N / 8), whose dot-product
-// partial its owner's warps sum in a fixed order.  A CTA of the cluster owns 8 / C consecutive
-// partitions and slices; the partitions' partial rows and the slices'
-// partials are added in part order through distributed shared memory after a
-// cluster barrier.  So a member's solution is the same bits for any C, alone
+// partial its owner's warps sum in a fixed order.  A CTA of the cluster owns
+// 8 / C consecutive partitions and slices; the partitions' partial rows and the
+// slices' partials are added in part order through distributed shared memory
+// after a cluster barrier.  So a member's solution is the same bits for any C, alone
 // and in any pack (it differs from rf_solve's in summation order only), and a
 // pack can give its large members more SMs when the GPU has them to spare.
 //

@@ -220,9 +220,13 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
 // 256: barriers of four warps, more CTAs to fill them; N=4000 3.09 -> 2.42 ms).
 // Matrix-free product and dense output: 256, where the product's 160 and the
 // block stores' 800 tasks of a batch split better (N=2500 product 0.90 against
-// 1.23 ms, N=2000 dense 1.55 against 1.77); 128 for more than 5 terms, whose G
-// and T of 32 pairs would leave one CTA per SM.
-constexpr int num_threads(int M, int mode) { return mode == kAsmStructF16 || mode == kAsmStructBF16 || M > 5 ? 128 : 256; }
+// 1.23 ms, N=2000 dense 1.55 against 1.77).  More than 5 terms: batches of 16
+// pairs, since G and T of 32 would leave one CTA per SM, on 128 threads; on 256 for
+// 8 terms, whose 144 force-term sums of a batch need a thread each (whole steps of
+// 37 and 1500 fibers, matrix-free: 0.54 and 18.2 ms, with 160 threads 0.68 and 19.7).
+constexpr int num_threads(int M, int mode) {
+  return M > 7 ? 256 : mode == kAsmStructF16 || mode == kAsmStructBF16 || M > 5 ? 128 : 256;
+}
 
 template <int M, int Q, int NTH>
 struct NumShape {
@@ -232,7 +236,8 @@ struct NumShape {
   static constexpr int NC2 = 6 * KP;                       // G columns, pairs of floats
   static constexpr int NT = NTH;
   static constexpr int FN = kFarNodes;
-  static constexpr int PB = NT / FN < TI * TI ? NT / FN : TI * TI;   // far pairs per batch
+  static constexpr int FB = (M > 5 ? 128 : NT) / FN;
+  static constexpr int PB = FB < TI * TI ? FB : TI * TI;   // far pairs per batch
   static constexpr int JB = PB / TI;                       // j of a batch
   static constexpr int GSF = PB * FN + PB % 32;            // G column stride (float2): lanes (col, pair)
   static constexpr int NS = NT / Q < TI ? NT / Q : TI;     // near pairs per group
@@ -248,6 +253,7 @@ struct NumShape {
   static constexpr int TFLOATS = JB * JS > PB * TP ? JB * JS : PB * TP;
   static constexpr size_t kSmem = sizeof(float) * (GFLOATS + TFLOATS);
   static_assert(PB % TI == 0 && TI % JB == 0 && 32 % PB == 0, "batches are whole j and part of one mask word");
+  static_assert(PB * FN <= NT && PB * K1 <= NT, "a far point and an i-side sum (force terms, or fewer: z) per thread");
   static_assert(JS % 4 == 0 && NQ32 * TI % 4 == 0, "a j's values are copied out from a 16-byte boundary");
 };
 
@@ -623,7 +629,7 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
 }
 
 template <int M, int Q, int MODE, bool P2>
-__global__ void __launch_bounds__(num_threads(M, MODE), M > 5 ? 4 : num_threads(M, MODE) == 128 ? 6 : 3)
+__global__ void __launch_bounds__(num_threads(M, MODE), M > 7 ? 2 : M > 5 ? 4 : num_threads(M, MODE) == 128 ? 6 : 3)
 k_assemble_pairs(const Tables tab, int N, const float4* __restrict__ ori, AsmOut out) {
   if (MODE == kAsmApply && out.skip != nullptr && *out.skip) return;
   int I, J;

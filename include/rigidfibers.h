@@ -173,7 +173,7 @@ int rf_run(rf_handle* h, int first_timestep, int nsteps);
  * 5 force terms, 8x3 quadrature, at most 256 fibers, one restart length.  A
  * member's result depends only on its own data, so it is the same alone and
  * in any pack (it may differ from rf_solve's in the last bits: the sums run
- * in another order).  Returns RF_E_NAN / RF_E_NOCONV if a member ended so;
+ * in another order).  Returns RF_E_TIMEOUT / RF_E_NAN / RF_E_NOCONV if a member ended so;
  * rf_last_stats has each member's counts. */
 int rf_solve_packed(rf_handle** handles, int n);
 /* One time step of n suspensions with a packed solve: rf_assemble on each,
@@ -405,9 +405,10 @@ int rf_server_destroy(rf_server* s);
 
 /* Fault injection for tests (no counterpart in the reference, which prints and
  * continues).  rf_debug_set_device_wait_limit(0) makes the first bounded
- * device-side wait of the TMA-pipelined matvec and of the tensor-core LU
- * update give up at once, so the calls return RF_E_TIMEOUT and the handle stays
- * usable; -1 restores the limits (2^24 polls, one second).
+ * device-side wait of the TMA-pipelined matvec, of the packed solve, of the
+ * triangular solves and of the tensor-core LU update give up at once, so the
+ * calls return RF_E_TIMEOUT and the handle stays usable; -1 restores the limits
+ * (2^24 polls, one second).
  * rf_debug_fail_allocation_after(n): the n-th device allocation of rf_create
  * from now on fails (RF_E_OOM); -1 disables. */
 int rf_debug_set_device_wait_limit(int64_t limit);

@@ -1422,6 +1422,8 @@ static void pack_member(rf_handle* h, int* out, double* relres, PackMember* q) {
   q->S32 = h->S32;
   q->ori = h->ori32;
   q->b = h->b;
+  const int64_t lim = device_wait_limit();
+  q->wait_ns = lim < 0 ? 1000000000ull : (uint64_t)lim;
   q->x64 = h->x64;
   q->x = h->x;
   q->V = h->V;
@@ -1444,8 +1446,9 @@ static int pack_record_solve(rf_handle* h, const int* o, double relres) {
   h->stats.refinement_steps = o[2];
   h->stats.relative_residual = relres;
   h->stats.graph_replays = 0;
-  h->pack_status = o[3] == 0 ? RF_OK : (o[3] == 1 ? RF_E_NOCONV : RF_E_NAN);
-  if (h->pack_status != RF_E_NAN) h->solved = true;
+  h->pack_status = o[3] == 0 ? RF_OK : o[3] == 1 ? RF_E_NOCONV : o[3] == 3 ? RF_E_TIMEOUT : RF_E_NAN;
+  if (o[3] == 3) set_last_error_str("a bounded device-side wait timed out");
+  if (o[3] < 2) h->solved = true;
   return h->pack_status;
 }
 
@@ -1494,7 +1497,7 @@ int rf_solve_packed(rf_handle** hs, int n) {
     rf_handle* h = hs[i];
     h->launches += (i == 0) ? 1 : 0;
     const int s = pack_record_solve(h, &out[(size_t)i * 4], rel[(size_t)i]);
-    if (s == RF_E_NAN) worst = RF_E_NAN;
+    if (s == RF_E_TIMEOUT || (s == RF_E_NAN && worst != RF_E_TIMEOUT)) worst = s;
     else if (s == RF_E_NOCONV && worst == RF_OK) worst = RF_E_NOCONV;
   }
   return worst;
@@ -1505,8 +1508,8 @@ int rf_solve_packed(rf_handle** hs, int n) {
 // the packed assembly (k_pack_assemble, k_pack_force_terms); the packed solve
 // of all members; per group the packed velocities and update (k_pack_velocity,
 // k_pack_finish).  One upload of the descriptors, one download of the
-// outcomes, one synchronisation.  A member whose solve ends non-finite keeps
-// its state; one whose velocities are not finite has taken the step and
+// outcomes, one synchronisation.  A member whose solve fails (non-finite, timed
+// out) keeps its state; one whose velocities are not finite has taken the step and
 // reports RF_E_NAN (as rf_step's stages do).
 int rf_step_packed(rf_handle** hs, const int* timesteps, int n, int* status) {
   if (!hs || !timesteps || !status || n < 1) return RF_E_INPUT;
@@ -1642,7 +1645,7 @@ int rf_step_packed(rf_handle** hs, const int* timesteps, int n, int* status) {
     h->assembled = true;
     h->solved = false;
     int s = pack_record_solve(h, &out[(size_t)i * 4], rel[i]);
-    if (s != RF_E_NAN) {
+    if (s == RF_OK || s == RF_E_NOCONV) {
       // velocities computed, state rotated in place (as rf_update_velocities + rf_update_fibers)
       h->vlast = h->vcur;
       h->vel_fresh = false;

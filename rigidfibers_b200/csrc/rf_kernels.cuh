@@ -113,7 +113,9 @@ struct PackMember {
   float* x;                      // solution (FP32 copy)
   float* V;                      // Krylov basis, m + 1 columns of ldv floats
   int64_t ldv;
-  int* out;                      // iterations, restarts, refinements, status (0 ok, 1 no convergence, 2 non-finite)
+  uint64_t wait_ns;              // limit of the wait for a tile's records (0: give up at once)
+  int* out;                      // iterations, restarts, refinements, status (0 ok, 1 no convergence, 2 non-finite,
+                                 // 3 a bounded wait gave up)
   double* relres;                // ||b - A x|| / ||b|| at the last check
   float coef[5], eig[5];         // C_k = coef_k (I - E_k t t^T), k >= 1; coef_0 t t^T
 };
@@ -148,7 +150,7 @@ struct PackStepMember {
   int N, first;               // fibers; 1 on a first (Euler) step
   int asm_start, vel_start;   // first block of the member in the group's grids
   double dt;
-  const int* solve_status;    // the packed solve's status word (2: non-finite, the member sits out)
+  const int* solve_status;    // the packed solve's status word (2 and 3: it failed, the member sits out)
   int* vbad;                  // set to 1 when a velocity is not finite, else 0
   double4 *pos64, *pos64_prev, *ori64, *ori64_prev;   // FP64 state: current, previous
   float4 *pos32, *ori32;      // FP32 copies of the current state

@@ -63,21 +63,31 @@ __host__ __device__ __forceinline__ int pack_tail_offset(int Rmax, int slots) { 
 }
 
 __device__ __forceinline__ uint32_t psmem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// wait for an mbarrier's phase; false after a second
-__device__ __forceinline__ bool pack_wait(uint64_t* bar, uint32_t parity) {
-  uint64_t t0 = 0, now;
+// Wait for an mbarrier's phase.  Past limit_ns (0: at once) *late is set, and the
+// wait goes on for a second, so that the copy does not land on what comes next.
+constexpr uint64_t kPackDrainNs = 1000000000ull;
+__device__ __forceinline__ void pack_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns, int* late) {
+  uint64_t t0 = 0, now, left = limit_ns;
+  bool over = false;
   for (int n = 0;; ++n) {
+    if (left == 0) {
+      if (over) return;
+      over = true;
+      *late = 1;   // every writer stores the same value
+      left = kPackDrainNs;
+      t0 = 0;
+    }
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done)
         : "r"(psmem(bar)), "r"(parity)
         : "memory");
-    if (done) return true;
+    if (done) return;
     if ((n & 63) == 63) {
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
-      if (now - t0 > 1000000000ull) return false;
+      if (now - t0 > left) left = 0;
     }
   }
 }
@@ -196,7 +206,8 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
   double* dpart = hh2 + m + 2;                                  // [3][kParts][m+2]
   double* red = tail;                                           // warp partials, outside the products
   double* scal = dpart + 3 * kParts * (m + 2);
-  int* flags = reinterpret_cast<int*>(scal + 2);                // [0] cycle done, [1] converged, [2] non-finite
+  // [0] cycle done, [2] non-finite, [3] a wait for records of a product gave up ([1]: of one not wanted)
+  int* flags = reinterpret_cast<int*>(scal + 2);
   float* V = P.V;
   const int64_t ldv = P.ldv;
   const int i16 = t & 15, j16 = t >> 4;
@@ -211,9 +222,9 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (t == 0) flags[3] = 0;
   __syncthreads();
   uint32_t phase = 0;                                          // of this warp's copies
-  bool lost = false;                                           // one of them never arrived
   int rb = 0;                                                  // reduction buffer in use (of 3)
   // a cluster barrier, or the block barrier when the member has one CTA
   auto csync = [&]() {
@@ -337,10 +348,11 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     for (int q = t; q < spc * Rmax; q += kPT) zpf[q] = 0.f;
     __syncthreads();
   };
-  // the staged product is not wanted: take in the records that were fetched
+  // the staged product is not wanted: the records that were fetched must still
+  // arrive before their room is used again or the CTA ends
   auto unstage = [&]() {
     if (p0 < ntiles) {
-      lost |= !pack_wait(&copied[warp], phase);
+      pack_wait(&copied[warp], phase, kPackDrainNs, &flags[1]);
       phase ^= 1;
     }
   };
@@ -359,7 +371,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
       float* zs = zpf + (size_t)(L % kParts - p0) * Rmax;
       while (I > J) I -= ++J;   // storage tile L = J (J + 1) / 2 + I
       const int i = I * 16 + i16, j = J * 16 + j16;
-      lost |= !pack_wait(&copied[warp], phase);
+      pack_wait(&copied[warp], phase, P.wait_ns, &flags[3]);
       phase ^= 1;
       uint32_t wv[kNW];
 #pragma unroll
@@ -383,7 +395,6 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
         if (P.smode == 2) ppair16<__nv_bfloat16>(wv, xi, xj, zi, zj);
         else ppair16<__half>(wv, xi, xj, zi, zj);
       }
-      if (lost) zj[0] = nanf("");   // the solve ends as non-finite
       const float sj = psum16(zj, lane);   // z_j over this half-warp's 16 i
       const bool b4 = lane & 16;
       float u8[8];                          // z_i over this warp's two j: one halving exchange
@@ -411,6 +422,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
       L = Ln;
     }
     csync();                                                   // every partition's rows are complete
+    const bool late = flags[3] != 0;                           // the solve ends as non-finite, in every CTA
     for (int u = t; u < (q1 - q0) / 3; u += kPT) {
       const int r0 = q0 + 3 * u, i = r0 / kPM3, k = (r0 % kPM3) / 3;
       float z3[3] = {0.f, 0.f, 0.f};
@@ -428,7 +440,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const float cz = k == 0 ? coef * t3[a] * tz : coef * (z3[a] - E * t3[a] * tz);
-        w[r0 + a] = sxf[r0 + a] + cz;
+        w[r0 + a] = late ? nanf("") : sxf[r0 + a] + cz;
       }
     }
   };
@@ -639,6 +651,9 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
     ++restarts;
   }
   status = bad ? 2 : (conv ? 0 : 1);
+  if (bad && rank == 0 && t == 0)
+    for (int r = 0; r < C; ++r)
+      if (at_rank(flags, r)[3]) status = 3;
   for (int q = q0 + t; q < q1; q += kPT) P.x[q] = (float)P.x64[q];
   if (rank == 0 && t == 0) {
     P.out[0] = total;

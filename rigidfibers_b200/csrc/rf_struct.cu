@@ -948,15 +948,15 @@ k_struct_velocity_finalize(const Tables tab, int N, const float4* __restrict__ o
 }
 
 // ---- packed step: velocities and update of every member of one group -----
-// Members whose packed solve ended non-finite (status 2) sit out: their state
-// stays as it is.  Per member the arithmetic is the single-suspension path's
+// Members whose packed solve failed (non-finite or timed out, status 2 and 3) sit
+// out: their state stays as it is.  Per member the arithmetic is the single-suspension path's
 // (k_struct_velocity, k_struct_velocity_finalize, the non-finite guard,
 // k_update_fibers), so a member's step is bit for bit the one it takes alone.
 __global__ void __launch_bounds__(256)
 k_pack_velocity(const PackStepMember* __restrict__ mem, int n) {
   const int L = (int)blockIdx.x;
   const PackStepMember& p = mem[pack_member_of(n, L, [&](int m) { return mem[m].vel_start; })];
-  if (*p.solve_status == 2) return;
+  if (*p.solve_status >= 2) return;
   struct_velocity_tile<5, 8>(p.N, p.S32, p.x, p.vpart, (unsigned)(L - p.vel_start));
 }
 
@@ -964,7 +964,7 @@ k_pack_velocity(const PackStepMember* __restrict__ mem, int n) {
 __global__ void __launch_bounds__(128)
 k_pack_finish(const Tables tab, const PackStepMember* __restrict__ mem) {
   const PackStepMember& p = mem[blockIdx.x];
-  if (*p.solve_status == 2) return;
+  if (*p.solve_status >= 2) return;
   const int N = p.N, nparts = (N + kStoreTile - 1) / kStoreTile;
   int bad = 0;
   for (int i = threadIdx.x; i < N; i += blockDim.x) {

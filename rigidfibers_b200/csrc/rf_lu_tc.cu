@@ -1012,6 +1012,9 @@ struct TrsvArgs {
 constexpr int kTrsvThreads = 512;
 constexpr int kTrsvMaxSmem = 200 * 1024;   // 400 owned blocks of a CTA
 
+// SHARED: the owned blocks' right-hand sides in shared memory; else, for grids
+// capped so far that a CTA owns more of them than fit, where they are in y.
+template <bool SHARED>
 __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
   extern __shared__ float ys[];            // [owned blocks][128]
   __shared__ float xs[kPanel];
@@ -1024,10 +1027,11 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
   // owns the positions p, p + P, ..
   auto block_at = [&](int q) { return a.lower ? q : nb - 1 - q; };
   auto rows_of = [&](int b) { return (int)min((int64_t)kPanel, R - (int64_t)b * kPanel); };
-  for (int q = p, o = 0; q < nb; q += P, ++o) {
-    const int b = block_at(q);
-    if (tid < kPanel) ys[o * kPanel + tid] = tid < rows_of(b) ? a.y[(int64_t)b * kPanel + tid] : 0.f;
-  }
+  if constexpr (SHARED)
+    for (int q = p, o = 0; q < nb; q += P, ++o) {
+      const int b = block_at(q);
+      if (tid < kPanel) ys[o * kPanel + tid] = tid < rows_of(b) ? a.y[(int64_t)b * kPanel + tid] : 0.f;
+    }
   if (tid == 0) fail = 0;
   __syncthreads();
   auto load_block = [&](int rb, int cb, float (&m)[32]) {   // rows of block rb, columns of block cb
@@ -1036,14 +1040,15 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
 #pragma unroll
     for (int c = 0; c < 32; ++c) m[c] = (i < nq && h * 32 + c < nr) ? __ldcs(col + (int64_t)c * a.lda) : 0.f;
   };
-  // y -= m xs for the owned block o (thread (i, h) holds 32 columns of row i)
-  auto update = [&](const float (&m)[32], int o) {
+  // y -= m xs for block b, the o-th owned (thread (i, h) holds 32 columns of row i)
+  auto update = [&](const float (&m)[32], int b, int o) {
     float v = 0.f;
 #pragma unroll
     for (int c = 0; c < 32; ++c) v = fmaf(m[c], xs[h * 32 + c], v);
     part[h][i] = v;
     __syncthreads();
-    if (tid < kPanel) ys[o * kPanel + tid] -= (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
+    float* yo = SHARED ? ys + o * kPanel : a.y + (int64_t)b * kPanel;
+    if (tid < (SHARED ? kPanel : rows_of(b))) yo[tid] -= (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]);
     __syncthreads();
   };
   float inv[32];
@@ -1052,11 +1057,13 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
 #pragma unroll
     for (int q = 0; q < 32; ++q) inv[q] = __ldcs(s + (int64_t)(h * 32 + q) * kPanel + i);
   };
-  // x_b from the owned block o: into y and xs, then the flag
+  // x_b from block b, the o-th owned: into y, then the flag
   auto publish = [&](int b, int o) {
+    const float* yo = SHARED ? ys + o * kPanel : a.y + (int64_t)b * kPanel;
+    const int rows = SHARED ? kPanel : rows_of(b);
     float v = 0.f;
 #pragma unroll
-    for (int q = 0; q < 32; ++q) v = fmaf(inv[q], ys[o * kPanel + h * 32 + q], v);
+    for (int q = 0; q < 32; ++q) v = fmaf(inv[q], SHARED || h * 32 + q < rows ? yo[h * 32 + q] : 0.f, v);
     part[h][i] = v;
     __syncthreads();
     if (tid < kPanel) {
@@ -1097,7 +1104,7 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
     if (fail) return;   // the same in every thread
     if (tid < kPanel) xs[tid] = tid < rows_of(b) ? __ldcg(a.y + (int64_t)b * kPanel + tid) : 0.f;
     __syncthreads();
-    update(m, own);
+    update(m, block_at(mine), own);
     int q2 = mine + P, o2 = own + 1;
     if (next) {
       publish(block_at(mine), own);
@@ -1106,7 +1113,7 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
     }
     for (; q2 < nb; q2 += P, ++o2) {
       load_block(block_at(q2), b, m);
-      update(m, o2);
+      update(m, block_at(q2), o2);
     }
   }
 }
@@ -1262,17 +1269,15 @@ int lu_solve_tc(const LuSetup& s, const float* rhs, float* x, cudaStream_t st) {
   const int P = std::max(1, std::min(std::min(s.coop_blocks, t.nblocks), sms));
   const size_t smem = sizeof(float) * kPanel * (size_t)ceil_div(t.nblocks, P);
   static const cudaError_t attr =
-      cudaFuncSetAttribute(k_trsv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrsvMaxSmem);
+      cudaFuncSetAttribute(k_trsv_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrsvMaxSmem);
   RF_CUDA_TRY(attr);
-  if (smem > (size_t)kTrsvMaxSmem) {
-    set_last_error_str("lu: too many row blocks per multiprocessor");
-    return RF_E_UNSUPPORTED;
-  }
+  const bool shared = smem <= (size_t)kTrsvMaxSmem;
+  const void* fn = shared ? (const void*)k_trsv_tc<true> : (const void*)k_trsv_tc<false>;
   for (int lower = 1; lower >= 0; --lower) {
     t.lower = lower;
     RF_CUDA_TRY(cudaMemsetAsync(t.flag, 0, (size_t)t.nblocks * sizeof(int), st));
     void* args[] = {&t};
-    RF_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_trsv_tc, dim3(P), dim3(kTrsvThreads), args, smem, st));
+    RF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(P), dim3(kTrsvThreads), args, shared ? smem : 0, st));
   }
   return RF_OK;
 }

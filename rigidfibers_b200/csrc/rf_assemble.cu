@@ -330,7 +330,7 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
       sD[pr][1] = dy;
       sD[pr][2] = dz;
       const bool valid = i0 + il < N && j0 + jl < N && (!diag || il < jl);
-      near_pair = valid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < tab.far_d2;
+      near_pair = valid && !far_pair(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), tab.far_d2);
       sKind[pr] = near_pair ? 2 : valid ? 1 : 0;
     }
     const unsigned m = __ballot_sync(0xffffffffu, near_pair);
@@ -722,7 +722,7 @@ __device__ __forceinline__ void analytical_near(const Tables& tab, int N, const 
   int count = 0;
   for (int js = 0; js < N; js += NT) {
     const int j = js + tid;
-    const bool near = j < N && j != i && centre_dist2(xi, out.pos64[j]) < tab.far_d2;
+    const bool near = j < N && j != i && !far_pair(centre_dist2(xi, out.pos64[j]), tab.far_d2);
     const unsigned m = __ballot_sync(0xffffffffu, near);
     if (lane == 0) warp_near[warp] = __popc(m);
     __syncthreads();
@@ -799,7 +799,7 @@ k_assemble_analytical(const Tables tab, int N, const float4* __restrict__ ori, A
     const int il = pr % TI, jl = pr / TI;
     const bool valid = i0 + il < N && j0 + jl < N && (!diag || il != jl);
     const float d2 = centre_dist2(out.pos64[min(i0 + il, N - 1)], out.pos64[min(j0 + jl, N - 1)]);
-    sKind[pr] = !valid ? 0 : d2 < tab.far_d2 ? 2 : 1;
+    sKind[pr] = !valid ? 0 : far_pair(d2, tab.far_d2) ? 1 : 2;
   }
   const float fz = tab.fz_half;
   // force-term accumulator of task (tl, k) = (tid / K1, tid % K1): F_i[k]

@@ -29,7 +29,7 @@ struct Tables {
   // {pts, w}, which gives that sum exactly for polynomials of degree
   // 2 kFarNodes - 1, hence the sums against P_0..P_M of any kernel that is
   // smooth on the fiber.  far_W[k][q] = weight x P_k, far_W2 as W2; pairs with
-  // |x_i - x_j|^2 >= far_d2 take it.
+  // |x_i - x_j|^2 >= far_d2 take it (far_pair).
   float far_pts[kFarNodes];
   float far_W[kMaxTerms + 1][kFarNodes];
   float2 far_W2[kMaxTerms / 2 + 1][kFarNodes / 2];
@@ -91,6 +91,16 @@ __device__ __forceinline__ double f2d(float v) {
   double d;
   asm("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(v));
   return d;
+}
+
+// Whether a pair whose centres are sqrt(d2) apart takes the far rule.  A pair
+// whose distance is not a number or too large for FP32 squares takes the full
+// rule: its reciprocal root of infinity is 0 and the kernel vanishes, where the
+// far rule's Newton step would form infinity times 0.
+constexpr float kFarMaxD2 = 1e37f;
+__device__ __forceinline__ bool far_pair(float d2, float far_d2) {
+  // squares are not negative: their bit patterns order as they do, NaN and infinity last
+  return __float_as_uint(d2) - __float_as_uint(far_d2) <= __float_as_uint(kFarMaxD2) - __float_as_uint(far_d2);
 }
 
 // Symmetric 3x3 stored as (11, 22, 33, 12, 13, 23) -- the order of

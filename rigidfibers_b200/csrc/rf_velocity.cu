@@ -121,7 +121,7 @@ __device__ __forceinline__ void velocity_far_block(const Tables& tab, int N, con
       // the centre difference in FP64, rounded once (as in the assembly): the
       // error scales with the fibers' distance, not with their distance from the origin
       const float dx = (float)(xi[0] - sXj[jl][0]), dy = (float)(xi[1] - sXj[jl][1]), dz = (float)(xi[2] - sXj[jl][2]);
-      if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < far_d2) continue;   // near, or i itself
+      if (!far_pair(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), far_d2)) continue;   // near, or i itself
       float acc[3] = {0.f, 0.f, 0.f};
 #pragma unroll
       for (int q = 0; q < FN; ++q)
@@ -194,7 +194,7 @@ __device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, con
     if (j < jend) {
       const double4 xj = pos64[j];
       d[0] = (float)(xi.x - xj.x); d[1] = (float)(xi.y - xj.y); d[2] = (float)(xi.z - xj.z);
-      near = j != i && fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2])) < far_d2;
+      near = j != i && !far_pair(fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2])), far_d2);
     }
     for (unsigned m = __ballot_sync(0xffffffffu, near); m != 0; m &= m - 1) {
       const int src = __ffs(m) - 1, jj = js + src;
@@ -322,7 +322,7 @@ k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, 
       const int jend = min(N, (chunk + 1) * v.jchunk);
       for (int j = chunk * v.jchunk; j < jend; ++j) {
         const double4 xj = pos[j];
-        if (j == i || dist2(xi, xj) < far_d2) continue;
+        if (!far_pair(dist2(xi, xj), far_d2)) continue;   // near, or i itself
         const double R0[3] = {pt[0] - xj.x, pt[1] - xj.y, pt[2] - xj.z};
         analytic_apply<M>(R0, ori[j], coeff + (int64_t)j * M3, e2, fz, g);
       }
@@ -349,7 +349,7 @@ k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, 
   const int jend = min(N, (seg + 1) * v.jseg);
   for (int js = seg * v.jseg; js < jend; js += 32) {
     const int j = js + lane;
-    const bool near = j < jend && j != i && dist2(xi, pos[j]) < far_d2;
+    const bool near = j < jend && j != i && !far_pair(dist2(xi, pos[j]), far_d2);
     for (unsigned m = __ballot_sync(0xffffffffu, near); m != 0; m &= m - 1) {
       const int jj = js + __ffs(m) - 1;
       const double4 xj = pos[jj], tj = ori[jj];

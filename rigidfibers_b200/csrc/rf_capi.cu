@@ -2148,8 +2148,10 @@ int rf_dense_lu_solve(const float* A, const float* b, float* x, int64_t R, doubl
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaStream_t st = (cudaStream_t)stream;
   LuSetup L{};
+  // a stream and its events for one call cost ~150 us, a panel's work beside the
+  // diagonal block gains ~19: from nine panels on
   LuLane lane;
-  L.lane = &lane;
+  L.lane = R > 1024 ? &lane : nullptr;
   L.R = R;
   L.lda = R;
   L.ldlu = ceil_div(R, 32) * 32;   // factors with 128-byte aligned columns (the tensor-core path's TMA needs

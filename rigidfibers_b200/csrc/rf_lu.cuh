@@ -44,7 +44,7 @@ struct LuSetup {
   float* inv = nullptr;    // lu_tc_inv_floats(): the diagonal block's L^-1 and U^-T
   int* flags = nullptr;    // 2: largest |l| (float bits), status
   float* sinv = nullptr;   // lu_tc_sinv_floats(R): each diagonal block's L^-1 and U^-1 (triangular solves)
-  LuLane* lane = nullptr;
+  LuLane* lane = nullptr;  // null: the factorization runs on one stream
   bool use_tc = true;
 };
 

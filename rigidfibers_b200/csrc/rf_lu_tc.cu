@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_lu_diag(float* __restrict__ A,
   if (tid == 0) zero_pivot = 0;
   __syncthreads();
   float vmax = 0.f;
-  for (int o = 0; o < kPanel; o += kSub) {
+  for (int o = 0; o < w; o += kSub) {   // what lies beyond w is the identity
     if (warp == 0) {
       // the 32 x 32 sub-block: lane = row
       float r[kSub];
@@ -1000,7 +1000,8 @@ struct TrsvArgs {
   int64_t lda, R;
   const float* sinv;   // per block: L^-1 column-major, then U^-1 column-major (2 x 128 x 128)
   float* y;            // right-hand side in, solution out
-  int* flag;           // nblocks words, zero on entry: x_b is in y
+  int* flag;           // nblocks words, none equal to `done` on entry: x_b is in y
+  int done;
   int* status;         // -1 on a timed-out wait
   uint64_t wait_ns;
   int nblocks;
@@ -1072,7 +1073,7 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
       __threadfence();
     }
     __syncthreads();
-    if (tid == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(a.flag + b), "r"(1) : "memory");
+    if (tid == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(a.flag + b), "r"(a.done) : "memory");
   };
   int mine = p, own = 0;   // this CTA's next position to solve, and its slot
   if (mine == 0) {
@@ -1092,7 +1093,7 @@ __global__ void __launch_bounds__(kTrsvThreads, 1) k_trsv_tc(TrsvArgs a) {
       for (;;) {
         int f;
         asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(f) : "l"(a.flag + b) : "memory");
-        if (f != 0) break;
+        if (f == a.done) break;
         if (now_ns() - t0 > a.wait_ns) {
           fail = 1;
           atomicExch(a.status, -1);
@@ -1273,9 +1274,10 @@ int lu_solve_tc(const LuSetup& s, const float* rhs, float* x, cudaStream_t st) {
   RF_CUDA_TRY(attr);
   const bool shared = smem <= (size_t)kTrsvMaxSmem;
   const void* fn = shared ? (const void*)k_trsv_tc<true> : (const void*)k_trsv_tc<false>;
+  RF_CUDA_TRY(cudaMemsetAsync(t.flag, 0, (size_t)t.nblocks * sizeof(int), st));
   for (int lower = 1; lower >= 0; --lower) {
     t.lower = lower;
-    RF_CUDA_TRY(cudaMemsetAsync(t.flag, 0, (size_t)t.nblocks * sizeof(int), st));
+    t.done = lower ? 1 : 2;   // the lower sweep leaves 1 in every flag
     void* args[] = {&t};
     RF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(P), dim3(kTrsvThreads), args, shared ? smem : 0, st));
   }
@@ -1290,8 +1292,7 @@ int lu_solve_tc(const LuSetup& s, const float* rhs, float* x, cudaStream_t st) {
 int lu_factor_tc(const LuSetup& s, cudaStream_t st, bool* clean, int* launches, float* max_l) {
   const int64_t R = s.R, lda = s.ldlu ? s.ldlu : s.lda;
   *clean = false;
-  if ((lda % 4) != 0 || (reinterpret_cast<uintptr_t>(s.LU) % 16) != 0 || !s.LT || !s.inv || !s.flags || !s.sinv ||
-      !s.lane) {
+  if ((lda % 4) != 0 || (reinterpret_cast<uintptr_t>(s.LU) % 16) != 0 || !s.LT || !s.inv || !s.flags || !s.sinv) {
     set_last_error_str("lu: tensor-core factorization needs a 16-byte aligned matrix and its buffers");
     return RF_E_UNSUPPORTED;
   }
@@ -1335,8 +1336,12 @@ int lu_factor_tc(const LuSetup& s, cudaStream_t st, bool* clean, int* launches, 
     t.ldlt = kLtCols;
     return t;
   };
-  LuLane& ln = *s.lane;
-  RF_TRY_RF(ln.open());
+  // the side stream, if the caller has one (a matrix of one panel has no use for it)
+  LuLane none;
+  LuLane& ln = s.lane && R > kPanel ? *s.lane : none;
+  const bool lane = &ln != &none;
+  if (lane) RF_TRY_RF(ln.open());
+  const cudaStream_t side = lane ? ln.side : st;
   // a failed launch leaves no work behind on the side stream: the caller goes on
   // with the same buffers
   struct Drain {
@@ -1345,7 +1350,7 @@ int lu_factor_tc(const LuSetup& s, cudaStream_t st, bool* clean, int* launches, 
     ~Drain() {
       if (armed) cudaStreamSynchronize(side);
     }
-  } drain{ln.side};
+  } drain{side, lane};
   // A21 of the panel at column k (width w) as rows of LT columns lt_col ..
   auto to_rows = [&](int64_t k, int w, int lt_col, cudaStream_t on) -> int {
     const int64_t m = R - k - w;
@@ -1441,18 +1446,18 @@ int lu_factor_tc(const LuSetup& s, cudaStream_t st, bool* clean, int* launches, 
       if (p > 0) RF_TRY_RF(update_cols(kk, kk, kk + w, k, kPanel * p));
       end = kk + w;
       if (end < R) {
-        RF_CUDA_TRY(cudaEventRecord(ln.forked, st));
-        RF_CUDA_TRY(cudaStreamWaitEvent(ln.side, ln.forked, 0));
-        RF_TRY_RF(to_rows(kk, w, kPanel * p, ln.side));
-        RF_CUDA_TRY(cudaEventRecord(ln.rows, ln.side));
-        if (p > 0) RF_TRY_RF(update(kk, end, end, k, kPanel * p, ln.side));
-        RF_CUDA_TRY(cudaEventRecord(ln.right, ln.side));
+        if (lane) RF_CUDA_TRY(cudaEventRecord(ln.forked, st));
+        if (lane) RF_CUDA_TRY(cudaStreamWaitEvent(side, ln.forked, 0));
+        RF_TRY_RF(to_rows(kk, w, kPanel * p, side));
+        if (lane) RF_CUDA_TRY(cudaEventRecord(ln.rows, side));
+        if (p > 0) RF_TRY_RF(update(kk, end, end, k, kPanel * p, side));
+        if (lane) RF_CUDA_TRY(cudaEventRecord(ln.right, side));
       }
       RF_TRY_RF(diagonal(kk, w));
       if (end >= R) break;
-      RF_CUDA_TRY(cudaStreamWaitEvent(st, ln.rows, 0));
+      if (lane) RF_CUDA_TRY(cudaStreamWaitEvent(st, ln.rows, 0));
       RF_TRY_RF(l21(kk, w, kPanel * p));
-      RF_CUDA_TRY(cudaStreamWaitEvent(st, ln.right, 0));
+      if (lane) RF_CUDA_TRY(cudaStreamWaitEvent(st, ln.right, 0));
       RF_TRY_RF(u12(kk, w, end));
     }
     if (end >= R) break;

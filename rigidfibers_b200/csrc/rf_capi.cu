@@ -1380,9 +1380,6 @@ static int pack_order_streams(rf_handle** hs, int n, cudaStream_t st) {
   for (int i = 0; i < n; ++i) {
     rf_handle* h = hs[i];
     if (h->st == st) continue;
-    const cudaError_t idle = cudaStreamQuery(h->st);
-    if (idle == cudaSuccess) continue;   // nothing to wait for: the usual case, the last pack was waited for
-    if (idle == cudaErrorNotReady) (void)cudaGetLastError();
     if (!h->order_ev) RF_CUDA_TRY(cudaEventCreateWithFlags(&h->order_ev, cudaEventDisableTiming));
     RF_CUDA_TRY(cudaEventRecord(h->order_ev, h->st));
     RF_CUDA_TRY(cudaStreamWaitEvent(st, h->order_ev, 0));

@@ -199,19 +199,28 @@ int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, cons
                                int* vflag, cudaStream_t st);
 
 // Sums of the velocity partial rows vpart[row][i][6]: rows row = g (mod 4) in
-// order for each group g, then the groups in order.  velocity_row_sum: component
-// c of fiber i by one thread; velocity_rows_block: 32 fibers from i0 by a block
-// of kVelSumThreads threads (8 loads per thread in flight), the same sums.
+// order for each group g, then the groups in order.  velocity_row_sums: fiber i by
+// one thread (24 loads in flight); velocity_rows_block: 32 fibers from i0 by a
+// block of kVelSumThreads threads (8 loads per thread in flight), the same sums.
 constexpr int kVelSumFibers = 32, kVelSumGroups = 4;
 constexpr int kVelSumThreads = kVelSumFibers * 6 * kVelSumGroups;
-__device__ __forceinline__ float velocity_row_sum(const float* __restrict__ vpart, int nrows, int N, int i, int c) {
-  float r[kVelSumGroups];
+__device__ __forceinline__ void velocity_row_sums(const float* __restrict__ vpart, int nrows, int N, int i,
+                                                  float (&S)[6]) {
+  float r[kVelSumGroups][6] = {};
+  for (int p = 0; p < nrows; p += kVelSumGroups) {
+    float v[kVelSumGroups][6];
 #pragma unroll
-  for (int g = 0; g < kVelSumGroups; ++g) {
-    r[g] = 0.f;
-    for (int p = g; p < nrows; p += kVelSumGroups) r[g] = __fadd_rn(r[g], vpart[((int64_t)p * N + i) * 6 + c]);
+    for (int g = 0; g < kVelSumGroups; ++g)
+#pragma unroll
+      for (int c = 0; c < 6; ++c) v[g][c] = p + g < nrows ? vpart[((int64_t)(p + g) * N + i) * 6 + c] : 0.f;
+#pragma unroll
+    for (int g = 0; g < kVelSumGroups; ++g)
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+        if (p + g < nrows) r[g][c] = __fadd_rn(r[g][c], v[g][c]);
   }
-  return __fadd_rn(__fadd_rn(__fadd_rn(r[0], r[1]), r[2]), r[3]);
+#pragma unroll
+  for (int c = 0; c < 6; ++c) S[c] = __fadd_rn(__fadd_rn(__fadd_rn(r[0][c], r[1][c]), r[2][c]), r[3][c]);
 }
 __device__ __forceinline__ void velocity_rows_block(const float* __restrict__ vpart, int nrows, int N, int i0,
                                                     float (*sums)[7]) {

@@ -970,8 +970,7 @@ k_pack_finish(const Tables tab, const PackStepMember* __restrict__ mem) {
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     float4 u, w;
     float S[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) S[c] = velocity_row_sum(p.vpart, nparts, N, i, c);
+    velocity_row_sums(p.vpart, nparts, N, i, S);
     struct_velocity_fiber(tab, p.ori32, p.F, S, i, u, w);
     p.tv[i] = u;
     p.rv[i] = w;

@@ -108,31 +108,32 @@ __device__ __forceinline__ void psym(const T (&t)[6], const T* v, T* acc) {
   acc[2] = pfma(t[2], v[2], pfma(t[5], v[1], pfma(t[4], v[0], acc[2])));
 }
 
-// v[16] summed over the 16 lanes that differ in lane bits 0..3 (four halving
-// exchanges); lane l gets the sum of v[l & 15].
-template <typename T>
-__device__ __forceinline__ T psum16(const T (&v)[16], int lane) {
-  const bool b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
-  T a[8];
+// v[G], G = 4, 8 or 16, summed over the 16 lanes that differ in lane bits 0..3 by
+// halving exchanges (then plain ones); lane l gets the sum of v[(l & 15) / (16 / G)].
+// The lanes are added in the same order for every G.
+template <int H, int O, typename T, int G>
+__device__ __forceinline__ void psum_step(T (&a)[G], int lane) {
+  if constexpr (O > 0) {
+    if constexpr (H > 0) {
+      const bool up = lane & O;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const T s = b3 ? v[k] : v[k + 8], kp = b3 ? v[k + 8] : v[k];
-    a[k] = kp + pshfl(s, 8);
+      for (int k = 0; k < H; ++k) {
+        const T s = up ? a[k] : a[k + H], kp = up ? a[k + H] : a[k];
+        a[k] = kp + pshfl(s, O);
+      }
+    } else {
+      a[0] += pshfl(a[0], O);
+    }
+    psum_step<H / 2, O / 2>(a, lane);
   }
-  T b[4];
+}
+template <typename T, int G>
+__device__ __forceinline__ T psum(const T (&v)[G], int lane) {
+  T a[G];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const T s = b2 ? a[k] : a[k + 4], kp = b2 ? a[k + 4] : a[k];
-    b[k] = kp + pshfl(s, 4);
-  }
-  T c[2];
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const T s = b1 ? b[k] : b[k + 2], kp = b1 ? b[k + 2] : b[k];
-    c[k] = kp + pshfl(s, 2);
-  }
-  const T s = b0 ? c[0] : c[1], kp = b0 ? c[1] : c[0];
-  return kp + pshfl(s, 1);
+  for (int k = 0; k < G; ++k) a[k] = v[k];
+  psum_step<G / 2, 8>(a, lane);
+  return a[0];
 }
 
 template <typename H16>
@@ -238,15 +239,16 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
   };
 
   // out[k] = sum over the member's rows of a[r] * V_k[r] for k < nv, FP64, and with
-  // `norm` out[nv] = sum of a[r]^2.  A slice's partial is that of up to 8 virtual
-  // warps: lane l of virtual warp w adds rows 32 w + l, 32 (w + 8) + l, .. of the
-  // slice (all basis loads of 16 values in flight), the lanes meet in halving
-  // exchanges, the virtual warps add in order; the CTA's warps share all its
-  // slices' virtual warps.  The partials go into the owning CTA's buffer; after
-  // the cluster barrier every CTA adds the 8 of them in slice order.  Three
-  // buffers in turn: a buffer is written again only after two more cluster
-  // barriers, when every CTA has read it.
-  const int nvw = min(8, (kPM3 * ((N + kParts - 1) / kParts) + 31) / 32);
+  // `norm` out[nv] = sum of a[r]^2.  A slice's partial is that of nvw virtual warps
+  // (1 up to 32 fibers, 8 from 233 on: at most two rows a lane): lane l of virtual
+  // warp w adds rows 32 w + l and 32 (w + nvw) + l of the slice, the lanes meet in
+  // halving exchanges, the virtual warps add in order; the CTA's warps share all
+  // its slices' virtual warps.  4, 8 or 16 values at a time (32 fibers: 1.8k cycles
+  // a call with 16 for any number, of which most cycles hold few values).  The
+  // partials go into the owning CTA's buffer; after the cluster barrier every CTA
+  // adds the 8 of them in slice order.  Three buffers in turn: a buffer is written
+  // again only after two more cluster barriers, when every CTA has read it.
+  const int nvw = min(8, (kPM3 * ((N + kParts - 1) / kParts) + 63) / 64);
   auto cdots = [&](const float* a, int nv, bool norm, double* out) {
     __syncthreads();                                           // this CTA's rows of a are written
     double* part = dpart + (size_t)rb * kParts * (m + 2);
@@ -258,28 +260,38 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
       for (int e = warp; e < cnt * nvw; e += kPT / 32) {
         const int s = p0 + s0 + e / nvw;
         const int r0 = kPM3 * ((s * N) / kParts), r1 = kPM3 * (((s + 1) * N) / kParts);
-        for (int g = 0; g < npad; g += 16) {
-          double acc[16];
+        // G values from g on, of this virtual warp's rows of the slice
+        auto values = [&](auto width, int g) {
+          constexpr int G = decltype(width)::value;
+          double acc[G];
 #pragma unroll
-          for (int u = 0; u < 16; ++u) acc[u] = 0.0;
-          for (int r = r0 + (e % nvw) * 32 + lane; r < r1; r += 8 * 32) {
+          for (int u = 0; u < G; ++u) acc[u] = 0.0;
+          for (int r = r0 + (e % nvw) * 32 + lane; r < r1; r += nvw * 32) {
             const float af = a[r];
             const double ar = (double)af;
-            float v[16];
+            float v[G];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
+            for (int u = 0; u < G; ++u) {
               const int k = g + u;
               v[u] = k < nv ? V[(int64_t)k * ldv + r] : k < n ? af : 0.f;
             }
 #pragma unroll
-            for (int u = 0; u < 16; ++u) acc[u] = fma(ar, (double)v[u], acc[u]);
+            for (int u = 0; u < G; ++u) acc[u] = fma(ar, (double)v[u], acc[u]);
           }
-          // lane l gets the warp's sum of value l & 15 (of both half-warps)
-          double v = psum16(acc, lane);
+          double v = psum(acc, lane);
           v += pshfl(v, 16);
-          if (lane < 16) red[(size_t)e * npad + g + lane] = v;
-        }
+          const int k = g + lane / (16 / G);
+          if (lane < 16 && lane % (16 / G) == 0 && k < n) {
+            if (nvw == 1) part[s * (m + 2) + k] = v;
+            else red[(size_t)e * npad + k] = v;
+          }
+        };
+        if (n <= 4) values(std::integral_constant<int, 4>(), 0);
+        else if (n <= 8) values(std::integral_constant<int, 8>(), 0);
+        else
+          for (int g = 0; g < npad; g += 16) values(std::integral_constant<int, 16>(), g);
       }
+      if (nvw == 1) continue;   // a slice is one virtual warp
       __syncthreads();
       for (int e = t; e < cnt * n; e += kPT) {
         const int sl = e / n, k = e % n;
@@ -395,7 +407,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
         if (P.smode == 2) ppair16<__nv_bfloat16>(wv, xi, xj, zi, zj);
         else ppair16<__half>(wv, xi, xj, zi, zj);
       }
-      const float sj = psum16(zj, lane);   // z_j over this half-warp's 16 i
+      const float sj = psum(zj, lane);   // z_j over this half-warp's 16 i
       const bool b4 = lane & 16;
       float u8[8];                          // z_i over this warp's two j: one halving exchange
 #pragma unroll
@@ -485,7 +497,7 @@ __global__ void __launch_bounds__(kPT) k_pack_gmres_ir(const PackMember* __restr
           }
         }
       }
-      const double sj = psum16(zj, lane);
+      const double sj = psum(zj, lane);
       const bool b4 = lane & 16;
       double u8[8];
 #pragma unroll

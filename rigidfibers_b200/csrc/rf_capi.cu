@@ -735,7 +735,7 @@ static int allocate_buffers(rf_handle* h, const rf_config* cfg) {
   }
   // velocities
   if (!rc) rc = h->alloc((void**)&h->fw, (size_t)N * (h->Q + kFarNodes) * sizeof(float4));
-  if (!rc) rc = h->alloc((void**)&h->vpart, (size_t)velocity_rows(N) * N * 6 * sizeof(float));
+  if (!rc) rc = h->alloc((void**)&h->vpart, (size_t)velocity_rows(N, h->Q) * N * 6 * sizeof(float));
   if (!rc) rc = h->alloc((void**)&h->vflag, sizeof(int));
   if (!rc && !h->dry && !(h->host_vflag = static_cast<int*>(pinned_pool().get(sizeof(int))))) rc = RF_E_OOM;
   h->io_size = io_bytes(N, R);

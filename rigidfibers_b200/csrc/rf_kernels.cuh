@@ -188,8 +188,8 @@ namespace rf {
 cudaError_t handle_pool(int dev, cudaMemPool_t* out);
 void pools_acquire();
 void pools_release();
-// fw: N * (Q + kFarNodes) float4 scratch; vpart: velocity_rows(N) * N * 6 floats scratch.
-int velocity_rows(int N);
+// fw: N * (Q + kFarNodes) float4 scratch; vpart: velocity_rows(N, Q) * N * 6 floats scratch.
+int velocity_rows(int N, int Q);
 // pos64: the FP64 centres, from which the pair separations are formed
 int launch_velocity_numerical(const Tables& tab, int N, const double4* pos64, const float4* ori, const float* x,
                               float4* fw, float* vpart, float4* tvel, float4* rvel, int* vflag, cudaStream_t st);

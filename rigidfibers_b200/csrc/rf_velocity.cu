@@ -175,11 +175,15 @@ __device__ __forceinline__ void near_row_sums(const Tables& tab, const float (&g
 }
 
 // One warp: fiber i's near sources of one segment, found 32 centres at a time and
-// taken in index order, lane = quadrature point of i (Q = 48: two passes)
+// taken in index order, lane = quadrature point of i (Q = 48: two passes).  A
+// source's densities pass through the warp's Q float4 of shared memory, the next
+// one's on their way meanwhile: read where they are used, each batch of a few was
+// a trip to L2 of its own (100 fibers: the velocities 52.7 us, 40.7 so).
 template <int Q>
 __device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, const double4* __restrict__ pos64,
                                                    const float4* __restrict__ ori, const float4* __restrict__ fw,
-                                                   int i, int jbeg, int jend, float* __restrict__ row) {
+                                                   int i, int jbeg, int jend, float4* __restrict__ sf,
+                                                   float* __restrict__ row) {
   constexpr int NP = (Q + 31) / 32;   // points per lane
   const int lane = threadIdx.x & 31;
   const int P = Q + kFarNodes;
@@ -187,6 +191,13 @@ __device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, con
   const float4 ti = ori[i];
   const float e2 = tab.e2, e2x3 = -3.f * tab.e2, far_d2 = tab.far_d2;
   float g[NP][3] = {};
+  float4 f[NP], t = ti;
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int h = 0; h < NP; ++h)
+      if (lane + 32 * h < Q) f[h] = fw[(int64_t)j * P + lane + 32 * h];
+    t = ori[j];
+  };
   for (int js = jbeg; js < jend; js += 32) {
     const int j = js + lane;
     float d[3] = {0.f, 0.f, 0.f};
@@ -196,11 +207,20 @@ __device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, con
       d[0] = (float)(xi.x - xj.x); d[1] = (float)(xi.y - xj.y); d[2] = (float)(xi.z - xj.z);
       near = j != i && !far_pair(fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2])), far_d2);
     }
-    for (unsigned m = __ballot_sync(0xffffffffu, near); m != 0; m &= m - 1) {
-      const int src = __ffs(m) - 1, jj = js + src;
+    unsigned m = __ballot_sync(0xffffffffu, near);
+    if (m != 0) fetch(js + __ffs(m) - 1);
+    while (m != 0) {
+      const int src = __ffs(m) - 1;
+      const float4 tj = t;
+      __syncwarp();   // the source before this one is read
+#pragma unroll
+      for (int h = 0; h < NP; ++h)
+        if (lane + 32 * h < Q) sf[lane + 32 * h] = f[h];
+      __syncwarp();
+      m &= m - 1;
+      if (m != 0) fetch(js + __ffs(m) - 1);
       const float dx = __shfl_sync(0xffffffffu, d[0], src), dy = __shfl_sync(0xffffffffu, d[1], src),
                   dz = __shfl_sync(0xffffffffu, d[2], src);
-      const float4 tj = ori[jj];
 #pragma unroll
       for (int h = 0; h < NP; ++h) {
         const int q = lane + 32 * h;
@@ -212,7 +232,7 @@ __device__ __forceinline__ void velocity_near_warp(const Tables& tab, int N, con
           for (int p = 0; p < Q; ++p) {
             const float sp = tab.pts[p];
             stokeslet_apply<false>(px, py, pz, make_float4(sp * tj.x, sp * tj.y, sp * tj.z, 0.f),
-                                   fw[(int64_t)jj * P + p], e2, e2x3, acc);
+                                   sf[p], e2, e2x3, acc);
           }
 #pragma unroll
           for (int a = 0; a < 3; ++a) g[h][a] += acc[a];
@@ -232,10 +252,11 @@ k_velocity_numerical(const Tables tab, int N, const double4* __restrict__ pos64,
     velocity_far_block(tab, N, pos64, ori, fw, b / v.chunks, b % v.chunks, v.jchunk, vpart);
     return;
   }
+  __shared__ float4 sf[kVelThreads / 32][Q];
   const int w = (int)blockIdx.x * (kVelThreads / 32) + (int)(threadIdx.x >> 5);
   const int i = w / v.segs, seg = w % v.segs;
   if (i < N)
-    velocity_near_warp<Q>(tab, N, pos64, ori, fw, i, seg * v.jseg, min(N, (seg + 1) * v.jseg),
+    velocity_near_warp<Q>(tab, N, pos64, ori, fw, i, seg * v.jseg, min(N, (seg + 1) * v.jseg), sf[threadIdx.x >> 5],
                           vpart + (int64_t)(v.chunks + seg) * N * 6);
 }
 
@@ -368,29 +389,35 @@ k_velocity_analytical(const Tables tab, int N, const double4* __restrict__ pos, 
 }
 
 // Far: enough fiber-tile x chunk blocks to fill the GPU four times over, at least 8
-// sources each; near: N warps alone leave the GPU idle below a few thousand fibers
-static VelSplit velocity_split(int N, int fibers, int threads) {
+// sources each; near: N warps alone leave the GPU idle below a few thousand fibers,
+// so segments of at least near_min sources.
+static VelSplit velocity_split(int N, int fibers, int threads, int near_min) {
   VelSplit v;
-  const int tiles = (int)ceil_div(N, fibers), most = (int)ceil_div(N, 8);
-  v.chunks = std::max(1, std::min((int)ceil_div(148 * 4 * 4, tiles), most));
+  const int tiles = (int)ceil_div(N, fibers);
+  v.chunks = std::max(1, std::min((int)ceil_div(148 * 4 * 4, tiles), (int)ceil_div(N, 8)));
   v.jchunk = (int)ceil_div(N, v.chunks);
   v.far_blocks = tiles * v.chunks;
-  v.segs = std::max(1, std::min((int)ceil_div(148 * 16, N), most));
+  v.segs = std::max(1, std::min((int)ceil_div(148 * 16, N), (int)ceil_div(N, near_min)));
   v.jseg = (int)ceil_div(N, v.segs);
   v.near_blocks = (int)ceil_div((int64_t)N * v.segs, threads / 32);
   return v;
 }
+// A near source costs a warp Q points on ceil(Q / 32) points a lane, so with 48
+// points (4 times the work of 24) a segment is 4 times shorter (30 fibers, all
+// near: 66 us with 8 sources, 50 with 2).
+static VelSplit numerical_split(int N, int Q) { return velocity_split(N, kVelFibers, kVelThreads, Q > 32 ? 2 : 8); }
+static VelSplit analytical_split(int N) { return velocity_split(N, kAnaFibers, kAnaThreads, 8); }
 
 // partial rows of either velocity path (vpart: this many rows of 6 N floats)
-int velocity_rows(int N) {
-  const VelSplit n = velocity_split(N, kVelFibers, kVelThreads), a = velocity_split(N, kAnaFibers, kAnaThreads);
+int velocity_rows(int N, int Q) {
+  const VelSplit n = numerical_split(N, Q), a = analytical_split(N);
   return std::max(n.chunks + n.segs, a.chunks + a.segs);
 }
 
 int launch_velocity_analytical(const Tables& tab, int N, const float4* ori, const double4* pos64,
                                const double4* ori64, const float* x, float* vpart, float4* tvel, float4* rvel,
                                int* vflag, cudaStream_t st) {
-  const VelSplit v = velocity_split(N, kAnaFibers, kAnaThreads);
+  const VelSplit v = analytical_split(N);
   const unsigned nb = (unsigned)(v.far_blocks + v.near_blocks);
   bool done = false;
 #define RF_VA_CASE(MM, QQ)                                                                              \
@@ -417,7 +444,7 @@ int launch_velocity_numerical(const Tables& tab, int N, const double4* pos64, co
   k_source_density<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)N * (Q + kFarNodes), 256), 148 * 16), 256, 0, st>>>(
       tab, N, x, fw, vflag);
   RF_LAUNCH_CHECK();
-  const VelSplit v = velocity_split(N, kVelFibers, kVelThreads);
+  const VelSplit v = numerical_split(N, Q);
   const unsigned nb = (unsigned)(v.far_blocks + v.near_blocks);
   switch (Q) {
     case 12: k_velocity_numerical<12><<<nb, kVelThreads, 0, st>>>(tab, N, pos64, ori, fw, v, vpart); break;

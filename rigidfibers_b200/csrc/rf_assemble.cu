@@ -221,11 +221,17 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
 // Matrix-free product and dense output: 256, where the product's 160 and the
 // block stores' 800 tasks of a batch split better (N=2500 product 0.90 against
 // 1.23 ms, N=2000 dense 1.55 against 1.77).  More than 5 terms: batches of 16
-// pairs, since G and T of 32 would leave one CTA per SM, on 128 threads; on 256 for
-// 8 terms, whose 144 force-term sums of a batch need a thread each (whole steps of
-// 37 and 1500 fibers, matrix-free: 0.54 and 18.2 ms, with 160 threads 0.68 and 19.7).
+// pairs, since G and T of 32 would leave one CTA per SM, on 128 threads; on 192 for
+// the product, which takes 8 near pairs at once then instead of 5 (whole steps of 37
+// and 1500 fibers, 6 terms: 0.43 and 10.5 ms against 0.50 and 10.9); on 256 for 8
+// terms, whose 144 force-term sums of a batch need a thread each (whole matrix-free
+// steps of 37 and 1500 fibers: 0.54 and 18.2 ms, with 160 threads 0.68 and 19.7).
 constexpr int num_threads(int M, int mode) {
-  return M > 7 ? 256 : mode == kAsmStructF16 || mode == kAsmStructBF16 || M > 5 ? 128 : 256;
+  return M > 7 ? 256 : mode == kAsmStructF16 || mode == kAsmStructBF16 ? 128 : M <= 5 ? 256 : mode == kAsmApply ? 192 : 128;
+}
+constexpr int min_ctas(int M, int mode) {
+  const int threads = num_threads(M, mode);
+  return M > 7 ? 2 : threads == 192 ? 3 : M > 5 ? 4 : threads == 128 ? 6 : 3;
 }
 
 template <int M, int Q, int NTH>
@@ -629,7 +635,7 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
 }
 
 template <int M, int Q, int MODE, bool P2>
-__global__ void __launch_bounds__(num_threads(M, MODE), M > 7 ? 2 : M > 5 ? 4 : num_threads(M, MODE) == 128 ? 6 : 3)
+__global__ void __launch_bounds__(num_threads(M, MODE), min_ctas(M, MODE))
 k_assemble_pairs(const Tables tab, int N, const float4* __restrict__ ori, AsmOut out) {
   if (MODE == kAsmApply && out.skip != nullptr && *out.skip) return;
   int I, J;

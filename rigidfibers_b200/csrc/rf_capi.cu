@@ -1701,12 +1701,14 @@ int rf_get_velocities(rf_handle* h, double* tvel, double* rvel) {
   return fetch_rows(h, h->tv[h->vlast], h->rv[h->vlast], false, tvel, rvel);
 }
 
+// one float a row: a copy into the page-locked block is sooner done than a kernel
+// that writes it (N=100: 13.4 us against 16.6; N=4000: 40 and 45)
 static int fetch_vec(rf_handle* h, const float* dev, double* out) {
   float* io = static_cast<float*>(h->host_io);
   const int64_t per = (int64_t)(io_bytes(h->N, h->R) / sizeof(float));
   for (int64_t r0 = 0; r0 < h->R; r0 += per) {
     const int64_t n = std::min(per, h->R - r0);
-    RF_TRY(launch_vector_out(dev + r0, (int)n, io, h->st));
+    RF_CUDA_TRY(cudaMemcpyAsync(io, dev + r0, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, h->st));
     RF_CUDA_TRY(cudaStreamSynchronize(h->st));
     for (int64_t r = 0; r < n; ++r) out[r0 + r] = io[r];
   }

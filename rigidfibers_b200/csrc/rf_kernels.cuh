@@ -302,5 +302,4 @@ int launch_state_in(const double* host, int n, int i0, double4* p0, double4* p1,
                     float4* o32, cudaStream_t st);
 int launch_rows_out(const double4* u, const double4* v, int n, int i0, double* host, cudaStream_t st);
 int launch_rows_out(const float4* u, const float4* v, int n, int i0, double* host, cudaStream_t st);
-int launch_vector_out(const float* x, int n, float* host, cudaStream_t st);
 }  // namespace rf

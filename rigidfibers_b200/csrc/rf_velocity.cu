@@ -525,11 +525,6 @@ __global__ void __launch_bounds__(256) k_rows_out(const T* __restrict__ u, const
   host[e] = (double)(e >= 3 * n ? v : u)[4 * (int64_t)(i0 + k / 3) + k % 3];
 }
 
-__global__ void __launch_bounds__(256) k_vector_out(const float* __restrict__ x, int n, float* __restrict__ host) {
-  const int e = blockIdx.x * 256 + threadIdx.x;
-  if (e < n) host[e] = x[e];
-}
-
 int launch_state_in(const double* host, int n, int i0, double4* p0, double4* p1, double4* o0, double4* o1, float4* p32,
                     float4* o32, cudaStream_t st) {
   k_state_in<<<(unsigned)ceil_div(6 * n, 256), 256, 0, st>>>(host, n, i0, p0, p1, o0, o1, p32, o32);
@@ -547,12 +542,6 @@ int launch_rows_out(const double4* u, const double4* v, int n, int i0, double* h
 int launch_rows_out(const float4* u, const float4* v, int n, int i0, double* host, cudaStream_t st) {
   k_rows_out<<<(unsigned)ceil_div(6 * n, 256), 256, 0, st>>>(reinterpret_cast<const float*>(u),
                                                              reinterpret_cast<const float*>(v), n, i0, host);
-  RF_LAUNCH_CHECK();
-  return RF_OK;
-}
-
-int launch_vector_out(const float* x, int n, float* host, cudaStream_t st) {
-  k_vector_out<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(x, n, host);
   RF_LAUNCH_CHECK();
   return RF_OK;
 }

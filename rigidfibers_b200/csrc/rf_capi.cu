@@ -598,8 +598,22 @@ static size_t io_bytes(int N, int64_t R) {
   return std::min(kIoBytes, std::max((size_t)N * 6 * sizeof(double), (size_t)R * sizeof(float)));
 }
 
+// The calling thread on the handle's device (kernels launch on the current one's
+// streams only; copies do not care) until the end of the scope.
+struct DeviceScope {
+  int before = -1;
+  explicit DeviceScope(int dev) {
+    int cur = 0;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) before = cur;
+  }
+  ~DeviceScope() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 int rf_set_state(rf_handle* h, const double* pos, const double* ori) {
   if (!h || !pos || !ori) return RF_E_INPUT;
+  DeviceScope on(h->dev);
   double* io = static_cast<double*>(h->host_io);
   const int per = (int)(io_bytes(h->N, h->R) / (6 * sizeof(double)));
   for (int i0 = 0; i0 < h->N; i0 += per) {
@@ -1677,6 +1691,7 @@ int rf_run(rf_handle* h, int first_timestep, int nsteps) {
 
 // 3 doubles a fiber of u and of v (double4 or float4 a fiber on the device)
 static int fetch_rows(rf_handle* h, const void* u, const void* v, bool is_double, double* out_u, double* out_v) {
+  DeviceScope on(h->dev);
   double* io = static_cast<double*>(h->host_io);
   const int per = (int)(io_bytes(h->N, h->R) / (6 * sizeof(double)));
   for (int i0 = 0; i0 < h->N; i0 += per) {

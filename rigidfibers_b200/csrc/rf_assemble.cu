@@ -112,24 +112,39 @@ struct AsmOut {
 // the two lanes against the weight pair W2[i][q] (the even part for P_2i, the
 // odd part for P_2i+1), and their six components are recombined and stored as
 // pairs: gcol[(i * 6 + c) * GS2] = (P_2i, P_2i+1).
-// FAR: the rule of the far pairs (far_pts, far_W2) instead of the full one.
-template <int K1, int Q, int GS2, bool P2, bool FAR>
-__device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const float p[3], const float4 tj, float e2,
-                                                    float e2x3, float2* __restrict__ gcol) {
+// FAR: the rule of the far pairs (far_pts, far_W2) instead of the full one, with a
+// Newton step on the reciprocal root (NEWTON) or with a0 taken off A_0 from the start.
+
+// the point (x, y, z) on t's axis: d and s*
+__device__ __forceinline__ float4 project(float x, float y, float z, const float4 t) {
+  float ss = fmaf(x, t.x, fmaf(y, t.y, z * t.z));
+  float dx = fmaf(-ss, t.x, x), dy = fmaf(-ss, t.y, y), dz = fmaf(-ss, t.z, z);
+  const float dl = fmaf(dx, t.x, fmaf(dy, t.y, dz * t.z));
+  ss += dl;
+  dx = fmaf(-dl, t.x, dx);
+  dy = fmaf(-dl, t.y, dy);
+  dz = fmaf(-dl, t.z, dz);
+  return make_float4(dx, dy, dz, ss);
+}
+
+// 2 / |x_i - x_j|
+__device__ __forceinline__ float mean_kernel(float x, float y, float z) {
+  return 2.f * rsqrtf(fmaf(x, x, fmaf(y, y, z * z)));
+}
+
+// d: project() of the point
+template <int K1, int Q, int GS2, bool P2, bool FAR, bool NEWTON = false>
+__device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const float4 d, const float4 tj, float e2,
+                                                    float e2x3, float a0, float2* __restrict__ gcol) {
   static_assert(P2 || !FAR, "the far rule runs packed");
   constexpr int H = Q / 2, KP = (K1 + 1) / 2;
   const float* const pts = FAR ? tab.far_pts : tab.pts;
-  float ss = fmaf(p[0], tj.x, fmaf(p[1], tj.y, p[2] * tj.z));
-  float dx = fmaf(-ss, tj.x, p[0]), dy = fmaf(-ss, tj.y, p[1]), dz = fmaf(-ss, tj.z, p[2]);
-  const float dl = fmaf(dx, tj.x, fmaf(dy, tj.y, dz * tj.z));
-  ss += dl;
-  dx = fmaf(-dl, tj.x, dx);
-  dy = fmaf(-dl, tj.y, dy);
-  dz = fmaf(-dl, tj.z, dz);
+  const float dx = d.x, dy = d.y, dz = d.z, ss = d.w;
   const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
   float2 mA[KP], m0[KP], m1[KP], m2[KP];
 #pragma unroll
   for (int i = 0; i < KP; ++i) mA[i] = m0[i] = m1[i] = m2[i] = make_float2(0.f, 0.f);
+  if (FAR) mA[0].x = -a0;
   // the full rule's 12 folded points unrolled whole would spill
   constexpr int kUnroll = FAR ? H : 3;
 #pragma unroll kUnroll
@@ -139,9 +154,7 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
       const float2 u = __fadd2_rn(make_float2(ss, ss), make_float2(-pts[q], -pts[Q - 1 - q]));
       const float2 r2 = __ffma2_rn(u, u, make_float2(dd, dd));
       float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-      if constexpr (FAR) {
-        // one Newton step: a ninth of the kernel values carry a ninth of the
-        // averaging of their roundings, so each is made more exact
+      if constexpr (NEWTON) {
         const float2 e = __ffma2_rn(__fmul2_rn(r2, inv), make_float2(-inv.x, -inv.y), make_float2(1.f, 1.f));
         inv = __ffma2_rn(__fmul2_rn(inv, make_float2(0.5f, 0.5f)), e, inv);
       }
@@ -210,12 +223,29 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
 // instead of Q^2 = 576, within 3e-10 of the full rule's blocks (below their
 // FP32 rounding).  The others take the full rule.
 //
+// A third of the points average the roundings of G a third as well, and the blocks
+// of P_1 and up against P_0 (the right-hand side) are small differences of G.  A
+// Newton step on the reciprocal root makes up for it in sums over hundreds of pairs
+// (forces of 400 dilute fibers against 64 bits: 2.0e-6, 2.4e-6 without the far rule),
+// not in smaller ones (8 to 24 packed members of 16 to 128: 1.3e-6 against 1.2e-6).
+// Up to kFarSmall fibers what all points of fiber i share is therefore taken out of
+// the sums: a point's projection on fiber j's axis is the centre difference's plus s
+// times t_i's, and 2 / |x_i - x_j|, about the sum of W_0 a, is taken off G[.][P_0]'s
+// diagonal components where their sum starts and put back into T[P_0][P_0]
+// (far_sum).  Roundings of T[k][P_0], k = 1 .. 5, times the distance (FP32 emulation):
+// 3.9 5.6 2.3 2.9 1.8 e-8 by the full rule, 5.2 5.2 3.5 3.6 2.8 by the far rule with
+// the step, 4.1 3.3 2.8 2.3 2.3 so (the step is left out); the packs' forces 1.0e-6.
+// Larger systems and the product keep the step, with which their errors are below
+// the full rule's; the choice costs them 0.7 % of the assembly (N=4000: 2.44 ms).
+//
 // Bound: FP32 issue in the matrix-free product, HBM stores in the structured
 // assembly.  The far pairs run in batches of whole j (2 or 4 of the tile: 16 or
 // 32 pairs x 8 points = the CTA's threads), so that every phase has one unit per
 // thread and lane = pair keeps shared memory free of conflicts; the near pairs
 // of those rows are compacted and run in groups of up to TI pairs x Q points.
 // ---------------------------------------------------------------------------
+constexpr int kFarSmall = kPackMaxFibers;
+
 // Threads per CTA.  Structured output: 128 (six CTAs per SM instead of three of
 // 256: barriers of four warps, more CTAs to fill them; N=4000 3.09 -> 2.42 ms).
 // Matrix-free product and dense output: 256, where the product's 160 and the
@@ -308,6 +338,7 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
   __shared__ float sFj[TI * FF];             // force terms of the tile's j
 
   const bool diag = (I == J);
+  const bool small = !APPLY && N <= kFarSmall;
   const int tid = threadIdx.x, lane = tid & 31;
   const int i0 = I * TI, j0 = J * TI;
   // kAsmApply with a vector applies the blocks; without one it forms the force terms
@@ -415,13 +446,21 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
     // u = qi * PB + pair; zeros for the others
     if (tid < PB * S::FN) {
       const int p = tid % PB, qi = tid / PB;
-      const int pr = jb * TI + p, il = p % TI;
+      const int pr = jb * TI + p;
       float2* const gcol = sG + tid;
       if (sKind[pr] == 1) {
-        const float4 ti = sTi[il];
+        const float4 ti = sTi[pr % TI], tj = sTj[pr / TI];
         const float si = tab.far_pts[qi];
-        const float pp[3] = {fmaf(si, ti.x, sD[pr][0]), fmaf(si, ti.y, sD[pr][1]), fmaf(si, ti.z, sD[pr][2])};
-        stokeslet_moments_G<K1, S::FN, S::GSF, true, true>(tab, pp, sTj[pr / TI], e2, e2x3, gcol);
+        const float dx = sD[pr][0], dy = sD[pr][1], dz = sD[pr][2];
+        if (small) {
+          const float4 d = project(dx, dy, dz, tj), e = project(ti.x, ti.y, ti.z, tj);
+          stokeslet_moments_G<K1, S::FN, S::GSF, true, true>(
+              tab, make_float4(fmaf(si, e.x, d.x), fmaf(si, e.y, d.y), fmaf(si, e.z, d.z), fmaf(si, e.w, d.w)), tj, e2,
+              e2x3, mean_kernel(dx, dy, dz), gcol);
+        } else {
+          stokeslet_moments_G<K1, S::FN, S::GSF, true, true, true>(
+              tab, project(fmaf(si, ti.x, dx), fmaf(si, ti.y, dy), fmaf(si, ti.z, dz), tj), tj, e2, e2x3, 0.f, gcol);
+        }
       } else {
 #pragma unroll
         for (int c = 0; c < NC2; ++c) gcol[c * S::GSF] = make_float2(0.f, 0.f);
@@ -436,6 +475,14 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
       contract(sG + col * S::GSF + p, std::integral_constant<int, S::FN>(), std::true_type(), PB, col,
                t_of(p / TI, p % TI));
     }
+    if (small && tid < 3 * PB) {   // what P_0's diagonal components lack, in this thread's first column
+      const int col = tid / PB, p = tid % PB, pr = jb * TI + p;
+      float* const t = t_of(p / TI, p % TI);
+      const float a0 = sKind[pr] == 1 ? mean_kernel(sD[pr][0], sD[pr][1], sD[pr][2]) : 0.f;
+#pragma unroll
+      for (int k = 0; k < K1; k += k == 0 ? 6 : 2)   // the sums of W_2 and W_4 are 0
+        t[((QT ? s32_block(M, k, 0) : k * K1) * 6 + col) * (QT ? TI : 1)] += a0 * tab.far_sum[k];
+    }
     // ---- near pairs of these rows, in groups of up to NS, into the same T
     const unsigned bits = (sMask[jb * TI / 32] >> (jb * TI % 32)) & (PB == 32 ? 0xffffffffu : (1u << PB % 32) - 1u);
     const int near1 = near0 + __popc(bits);
@@ -445,10 +492,11 @@ __device__ __forceinline__ void assemble_pair_tile(const Tables& tab, int N, con
       if (tid < cnt * Q) {
         const int slot = tid / Q, qi = tid % Q;
         const int pr = sNear[n0 + slot];
-        const float4 ti = sTi[pr % TI];
+        const float4 ti = sTi[pr % TI], tj = sTj[pr / TI];
         const float si = tab.pts[qi];
-        const float pp[3] = {fmaf(si, ti.x, sD[pr][0]), fmaf(si, ti.y, sD[pr][1]), fmaf(si, ti.z, sD[pr][2])};
-        stokeslet_moments_G<K1, Q, S::GSN, P2, false>(tab, pp, sTj[pr / TI], e2, e2x3, sG + slot * S::QP + qi);
+        const float px = fmaf(si, ti.x, sD[pr][0]), py = fmaf(si, ti.y, sD[pr][1]), pz = fmaf(si, ti.z, sD[pr][2]);
+        stokeslet_moments_G<K1, Q, S::GSN, P2, false>(tab, project(px, py, pz, tj), tj, e2, e2x3, 0.f,
+                                                      sG + slot * S::QP + qi);
       }
       __syncthreads();
       for (int task = tid; task < cnt * NC2; task += NT) {   // lanes = columns

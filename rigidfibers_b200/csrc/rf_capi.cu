@@ -278,6 +278,9 @@ static Tables make_tables(const rf_config& c) {
       t.far_W[k][kFarNodes - 1 - q] = (k & 1) ? -t.far_W[k][q] : t.far_W[k][q];
       (k % 2 ? t.far_W2[k / 2][q].y : t.far_W2[k / 2][q].x) = t.far_W[k][q];
     }
+    double sum = 0.0;
+    for (int q = 0; q < kFarNodes; ++q) sum += t.far_W[k][q];
+    t.far_sum[k] = (float)sum;
   }
   // Centre distance from which the far rule's blocks are the full rule's to
   // 3e-10 of their largest entry (both in FP64, collinear and random

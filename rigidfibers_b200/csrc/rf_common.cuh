@@ -33,6 +33,7 @@ struct Tables {
   float far_pts[kFarNodes];
   float far_W[kMaxTerms + 1][kFarNodes];
   float2 far_W2[kMaxTerms / 2 + 1][kFarNodes / 2];
+  float far_sum[kMaxTerms + 1];       // sum over the points of far_W[k] (2, then 0 up to P_5)
   float far_d2;
   float gamma[kMaxTerms];   // gamma[0] = D1 (force index 0), gamma[k] for k>=1
   float eigen[kMaxTerms];   // E_k; unused for k = 0
@@ -96,7 +97,7 @@ __device__ __forceinline__ double f2d(float v) {
 // Whether a pair whose centres are sqrt(d2) apart takes the far rule.  A pair
 // whose distance is not a number or too large for FP32 squares takes the full
 // rule: its reciprocal root of infinity is 0 and the kernel vanishes, where the
-// far rule's Newton step would form infinity times 0.
+// far velocities' Newton step would form infinity times 0.
 constexpr float kFarMaxD2 = 1e37f;
 __device__ __forceinline__ bool far_pair(float d2, float far_d2) {
   // squares are not negative: their bit patterns order as they do, NaN and infinity last

@@ -284,9 +284,10 @@ static Tables make_tables(const rf_config& c) {
   }
   // Centre distance from which the far rule's blocks are the full rule's to
   // 3e-10 of their largest entry (both in FP64, collinear and random
-  // orientations): below the FP32 rounding of the blocks, ~2e-9.  8 points, M = 5
-  // terms, 24 points per fiber: 2.4e-8 at 3.0, 2.0e-9 at 3.5, 2.6e-10 at 4.0;
-  // M = 8: 6.4e-9 at 5.0, 3.2e-10 at 7.0.  12 and 48 points per fiber: the same.
+  // orientations): a hundredth of the FP32 rounding of an entry of that size,
+  // 3e-8 to 6e-8.  8 points, M = 5 terms, 24 points per fiber: 2.4e-8 at 3.0,
+  // 2.0e-9 at 3.5, 2.6e-10 at 4.0; M = 8: 6.4e-9 at 5.0, 3.2e-10 at 7.0.  12 and 48
+  // points per fiber: the same.
   const double far = M <= 5 ? 4.0 : 7.0;
   t.far_d2 = (float)(far * far);
   const double eps = c.slenderness;

@@ -226,15 +226,15 @@ __device__ __forceinline__ void stokeslet_moments_G(const Tables& tab, const flo
 // A third of the points average the roundings of G a third as well, and the blocks
 // of P_1 and up against P_0 (the right-hand side) are small differences of G.  A
 // Newton step on the reciprocal root makes up for it in sums over hundreds of pairs
-// (forces of 400 dilute fibers against 64 bits: 2.0e-6, 2.4e-6 without the far rule),
-// not in smaller ones (8 to 24 packed members of 16 to 128: 1.3e-6 against 1.2e-6).
+// (forces of 400 dilute fibers against 64 bits: 1.7e-6, 2.1e-6 without the far rule),
+// not in smaller ones (nine packs of 8 and 12 members: 1.27e-6 against 1.16e-6).
 // Up to kFarSmall fibers what all points of fiber i share is therefore taken out of
 // the sums: a point's projection on fiber j's axis is the centre difference's plus s
 // times t_i's, and 2 / |x_i - x_j|, about the sum of W_0 a, is taken off G[.][P_0]'s
 // diagonal components where their sum starts and put back into T[P_0][P_0]
 // (far_sum).  Roundings of T[k][P_0], k = 1 .. 5, times the distance (FP32 emulation):
 // 3.9 5.6 2.3 2.9 1.8 e-8 by the full rule, 5.2 5.2 3.5 3.6 2.8 by the far rule with
-// the step, 4.1 3.3 2.8 2.3 2.3 so (the step is left out); the packs' forces 1.0e-6.
+// the step, 4.1 3.3 2.8 2.3 2.3 so (the step is left out); the packs' forces 0.98e-6.
 // Larger systems and the product keep the step, with which their errors are below
 // the full rule's; the choice costs them 0.7 % of the assembly (N=4000: 2.44 ms).
 //
